@@ -20,7 +20,7 @@ namespace {
 
 enum Slot {
   S_CHUNKS, S_UNITS, S_FLAGS, S_TOT, S_INFO, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
-  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_NUM
+  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_NUM
 };
 
 constexpr int kMaxDim = 512;
@@ -63,6 +63,7 @@ struct bmf_batch {
   uint32_t* d_flags = nullptr;
   uint32_t* d_tot = nullptr;
   int64_t* d_totals = nullptr;
+  int* d_ticket = nullptr;  // launch_chunk_scan's
   float* d_dens = nullptr;
   uint32_t* d_words = nullptr;
   WordScratch ws{};
@@ -221,18 +222,21 @@ bmf_status upload_single(bmf_ctx* ctx, const ChunkDev& c, cudaStream_t st, Chunk
   return BMF_OK;
 }
 
-// Count -> scan -> offsets -> emit for chunks already labelled.  Totals land
-// in d_totals[0..1] (vertices, indices); flags must be set.
-bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunks, int n_chunks, const int* d_units,
-                        int n_units, const uint32_t* d_words, const float* d_dens, const uint32_t* d_flags,
-                        int64_t words_total, const MeshOut& mo, int64_t* d_info, int64_t* d_totals,
-                        cudaStream_t st, WordScratch* ws_out = nullptr) {
+// Count -> chunk scan -> emit for one labelled chunk.  Totals land in
+// d_totals (kTotals entries).  flags_ready: the fill set d_flags; else they
+// are cleared here and the count sets them.
+bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunks, const int* d_units, int n_units,
+                        const uint32_t* d_words, const float* d_dens, uint32_t* d_flags, bool flags_ready,
+                        int64_t words_total, const MeshOut& mo, int64_t* d_totals, cudaStream_t st,
+                        WordScratch* ws_out = nullptr) {
+  constexpr int n_chunks = 1;
   WordScratch ws{};
   uint32_t* tot = nullptr;
   bmf_status s;
   if ((s = scratch(ctx, S_VCNT, (size_t)words_total, &ws.vcnt)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_ICNT, (size_t)words_total, &ws.icnt)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_GPL, (size_t)words_total * 3, &ws.gpl)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_PB, (size_t)n_units, &ws.pb)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_TOT, (size_t)n_chunks * 2, &tot)) != BMF_OK) return s;
   {
     // work list of active cells: each one owns a vertex or emits a primitive
@@ -243,11 +247,11 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunk
     ws.ccount = (uint32_t*)(list + ws.clist_cap);
   }
   if (ws_out) *ws_out = ws;
-  launch_count(mode, d_chunks, n_chunks, d_units, n_units, d_words, d_flags, ws, st);
+  if (!flags_ready) BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
+  launch_count(mode, d_chunks, n_chunks, d_units, n_units, d_words, flags_ready ? d_flags : nullptr, ws, st,
+               flags_ready ? nullptr : d_flags);
   BMF_LAUNCHED(ctx, 1);
-  launch_scan_chunks(d_chunks, n_chunks, ws, tot, st);
-  BMF_LAUNCHED(ctx, 1);
-  launch_chunk_offsets(d_chunks, n_chunks, tot, d_flags, mo.vcap, mo.icap, d_info, d_totals, st);
+  launch_chunk_scan(d_chunks, n_chunks, ws, tot, d_flags, mo.vcap, mo.icap, nullptr, d_totals, nullptr, st);
   BMF_LAUNCHED(ctx, 1);
   BMF_LAUNCHED(ctx, launch_emit(mode, placement, d_chunks, n_chunks, d_units, n_units, d_words, d_dens, d_flags, ws,
                                 mo, d_totals, st));
@@ -417,23 +421,19 @@ bmf_status bmf_polygonize(bmf_ctx* ctx, int32_t dim, const float* d_density, con
   int64_t* d_totals;
   if ((s = upload_single(ctx, c, st, &d_c, &d_u)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_FLAGS, 1, &d_flags)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_TOTALS, 2, &d_totals)) != BMF_OK) return s;
-  launch_word_flags(d_c, 1, d_words, d_flags, st);
-  BMF_LAUNCHED(ctx, 1);
+  if ((s = scratch(ctx, S_TOTALS, kTotals, &d_totals)) != BMF_OK) return s;
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   if (mode == BMF_MODE_Q && placement == BMF_PLACE_QEF &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
-  if ((s = extract_core(ctx, mode, placement, d_c, 1, d_u, dim, d_words, d_density, d_flags,
-                        (int64_t)dim * dim * c.zc, mo, nullptr, d_totals, st)) != BMF_OK)
+  if ((s = extract_core(ctx, mode, placement, d_c, d_u, dim, d_words, d_density, d_flags, false,
+                        (int64_t)dim * dim * c.zc, mo, d_totals, st)) != BMF_OK)
     return s;
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned + 2, d_flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, kTotals * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   BMF_CUDA(ctx, cudaStreamSynchronize(st));
   out->n_verts = ctx->h_pinned[0];
   out->n_idx = ctx->h_pinned[1];
-  const uint32_t f = (uint32_t)ctx->h_pinned[2];
-  out->contains_mesh = ((f & 1u) || ((f & 6u) == 6u)) ? 1 : 0;
+  out->contains_mesh = (int32_t)ctx->h_pinned[2];
   out->prim_size = mode == BMF_MODE_R ? 3 : 4;
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_polygonize: output capacity exceeded (needed counts reported)");
@@ -514,7 +514,7 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   uint32_t* d_words;
   if ((s = upload_single(ctx, c, st, &d_c, &d_u)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_FLAGS, 1, &d_flags)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_TOTALS, 2, &d_totals)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_TOTALS, kTotals, &d_totals)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_DENS, (size_t)dim * dim * dim, &d_dens)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_WORDS, (size_t)dim * dim * c.zc, &d_words)) != BMF_OK) return s;
   BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
@@ -526,16 +526,14 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
   WordScratch ws{};
-  if ((s = extract_core(ctx, opts->mode, opts->placement, d_c, 1, d_u, dim, d_words, d_dens, d_flags,
-                        (int64_t)dim * dim * c.zc, mo, nullptr, d_totals, st, &ws)) != BMF_OK)
+  if ((s = extract_core(ctx, opts->mode, opts->placement, d_c, d_u, dim, d_words, d_dens, d_flags, true,
+                        (int64_t)dim * dim * c.zc, mo, d_totals, st, &ws)) != BMF_OK)
     return s;
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned + 2, d_flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, kTotals * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   BMF_CUDA(ctx, cudaStreamSynchronize(st));
   out->n_verts = ctx->h_pinned[0];
   out->n_idx = ctx->h_pinned[1];
-  const uint32_t f = (uint32_t)ctx->h_pinned[2];
-  out->contains_mesh = ((f & 1u) || ((f & 6u) == 6u)) ? 1 : 0;
+  out->contains_mesh = (int32_t)ctx->h_pinned[2];
   out->prim_size = opts->mode == BMF_MODE_R ? 3 : 4;
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_extract_chunk: output capacity exceeded (needed counts reported)");
@@ -584,6 +582,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
     dens += (int64_t)c.dim * c.dim * c.dim;
     words += (int64_t)c.dim * c.dim * c.zc;
     units[i] = n_units;
+    c.unit0 = n_units;
     n_units += c.dim;
     b->max_dim = c.dim > b->max_dim ? c.dim : b->max_dim;
     b->h_chunks[i] = c;
@@ -600,7 +599,10 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if ((s = bail(cudaMalloc(&b->d_units, sizeof(int) * (n_chunks + 1)), "units")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_flags, sizeof(uint32_t) * n_chunks), "flags")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_tot, sizeof(uint32_t) * 2 * n_chunks), "tot")) != BMF_OK) return s;
-  if ((s = bail(cudaMalloc(&b->d_totals, sizeof(int64_t) * 2), "totals")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->d_totals, sizeof(int64_t) * kTotals), "totals")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->d_ticket, sizeof(int)), "scan ticket")) != BMF_OK) return s;
+  if ((s = bail(cudaMemset(b->d_ticket, 0, sizeof(int)), "scan ticket")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->ws.pb, sizeof(uint2) * n_units), "plane bases")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_dens, sizeof(float) * dens), "density")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_words, sizeof(uint32_t) * words), "words")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->ws.vcnt, sizeof(uint32_t) * words), "vcnt")) != BMF_OK) return s;
@@ -785,12 +787,11 @@ bmf_status batch_record(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st,
   launch_count(b->opts.mode, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_flags, b->ws, st);
   const bool band = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;  // the 2D column fill needs no fix-up
   if (band) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
-  launch_scan_chunks(b->d_chunks, b->n, b->ws, b->d_tot, st, b->d_order);
-  launch_chunk_offsets(b->d_chunks, b->n, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                       b->d_totals, st);
+  launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
+                    b->d_totals, b->d_ticket, st);
   MeshOut mo{out->d_pos, out->d_nrm, proc ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr,
              out->d_idx, proc ? b->d_idxg : nullptr, out->vcap, out->icap, batch_keys(b) ? b->d_vkey : nullptr};
-  int64_t k = (band ? 5 : 4) + (b->d_cols ? 1 : 0);
+  int64_t k = (band ? 4 : 3) + (b->d_cols ? 1 : 0);
   k += launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_dens,
                    b->d_flags, b->ws, mo, b->d_totals, st);
   // indices and chunk table are final here (bmf_batch_wait_extraction); an
@@ -968,10 +969,9 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   const bool fixup = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;
   if (fixup) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[7], st));
-  launch_scan_chunks(b->d_chunks, b->n, b->ws, b->d_tot, st, b->d_order);
-  BMF_CUDA(ctx, cudaEventRecord(ev[3], st));
-  launch_chunk_offsets(b->d_chunks, b->n, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                       b->d_totals, st);
+  BMF_CUDA(ctx, cudaEventRecord(ev[3], st));  // the word scan is part of the count
+  launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
+                    b->d_totals, b->d_ticket, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[4], st));
   MeshOut mo{out->d_pos, out->d_nrm, proc ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr,
              out->d_idx, proc ? b->d_idxg : nullptr, out->vcap, out->icap, batch_keys(b) ? b->d_vkey : nullptr};
@@ -997,7 +997,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[2], ev[7], ev[3]));
   for (int k = 3; k < 6; ++k) BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[k], ev[k], ev[k + 1]));
   for (auto& e : ev) cudaEventDestroy(e);
-  ctx->launches += (fixup ? 5 : 4) + (b->d_cols ? 1 : 0) + ek + pk;
+  ctx->launches += (fixup ? 4 : 3) + (b->d_cols ? 1 : 0) + ek + pk;
   return BMF_OK;
 }
 
@@ -1163,6 +1163,7 @@ struct bmf_fit {
   int* d_units = nullptr;
   uint32_t *d_flags = nullptr, *d_tot = nullptr, *d_words = nullptr;
   int64_t* d_totals = nullptr;
+  int* d_ticket = nullptr;  // launch_chunk_scan's
   WordScratch ws{};
   ProcessScratch ps{};
   uint32_t *d_idxg = nullptr, *d_vkey = nullptr;
@@ -1187,7 +1188,7 @@ bmf_status bmf_fit_destroy(bmf_fit* f) {
   void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.icnt,
                   f->ws.gpl, f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
                   f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_qlist, f->d_qseed, f->d_clist, f->d_order,
-                  f->d_pqueue, f->d_qflag, f->d_lpart};
+                  f->d_pqueue, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (f->h_pinned) cudaFreeHost(f->h_pinned);
@@ -1225,8 +1226,8 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
     c.zc = zc;
     c.dens = (int64_t)i * dim * dim * dim;
     c.words = (int64_t)i * dim * dim * zc;
+    units[i] = c.unit0 = i * dim;
     hc[i] = c;
-    units[i] = i * dim;
   }
   units[n_chunks] = n_chunks * dim;
   const int64_t np = icap / 4;
@@ -1235,7 +1236,10 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_flags, sizeof(uint32_t) * n_chunks) == cudaSuccess &&
             cudaMalloc(&f->d_tot, sizeof(uint32_t) * 2 * n_chunks) == cudaSuccess &&
             cudaMalloc(&f->d_words, sizeof(uint32_t) * words) == cudaSuccess &&
-            cudaMalloc(&f->d_totals, sizeof(int64_t) * 2) == cudaSuccess &&
+            cudaMalloc(&f->d_totals, sizeof(int64_t) * kTotals) == cudaSuccess &&
+            cudaMalloc(&f->d_ticket, sizeof(int)) == cudaSuccess &&
+            cudaMemset(f->d_ticket, 0, sizeof(int)) == cudaSuccess &&
+            cudaMalloc(&f->ws.pb, sizeof(uint2) * n_chunks * dim) == cudaSuccess &&
             cudaMalloc(&f->ws.vcnt, sizeof(uint32_t) * words) == cudaSuccess &&
             cudaMalloc(&f->ws.icnt, sizeof(uint32_t) * words) == cudaSuccess &&
             cudaMalloc(&f->ws.gpl, sizeof(uint32_t) * 3 * words) == cudaSuccess &&
@@ -1287,8 +1291,8 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   launch_sample_label(f->d_chunks, f->n, f->d_units, f->n * f->dim, f->dim, fd, d_density, nullptr, f->d_words,
                       f->d_flags, st);
   launch_count(BMF_MODE_Q, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words, f->d_flags, f->ws, st);
-  launch_scan_chunks(f->d_chunks, f->n, f->ws, f->d_tot, st);
-  launch_chunk_offsets(f->d_chunks, f->n, f->d_tot, f->d_flags, f->vcap, f->icap, d_chunk_info, f->d_totals, st);
+  launch_chunk_scan(f->d_chunks, f->n, f->ws, f->d_tot, f->d_flags, f->vcap, f->icap, d_chunk_info, f->d_totals,
+                    f->d_ticket, st);
   MeshOut mo{d_pos, nullptr, f->d_boundary, f->d_valence, d_idx, f->d_idxg, f->vcap, f->icap, f->d_vkey};
   if (f->d_qflag && f->placement == BMF_PLACE_QEF) {  // the wide adjoint reads the forward's QEF branches
     mo.qflag = f->d_qflag;
@@ -1296,7 +1300,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
     mo.qcount = f->d_qlist + f->vcap;
     mo.qseed = f->d_qseed;
   }
-  int k = 4 + launch_emit(BMF_MODE_Q, f->placement, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words,
+  int k = 3 + launch_emit(BMF_MODE_Q, f->placement, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words,
                           d_density, f->d_flags, f->ws, mo, f->d_totals, st);
   if (f->iters > 0) {
     StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->d_words, f->ws, f->d_vkey};
@@ -1385,7 +1389,7 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
                   b->ws.vcnt, b->ws.icnt, b->ws.gpl, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
                   b->d_fill_items, b->d_queue, b->d_order, b->d_pqueue, b->d_clist, b->d_exact, b->d_fix,
-                  b->d_cols};
+                  b->d_cols, b->d_ticket, b->ws.pb};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);

@@ -48,6 +48,8 @@ struct ChunkDev {
   float ox, oy, oz, scale;
   int dim;        // samples per axis
   int zc;         // 32-bit occupancy words per (x, y) line = ceil(dim / 32)
+  int unit0;      // index of the chunk's first x-plane among the batch's planes (WordScratch::pb)
+  int pad;
   int64_t dens;   // offset of the chunk's density block (floats); -1 = not materialised
   int64_t words;  // offset of the chunk's occupancy words (u32)
   int64_t vout;   // offset of the chunk's vertices in the output arena

@@ -11,8 +11,9 @@
 //     X = W[x][y] ^ W[x+1][y],  Y = W[x][y] ^ W[x][y+1],  Z = W ^ (W >> 1 | next << 31)
 // so a word hosts popc(X)+popc(Y)+popc(Z) vertices, and the vertex id of cell z's
 // axis-a crossing is   base(word) + popc((X|Y|Z bits of cells < z)) + (own earlier axes).
-// base(word) is an exclusive scan of the per-word counts in (x, y, zb) order,
-// which is exactly the reference's sequential order.  Triangles are counted
+// base(word) is the exclusive sum of the per-word counts in (x, y, zb) order --
+// of the planes before x (ws.pb) plus of the plane's words before it (ws.vcnt)
+// -- which is exactly the reference's sequential order.  Triangles are counted
 // and placed the same way, so vertex and index buffers come out bit-identical
 // to the reference without any per-cell index volume (IndexesBlock) or cell
 // list (DMC_CellsBlock).
@@ -23,11 +24,17 @@
 
 namespace bmf {
 
+// Chunk of x-plane u, by a whole warp: 32 candidates per step (a dependent load
+// per factor of 32 in the chunk count, not per factor of 2).
 __device__ __forceinline__ int find_chunk_e(const int* __restrict__ unit_start, int n_chunks, int u) {
-  int lo = 0, hi = n_chunks - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(unit_start + mid) <= u) lo = mid; else hi = mid - 1;
+  const int lane = threadIdx.x & 31;
+  int lo = 0, n = n_chunks;
+  while (n > 1) {
+    const int step = (n + 31) >> 5, cand = lane * step;
+    const uint32_t le = __ballot_sync(kFull, cand < n && __ldg(unit_start + lo + cand) <= u);
+    const int at = (__popc(le) - 1) * step;  // unit_start ascends: le is a prefix of the lanes, lane 0 in it
+    lo += at;
+    n = min(step, n - at);
   }
   return lo;
 }
@@ -129,7 +136,14 @@ __device__ __forceinline__ void q_quad_words(const uint32_t* W, int dim, int zc,
 }
 
 // ---------------------------------------------------------------------------
-// K2: per-word counts, one thread per occupancy word.
+// K2: per-word counts, one thread per occupancy word, one CTA per x-plane.
+//
+// The CTA walks its plane's words in order and keeps the running sums, so a
+// word's count leaves as the sum of the plane's words before it, and the
+// plane's totals go to ws.pb: a scan over a chunk's planes (k_chunk_scan, at
+// most 512 pairs) then replaces a pass over all words (read and written back:
+// 0.28 ms of a 4096-chunk update, 65 us of one 129^3 chunk, whose words one
+// CTA scanned).  Quiet words write nothing.
 //
 // Everything a word contributes is bit arithmetic on the eight line words
 // around it (lines (x..x+1, y..y+1), blocks zb and zb + 1): its owned
@@ -173,7 +187,11 @@ constexpr EdgeTris make_edge_tris() {
 }
 static __device__ const EdgeTris g_edge_tris = make_edge_tris();
 
-constexpr int kCountThreads = 64;
+// Threads per plane: 64 keeps every lane of a small plane's CTA busy and lets
+// a whole update's planes fill the GPU; with few planes (a chunk or a small
+// batch) 256 shorten the walk over a plane's words (129^3: 645 words).
+constexpr int kCountThreads = 64, kCountThreadsFew = 256;
+constexpr int kCountFewUnits = 2048;
 
 // Cells z of block zb with z <= hi (bits [0, hi - 32 zb]).
 __device__ __forceinline__ uint32_t zbits_upto(int hi, int zb) {
@@ -181,36 +199,42 @@ __device__ __forceinline__ uint32_t zbits_upto(int hi, int zb) {
   return n >= 32 ? kFull : (n <= 0 ? 0u : ((1u << n) - 1u));
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kCountThreads) k_count(const ChunkDev* __restrict__ chunks, int n_chunks,
-                                                         const int* __restrict__ unit_start,
-                                                         const uint32_t* __restrict__ words,
-                                                         const uint32_t* __restrict__ flags, WordScratch ws) {
+template <int MODE, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_count(const ChunkDev* __restrict__ chunks, int n_chunks,
+                                                   const int* __restrict__ unit_start,
+                                                   const uint32_t* __restrict__ words,
+                                                   const uint32_t* __restrict__ flags,
+                                                   uint32_t* __restrict__ flags_out, WordScratch ws) {
+  constexpr int kWarps = THREADS / 32;
   __shared__ uint32_t s_cnt[64];
-  __shared__ int s_c;
+  __shared__ uint2 s_sum[2][kWarps];  // per warp {vertices, indices} of this step's words, two steps in turn
   const int u = blockIdx.x;
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) s_cnt[i] = g_case_counts.w[i];
-  if (threadIdx.x == 0) s_c = find_chunk_e(unit_start, n_chunks, u);
+  const int c = find_chunk_e(unit_start, n_chunks, u);
+  // a chunk without a mesh has equal words everywhere: nothing to count
+  if (flags && !contains_mesh(__ldg(flags + c))) {
+    if (threadIdx.x == 0) ws.pb[u] = make_uint2(0u, 0u);
+    return;
+  }
+  for (int i = threadIdx.x; i < 64; i += THREADS) s_cnt[i] = g_case_counts.w[i];
   __syncthreads();
-  const int c = s_c;
   const ChunkDev ch = chunks[c];
   const int x = u - __ldg(unit_start + c);
   const int dim = ch.dim, zc = ch.zc, nw = dim * zc;
   const uint32_t* W = words + ch.words;
-  const bool cm = contains_mesh(__ldg(flags + c));
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t carry_v = 0u, carry_i = 0u, fl = 0u;
   const bool listing = ws.clist != nullptr;
   const bool xin = x + 1 < dim;  // line x + 1 exists (cells and x-crossings of this plane)
   // a word's y is its index times the rounded-up 2^32 / zc, high half: exact
   // while index * zc < 2^32
   const uint64_t zmagic = ((1ull << 32) + (uint64_t)zc - 1u) / (uint64_t)zc;
   const uint32_t* Wx = W + (int64_t)x * nw;  // the plane's words
-  for (int base = 0; base < nw; base += kCountThreads) {
+  for (int base = 0, step = 0; base < nw; base += THREADS, step ^= 1) {
     const int wi = base + threadIdx.x;
     const int y = (int)(((uint64_t)(uint32_t)wi * zmagic) >> 32), zb = wi - y * zc;
     uint32_t vc = 0u, ic = 0u, p0 = 0u, p1 = 0u, p2 = 0u, act = 0u;
     uint32_t f00 = 0u, f10 = 0u, f01 = 0u, fnx = 0u;  // band fill: samples to make exact
-    if (wi < nw && cm) {
+    if (wi < nw) {
       const bool yin = y + 1 < dim, nin = zb + 1 < zc;
       const uint32_t* L00 = Wx + wi;  // the word (x, y, zb)
       const uint32_t w00 = __ldg(L00), n00 = nin ? __ldg(L00 + 1) : 0u;
@@ -218,6 +242,7 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const ChunkDev* __restr
       const uint32_t* L10 = L00 + (int64_t)dim * zc;
       const uint32_t w10 = xin ? __ldg(L10) : 0u, n10 = (xin && nin) ? __ldg(L10 + 1) : 0u;
       const uint32_t w11 = (xin && yin) ? __ldg(L10 + zc) : 0u, n11 = (xin && yin && nin) ? __ldg(L10 + zc + 1) : 0u;
+      fl |= (w00 != 0u && w00 != kFull) ? 1u : (w00 == kFull ? 2u : 4u);
       // corner words: bit l = corner (dx, dy, dz) of cell 32 zb + l
       const uint32_t a0 = w00, a1 = (w00 >> 1) | (n00 << 31), b0 = w01, b1 = (w01 >> 1) | (n01 << 31);
       const uint32_t c0 = w10, c1 = (w10 >> 1) | (n10 << 31), d0 = w11, d1 = (w11 >> 1) | (n11 << 31);
@@ -267,11 +292,32 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const ChunkDev* __restr
         act = p0 | p1 | p2 | Xi | Yi | Zi;
       }
     }
-    if (wi < nw) {
-      const int64_t o = ch.words + (int64_t)x * nw + wi;
-      ws.vcnt[o] = vc;
-      ws.icnt[o] = ic;
-      if (ws.gpl) {
+    {
+      // the plane's running sums; indices per plane stay below 2^32 (at most
+      // 15 per cell, 2^18 cells)
+      uint32_t iv = vc, ii = ic;
+      const bool any_act = __any_sync(kFull, act != 0u);
+      if (any_act) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const uint32_t a = __shfl_up_sync(kFull, iv, off), b = __shfl_up_sync(kFull, ii, off);
+          if (lane >= off) { iv += a; ii += b; }
+        }
+      }
+      if (lane == 31) s_sum[step][warp] = make_uint2(iv, ii);
+      __syncthreads();
+      uint32_t bv = carry_v, bi = carry_i;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const uint2 t = s_sum[step][w];
+        if (w < warp) { bv += t.x; bi += t.y; }
+        carry_v += t.x;
+        carry_i += t.y;
+      }
+      if (act) {
+        const int64_t o = ch.words + (int64_t)x * nw + wi;
+        ws.vcnt[o] = bv + iv - vc;
+        ws.icnt[o] = bi + ii - ic;
         ws.gpl[3 * o] = p0;
         ws.gpl[3 * o + 1] = p1;
         ws.gpl[3 * o + 2] = p2;
@@ -332,107 +378,80 @@ __global__ void __launch_bounds__(kCountThreads) k_count(const ChunkDev* __restr
       }
     }
   }
+  if (threadIdx.x == 0) ws.pb[u] = make_uint2(carry_v, carry_i);
+  if (flags_out) {
+    fl = __reduce_or_sync(kFull, fl);
+    if (lane == 0 && fl) atomicOr(flags_out + c, fl);
+  }
 }
 
 // ---------------------------------------------------------------------------
-// K3: exclusive scan of each chunk's per-word counts (one CTA per chunk).
+// K3: plane totals -> plane bases per chunk (one warp per chunk), then chunk
+// totals -> arena offsets, info table and totals, by the CTA that finishes
+// last (one for up to 32 chunks).  Latency only: a few KB per chunk.  As one
+// CTA with a shared-memory scan after a separate word scan the offsets of 4096
+// chunks took 28 us.
 // ---------------------------------------------------------------------------
-template <int NT>
-__device__ __forceinline__ void block_excl_scan2(uint32_t& a, uint32_t& b, uint32_t& tot_a, uint32_t& tot_b) {
-  __shared__ uint32_t sa[NT / 32], sb[NT / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t ia = a, ib = b;
+constexpr int kScanThreads = 1024, kScanWarps = kScanThreads / 32;
+
+template <typename T>
+__device__ __forceinline__ T warp_incl_sum(T v, int lane) {
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t na = __shfl_up_sync(kFull, ia, o), nb = __shfl_up_sync(kFull, ib, o);
-    if (lane >= o) { ia += na; ib += nb; }
+    const T n = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += n;
   }
-  if (lane == 31) { sa[warp] = ia; sb[warp] = ib; }
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t va = lane < NT / 32 ? sa[lane] : 0u, vb = lane < NT / 32 ? sb[lane] : 0u;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t na = __shfl_up_sync(kFull, va, o), nb = __shfl_up_sync(kFull, vb, o);
-      if (lane >= o) { va += na; vb += nb; }
-    }
-    if (lane < NT / 32) { sa[lane] = va; sb[lane] = vb; }
-  }
-  __syncthreads();
-  const uint32_t wa = warp ? sa[warp - 1] : 0u, wb = warp ? sb[warp - 1] : 0u;
-  tot_a = sa[NT / 32 - 1];
-  tot_b = sb[NT / 32 - 1];
-  a = wa + ia - a;
-  b = wb + ib - b;
-  __syncthreads();
+  return v;
 }
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 2;
-
-// order (nullable): CTA i scans chunk order[i] -- largest chunks first, so the
-// longest scans do not start last.
-__global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const ChunkDev* __restrict__ chunks, WordScratch ws,
-                                                            uint32_t* __restrict__ tot, const int* __restrict__ order) {
-  const int cid = order ? __ldg(order + blockIdx.x) : (int)blockIdx.x;
-  const ChunkDev ch = chunks[cid];
-  const int64_t n = (int64_t)ch.dim * ch.dim * ch.zc;
-  uint32_t* v = ws.vcnt + ch.words;
-  uint32_t* ic = ws.icnt + ch.words;
-  uint32_t carry_v = 0, carry_i = 0;
-  for (int64_t base = 0; base < n; base += (int64_t)kScanThreads * kScanItems) {
-    const int64_t i0 = base + (int64_t)threadIdx.x * kScanItems;
-    uint32_t lv[kScanItems], li[kScanItems], sv = 0, si = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      lv[k] = (i0 + k < n) ? v[i0 + k] : 0u;
-      li[k] = (i0 + k < n) ? ic[i0 + k] : 0u;
-      sv += lv[k];
-      si += li[k];
+__global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restrict__ chunks, int n, uint2* __restrict__ pb,
+                                                             uint32_t* tot, const uint32_t* __restrict__ flags,
+                                                             int64_t vcap, int64_t icap, int64_t* __restrict__ info,
+                                                             int64_t* __restrict__ totals, int* __restrict__ ticket) {
+  __shared__ int64_t s_v[kScanWarps], s_i[kScanWarps];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int mine = blockIdx.x * kScanWarps + warp;
+  if (mine < n) {
+    const int dim = chunks[mine].dim;
+    uint2* p = pb + chunks[mine].unit0;
+    uint32_t cv = 0u, ci = 0u;
+    for (int b = 0; b < dim; b += 32) {
+      const bool in = b + lane < dim;
+      const uint2 t = in ? p[b + lane] : make_uint2(0u, 0u);
+      const uint32_t iv = warp_incl_sum(t.x, lane), ii = warp_incl_sum(t.y, lane);
+      if (in) p[b + lane] = make_uint2(cv + iv - t.x, ci + ii - t.y);
+      cv += __shfl_sync(kFull, iv, 31);
+      ci += __shfl_sync(kFull, ii, 31);
     }
-    uint32_t ev = sv, ei = si, tv, ti;
-    block_excl_scan2<kScanThreads>(ev, ei, tv, ti);
-    ev += carry_v;
-    ei += carry_i;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (i0 + k < n) {
-        v[i0 + k] = ev;
-        ic[i0 + k] = ei;
-      }
-      ev += lv[k];
-      ei += li[k];
+    if (lane == 0) {
+      tot[2 * mine] = cv;
+      tot[2 * mine + 1] = ci;
     }
-    carry_v += tv;
-    carry_i += ti;
   }
-  if (threadIdx.x == 0) {
-    tot[2 * cid] = carry_v;
-    tot[2 * cid + 1] = carry_i;
-  }
-}
-
-// Chunk offsets in the output arena + per-chunk info (single CTA).
-__global__ void __launch_bounds__(1024) k_chunk_offsets(ChunkDev* __restrict__ chunks, int n, const uint32_t* tot,
-                                                        const uint32_t* flags, int64_t vcap, int64_t icap,
-                                                        int64_t* info, int64_t* totals) {
-  __shared__ int64_t s_v[1024], s_i[1024];
+  __threadfence();  // this CTA's totals before its ticket
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = gridDim.x == 1 || atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();  // the other CTAs' totals after their tickets
   int64_t carry_v = 0, carry_i = 0;
-  for (int base = 0; base < n; base += 1024) {
+  for (int base = 0; base < n; base += kScanThreads) {
     const int c = base + threadIdx.x;
-    const int64_t v = c < n ? (int64_t)tot[2 * c] : 0, i = c < n ? (int64_t)tot[2 * c + 1] : 0;
-    s_v[threadIdx.x] = v;
-    s_i[threadIdx.x] = i;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const int64_t av = threadIdx.x >= o ? s_v[threadIdx.x - o] : 0, ai = threadIdx.x >= o ? s_i[threadIdx.x - o] : 0;
-      __syncthreads();
-      s_v[threadIdx.x] += av;
-      s_i[threadIdx.x] += ai;
-      __syncthreads();
+    const int64_t v = c < n ? (int64_t)__ldcg(tot + 2 * c) : 0, i = c < n ? (int64_t)__ldcg(tot + 2 * c + 1) : 0;
+    const int64_t iv = warp_incl_sum(v, lane), ii = warp_incl_sum(i, lane);
+    if (lane == 31) {
+      s_v[warp] = iv;
+      s_i[warp] = ii;
     }
+    __syncthreads();
+    if (warp == 0) {
+      s_v[lane] = warp_incl_sum(s_v[lane], lane);
+      s_i[lane] = warp_incl_sum(s_i[lane], lane);
+    }
+    __syncthreads();
     if (c < n) {
-      const int64_t vo = carry_v + s_v[threadIdx.x] - v, io = carry_i + s_i[threadIdx.x] - i;
+      const int64_t vo = carry_v + (warp ? s_v[warp - 1] : 0) + iv - v, io = carry_i + (warp ? s_i[warp - 1] : 0) + ii - i;
       chunks[c].vout = vo;
       chunks[c].iout = io;
       if (info) {
@@ -444,32 +463,21 @@ __global__ void __launch_bounds__(1024) k_chunk_offsets(ChunkDev* __restrict__ c
         info[6 * c + 5] = (vo + v > vcap || io + i > icap) ? 3 : 0;
       }
     }
-    carry_v += s_v[1023];
-    carry_i += s_i[1023];
+    carry_v += s_v[kScanWarps - 1];
+    carry_i += s_i[kScanWarps - 1];
     __syncthreads();
   }
-  if (threadIdx.x == 0 && totals) {
+  if (threadIdx.x == 0) {
     totals[0] = carry_v;
     totals[1] = carry_i;
+    totals[2] = contains_mesh(flags[0]) ? 1 : 0;
+    if (gridDim.x > 1) *ticket = 0;
   }
 }
 
 // ---------------------------------------------------------------------------
 // K4: emission
 // ---------------------------------------------------------------------------
-
-// Vertex id (chunk-local) of the axis-a crossing owned by sample (x, y, z).
-__device__ __forceinline__ uint32_t r_vertex_id(const uint32_t* W, const uint32_t* vbase, int dim, int zc, int x, int y,
-                                                int z, int a) {
-  const int zb = z >> 5, l = z & 31;
-  const uint32_t X = xcross_word(W, dim, zc, x, y, zb), Y = ycross_word(W, dim, zc, x, y, zb);
-  const uint32_t Z = zcross_word(W, dim, zc, x, y, zb);
-  const uint32_t lt = lane_lt(l);
-  uint32_t id = __ldg(vbase + ((int64_t)x * dim + y) * zc + zb) + __popc(X & lt) + __popc(Y & lt) + __popc(Z & lt);
-  if (a >= 1) id += (X >> l) & 1u;
-  if (a >= 2) id += (Y >> l) & 1u;
-  return id;
-}
 
 // Per-warp staging of a busy word's neighbourhood (Mode R emit): the
 // occupancy words of lines (x-1+i, y-1+j), i, j in 0..3, for blocks zb-1, zb,
@@ -481,8 +489,8 @@ struct NbCache {
   uint32_t vb[8];  // [i][j][b], b = block - zb
 };
 
-__device__ __forceinline__ void nb_load(NbCache& c, const uint32_t* W, const uint32_t* vbase, int dim, int zc, int x,
-                                        int y, int zb, int lane) {
+__device__ __forceinline__ void nb_load(NbCache& c, const uint32_t* W, const uint32_t* vbase, const uint2* pb, int dim,
+                                        int zc, int x, int y, int zb, int lane) {
   __syncwarp();  // every lane is done with the previous word's cache
   for (int k = lane; k < 48; k += 32) {
     const int i = k / 12, j = (k / 3) & 3, b = k % 3;
@@ -490,7 +498,7 @@ __device__ __forceinline__ void nb_load(NbCache& c, const uint32_t* W, const uin
   }
   if (lane < 8) {
     const int xx = x + (lane >> 2), yy = y + ((lane >> 1) & 1), bb = zb + (lane & 1);
-    c.vb[lane] = (xx < dim && yy < dim && bb < zc) ? __ldg(vbase + ((int64_t)xx * dim + yy) * zc + bb) : 0u;
+    c.vb[lane] = (xx < dim && yy < dim && bb < zc) ? __ldg(vbase + ((int64_t)xx * dim + yy) * zc + bb) + pb[xx].x : 0u;
   }
   __syncwarp();
 }
@@ -508,7 +516,7 @@ __device__ __forceinline__ int nb_mask(const NbCache& c, int ci, int cj, int zr)
   return m;
 }
 
-// r_vertex_id from the cache: the axis-a crossing owned by sample
+// Vertex id (chunk-local) of the axis-a crossing owned by sample
 // (x+i, y+j, zabs), i, j in {0, 1}, zabs in [32zb, 32zb+32].
 __device__ __forceinline__ uint32_t nb_vertex_id(const NbCache& c, int dim, int x, int y, int zb, int i, int j,
                                                  int zabs, int a) {
@@ -530,12 +538,12 @@ __device__ __forceinline__ uint32_t nb_vertex_id(const NbCache& c, int dim, int 
 }
 
 // Mode Q vertex base of cell (x, y, z).
-__device__ __forceinline__ uint32_t q_vertex_base(const uint32_t* vbase, const uint32_t* gpl, int dim, int zc, int x,
-                                                  int y, int z) {
+__device__ __forceinline__ uint32_t q_vertex_base(const uint32_t* vbase, const uint32_t* gpl, const uint2* pb, int dim,
+                                                  int zc, int x, int y, int z) {
   const int64_t wi = ((int64_t)x * dim + y) * zc + (z >> 5);
   const uint32_t lt = lane_lt(z & 31);
-  return __ldg(vbase + wi) + __popc(__ldg(gpl + 3 * wi) & lt) + 2 * __popc(__ldg(gpl + 3 * wi + 1) & lt) +
-         4 * __popc(__ldg(gpl + 3 * wi + 2) & lt);
+  return __ldg(&pb[x].x) + __ldg(vbase + wi) + __popc(__ldg(gpl + 3 * wi) & lt) +
+         2 * __popc(__ldg(gpl + 3 * wi + 1) & lt) + 4 * __popc(__ldg(gpl + 3 * wi + 2) & lt);
 }
 
 template <int MODE, int PLACE>
@@ -553,6 +561,8 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
   const uint32_t* W = words + ch.words;
   const uint32_t* vbase = ws.vcnt + ch.words;
   const uint32_t* ibase = ws.icnt + ch.words;
+  const uint2* pb = ws.pb + ch.unit0;
+  const uint2 pbx = pb[x];
   const float* D = dens + ch.dens;
   const uint32_t lt = lane_lt(lane);
   __shared__ int s_busy[kWordBlock];
@@ -579,13 +589,13 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
     lw.load(W, dim, zc, x, y, zb);
     if (MODE == 0) {
       NbCache& nb = s_nb[warp];
-      nb_load(nb, W, vbase, dim, zc, x, y, zb, lane);
+      nb_load(nb, W, vbase, pb, dim, zc, x, y, zb, lane);
       // ---- vertices: calculate_cell / calculate_isovertex order ----
       const uint32_t X = (x + 1 < dim) ? (lw.w00 ^ lw.w10) : 0u;
       const uint32_t Y = (y + 1 < dim) ? (lw.w00 ^ lw.w01) : 0u;
       const uint32_t Z = zcross_word(W, dim, zc, x, y, zb);
       if ((X | Y | Z) != 0u) {
-        uint32_t vid = __ldg(vbase + wo) + __popc(X & lt) + __popc(Y & lt) + __popc(Z & lt);
+        uint32_t vid = pbx.x + __ldg(vbase + wo) + __popc(X & lt) + __popc(Y & lt) + __popc(Z & lt);
         const uint32_t own = ((X >> lane) & 1u) | (((Y >> lane) & 1u) << 1) | (((Z >> lane) & 1u) << 2);
         for (int a = 0; a < 3; ++a) {
           if (!((own >> a) & 1u)) continue;
@@ -633,7 +643,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const int t3 = 3 * (int)(tw >> 60);
       if (__ballot_sync(kFull, t3 != 0) == 0u) continue;
       const int incl = warp_incl_scan(t3);
-      int64_t gi = ch.iout + (int64_t)__ldg(ibase + wo) + (incl - t3);
+      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(ibase + wo)) + (incl - t3);
       for (int i = 0; i < t3; ++i, ++gi) {
         const int e = tri_edge(tw, i);
         const uint32_t vid = nb_vertex_id(nb, dim, x, y, zb, c_edge_owner[e][0], c_edge_owner[e][1],
@@ -650,7 +660,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const int ng = group_count(mask);
       const int64_t gpo = 3 * (ch.words + wo);
       if (ng) {
-        uint32_t vid = __ldg(vbase + wo) + __popc(__ldg(ws.gpl + gpo) & lt) +
+        uint32_t vid = pbx.x + __ldg(vbase + wo) + __popc(__ldg(ws.gpl + gpo) & lt) +
                        2 * __popc(__ldg(ws.gpl + gpo + 1) & lt) + 4 * __popc(__ldg(ws.gpl + gpo + 2) & lt);
         const int nc = dim - 1;
         const uint8_t bnd = (x == 0 || y == 0 || z == 0 || x == nc - 1 || y == nc - 1 || z == nc - 1);
@@ -688,7 +698,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const int nq = __popc(own);
       if (__ballot_sync(kFull, nq != 0) == 0u) continue;
       const int incl = warp_incl_scan(4 * nq);
-      int64_t gi = ch.iout + (int64_t)__ldg(ibase + wo) + (incl - 4 * nq);
+      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(ibase + wo)) + (incl - 4 * nq);
       const bool in0 = ((lw.w00 >> lane) & 1u) != 0u;
       for (int a = 0; a < 3; ++a) {
         if (!((own >> a) & 1)) continue;
@@ -705,7 +715,8 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
           lo[cax] = -oc;
           const int e = a == 0 ? 2 * lo[1] + lo[2] : (a == 1 ? 4 + 2 * lo[0] + lo[2] : 8 + 2 * lo[0] + lo[1]);
           const int cm = cell_mask_at(W, dim, zc, cc[0], cc[1], cc[2]);
-          q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, dim, zc, cc[0], cc[1], cc[2]) + (uint32_t)group_of(cm, e);
+          q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, pb, dim, zc, cc[0], cc[1], cc[2]) +
+                 (uint32_t)group_of(cm, e);
         }
         if (!in0) {
           const uint32_t t = q[1];
@@ -804,7 +815,7 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
   const int64_t iout = ch.iout;
   const uint32_t* W = words + ch.words;
   const uint32_t* ibase = ws.icnt + ch.words;
-  const uint32_t* pl = ws.gpl + 3 * ch.words;
+  const uint32_t* pl = ws.gpl + 3 * ch.words;  // (Mode R: ibase holds primitive bases by now)
   int x, y, z, k;
   vertex_key_decode(key, x, y, z, k);
   // the chunk's first primitive (its index offset and word bases are
@@ -843,7 +854,7 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
       const uint32_t lt = lane_lt(cz & 31);
       const uint32_t pre = __popc(__ldg(pl + 3 * wi) & lt) + 2 * __popc(__ldg(pl + 3 * wi + 1) & lt) +
                            4 * __popc(__ldg(pl + 3 * wi + 2) & lt);
-      const int64_t first = pbase + __ldg(ibase + wi) / 3u + pre;
+      const int64_t first = pbase + __ldg(ibase + wi) + pre;
       for (; tm && n < room; tm &= tm - 1u) out[n++] = (OUT)(first + __ffs(tm) - 1 - rel);
     }
   } else {
@@ -864,7 +875,7 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
       if (a >= 1) pre += (Xi >> l) & 1u;
       if (a >= 2) pre += (Yi >> l) & 1u;
       const int wi = (sx * dim + sy) * zc + (sz >> 5);
-      uint32_t id = (uint32_t)(pbase + __ldg(ibase + wi) / 4u + pre);
+      uint32_t id = (uint32_t)(pbase + (__ldg(&ws.pb[ch.unit0 + sx].y) + __ldg(ibase + wi)) / 4u + pre);
       int j = n++;  // insertion into the sorted prefix
       while (j > 0 && ids[j - 1] > id) { ids[j] = ids[j - 1]; --j; }
       ids[j] = id;
@@ -1046,21 +1057,25 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
 }
 
 void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
-                  const uint32_t* words, const uint32_t* flags, WordScratch ws, cudaStream_t st) {
+                  const uint32_t* words, const uint32_t* flags, WordScratch ws, cudaStream_t st,
+                  uint32_t* flags_out) {
   if (ws.clist) cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t), st);
   if (ws.exact) cudaMemsetAsync(ws.fcount, 0, sizeof(uint32_t), st);
-  if (mode == 0) k_count<0><<<n_units, kCountThreads, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, flags, ws);
-  else k_count<1><<<n_units, kCountThreads, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, flags, ws);
+#define BMF_COUNT(M, T) \
+  k_count<M, T><<<n_units, T, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, flags, flags_out, ws)
+  if (n_units < kCountFewUnits) {
+    if (mode == 0) BMF_COUNT(0, kCountThreadsFew); else BMF_COUNT(1, kCountThreadsFew);
+  } else {
+    if (mode == 0) BMF_COUNT(0, kCountThreads); else BMF_COUNT(1, kCountThreads);
+  }
+#undef BMF_COUNT
 }
 
-void launch_scan_chunks(const ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, cudaStream_t st,
-                        const int* d_order) {
-  k_scan_chunks<<<n_chunks, kScanThreads, 0, st>>>(d_chunks, ws, d_tot, d_order);
-}
-
-void launch_chunk_offsets(ChunkDev* d_chunks, int n_chunks, const uint32_t* d_tot, const uint32_t* flags,
-                          int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, cudaStream_t st) {
-  k_chunk_offsets<<<1, 1024, 0, st>>>(d_chunks, n_chunks, d_tot, flags, vcap, icap, d_info, d_totals);
+void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
+                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
+                       cudaStream_t st) {
+  k_chunk_scan<<<(n_chunks + kScanWarps - 1) / kScanWarps, kScanThreads, 0, st>>>(
+      d_chunks, n_chunks, ws.pb, d_tot, flags, vcap, icap, d_info, d_totals, d_ticket);
 }
 
 // k-th set bit (from 0) of m; m must have more than k set bits.
@@ -1192,6 +1207,8 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
   for (int64_t t0 = ((int64_t)blockIdx.x * kEmitWarps + warp) * kTileWords; t0 < n; t0 += nwarps * kTileWords) {
     const int nt = (int)min((int64_t)kTileWords, n - t0);
     // 1. the tile's words
+    uint2 pb0 = make_uint2(0u, 0u);  // this lane's word: its plane's bases, the next plane's vertex base
+    uint32_t pv1 = 0u;
     if (lane < nt) {
       const uint2 e = ws.clist[t0 + lane];
       const ChunkDev& ch = chunks[e.x];
@@ -1202,6 +1219,9 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
       R.x[lane] = xy / dim;
       R.dim[lane] = dim;
       R.zc[lane] = zc;
+      const uint2* pb = ws.pb + ch.unit0 + R.x[lane];
+      pb0 = __ldg(pb);
+      if (R.x[lane] + 1 < dim) pv1 = __ldg(&pb[1].x);
       R.cw[lane] = ch.words;
       R.dens[lane] = ch.dens;
       R.vout[lane] = ch.vout;
@@ -1258,7 +1278,17 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
     {
       uint32_t packed = 0u;
       if (lane < nt) {
-        const NbCache& nb = R.nb[lane];
+        NbCache& nb = R.nb[lane];
+        // word bases: within the plane + the plane's
+        const uint32_t ib = R.ib[lane] + pb0.y;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          nb.vb[k] += pb0.x;
+          nb.vb[4 + k] += pv1;
+        }
+        R.ib[lane] = ib;
+        if (out.vkey)  // the adjacency build reads the word's primitive base
+          ws.icnt[R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane]] = ib / 3u;
         const int dim = R.dim[lane], x = R.x[lane], y = R.y[lane], zb = R.zb[lane];
         const uint32_t wc = nb.w[(1 * 4 + 1) * 3 + 1];
         const uint32_t X = (x + 1 < dim) ? wc ^ nb.w[(2 * 4 + 1) * 3 + 1] : 0u;
@@ -1440,6 +1470,7 @@ __global__ void __launch_bounds__(256, 3) k_emit_cells_q(const ChunkDev* __restr
     const uint32_t lt = lane_lt(lane);
     const uint32_t* W = words + ch.words;
     const uint32_t* vbase = ws.vcnt + ch.words;
+    const uint2* pb = ws.pb + ch.unit0;
     const float* D = dens + ch.dens;
     const int64_t wo = ((int64_t)x * dim + y) * zc + zb;
     const bool interior = x <= dim - 2 && y <= dim - 2 && z <= dim - 2;
@@ -1448,8 +1479,8 @@ __global__ void __launch_bounds__(256, 3) k_emit_cells_q(const ChunkDev* __restr
     const int ng = (int)((gw >> 48) & 0xF);
     if (ng) {
       const uint32_t* pl = ws.gpl + 3 * (ch.words + wo);
-      uint32_t vid = __ldg(vbase + wo) + __popc(__ldg(pl) & lt) + 2 * __popc(__ldg(pl + 1) & lt) +
-                     4 * __popc(__ldg(pl + 2) & lt);
+      uint32_t vid = __ldg(&pb[x].x) + __ldg(vbase + wo) + __popc(__ldg(pl) & lt) +
+                     2 * __popc(__ldg(pl + 1) & lt) + 4 * __popc(__ldg(pl + 2) & lt);
       const int nc = dim - 1;
       const uint8_t bnd = (x == 0 || y == 0 || z == 0 || x == nc - 1 || y == nc - 1 || z == nc - 1);
       for (int g = 0; g < ng; ++g, ++vid) {
@@ -1480,7 +1511,7 @@ __global__ void __launch_bounds__(256, 3) k_emit_cells_q(const ChunkDev* __restr
     q_quad_words(W, dim, zc, x, y, zb, Xi, Yi, Zi);
     const int own = (int)(((Xi >> lane) & 1u) | (((Yi >> lane) & 1u) << 1) | (((Zi >> lane) & 1u) << 2));
     if (!own) continue;
-    int64_t gi = ch.iout + (int64_t)__ldg(ws.icnt + ch.words + wo) +
+    int64_t gi = ch.iout + (int64_t)(__ldg(&pb[x].y) + __ldg(ws.icnt + ch.words + wo)) +
                  4 * (int64_t)(__popc(Xi & lt) + __popc(Yi & lt) + __popc(Zi & lt));
     const bool in0 = ((word_at(W, dim, zc, x, y, zb) >> lane) & 1u) != 0u;
     for (int a = 0; a < 3; ++a) {
@@ -1498,7 +1529,7 @@ __global__ void __launch_bounds__(256, 3) k_emit_cells_q(const ChunkDev* __restr
         lo[cax] = -oc;
         const int e = a == 0 ? 2 * lo[1] + lo[2] : (a == 1 ? 4 + 2 * lo[0] + lo[2] : 8 + 2 * lo[0] + lo[1]);
         const int cm = cell_mask_at(W, dim, zc, cc[0], cc[1], cc[2]);
-        q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, dim, zc, cc[0], cc[1], cc[2]) +
+        q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, pb, dim, zc, cc[0], cc[1], cc[2]) +
                (uint32_t)((T.grp[cm] >> (4 * e)) & 0xF);
       }
       if (!in0) {

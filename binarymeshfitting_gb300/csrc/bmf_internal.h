@@ -53,8 +53,11 @@ struct MeshOut {
 // Per-word scratch of the extraction kernels, indexed like the occupancy
 // words (chunk.words + (x*dim + y)*zc + zb).
 struct WordScratch {
-  uint32_t* vcnt;   // vertices hosted by the word's 32 cells; scanned in place to the chunk-local base
-  uint32_t* icnt;   // indices emitted by the word's cells; scanned in place
+  // The count kernel writes these three for busy words only (words that own a
+  // vertex or emit a primitive); nothing reads them for any other word.
+  uint32_t* vcnt;   // vertices of the x-plane's words before this one (a word's base is pb[plane].x + vcnt)
+  uint32_t* icnt;   // indices of the x-plane's words before this one; Mode R's emit replaces it by the word's
+                    // chunk-local primitive base, which the adjacency reads
   uint32_t* gpl;    // 3 bit-planes of the per-cell triangle (Mode R) / vertex-group (Mode Q) count
   // Work list (nullable), in no particular order; *ccount (zeroed before the
   // count kernel) entries, at most clist_cap kept.  Mode R: every busy word
@@ -65,6 +68,9 @@ struct WordScratch {
   uint2* clist;
   uint32_t* ccount;
   int64_t clist_cap;
+  // Per x-plane (ChunkDev::unit0 + x): its {vertex, index} totals (count
+  // kernel), then their exclusive sums over the chunk's planes (k_chunk_scan)
+  uint2* pb;
   // Band fill (Mode R, nullable): its exactness mask, and the list of samples
   // the count kernel finds at an end of a crossing with an inexact density,
   // as {chunk, sample index in the chunk}; *fcount (zeroed before the count
@@ -130,21 +136,21 @@ int fill_terrain_items(int dim);          // items of one chunk
 int fill_terrain_lines();                 // lines per item
 int fill_terrain_resident_ctas(int run, int octaves, bool band);  // persistent grid: SMs x resident CTAs per SM
 void launch_cell_masks(int dim, const uint32_t* W, uint8_t* masks, cudaStream_t st);
-// contains_mesh flags of chunks whose words were produced elsewhere.
-void launch_word_flags(const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, uint32_t* flags,
-                       cudaStream_t st);
-
-// Extraction: count -> per-chunk scan -> (chunk offsets) -> emit.
+// Extraction: count -> chunk scan -> emit.  flags: the contains_mesh flags the
+// fill wrote; flags_out (instead, with flags null): words produced elsewhere,
+// whose flags the count kernel adds up here (cleared by the caller).
 void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
-                  const uint32_t* words, const uint32_t* flags, WordScratch ws, cudaStream_t st);
-// Scans each chunk's word counts; writes chunk totals (vertices, indices) to
-// d_tot[2c].  d_order (optional): a permutation of the chunks, largest first.
-void launch_scan_chunks(const ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, cudaStream_t st,
-                        const int* d_order = nullptr);
-// Exclusive scan of the chunk totals into chunk.vout / chunk.iout, and the
-// per-chunk info table {voff, vcount, ioff, icount, contains_mesh, status}.
-void launch_chunk_offsets(ChunkDev* d_chunks, int n_chunks, const uint32_t* d_tot, const uint32_t* flags,
-                          int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, cudaStream_t st);
+                  const uint32_t* words, const uint32_t* flags, WordScratch ws, cudaStream_t st,
+                  uint32_t* flags_out = nullptr);
+// Scans each chunk's plane totals in ws.pb, writes chunk totals (vertices,
+// indices) to d_tot[2c], and scans those into chunk.vout / chunk.iout, the
+// per-chunk info table {voff, vcount, ioff, icount, contains_mesh, status} and
+// d_totals {vertices, indices, contains_mesh of chunk 0}.  d_ticket: one int,
+// zero before the first call and left zero by each.
+constexpr int kTotals = 3;
+void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
+                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
+                       cudaStream_t st);
 // Returns the kernels launched: Mode Q QEF placement with vertex keys and
 // d_counts (total vertices on the device) adds the per-vertex k_place_qef.
 int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start,

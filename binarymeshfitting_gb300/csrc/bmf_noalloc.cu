@@ -41,9 +41,11 @@ namespace {
 constexpr int kNoAllocMaxDim = BMF_NOALLOC_MAX_DIM;
 constexpr int64_t kMaxWords = (int64_t)kNoAllocMaxDim * kNoAllocMaxDim * ((kNoAllocMaxDim + 31) / 32);
 // Layout (u32 units): [0, 64) chunk record + unit range + flags + chunk totals
-// + device totals; then vcnt, icnt and the 3 bit-planes, one entry per word.
+// + device totals; then the plane bases (2 per x-plane), vcnt, icnt and the 3
+// bit-planes, one entry per word.
 constexpr int64_t kHeader = 64;
-constexpr int64_t kScratchWords = kHeader + 5 * kMaxWords;
+constexpr int64_t kPlanes = kHeader + 2 * kNoAllocMaxDim;
+constexpr int64_t kScratchWords = kPlanes + 5 * kMaxWords;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kScratchWords];
 
@@ -93,32 +95,30 @@ extern "C" bmf_status bmf_polygonize_noalloc(int32_t dim, const float* d_density
   int* d_u = (int*)(base + 32);                         // [32, 34)
   uint32_t* d_flags = base + 34;                        // [34, 35)
   uint32_t* d_tot = base + 36;                          // [36, 38)
-  int64_t* d_totals = (int64_t*)(base + 40);            // [40, 44), 8-byte aligned
+  int64_t* d_totals = (int64_t*)(base + 40);            // [40, 46), 8-byte aligned
   const int zc = (dim + 31) / 32;
   const int64_t nw = (int64_t)dim * dim * zc;
-  WordScratch ws{base + kHeader, base + kHeader + nw, base + kHeader + 2 * nw};
+  WordScratch ws{base + kPlanes, base + kPlanes + nw, base + kPlanes + 2 * nw};
+  ws.pb = (uint2*)(base + kHeader);
 
   ChunkDev c{};
   c.scale = 1.0f;
   c.dim = dim;
   c.zc = zc;
   k_noalloc_header<<<1, 1, 0, st>>>(c, d_c, d_u);
-  launch_word_flags(d_c, 1, d_words, d_flags, st);  // clears and sets the flags
-  launch_count(mode, d_c, 1, d_u, dim, d_words, d_flags, ws, st);
-  launch_scan_chunks(d_c, 1, ws, d_tot, st);
-  launch_chunk_offsets(d_c, 1, d_tot, d_flags, out->vcap, out->icap, nullptr, d_totals, st);
+  cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st);
+  launch_count(mode, d_c, 1, d_u, dim, d_words, nullptr, ws, st, d_flags);  // sets the flags
+  launch_chunk_scan(d_c, 1, ws, d_tot, d_flags, out->vcap, out->icap, nullptr, d_totals, nullptr, st);
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   launch_emit(mode, placement, d_c, 1, d_u, dim, d_words, d_density, d_flags, ws, mo, nullptr, st);
   if (cudaPeekAtLastError() != cudaSuccess) return BMF_ERR_CUDA;
-  int64_t totals[2] = {0, 0};
-  uint32_t flags = 0;
+  int64_t totals[kTotals] = {0, 0, 0};
   if (cudaMemcpyAsync(totals, d_totals, sizeof(totals), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return BMF_ERR_CUDA;
   out->n_verts = totals[0];
   out->n_idx = totals[1];
-  out->contains_mesh = ((flags & 1u) || ((flags & 6u) == 6u)) ? 1 : 0;
+  out->contains_mesh = (int32_t)totals[2];
   out->prim_size = mode == BMF_MODE_R ? 3 : 4;
   if (out->n_verts > out->vcap || out->n_idx > out->icap) return BMF_ERR_CAPACITY;
   return BMF_OK;

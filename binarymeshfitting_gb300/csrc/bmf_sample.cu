@@ -674,26 +674,6 @@ __global__ void k_cell_masks(int dim, int zc, const uint32_t* __restrict__ W, ui
   }
 }
 
-// contains_mesh flags from existing words (one CTA per chunk).
-__global__ void k_word_flags(const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ words,
-                             uint32_t* __restrict__ flags) {
-  const ChunkDev ch = chunks[blockIdx.x];
-  const int64_t n = (int64_t)ch.dim * ch.dim * ch.zc;
-  uint32_t f = 0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint32_t w = words[ch.words + i];
-    f |= (w != 0u && w != kFull) ? 1u : (w == kFull ? 2u : 4u);
-  }
-  f = __reduce_or_sync(kFull, f);
-  if ((threadIdx.x & 31) == 0 && f) atomicOr(flags + blockIdx.x, f);
-}
-
-void launch_word_flags(const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, uint32_t* flags,
-                       cudaStream_t st) {
-  cudaMemsetAsync(flags, 0, sizeof(uint32_t) * n_chunks, st);
-  k_word_flags<<<n_chunks, 256, 0, st>>>(d_chunks, words, flags);
-}
-
 // The 2D heightmap's (x, z) column heights of a batch, one thread per column
 // over items of kColumnItem consecutive columns of one chunk ({chunk, first
 // column}, column = x * dim + z), stored at chunk.words + column: every
