@@ -20,19 +20,10 @@ namespace {
 
 enum Slot {
   S_CHUNKS, S_UNITS, S_FLAGS, S_TOT, S_INFO, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
-  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_NUM
+  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_NUM
 };
 
 constexpr int kMaxDim = 512;
-// below this many chunks the sweeps run as whole-mesh kernels: one CTA per
-// chunk needs several chunks per resident CTA to balance.  Mode R batches of
-// the mixed-LOD update run chunk by chunk from 512 chunks (processing stage,
-// whole-mesh -> chunk by chunk: 512 chunks 1.79 -> 1.68 ms, 1024 chunks 2.48
-// -> 1.73, 1536 chunks 3.21 -> 2.03); Mode Q batches and fit plans from 2048
-// (Mode Q chunk by chunk: mixed 512 / 1024 chunks 1.59 -> 2.21 / 2.24 -> 2.75
-// ms, 512 equal chunks lose 3 %)
-constexpr int kChunkSweepMinChunks = 2048;
-constexpr int kChunkSweepMinChunksR = 512;
 // fit plans: the adjoint sweeps run chunk by chunk from this many chunks (one
 // 512-thread CTA per chunk, four per SM)
 constexpr int kChunkSweepBwdMinChunks = 256;
@@ -44,12 +35,16 @@ struct DevBuf {
 
 }  // namespace
 
+constexpr int kPinned = 64, kPinnedFailed = 32;  // h_pinned: entries, and the one that holds the sweeps' failure mark
+
 struct bmf_ctx {
   int device = 0;
   std::string err;
   int64_t launches = 0;
   DevBuf bufs[S_NUM];
   int64_t* h_pinned = nullptr;  // readback staging
+  TeamSync* team = nullptr;     // barrier of the whole-mesh sweep kernel
+  unsigned* team_failed() const { return (unsigned*)(h_pinned + kPinnedFailed); }
 };
 
 struct bmf_batch {
@@ -91,9 +86,9 @@ struct bmf_batch {
   int2* d_fill_items = nullptr;
   int n_fill_items = 0;
   int* d_queue = nullptr;
-  // the chunk-by-chunk sweeps: chunk indices by size, largest first, and their queue
-  int* d_order = nullptr;
-  int* d_pqueue = nullptr;
+  SweepForm form = kSweepLaunches;
+  SweepLists sweep;  // the chunk-by-chunk sweeps' work lists
+  TeamSync* team = nullptr;  // barrier of the whole-mesh sweep kernel
   int fill_grid = 0;
   int fill_mode = 0;
   int fill_run = 16;  // the tile height the autotuner picks on the mixed-LOD update
@@ -139,6 +134,15 @@ bmf_status cuda_check(bmf_ctx* ctx, cudaError_t e, const char* what) {
     bmf_status _s = cuda_check((ctx), cudaPeekAtLastError(), "kernel launch"); \
     if (_s != BMF_OK) return _s;                                               \
   } while (0)
+
+// After a synchronisation: did a wait of the whole-mesh sweep kernel run out?
+// (Only when its CTAs could not all make progress; the barrier is set anew.)
+bmf_status team_check(bmf_ctx* ctx, TeamSync* team) {
+  if (!team || !*(volatile unsigned*)ctx->team_failed()) return BMF_OK;
+  *ctx->team_failed() = 0;
+  cudaMemset(team, 0, sizeof(TeamSync));
+  return fail(ctx, BMF_ERR_CUDA, "a wait of the smoothing sweeps ran out: the mesh is not smoothed");
+}
 
 template <class T>
 bmf_status scratch(bmf_ctx* ctx, Slot s, size_t count, T** out) {
@@ -228,7 +232,7 @@ bmf_status upload_single(bmf_ctx* ctx, const ChunkDev& c, cudaStream_t st, Chunk
 bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunks, const int* d_units, int n_units,
                         const uint32_t* d_words, const float* d_dens, uint32_t* d_flags, bool flags_ready,
                         int64_t words_total, const MeshOut& mo, int64_t* d_totals, cudaStream_t st,
-                        WordScratch* ws_out = nullptr) {
+                        StructuredAdj* sa = nullptr) {
   constexpr int n_chunks = 1;
   WordScratch ws{};
   uint32_t* tot = nullptr;
@@ -246,7 +250,13 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunk
     ws.clist = list;
     ws.ccount = (uint32_t*)(list + ws.clist_cap);
   }
-  if (ws_out) *ws_out = ws;
+  if (sa) {
+    *sa = StructuredAdj{mode, d_chunks, n_chunks, d_words, ws, mo.vkey};
+    if (sweep_form(mode, 1, (int64_t)n_units * n_units, &sa->lists) == kSweepTeam) {
+      sa->team = ctx->team;
+      sa->team_failed = ctx->team_failed();
+    }
+  }
   if (!flags_ready) BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
   launch_count(mode, d_chunks, n_chunks, d_units, n_units, d_words, flags_ready ? d_flags : nullptr, ws, st,
                flags_ready ? nullptr : d_flags);
@@ -258,28 +268,38 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunk
   return BMF_OK;
 }
 
+// Face sweeps left out for a field (internal.h): none for the cuboid, whose
+// walls give half its vertices normals without a y part in every sweep -- each
+// would take primal_older_normal (1200 x 65^3: the sweeps 2.17 -> 2.87 ms).
+int field_skipped(int kind, int iters, int sn) {
+  return kind == BMF_FIELD_CUBOID ? 0 : sweep_skipped(iters, sn);
+}
+
 bmf_status mesh_valid(bmf_ctx* ctx, const bmf_mesh* m) {
   if (!m || !m->d_pos || !m->d_idx || m->vcap < 0 || m->icap < 0)
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "mesh output: d_pos and d_idx are required");
   return BMF_OK;
 }
 
+// x: the positions before the left-out face sweeps (x[0] the emitted mesh), or null
 bmf_status process_mesh(bmf_ctx* ctx, bmf_mesh* mesh, int iters, int pb, int sn, cudaStream_t st,
-                        const StructuredAdj* sa = nullptr) {
+                        const StructuredAdj* sa = nullptr, float* const* x = nullptr) {
   const int N = mesh->prim_size;
   if (N != 3 && N != 4) return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "prim_size must be 3 or 4");
   if (!mesh->d_valence || !mesh->d_boundary)
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_process needs d_valence and d_boundary");
   const int64_t nv = mesh->n_verts, n_prims = mesh->n_idx / N;
   // MeshProcessor::init returns early without work on an empty mesh (MeshProcessor.cpp:28-29)
-  if (iters <= 0 || nv == 0 || mesh->n_idx < N) return BMF_OK;
+  // (kept positions have to reach the output even then)
+  if (iters <= 0 || nv == 0 || (mesh->n_idx < N && !x)) return BMF_OK;
   ProcessScratch ps{};
   bmf_status s;
   if ((s = scratch(ctx, S_OFF, (size_t)nv + 1, &ps.off)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_CURSOR, (size_t)nv, &ps.cursor)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_ADJ, (size_t)n_prims * N, &ps.adj)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_DUALP, (size_t)n_prims * 3, &ps.dual_p)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_DUALN, (size_t)n_prims * 3, &ps.dual_n)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_DUALP, (size_t)n_prims * 4, &ps.dual_p)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_DUALN, (size_t)n_prims * 2, &ps.dual_n)) != BMF_OK) return s;
+  for (int k = 0; x && k < 3; ++k) ps.x[k] = x[k];
   if ((s = scratch(ctx, S_SCANTMP, (size_t)(nv / 4096 + 2), &ps.tmp)) != BMF_OK) return s;
   const int k = launch_process(N, nv, n_prims, nullptr, mesh->d_pos, mesh->d_nrm, mesh->d_boundary,
                                mesh->d_valence, mesh->d_idx, iters, pb, sn, ps, sa, st);
@@ -315,8 +335,14 @@ bmf_status bmf_create(const bmf_config* cfg, bmf_ctx** out) {
   if (cudaSetDevice(dev) != cudaSuccess) return BMF_ERR_CUDA;
   bmf_ctx* ctx = new bmf_ctx();
   ctx->device = dev;
-  if (cudaMallocHost(&ctx->h_pinned, 64 * sizeof(int64_t)) != cudaSuccess) {
+  if (cudaMallocHost(&ctx->h_pinned, kPinned * sizeof(int64_t)) != cudaSuccess) {
     delete ctx;
+    return BMF_ERR_OUT_OF_MEMORY;
+  }
+  std::memset(ctx->h_pinned, 0, kPinned * sizeof(int64_t));
+  if (cudaMalloc(&ctx->team, sizeof(TeamSync)) != cudaSuccess ||
+      cudaMemset(ctx->team, 0, sizeof(TeamSync)) != cudaSuccess) {
+    bmf_destroy(ctx);
     return BMF_ERR_OUT_OF_MEMORY;
   }
   *out = ctx;
@@ -329,6 +355,7 @@ bmf_status bmf_destroy(bmf_ctx* ctx) {
   for (auto& b : ctx->bufs)
     if (b.p) cudaFree(b.p);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+  if (ctx->team) cudaFree(ctx->team);
   delete ctx;
   return BMF_OK;
 }
@@ -525,9 +552,18 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   if ((opts->iters > 0 || (opts->mode == BMF_MODE_Q && opts->placement == BMF_PLACE_QEF)) &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
-  WordScratch ws{};
+  // sweeps that leave steps out read the mesh from x[0] and write out->d_pos
+  float* x[3] = {};
+  const int skip = field_skipped(field->kind, opts->iters, opts->smooth_normals && out->d_nrm);
+  for (int k = 0; skip && k <= skip; ++k)
+    if ((s = scratch(ctx, (Slot)(S_X0 + k), (size_t)out->vcap * 3, &x[k])) != BMF_OK) return s;
+  if (skip) {
+    mo.pos = x[0];
+    mo.nrm = nullptr;
+  }
+  StructuredAdj sa{};
   if ((s = extract_core(ctx, opts->mode, opts->placement, d_c, d_u, dim, d_words, d_dens, d_flags, true,
-                        (int64_t)dim * dim * c.zc, mo, d_totals, st, &ws)) != BMF_OK)
+                        (int64_t)dim * dim * c.zc, mo, d_totals, st, opts->iters > 0 ? &sa : nullptr)) != BMF_OK)
     return s;
   BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, kTotals * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   BMF_CUDA(ctx, cudaStreamSynchronize(st));
@@ -538,11 +574,12 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_extract_chunk: output capacity exceeded (needed counts reported)");
   // ChunkGenerator.cpp:112: processing only when the chunk has a mesh
-  if (opts->iters > 0 && out->contains_mesh && out->n_verts && out->n_idx) {
-    const StructuredAdj sa{opts->mode, d_c, 1, d_words, ws, mo.vkey};
-    if ((s = process_mesh(ctx, out, opts->iters, opts->process_boundary, opts->smooth_normals, st, &sa)) != BMF_OK)
+  if (opts->iters > 0 && out->contains_mesh && out->n_verts && (out->n_idx || skip)) {
+    if ((s = process_mesh(ctx, out, opts->iters, opts->process_boundary, opts->smooth_normals, st, &sa,
+                          skip ? x : nullptr)) != BMF_OK)
       return s;
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
+    return team_check(ctx, sa.team);
   }
   return BMF_OK;
 }
@@ -615,17 +652,24 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if ((s = bail(cudaMemcpy(b->d_units, units.data(), sizeof(int) * (n_chunks + 1), cudaMemcpyHostToDevice),
                 "upload units")) != BMF_OK)
     return s;
+  if (opts->iters > 0) {
+    int64_t columns = 0;
+    for (const ChunkDev& c : b->h_chunks) columns += (int64_t)c.dim * c.dim;
+    b->form = sweep_form(opts->mode, n_chunks, columns, &b->sweep);
+    if (b->form == kSweepChunks) {
+      if ((s = bail(cudaMalloc(&b->sweep.order, sizeof(int) * (n_chunks + kSweepHead)), "sweep lists")) != BMF_OK)
+        return s;
+      b->sweep.head = b->sweep.order + n_chunks;
+    }
+  }
+  if ((s = bail(cudaMalloc(&b->team, sizeof(TeamSync)), "sweep barrier")) != BMF_OK) return s;
+  if ((s = bail(cudaMemset(b->team, 0, sizeof(TeamSync)), "sweep barrier")) != BMF_OK) return s;
   // chunks by size, largest first (longest-processing-time order for the
-  // work queues of the fill and of the chunk-by-chunk sweeps)
+  // work queue of the fill)
   std::vector<int> order(n_chunks);
   for (int i = 0; i < n_chunks; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int c) { return b->h_chunks[a].dim > b->h_chunks[c].dim; });
-  if ((s = bail(cudaMalloc(&b->d_order, sizeof(int) * n_chunks), "chunk order")) != BMF_OK) return s;
-  if ((s = bail(cudaMalloc(&b->d_pqueue, sizeof(int)), "sweep queue")) != BMF_OK) return s;
-  if ((s = bail(cudaMemcpy(b->d_order, order.data(), sizeof(int) * n_chunks, cudaMemcpyHostToDevice),
-                "upload chunk order")) != BMF_OK)
-    return s;
   if (b->field.kind == BMF_FIELD_TERRAIN_FBM) {
     // line items in that order
     std::vector<int2> items;
@@ -745,19 +789,23 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   bmf_ctx* ctx = b->ctx;
   const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
   const int64_t np = icap / N;
-  void* ptrs[] = {b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p, b->ps.dual_n, b->ps.tmp,
-                  b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  void** ptrs[] = {(void**)&b->ps.off, (void**)&b->ps.adj, (void**)&b->ps.dual_p, (void**)&b->ps.dual_n,
+                   (void**)&b->ps.tmp, (void**)&b->ps.x[0], (void**)&b->ps.x[1], (void**)&b->ps.x[2],
+                   (void**)&b->d_idxg, (void**)&b->d_valence, (void**)&b->d_boundary, (void**)&b->d_vkey};
+  for (void** p : ptrs) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
   b->proc_vcap = b->proc_icap = 0;
   BMF_CUDA(ctx, cudaMalloc(&b->ps.off, sizeof(uint32_t) * (vcap + 1)));
-  BMF_CUDA(ctx, cudaMalloc(&b->ps.cursor, sizeof(uint32_t) * (vcap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->ps.adj, sizeof(uint32_t) * (np * N + 1)));
-  // 4 floats per primitive: the chunk-by-chunk sweeps keep (p, n.x) as one float4
   BMF_CUDA(ctx, cudaMalloc(&b->ps.dual_p, sizeof(float) * (4 * np + 4)));
-  BMF_CUDA(ctx, cudaMalloc(&b->ps.dual_n, sizeof(float) * (3 * np + 3)));
+  if (b->opts.smooth_normals) BMF_CUDA(ctx, cudaMalloc(&b->ps.dual_n, sizeof(float) * (2 * np + 2)));
+  if (const int skip = field_skipped(b->field.kind, b->opts.iters, b->opts.smooth_normals))
+    for (int k = 0; k <= skip; ++k) BMF_CUDA(ctx, cudaMalloc(&b->ps.x[k], sizeof(float) * 3 * (vcap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->ps.tmp, sizeof(uint32_t) * (vcap / 4096 + 2)));
-  BMF_CUDA(ctx, cudaMalloc(&b->d_idxg, sizeof(uint32_t) * (icap + 1)));
+  if (b->opts.iters > 0 && b->form != kSweepChunks)
+    BMF_CUDA(ctx, cudaMalloc(&b->d_idxg, sizeof(uint32_t) * (icap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->d_valence, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_boundary, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_vkey, sizeof(uint32_t) * (vcap + 1)));
@@ -766,16 +814,49 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   return BMF_OK;
 }
 
-// The structured adjacency of a batch; with enough chunks to fill the GPU
-// the sweeps run chunk by chunk (one CTA per chunk, largest chunks first).
+// The structured adjacency of a batch.
 StructuredAdj batch_adj(const bmf_batch* b) {
   StructuredAdj sa{b->opts.mode, b->d_chunks, b->n, b->d_words, b->ws, b->d_vkey};
-  if (b->n >= (b->opts.mode == BMF_MODE_R ? kChunkSweepMinChunksR : kChunkSweepMinChunks)) {
+  if (b->form == kSweepChunks) {
     sa.tot = b->d_tot;
-    sa.order = b->d_order;
-    sa.queue = b->d_pqueue;
+    sa.lists = b->sweep;
+  } else if (b->form == kSweepTeam) {
+    sa.team = b->team;
+    sa.team_failed = b->ctx->team_failed();
   }
   return sa;
+}
+
+// The plan's sweep scratch for this output; the positions before the left-out
+// face sweeps are kept only with normals.
+ProcessScratch batch_sweep_scratch(const bmf_batch* b, const bmf_batch_out* out) {
+  ProcessScratch ps = b->ps;
+  if (!field_skipped(b->field.kind, b->opts.iters, b->opts.smooth_normals && out->d_nrm))
+    for (float*& x : ps.x) x = nullptr;
+  return ps;
+}
+
+// Where the emit puts the mesh: with sweeps that leave steps out, the
+// positions go to the sweeps' first buffer, and the sweeps set every normal.
+MeshOut batch_mesh_out(const bmf_batch* b, const bmf_batch_out* out) {
+  const bool proc = b->opts.iters > 0;
+  const ProcessScratch ps = batch_sweep_scratch(b, out);
+  const bool keep = proc && ps.x[0];
+  // the chunk-by-chunk sweeps read the chunk-local indices
+  return MeshOut{keep ? ps.x[0] : out->d_pos, keep ? nullptr : out->d_nrm,
+                 proc && !out->d_boundary ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr, out->d_idx,
+                 proc && b->form != kSweepChunks ? b->d_idxg : nullptr, out->vcap, out->icap,
+                 batch_keys(b) ? b->d_vkey : nullptr};
+}
+
+// Enqueues the sweeps of one update; returns the kernels launched.
+int batch_sweeps(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st) {
+  const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
+  const StructuredAdj sa = batch_adj(b);
+  return launch_process(N, out->vcap, out->icap / N, b->d_totals, out->d_pos, out->d_nrm,
+                        out->d_boundary ? out->d_boundary : b->d_boundary, b->d_valence,
+                        b->form == kSweepChunks ? out->d_idx : b->d_idxg, b->opts.iters, b->opts.process_boundary,
+                        b->opts.smooth_normals, batch_sweep_scratch(b, out), &sa, st);
 }
 
 // Enqueues one whole update on st (captured into the graph, or run directly).
@@ -788,9 +869,8 @@ bmf_status batch_record(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st,
   const bool band = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;  // the 2D column fill needs no fix-up
   if (band) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                    b->d_totals, b->d_ticket, st);
-  MeshOut mo{out->d_pos, out->d_nrm, proc ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr,
-             out->d_idx, proc ? b->d_idxg : nullptr, out->vcap, out->icap, batch_keys(b) ? b->d_vkey : nullptr};
+                    b->d_totals, b->d_ticket, st, &b->sweep);
+  const MeshOut mo = batch_mesh_out(b, out);
   int64_t k = (band ? 4 : 3) + (b->d_cols ? 1 : 0);
   k += launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_dens,
                    b->d_flags, b->ws, mo, b->d_totals, st);
@@ -805,15 +885,7 @@ bmf_status batch_record(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st,
     else
       BMF_CUDA(ctx, cudaEventRecord(b->extract_done, st));
   }
-  if (proc) {
-    const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
-    const StructuredAdj sa = batch_adj(b);
-    k += launch_process(N, out->vcap, out->icap / N, b->d_totals, out->d_pos, out->d_nrm, b->d_boundary,
-                        b->d_valence, b->d_idxg, b->opts.iters, b->opts.process_boundary, b->opts.smooth_normals,
-                        b->ps, &sa, st);
-    if (out->d_boundary)
-      BMF_CUDA(ctx, cudaMemcpyAsync(out->d_boundary, b->d_boundary, (size_t)out->vcap, cudaMemcpyDeviceToDevice, st));
-  }
+  if (proc) k += batch_sweeps(b, out, st);
   BMF_CUDA(ctx, cudaPeekAtLastError());
   *kernels = k;
   return BMF_OK;
@@ -875,6 +947,7 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
     out->n_idx = b->h_pinned[1];
     if (out->n_verts > out->vcap || out->n_idx > out->icap)
       return fail(ctx, BMF_ERR_CAPACITY, "bmf_batch_run: output capacity exceeded (needed totals reported)");
+    if (b->form == kSweepTeam) return team_check(ctx, b->team);
   }
   return BMF_OK;
 }
@@ -903,7 +976,7 @@ bmf_status bmf_batch_wait(bmf_batch* b, bmf_batch_out* out, int32_t timeout_ms) 
   out->n_idx = b->h_pinned[1];
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_batch_wait: output capacity exceeded (needed totals reported)");
-  return BMF_OK;
+  return b->form == kSweepTeam ? team_check(ctx, b->team) : BMF_OK;
 }
 
 bmf_status bmf_batch_wait_extraction(bmf_batch* b, void* stream) {
@@ -971,21 +1044,14 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaEventRecord(ev[7], st));
   BMF_CUDA(ctx, cudaEventRecord(ev[3], st));  // the word scan is part of the count
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                    b->d_totals, b->d_ticket, st);
+                    b->d_totals, b->d_ticket, st, &b->sweep);
   BMF_CUDA(ctx, cudaEventRecord(ev[4], st));
-  MeshOut mo{out->d_pos, out->d_nrm, proc ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr,
-             out->d_idx, proc ? b->d_idxg : nullptr, out->vcap, out->icap, batch_keys(b) ? b->d_vkey : nullptr};
+  const MeshOut mo = batch_mesh_out(b, out);
   const int ek = launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words,
                              b->d_dens, b->d_flags, b->ws, mo, b->d_totals, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[5], st));
   int pk = 0;
-  if (proc) {
-    const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
-    const StructuredAdj sa = batch_adj(b);
-    pk = launch_process(N, out->vcap, out->icap / N, b->d_totals, out->d_pos, out->d_nrm, b->d_boundary,
-                        b->d_valence, b->d_idxg, b->opts.iters, b->opts.process_boundary, b->opts.smooth_normals,
-                        b->ps, &sa, st);
-  }
+  if (proc) pk = batch_sweeps(b, out, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[6], st));
   BMF_CUDA(ctx, cudaEventSynchronize(ev[6]));
   BMF_CUDA(ctx, cudaPeekAtLastError());
@@ -1118,18 +1184,12 @@ bmf_status bmf_batch_autotune(bmf_batch* b, bmf_batch_out* out, int32_t reps, vo
   // stage 2: the sweeps, on the mesh of one real update
   if (b->opts.iters > 0) {
     if ((s = bmf_batch_run(b, out, 0, 1, stream)) != BMF_OK) return s;
-    const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
-    const StructuredAdj sa = batch_adj(b);
     const int blocks[3] = {128, 256, 512};
     float best_ms = 1e30f;
     for (int bs : blocks) {
       b->ps.block = bs;
       float ms = 0.0f;
-      s = time_it([&] {
-        launch_process(N, out->vcap, out->icap / N, b->d_totals, out->d_pos, out->d_nrm, b->d_boundary,
-                       b->d_valence, b->d_idxg, b->opts.iters, b->opts.process_boundary, b->opts.smooth_normals,
-                       b->ps, &sa, st);
-      }, &ms);
+      s = time_it([&] { batch_sweeps(b, out, st); }, &ms);
       if (s != BMF_OK) return s;
       report.push_back(ms);
       if (ms < best_ms) {
@@ -1169,8 +1229,10 @@ struct bmf_fit {
   uint32_t *d_idxg = nullptr, *d_vkey = nullptr;
   uint8_t *d_valence = nullptr, *d_boundary = nullptr;
   float* d_g = nullptr;           // position-gradient work buffer
-  int* d_order = nullptr;         // chunk order of the chunk-by-chunk sweeps (identity) and its queue
+  SweepLists sweep;               // the chunk-by-chunk sweeps' work lists, and the adjoint's queue over them
   int* d_pqueue = nullptr;
+  SweepForm form = kSweepLaunches;  // the forward's sweeps
+  TeamSync* team = nullptr;       // barrier of the whole-mesh sweep kernel
   uint32_t* d_qlist = nullptr;    // QEF-placed vertices of the forward, for the wide backward (+ counter at [vcap])
   float* d_qseed = nullptr;       // their FP32 eigenvectors (9 per entry), recorded by the forward
   uint8_t* d_qflag = nullptr;     // per vertex: took the QEF branch in the forward
@@ -1187,8 +1249,8 @@ bmf_status bmf_fit_destroy(bmf_fit* f) {
   if (!f) return BMF_ERR_INVALID_ARGUMENT;
   void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.icnt,
                   f->ws.gpl, f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
-                  f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_qlist, f->d_qseed, f->d_clist, f->d_order,
-                  f->d_pqueue, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb};
+                  f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
+                  f->d_pqueue, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (f->h_pinned) cudaFreeHost(f->h_pinned);
@@ -1238,6 +1300,8 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_words, sizeof(uint32_t) * words) == cudaSuccess &&
             cudaMalloc(&f->d_totals, sizeof(int64_t) * kTotals) == cudaSuccess &&
             cudaMalloc(&f->d_ticket, sizeof(int)) == cudaSuccess &&
+            cudaMalloc(&f->team, sizeof(TeamSync)) == cudaSuccess &&
+            cudaMemset(f->team, 0, sizeof(TeamSync)) == cudaSuccess &&
             cudaMemset(f->d_ticket, 0, sizeof(int)) == cudaSuccess &&
             cudaMalloc(&f->ws.pb, sizeof(uint2) * n_chunks * dim) == cudaSuccess &&
             cudaMalloc(&f->ws.vcnt, sizeof(uint32_t) * words) == cudaSuccess &&
@@ -1252,7 +1316,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_valence, vcap + 1) == cudaSuccess && cudaMalloc(&f->d_boundary, vcap + 1) == cudaSuccess &&
             cudaMalloc(&f->d_g, sizeof(float) * 3 * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->d_qlist, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
-            cudaMalloc(&f->d_order, sizeof(int) * n_chunks) == cudaSuccess &&
+            cudaMalloc(&f->sweep.order, sizeof(int) * (n_chunks + kSweepHead)) == cudaSuccess &&
             cudaMalloc(&f->d_pqueue, sizeof(int)) == cudaSuccess &&
             (!(flags & (BMF_FIT_ADJOINT_F64 | BMF_FIT_ADJOINT_DF)) ||
              (cudaMalloc(&f->d_qseed, sizeof(float) * 9 * (vcap + 1)) == cudaSuccess &&
@@ -1262,11 +1326,8 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMallocHost(&f->h_pinned, sizeof(int64_t) * 4) == cudaSuccess &&
             cudaMemcpy(f->d_chunks, hc.data(), sizeof(ChunkDev) * n_chunks, cudaMemcpyHostToDevice) == cudaSuccess &&
             cudaMemcpy(f->d_units, units.data(), sizeof(int) * (n_chunks + 1), cudaMemcpyHostToDevice) == cudaSuccess;
-  if (ok) {  // every chunk has the same size: the sweep queue takes them in index order
-    std::vector<int> order(n_chunks);
-    for (int i = 0; i < n_chunks; ++i) order[i] = i;
-    ok = cudaMemcpy(f->d_order, order.data(), sizeof(int) * n_chunks, cudaMemcpyHostToDevice) == cudaSuccess;
-  }
+  f->sweep.head = f->sweep.order + n_chunks;
+  f->form = iters > 0 ? sweep_form(BMF_MODE_Q, n_chunks, (int64_t)n_chunks * dim * dim, &f->sweep) : kSweepLaunches;
   if (!ok) {
     bmf_fit_destroy(f);
     return fail(ctx, BMF_ERR_OUT_OF_MEMORY, "bmf_fit_create: device allocation failed");
@@ -1292,7 +1353,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
                       f->d_flags, st);
   launch_count(BMF_MODE_Q, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words, f->d_flags, f->ws, st);
   launch_chunk_scan(f->d_chunks, f->n, f->ws, f->d_tot, f->d_flags, f->vcap, f->icap, d_chunk_info, f->d_totals,
-                    f->d_ticket, st);
+                    f->d_ticket, st, &f->sweep);
   MeshOut mo{d_pos, nullptr, f->d_boundary, f->d_valence, d_idx, f->d_idxg, f->vcap, f->icap, f->d_vkey};
   if (f->d_qflag && f->placement == BMF_PLACE_QEF) {  // the wide adjoint reads the forward's QEF branches
     mo.qflag = f->d_qflag;
@@ -1304,14 +1365,16 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
                           d_density, f->d_flags, f->ws, mo, f->d_totals, st);
   if (f->iters > 0) {
     StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->d_words, f->ws, f->d_vkey};
-    if (f->n >= kChunkSweepMinChunks) {
+    if (f->form == kSweepChunks) {
       sa.tot = f->d_tot;
-      sa.order = f->d_order;
-      sa.queue = f->d_pqueue;
+      sa.lists = f->sweep;
       sa.wide_adj = true;  // bmf_fit_backward's adjoint sweeps read it
+    } else if (f->form == kSweepTeam) {
+      sa.team = f->team;
+      sa.team_failed = ctx->team_failed();
     }
-    k += launch_process(4, f->vcap, f->icap / 4, f->d_totals, d_pos, nullptr, f->d_boundary, f->d_valence, f->d_idxg,
-                        f->iters, 0, 0, f->ps, &sa, st);
+    k += launch_process(4, f->vcap, f->icap / 4, f->d_totals, d_pos, nullptr, f->d_boundary, f->d_valence,
+                        f->form == kSweepChunks ? d_idx : f->d_idxg, f->iters, 0, 0, f->ps, &sa, st);
   }
   BMF_LAUNCHED(ctx, k);
   f->last_density = d_density;
@@ -1322,6 +1385,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
     h_counts[1] = f->h_pinned[1];
     if (h_counts[0] > f->vcap || h_counts[1] > f->icap)
       return fail(ctx, BMF_ERR_CAPACITY, "bmf_fit_forward: output capacity exceeded (needed totals reported)");
+    if (f->form == kSweepTeam) return team_check(ctx, f->team);
   }
   return BMF_OK;
 }
@@ -1369,8 +1433,8 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
   StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->d_words, f->ws, f->d_vkey};
   if (f->n >= kChunkSweepBwdMinChunks) {
     sa.tot = f->d_tot;
-    sa.order = f->d_order;
-    sa.queue = f->d_pqueue;
+    sa.lists = f->sweep;
+    sa.bwd_queue = f->d_pqueue;
   }
   int k = launch_process_bwd(4, f->vcap, f->icap / 4, f->d_totals, f->d_boundary, f->d_valence, f->d_idxg, f->iters,
                              0, f->ps, f->d_g, &sa, st);
@@ -1388,8 +1452,8 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
   void* ptrs[] = {b->d_chunks, b->d_units, b->d_flags, b->d_tot, b->d_totals, b->d_dens, b->d_words,
                   b->ws.vcnt, b->ws.icnt, b->ws.gpl, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
-                  b->d_fill_items, b->d_queue, b->d_order, b->d_pqueue, b->d_clist, b->d_exact, b->d_fix,
-                  b->d_cols, b->d_ticket, b->ws.pb};
+                  b->d_fill_items, b->d_queue, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
+                  b->d_cols, b->d_ticket, b->ws.pb, b->team, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);

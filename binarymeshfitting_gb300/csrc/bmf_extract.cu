@@ -404,12 +404,20 @@ __device__ __forceinline__ T warp_incl_sum(T v, int lane) {
   return v;
 }
 
+// Size class of v >= 1 items: two per power of two.
+__device__ __forceinline__ int size_bin(uint32_t v) {
+  const int l = 31 - __clz(v);
+  return 2 * l + (l > 0 ? (int)((v >> (l - 1)) & 1u) : 0);
+}
+
 __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restrict__ chunks, int n, uint2* __restrict__ pb,
                                                              uint32_t* tot, const uint32_t* __restrict__ flags,
                                                              int64_t vcap, int64_t icap, int64_t* __restrict__ info,
-                                                             int64_t* __restrict__ totals, int* __restrict__ ticket) {
+                                                             int64_t* __restrict__ totals, int* __restrict__ ticket,
+                                                             SweepLists sweep) {
   __shared__ int64_t s_v[kScanWarps], s_i[kScanWarps];
   __shared__ bool s_last;
+  __shared__ int s_bin[64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int mine = blockIdx.x * kScanWarps + warp;
   if (mine < n) {
@@ -472,6 +480,35 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
     totals[1] = carry_i;
     totals[2] = contains_mesh(flags[0]) ? 1 : 0;
     if (gridDim.x > 1) *ticket = 0;
+  }
+  if (!sweep.order) return;
+  // the sweeps' work lists: a counting sort by size, largest first, without
+  // the empty chunks.  A chunk goes to a whole cluster when it holds more than
+  // a CTA's even share of the vertices: alone it would end after all others.
+  if (threadIdx.x < 64) s_bin[threadIdx.x] = 0;
+  __syncthreads();
+  for (int c = threadIdx.x; c < n; c += kScanThreads) {
+    const uint32_t v = __ldcg(tot + 2 * c);
+    if (v) atomicAdd(&s_bin[63 - size_bin(v)], 1);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int a = s_bin[2 * lane], b = s_bin[2 * lane + 1], incl = warp_incl_sum(a + b, lane);
+    const int64_t share = carry_v / sweep.ctas;
+    const int cut = sweep.cluster > 1 ? 63 - size_bin((uint32_t)max(min(share, (int64_t)0x7fffffff), (int64_t)512)) : 0;
+    const int big = __reduce_add_sync(kFull, (2 * lane < cut ? a : 0) + (2 * lane + 1 < cut ? b : 0));
+    s_bin[2 * lane] = incl - a - b;
+    s_bin[2 * lane + 1] = incl - b;
+    if (lane == 31) {
+      sweep.head[0] = big;
+      sweep.head[1] = incl;
+      sweep.head[2] = sweep.head[3] = 0;
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < n; c += kScanThreads) {
+    const uint32_t v = __ldcg(tot + 2 * c);
+    if (v) sweep.order[atomicAdd(&s_bin[63 - size_bin(v)], 1)] = c;
   }
 }
 
@@ -775,8 +812,8 @@ void launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_c
 // edge, whose primitive ids are ascending in linear cell order and, inside a
 // cell, in triangle-list order -- exactly the ascending-prim order
 // init_primitives produces.  A Mode Q vertex is used by one quad per interior
-// crossing edge of its group; those quad ids are sorted.  No atomics, no sort
-// pass, deterministic.
+// crossing edge of its group, walked in ascending quad order.  No atomics, no
+// sort, deterministic.
 // ---------------------------------------------------------------------------
 
 // Three consecutive inside bits z0..z0+2 of line (x, y) (zero outside the
@@ -860,9 +897,13 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
   } else {
     const int g = k;
     const int m = cell_mask_at(W, dim, zc, x, y, z);
-    uint32_t ids[12];
     const uint64_t gw = T.grp[m];
-    for (int e = 0; e < 12; ++e) {
+    // a quad's id grows with its edge's owner sample, then axis: walking the
+    // cell's edges in that order gives the list ascending
+    constexpr uint64_t kEdgeOrder = 0xB7A639251840ull;  // 0, 4, 8, 1, 5, 2, 9, 3, 6, 10, 7, 11 from the low nibble
+#pragma unroll 1
+    for (uint64_t eo = kEdgeOrder, i = 0; i < 12; ++i, eo >>= 4) {
+      const int e = (int)(eo & 0xF);
       if ((int)((gw >> (4 * e)) & 0xF) != g) continue;
       const int c0 = edge_c0(e), a = e >> 2;
       const int sx = x + ((c0 >> 2) & 1), sy = y + ((c0 >> 1) & 1), sz = z + (c0 & 1);
@@ -875,12 +916,9 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
       if (a >= 1) pre += (Xi >> l) & 1u;
       if (a >= 2) pre += (Yi >> l) & 1u;
       const int wi = (sx * dim + sy) * zc + (sz >> 5);
-      uint32_t id = (uint32_t)(pbase + (__ldg(&ws.pb[ch.unit0 + sx].y) + __ldg(ibase + wi)) / 4u + pre);
-      int j = n++;  // insertion into the sorted prefix
-      while (j > 0 && ids[j - 1] > id) { ids[j] = ids[j - 1]; --j; }
-      ids[j] = id;
+      const int64_t id = pbase + (__ldg(&ws.pb[ch.unit0 + sx].y) + __ldg(ibase + wi)) / 4u + pre;
+      if (n < room) out[n++] = (OUT)(id - rel);
     }
-    for (int i = 0; i < n && i < room; ++i) out[i] = (OUT)(ids[i] - rel);
   }
 }
 
@@ -909,51 +947,198 @@ void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const ui
 }
 
 // ---------------------------------------------------------------------------
-// K5+K6 chunk by chunk (batches): one CTA per chunk, from a queue ordered
-// largest first, runs the chunk's CSR offsets, its adjacency and every
-// dual / primal sweep with block barriers in between.  A chunk's vertices
-// only touch its own primitives, and the sum of its vertices' valences is its
-// index count, so the chunk's offsets are its index offset plus the exclusive
-// scan of its own valences -- the global scan's values.  Per primitive and
-// vertex the operations are those of k_adj_build, k_dual and k_primal, so
-// the results are identical.
+// K5+K6 chunk by chunk: a cluster of CTAs (a chunk that is large beside the
+// work of one CTA) or one CTA (the others) runs a chunk's CSR offsets, its
+// adjacency and every dual / primal sweep with barriers in between.  A chunk's
+// vertices only touch its own primitives, and the sum of its vertices'
+// valences is its index count, so the chunk's offsets are its index offset plus
+// the exclusive scan of its own valences -- the global scan's values.  Per
+// primitive and vertex the operations are those of k_adj_build, k_dual and
+// k_primal, so the results are identical.  In a cluster each CTA keeps a fixed
+// range of the chunk's vertices (its offsets and lists are then its own) and
+// of its primitives; dual and primal steps meet at cluster barriers.
+//
+// Bound by the latency of dependent gathers.  One launch instead of 4 + 2 iters
+// dependent small ones, and the update's largest chunks no longer run on one
+// CTA each at the end of a small or middle-sized update.
 // ---------------------------------------------------------------------------
+struct SweepArgs {
+  const ChunkDev* __restrict__ chunks;
+  const uint32_t* __restrict__ tot;
+  SweepLists lists;
+  const uint32_t* __restrict__ words;
+  WordScratch ws;
+  const uint32_t* __restrict__ vkey;
+  int64_t nv, n_prims, adj_cap;
+  const int64_t* __restrict__ d_counts;
+  uint32_t* __restrict__ off;
+  const uint8_t* __restrict__ valence;
+  uint32_t* __restrict__ adj;
+  const uint8_t* __restrict__ boundary;
+  const uint32_t* __restrict__ idx;  // chunk-local
+  SweepBufs b;
+  float *__restrict__ dual_p, *__restrict__ dual_n;
+  int iters, process_boundary, sn, wide_adj;
+};
+
+// One chunk (or a cluster CTA's part of it) in mesh-wide 32-bit ids: every
+// address is a kernel parameter plus a 32-bit index, so the loops below keep
+// few registers (the kernel has 32).
+struct ChunkPart {
+  uint32_t v0, p0, io;  // the chunk's first vertex, primitive and index
+  uint32_t nv, np;      // its vertices and primitives
+  uint32_t va, ve, pa, pe;  // this CTA's (from v0 / p0)
+};
+
+// Length of vertex v's list from offset o on: adj_next (MeshProcessor.cpp:247),
+// with a prebuilt adjacency init_valence; 0 for a vertex that is not moved.
+__device__ __forceinline__ uint32_t sweep_list_len(const SweepArgs& A, uint32_t v, uint32_t o) {
+  const uint32_t n = __ldg(A.valence + v), fz = __ldg(A.boundary + v);
+  const uint32_t m = (int64_t)o + n <= A.adj_cap ? n : (uint32_t)max((int64_t)0, A.adj_cap - (int64_t)o);
+  return !A.process_boundary && fz ? 0u : m;
+}
+
+// AT = uint16_t: lists of 16-bit ids relative to the chunk's first primitive,
+// in the first half of the chunk's own span of adj.
+template <typename AT>
+__device__ __forceinline__ const AT* sweep_list(const SweepArgs& A, const ChunkPart& c, uint32_t o) {
+  if (sizeof(AT) == 2) return reinterpret_cast<const AT*>(A.adj) + ((int64_t)o + c.io);
+  return reinterpret_cast<const AT*>(A.adj) + o;
+}
+
+template <int N>
+__device__ __forceinline__ void sweep_dual(const SweepArgs& A, const ChunkPart& c, const float* __restrict__ src,
+                                           int normals) {
+  for (uint32_t t = c.pa + threadIdx.x; t < c.pe; t += kSweepThreads) {
+    uint32_t v[N];
+    prim_corners<N, uint32_t>(c.p0 + t, c.nv, A.idx, v);
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] += c.v0;
+    dual_corners<N, true, uint32_t>(c.p0 + t, v, src, A.b.nrm, A.dual_p, A.dual_n, normals);
+  }
+}
+
+template <bool NORMALS, typename AT>
+__device__ __forceinline__ bool sweep_primal(const SweepArgs& A, const ChunkPart& c, const SweepStep& st) {
+  bool older = false;
+  const uint32_t rel = sizeof(AT) == 2 ? c.p0 : 0u;
+  const uint32_t lim = sizeof(AT) == 2 ? c.np : (uint32_t)min(A.n_prims, (int64_t)UINT32_MAX);
+  const uint32_t end = c.v0 + c.ve;
+  // whole warps: v - lane is the same for all lanes
+  for (uint32_t v = c.v0 + c.va + threadIdx.x; v - (threadIdx.x & 31u) < end; v += kSweepThreads) {
+    uint32_t o = 0u, n = 0u;
+    if (v < end) {
+      o = __ldca(A.off + v);
+      n = sweep_list_len(A, v, o);
+    }
+    float p[3], nn[3];
+    primal_sums<2, NORMALS, true>(sweep_list<AT>(A, c, o), n, lim, rel, A.dual_p, A.dual_n, p, nn);
+    if (n != 0u)
+      older |= primal_store<NORMALS>(v, n, p, nn, st.dst, A.b.nrm, st.set_colors, st.skipped);
+    else if (v < end)
+      primal_frozen<true>(v, st, A.b.nrm);
+  }
+  return older;
+}
+
+template <int N, typename AT>
+__device__ __forceinline__ void sweep_older(const SweepArgs& A, ChunkPart c, int skipped) {
+  const uint32_t rel = sizeof(AT) == 2 ? c.p0 : 0u;
+  const uint32_t lim = sizeof(AT) == 2 ? c.np : (uint32_t)min(A.n_prims, (int64_t)UINT32_MAX);
+  for (uint32_t v = c.v0 + c.va + threadIdx.x; v < c.v0 + c.ve; v += kSweepThreads) {
+    const uint32_t o = A.off[v], n = sweep_list_len(A, v, o);
+    const float* q = A.b.nrm + 3 * (int64_t)v;
+    if (n == 0 || q[0] != 0.0f || q[1] != 0.0f || q[2] != 0.0f) continue;
+    primal_older_normal<N, true>(v, sweep_list<AT>(A, c, o), n, lim, rel, A.idx, c.v0, c.nv, skipped, A.b.x[0],
+                                 A.b.x[1], A.iters, A.b.nrm);
+  }
+}
+
 template <int MODE, int N>
-__global__ void __launch_bounds__(chunk_sweep_threads<MODE>(), chunk_sweep_min_ctas<MODE>()) k_sweep_chunks(
-    const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, const int* __restrict__ order,
-    int n_chunks, int* __restrict__ queue, const uint32_t* __restrict__ words, WordScratch ws,
-    const uint32_t* __restrict__ vkey, int64_t nv, int64_t n_prims, int64_t adj_cap,
-    const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off, const uint8_t* __restrict__ valence,
-    uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary, const uint32_t* __restrict__ idx,
-    float* __restrict__ pos, float* __restrict__ nrm, float* __restrict__ dual_p, float* __restrict__ dual_n,
-    int iters, int process_boundary, int sn, int wide_adj) {
-  constexpr int kThreads = chunk_sweep_threads<MODE>(), kWarps = kThreads / 32;
+__global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
+    const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, SweepLists lists,
+    const uint32_t* __restrict__ words, WordScratch ws, const uint32_t* __restrict__ vkey, int64_t nv, int64_t n_prims,
+    int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
+    const uint8_t* __restrict__ valence, uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary,
+    const uint32_t* __restrict__ idx, SweepBufs b_, float* __restrict__ dual_p, float* __restrict__ dual_n, int iters,
+    int process_boundary, int sn, int wide_adj) {
+  const SweepArgs A{chunks, tot, lists, words, ws, vkey, nv, n_prims, adj_cap, d_counts, off, valence, adj, boundary,
+                    idx, b_, dual_p, dual_n, iters, process_boundary, sn, wide_adj};
+  constexpr int kThreads = kSweepThreads, kWarps = kThreads / 32;
   __shared__ SmemTabs T;
-  __shared__ uint32_t s_warp[kWarps];
+  __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_total;
-  __shared__ int s_item;
+  __shared__ uint32_t s_item;
+  __shared__ uint32_t s_seg[8];  // valence sum of each CTA's vertices
   load_tabs_some<false, false, MODE != 0, MODE == 0>(T);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t nvb = d_counts ? min(nv, d_counts[0]) : nv;
-  const int64_t npb = d_counts ? min(n_prims, d_counts[1] / N) : n_prims;
-  const int hard_norm_max = 10;
-  const int max_norms = (iters / 2 - 3 < hard_norm_max ? iters / 2 - 3 : hard_norm_max);
+  const int n_big = A.lists.head[0], n_list = A.lists.head[1];
+  bool wide = true;  // the cluster's items first, then single CTAs
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
-    __syncthreads();
-    const int it = s_item;
-    __syncthreads();  // everyone has read s_item before thread 0 takes the next
-    if (it >= n_chunks) break;
-    const int c = order[it];
-    const ChunkDev& ch = chunks[c];
-    const int64_t v0 = ch.vout, v1 = min(v0 + (int64_t)tot[2 * c], nvb);
-    const int64_t p0 = ch.iout / N, p1 = min((ch.iout + (int64_t)tot[2 * c + 1]) / N, npb);
+    int it;
+    if (wide) {
+      if (cluster_rank() == 0 && threadIdx.x == 0) {
+        const uint32_t k = (uint32_t)atomicAdd(A.lists.head + 2, 1);
+        for (uint32_t r = 0; r < cluster_size(); ++r) cluster_store(&s_item, r, k);
+      }
+      // everyone has read s_item before the next item's store: the item's own
+      // cluster barriers are in between
+      cluster_barrier();
+      it = (int)s_item;
+      if (it >= n_big) {
+        wide = false;
+        __syncthreads();  // s_item is read
+        continue;
+      }
+    } else {
+      if (threadIdx.x == 0) s_item = (uint32_t)atomicAdd(A.lists.head + 3, 1);
+      __syncthreads();
+      it = n_big + (int)s_item;
+      __syncthreads();  // everyone has read s_item before thread 0 takes the next
+      if (it >= n_list) break;
+    }
+    const int ci = A.lists.order[it];
+    const ChunkDev& ch = A.chunks[ci];
+    ChunkPart c;
+    {
+      const int64_t nvb = A.d_counts ? min(A.nv, A.d_counts[0]) : A.nv;
+      const int64_t npb = A.d_counts ? min(A.n_prims, A.d_counts[1] / N) : A.n_prims;
+      const int64_t v0 = ch.vout, p0 = ch.iout / N;
+      c.v0 = (uint32_t)v0;
+      c.p0 = (uint32_t)p0;
+      c.io = (uint32_t)ch.iout;
+      c.nv = (uint32_t)max((int64_t)0, min((int64_t)A.tot[2 * ci], nvb - v0));
+      c.np = (uint32_t)max((int64_t)0, min((ch.iout + (int64_t)A.tot[2 * ci + 1]) / N, npb) - p0);
+    }
+    // this CTA's vertices and primitives of the chunk (all of them for one CTA)
+    c.va = c.pa = 0u;
+    c.ve = c.nv;
+    c.pe = c.np;
     // CSR offsets (MeshProcessor.cpp:32-40), blockDim vertices per pass;
     // vertex v is always handled by the same thread below
-    uint32_t carry = (uint32_t)ch.iout;
-    for (int64_t b = v0; b < v1; b += kThreads) {
-      const int64_t v = b + threadIdx.x;
-      const uint32_t x = v < v1 ? (uint32_t)__ldg(valence + v) : 0u;
+    uint32_t carry = c.io;
+    if (wide) {
+      const uint32_t csize = cluster_size(), rank = cluster_rank();
+      const uint32_t vs = (c.nv + csize - 1u) / csize, ps = (c.np + csize - 1u) / csize;
+      c.va = min(rank * vs, c.nv);
+      c.ve = min(c.va + vs, c.nv);
+      c.pa = min(rank * ps, c.np);
+      c.pe = min(c.pa + ps, c.np);
+      uint32_t sum = 0u;
+      for (uint32_t v = c.va + threadIdx.x; v < c.ve; v += kThreads) sum += __ldg(A.valence + c.v0 + v);
+      sum = __reduce_add_sync(kFull, sum);
+      if (lane == 0) s_warp[warp] = sum;
+      __syncthreads();
+      if (warp == 0) {
+        sum = __reduce_add_sync(kFull, lane < kWarps ? s_warp[lane] : 0u);
+        if (lane < (int)csize) cluster_store(&s_seg[rank], lane, sum);
+      }
+      cluster_barrier();
+      for (uint32_t r = 0; r < rank; ++r) carry += s_seg[r];
+    }
+    for (uint32_t b = c.va; b < c.ve; b += kThreads) {
+      const uint32_t v = b + threadIdx.x;
+      const uint32_t x = v < c.ve ? (uint32_t)__ldg(A.valence + c.v0 + v) : 0u;
       uint32_t incl = x;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -970,70 +1155,294 @@ __global__ void __launch_bounds__(chunk_sweep_threads<MODE>(), chunk_sweep_min_c
           const uint32_t y = __shfl_up_sync(0xffffffffu, wi, d);
           if (lane >= d) wi += y;
         }
-        if (lane < kWarps) s_warp[lane] = wi - w;  // exclusive over warps
+        s_warp[lane] = wi - w;  // exclusive over warps
         if (lane == kWarps - 1) s_total = wi;
       }
       __syncthreads();
-      if (v < v1) off[v] = carry + s_warp[warp] + incl - x;
+      if (v < c.ve) A.off[c.v0 + v] = carry + s_warp[warp] + incl - x;
       carry += s_total;
       __syncthreads();
     }
-    // adjacency, in each vertex's own CSR range and inside adj
-    // a chunk of at most 65535 primitives keeps 16-bit chunk-relative ids, in
-    // the first half of its own span of adj (its lists hold as many entries
-    // as it has indices)
-    const bool compact = !wide_adj && p1 - p0 <= 65535;
-    uint16_t* adj16 = reinterpret_cast<uint16_t*>(adj + ch.iout);
-    for (int64_t v = v0 + threadIdx.x; v < v1; v += kThreads) {
-      const uint32_t o = off[v];
-      const int room = (int)max((int64_t)0, min((int64_t)__ldg(valence + v), adj_cap - (int64_t)o));
+    // adjacency, in each vertex's own CSR range and inside adj; a chunk of at
+    // most 65535 primitives keeps 16-bit ids
+    const bool compact = !A.wide_adj && c.np <= 65535u;
+    for (uint32_t v = c.v0 + c.va + threadIdx.x; v < c.v0 + c.ve; v += kThreads) {
+      const uint32_t o = A.off[v];
+      const int room = (int)max((int64_t)0, min((int64_t)__ldg(A.valence + v), A.adj_cap - (int64_t)o));
       if (compact)
-        adj_vertex<MODE, uint16_t>(T, ch, words, ws, __ldg(vkey + v), adj16 + (o - (uint32_t)ch.iout), room, p0);
+        adj_vertex<MODE, uint16_t>(T, ch, A.words, A.ws, __ldg(A.vkey + v),
+                                   const_cast<uint16_t*>(sweep_list<uint16_t>(A, c, o)), room, (int64_t)c.p0);
       else
-        adj_vertex<MODE>(T, ch, words, ws, __ldg(vkey + v), adj + o, room);
+        adj_vertex<MODE>(T, ch, A.words, A.ws, __ldg(A.vkey + v), A.adj + o, room);
     }
-    __syncthreads();
-    // the sweeps in 32-bit chunk-relative indices over chunk-based pointers
-    // (vertex ids, primitive ids and adjacency offsets stay mesh-wide)
-    const uint32_t np_c = (uint32_t)max((int64_t)0, p1 - p0), nv_c = (uint32_t)max((int64_t)0, v1 - v0);
-    const uint32_t nvb32 = (uint32_t)min(nvb, (int64_t)UINT32_MAX);
-    const uint32_t npl32 = (uint32_t)min(n_prims, (int64_t)UINT32_MAX);
-    const uint32_t* idx_c = idx + N * p0;
-    float* dp_c = dual_p + 4 * p0;
-    float* dn_c = dual_n + 2 * p0;
-    const uint32_t* off_c = off + v0;
-    const uint8_t* val_c = valence + v0;
-    const uint8_t* bnd_c = boundary + v0;
-    float* pos_c = pos + 3 * v0;
-    float* nrm_c = nrm ? nrm + 3 * v0 : nullptr;
-    for (int m = 0; m < iters; ++m) {
-      const int normal_mode = !sn ? 0 : ((m == 0 || m < max_norms || m < 3) ? 1 : 2);
-      const int set_colors = (m < iters - 1) ? ((m == 3) || (m == 0 && iters <= 3)) : 0;
-      for (uint32_t t = threadIdx.x; t < np_c; t += kThreads)
-        dual_prim<N, true, true>(t, nvb32, idx_c, pos, nrm, dp_c, dn_c, normal_mode);
-      __syncthreads();
-      if (compact) {
-        for (uint32_t v = threadIdx.x; v < nv_c; v += kThreads)
-          primal_vertex<true, true, uint32_t, uint16_t>(v, np_c, adj_cap, off_c, nullptr, val_c, adj, bnd_c, dp_c, dn_c,
-                                                        pos_c, nrm_c, process_boundary, sn, set_colors, ch.iout);
+    for (int m = 0; m < A.iters; ++m) {
+      const SweepStep st = sweep_step(m, A.iters, A.sn, A.b.keep(), A.b);
+      sweep_dual<N>(A, c, st.src, st.normals);
+      if (wide) cluster_barrier(); else __syncthreads();
+      bool older = false;
+      if (st.normals == 0) {
+        if (compact) sweep_primal<false, uint16_t>(A, c, st); else sweep_primal<false, uint32_t>(A, c, st);
       } else {
-        for (uint32_t v = threadIdx.x; v < nv_c; v += kThreads)
-          primal_vertex<true, true>(v, npl32, adj_cap, off_c, nullptr, val_c, adj, bnd_c, dual_p, dual_n, pos_c, nrm_c,
-                                    process_boundary, sn, set_colors);
+        older = compact ? sweep_primal<true, uint16_t>(A, c, st) : sweep_primal<true, uint32_t>(A, c, st);
       }
-      __syncthreads();
+      if (st.skipped && __syncthreads_or(older)) {
+        if (compact) sweep_older<N, uint16_t>(A, c, st.skipped); else sweep_older<N, uint32_t>(A, c, st.skipped);
+      }
+      if (wide) cluster_barrier(); else __syncthreads();
     }
   }
 }
 
+// ---------------------------------------------------------------------------
+// K5+K6 over the whole mesh in one cooperative launch, for meshes whose steps
+// are too short to be launched one by one (a chunk, a small update): CSR
+// offsets, adjacency and every dual / primal step, with a barrier over the
+// team's CTAs in between.  The team is as many of the launch's CTAs as the
+// mesh can use (kTeamVerts vertices each): fewer CTAs meet faster.  Every CTA
+// keeps a fixed range of the vertices and of the primitives; each thread keeps
+// its first vertex's list and its first two primitives' corners in registers,
+// so a step is one round of independent gathers from L2 (what the other SMs
+// wrote), the sums in list order, and the barrier.  Values and order of the
+// sums are those of k_adj_build, k_dual and k_primal.
+// ---------------------------------------------------------------------------
+constexpr int kTeamThreads = 512;
+constexpr int kTeamVerts = 256;  // vertices per CTA that make the team one CTA larger
+constexpr int kTeamRegs = 6;     // list entries gathered at once (and kept for a thread's first vertex)
+
+struct TeamArgs {
+  const ChunkDev* chunks;
+  int n_chunks;
+  const uint32_t* words;
+  WordScratch ws;
+  const uint32_t* vkey;
+  int64_t nv, n_prims;
+  const int64_t* d_counts;
+  uint32_t* off;
+  const uint8_t* valence;
+  uint32_t* adj;
+  const uint8_t* boundary;
+  const uint32_t* idx;
+  SweepBufs b;
+  float *dual_p, *dual_n;
+  int iters, process_boundary, sn;
+  TeamSync* sync;
+  unsigned* host_failed;  // pinned host memory
+};
+
+// Barrier over the team's CTAs (all resident: a cooperative launch).  The wait
+// is bounded: after kTeamSpins polls (a second or so) or once another CTA has
+// given up, the CTA marks the team failed and no longer waits anywhere; the
+// host finds the mark after its synchronisation.
+constexpr unsigned kTeamSpins = 1u << 22;
+__device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed, unsigned& target, unsigned team,
+                                             bool& dead) {
+  __syncthreads();
+  target += team;
+  if (threadIdx.x == 0 && team > 1 && !dead) {
+    __threadfence();  // the CTA's stores (ordered before by the block barrier) before the arrival
+    atomicAdd(&y->arrived, 1u);
+    unsigned v = 0;
+    for (unsigned spins = 0;; ++spins) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&y->arrived) : "memory");
+      if (v >= target) break;
+      if (spins >= kTeamSpins || ((spins & 1023u) == 1023u && *(volatile unsigned*)&y->failed)) {
+        *(volatile unsigned*)&y->failed = 1u;
+        *(volatile unsigned*)host_failed = 1u;
+        dead = true;  // this CTA waits nowhere any more
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+}
+
 template <int MODE, int N>
-static int sweep_chunks_grid() {
+__global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_constant__ TeamArgs A) {
+  constexpr int kWarps = kTeamThreads / 32;
+  __shared__ SmemTabs T;
+  __shared__ uint32_t s_warp[kWarps], s_total;
+  const uint32_t nv = (uint32_t)(A.d_counts ? min(A.nv, A.d_counts[0]) : A.nv);
+  const uint32_t np = (uint32_t)(A.d_counts ? min(A.n_prims, A.d_counts[1] / N) : A.n_prims);
+  const unsigned team = min(gridDim.x, max(1u, (nv + kTeamVerts - 1u) / kTeamVerts));
+  const unsigned rank = blockIdx.x;
+  if (rank >= team || nv == 0) return;
+  if (*(volatile unsigned*)&A.sync->failed) {  // a launch before gave up and the host has not seen it yet
+    if (threadIdx.x == 0) *(volatile unsigned*)A.host_failed = 1u;
+    return;
+  }
+  load_tabs_some<false, false, MODE != 0, MODE == 0>(T);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
+  const int iters = A.iters;
+  unsigned target = 0;
+  bool dead = false;
+  const uint32_t vs = (nv + team - 1u) / team, ps = (np + team - 1u) / team;
+  const uint32_t va = min(rank * vs, nv), ve = min(va + vs, nv), pa = min(rank * ps, np), pe = min(pa + ps, np);
+  const uint32_t cap = np * N;  // slots of adj
+  // CSR offsets (MeshProcessor.cpp:32-40): the CTAs' valence sums, then a scan of the own range
+  uint32_t sum = 0u;
+  for (uint32_t v = va + tid; v < ve; v += kTeamThreads) sum += __ldg(A.valence + v);
+  sum = __reduce_add_sync(kFull, sum);
+  if (lane == 0) s_warp[warp] = sum;
+  __syncthreads();
+  if (warp == 0) {
+    sum = __reduce_add_sync(kFull, lane < kWarps ? s_warp[lane] : 0u);
+    if (lane == 0) A.sync->seg[rank] = sum;
+  }
+  team_barrier(A.sync, A.host_failed, target, team, dead);
+  if (warp == 0) {
+    uint32_t c = 0u;
+    for (unsigned r = lane; r < rank; r += 32) c += __ldcg(A.sync->seg + r);
+    c = __reduce_add_sync(kFull, c);
+    if (lane == 0) s_total = c;
+  }
+  __syncthreads();
+  uint32_t carry = s_total;
+  __syncthreads();
+  for (uint32_t b = va; b < ve; b += kTeamThreads) {
+    const uint32_t v = b + tid, x = v < ve ? (uint32_t)__ldg(A.valence + v) : 0u;
+    const uint32_t incl = warp_incl_sum(x, lane);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t w = lane < kWarps ? s_warp[lane] : 0u, wi = warp_incl_sum(w, lane);
+      if (lane < kWarps) s_warp[lane] = wi - w;
+      if (lane == kWarps - 1) s_total = wi;
+    }
+    __syncthreads();
+    if (v < ve) {
+      const uint32_t o = carry + s_warp[warp] + incl - x;
+      A.off[v] = o;
+      const int room = o < cap ? (int)min(x, cap - o) : 0;
+      adj_vertex<MODE>(T, A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.words, A.ws, __ldg(A.vkey + v),
+                       A.adj + o, room);
+    }
+    carry += s_total;
+    __syncthreads();
+  }
+  // what a thread keeps over all steps: its first vertex's list and its first two primitives' corners
+  const auto list_of = [&](uint32_t v, uint32_t& n, uint32_t& o) {
+    o = A.off[v];
+    n = o < cap ? min((uint32_t)__ldg(A.valence + v), cap - o) : 0u;
+    if (!A.process_boundary && __ldg(A.boundary + v)) n = 0u;
+  };
+  const auto load_ids = [&](uint32_t o, uint32_t n, uint32_t ids[kTeamRegs]) {
+#pragma unroll
+    for (int k = 0; k < kTeamRegs; ++k) ids[k] = k < (int)n ? A.adj[o + k] : 0xffffffffu;
+  };
+  uint32_t n0 = 0u, o0 = 0u, ids0[kTeamRegs] = {}, c0[2][N];
+  const uint32_t v_own = va + tid, p_own = pa + tid;
+  if (v_own < ve) {
+    list_of(v_own, n0, o0);
+    load_ids(o0, n0, ids0);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (p_own + k * kTeamThreads < pe) prim_corners<N, uint32_t>(p_own + k * kTeamThreads, nv, A.idx, c0[k]);
+  const bool keep = A.b.keep();
+  for (int m = 0; m < iters; ++m) {
+    const SweepStep st = sweep_step(m, iters, A.sn, keep, A.b);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (p_own + k * kTeamThreads < pe)
+        dual_corners<N, true, uint32_t>(p_own + k * kTeamThreads, c0[k], st.src, A.b.nrm, A.dual_p, A.dual_n,
+                                        st.normals);
+    for (uint32_t t = p_own + 2 * kTeamThreads; t < pe; t += kTeamThreads)
+      dual_prim<N, true, uint32_t>(t, nv, A.idx, st.src, A.b.nrm, A.dual_p, A.dual_n, st.normals);
+    team_barrier(A.sync, A.host_failed, target, team, dead);
+    bool older = false;
+    for (uint32_t v = v_own; v - lane < ve; v += kTeamThreads) {
+      uint32_t n = n0, o = o0;
+      if (v != v_own) {
+        n = o = 0u;
+        if (v < ve) list_of(v, n, o);
+      }
+      const uint32_t* first = v == v_own ? ids0 : nullptr;
+      float p[3], nn[3];
+      if (st.normals == 0)
+        primal_sums<kTeamRegs, false, true>(A.adj + o, n, np, 0u, A.dual_p, A.dual_n, p, nn, first);
+      else
+        primal_sums<kTeamRegs, true, true>(A.adj + o, n, np, 0u, A.dual_p, A.dual_n, p, nn, first);
+      if (n == 0u) {
+        if (v < ve) primal_frozen<true>(v, st, A.b.nrm);
+      } else if (st.normals == 0) {
+        primal_store<false>(v, n, p, nn, st.dst, A.b.nrm, st.set_colors, 0);
+      } else {
+        older |= primal_store<true>(v, n, p, nn, st.dst, A.b.nrm, st.set_colors, st.skipped);
+      }
+    }
+    if (st.skipped && __syncthreads_or(older)) {
+      for (uint32_t v = v_own; v < ve; v += kTeamThreads) {
+        uint32_t n, o;
+        list_of(v, n, o);
+        const float* nv3 = A.b.nrm + 3 * (int64_t)v;
+        if (n == 0u || nv3[0] != 0.0f || nv3[1] != 0.0f || nv3[2] != 0.0f) continue;
+        primal_older_normal<N, true>(v, A.adj + o, n, np, 0u, A.idx, 0u, nv, st.skipped, A.b.x[0], A.b.x[1], iters, A.b.nrm);
+      }
+    }
+    if (m + 1 < iters) team_barrier(A.sync, A.host_failed, target, team, dead);
+  }
+  // the last CTA leaves the barrier ready for the next launch
+  __syncthreads();
+  if (tid == 0 && atomicAdd(&A.sync->left, 1u) == team - 1u) {
+    A.sync->arrived = 0u;
+    A.sync->left = 0u;
+  }
+}
+
+template <int MODE, int N>
+static int team_grid() {
   static std::atomic<int> grid[64] = {};
   return per_device_once(grid, [](int dev) {
-    int sms = 0, per_sm = 0;
+    int sms = 0, coop = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_chunks<MODE, N>, chunk_sweep_threads<MODE>(), 0);
-    return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_team<MODE, N>, kTeamThreads, 0);
+    return coop && per_sm > 0 ? min(sms, kTeamMax) : -1;
+  });
+}
+
+void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,
+                       float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
+                       int iters, int process_boundary, int smooth_normals, const ProcessScratch& s,
+                       cudaStream_t st) {
+  TeamArgs A{sa.chunks, sa.n_chunks, sa.words, sa.ws, sa.vkey, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
+             idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
+             smooth_normals, sa.team, sa.team_failed};
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.gridDim = dim3(sa.mode == 0 ? team_grid<0, 3>() : team_grid<1, 4>());
+  cfg.blockDim = dim3(kTeamThreads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (sa.mode == 0) cudaLaunchKernelEx(&cfg, k_sweep_team<0, 3>, A);
+  else cudaLaunchKernelEx(&cfg, k_sweep_team<1, 4>, A);
+}
+
+// Clusters of `size` (1, 2, 4 or 8) CTAs that can be resident at once (negative: none).
+template <int MODE, int N>
+static int sweep_max_clusters(int size) {
+  static std::atomic<int> slots[4][64] = {};
+  int lg = 0;
+  while ((1 << lg) < size) ++lg;
+  return per_device_once(slots[lg], [size](int dev) {
+    (void)dev;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = size;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_sweep_chunks<MODE, N>, &cfg) != cudaSuccess) n = 0;
+    cudaGetLastError();
+    return n > 0 ? n : -1;
   });
 }
 
@@ -1041,19 +1450,60 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st) {
-  cudaMemsetAsync(sa.queue, 0, sizeof(int), st);
-  const int64_t adj_cap = n_prims * N;
-#define BMF_SWEEP_CHUNKS(M, NN)                                                                                 \
-  k_sweep_chunks<M, NN><<<sweep_chunks_grid<M, NN>(), chunk_sweep_threads<M>(), 0, st>>>(                     \
-      sa.chunks, sa.tot, sa.order, sa.n_chunks, sa.queue, sa.words, sa.ws, sa.vkey, nv, n_prims, adj_cap,        \
-      d_counts, s.off, valence, s.adj, boundary, idx, pos, nrm, s.dual_p, s.dual_n, iters, process_boundary,      \
-      smooth_normals, sa.wide_adj ? 1 : 0)
-  if (sa.mode == 0) {
-    if (N == 3) BMF_SWEEP_CHUNKS(0, 3); else BMF_SWEEP_CHUNKS(0, 4);
-  } else {
-    if (N == 3) BMF_SWEEP_CHUNKS(1, 3); else BMF_SWEEP_CHUNKS(1, 4);
+  SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.words, sa.ws, sa.vkey, nv, n_prims, n_prims * N, d_counts, s.off,
+              valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters,
+              process_boundary, smooth_normals, sa.wide_adj ? 1 : 0};
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = sa.lists.cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(sa.lists.ctas);
+  cfg.blockDim = dim3(kSweepThreads);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const auto go = [&](auto kernel) {
+    cudaLaunchKernelEx(&cfg, kernel, A.chunks, A.tot, A.lists, A.words, A.ws, A.vkey, A.nv, A.n_prims, A.adj_cap,
+                       A.d_counts, A.off, A.valence, A.adj, A.boundary, A.idx, A.b, A.dual_p, A.dual_n, A.iters,
+                       A.process_boundary, A.sn, A.wide_adj);
+  };
+  if (sa.mode == 0) go(k_sweep_chunks<0, 3>);
+  else go(k_sweep_chunks<1, 4>);
+}
+
+// Where the lines lie (whole passes, us; launches / team / chunks with the
+// cluster size chosen here):
+//   one 33^3 chunk, Mode R            152 /  121 /    -
+//   one 257^3 chunk, Mode R           267 /  244 /    -       (66 k columns)
+//   fit, 8 x 65^3 (adjoint in all)    370 /  332 /  375
+//   fit, 32 x 65^3                    608 /  590 /  567       (135 k columns)
+//   mixed update, 48 chunks           299 /  328 /  460       (214 k columns)
+//   128 chunks Mode R / Q       522 / 771   631 / 833   688 / 1034
+//   256                       1019 / 1551  1389 / 1813 1004 / 1663
+//   384                       1414 / 2248  1967 / 2658 1333 / 2247
+//   512                       1779 / 2938  2465 / 3441 1643 / 2879
+//   1024                      3423 / 5629  4819 / 6657 2954 / 5459
+// A team pays off while a step is shorter than a launch; its 16 warps per SM
+// carry fewer gathers than full occupancy once steps are long.  A chunk per CTA
+// or cluster needs several chunks per resident CTA to balance.  Clusters of 4
+// against 2 and 1: 512 chunks 1643 / 1802 / 2434 us, 1024 chunks 2996 / 2954 /
+// 3456, 2048 chunks 5805 / 5764 / 5781.
+constexpr int64_t kTeamColumns = 140000;
+constexpr int kChunkSweepMin = 320, kChunkSweepPairs = 1024;
+
+SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s) {
+  if (columns <= kTeamColumns && (mode == 0 ? team_grid<0, 3>() : team_grid<1, 4>()) > 0) return kSweepTeam;
+  if (n_chunks >= kChunkSweepMin) {
+    for (int size = n_chunks >= kChunkSweepPairs ? 2 : 4; size >= 1; size >>= 1) {
+      const int clusters = mode == 0 ? sweep_max_clusters<0, 3>(size) : sweep_max_clusters<1, 4>(size);
+      if (clusters <= 0) continue;
+      s->cluster = size;
+      s->ctas = size * min(clusters, n_chunks);
+      return kSweepChunks;
+    }
   }
-#undef BMF_SWEEP_CHUNKS
+  return kSweepLaunches;
 }
 
 void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
@@ -1073,9 +1523,9 @@ void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d
 
 void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
                        int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
-                       cudaStream_t st) {
+                       cudaStream_t st, const SweepLists* sweep) {
   k_chunk_scan<<<(n_chunks + kScanWarps - 1) / kScanWarps, kScanThreads, 0, st>>>(
-      d_chunks, n_chunks, ws.pb, d_tot, flags, vcap, icap, d_info, d_totals, d_ticket);
+      d_chunks, n_chunks, ws.pb, d_tot, flags, vcap, icap, d_info, d_totals, d_ticket, sweep ? *sweep : SweepLists{});
 }
 
 // k-th set bit (from 0) of m; m must have more than k set bits.

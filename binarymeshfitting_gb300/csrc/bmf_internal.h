@@ -146,32 +146,103 @@ void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d
 // indices) to d_tot[2c], and scans those into chunk.vout / chunk.iout, the
 // per-chunk info table {voff, vcount, ioff, icount, contains_mesh, status} and
 // d_totals {vertices, indices, contains_mesh of chunk 0}.  d_ticket: one int,
-// zero before the first call and left zero by each.
+// zero before the first call and left zero by each (null for at most 32 chunks).
+// sweep (nullable): the work lists of the chunk-by-chunk sweeps.
 constexpr int kTotals = 3;
+// Work lists of the chunk-by-chunk sweeps: the chunks that have vertices, by
+// size (powers of sqrt 2), largest first.  The first n_big are taken by whole
+// clusters, the others by single CTAs.
+struct SweepLists {
+  int* order = nullptr;  // [n_chunks]
+  int* head = nullptr;   // {n_big, listed chunks, cluster queue, CTA queue}; the queues are zeroed with the lists
+  int cluster = 1;       // CTAs per cluster and CTAs in all of the launch that will take the lists
+  int ctas = 1;
+};
+constexpr int kSweepHead = 4;
+// The barrier of the whole-mesh sweep kernel's team of CTAs (zeroed once; each
+// launch leaves arrived and left zero) and the CTAs' valence sums.
+constexpr int kTeamMax = 256;
+struct TeamSync {
+  unsigned arrived, left, failed, pad;
+  uint32_t seg[kTeamMax];
+};
 void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
                        int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
-                       cudaStream_t st);
+                       cudaStream_t st, const SweepLists* sweep = nullptr);
+// How the sweeps of n_chunks chunks with `columns` (sum of dim^2) columns in all
+// run: one launch per step, one cooperative launch over the whole mesh, or
+// chunk by chunk (then cluster and ctas of *s are filled).
+enum SweepForm { kSweepLaunches, kSweepTeam, kSweepChunks };
+SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s);
 // Returns the kernels launched: Mode Q QEF placement with vertex keys and
 // d_counts (total vertices on the device) adds the per-vertex k_place_qef.
 int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start,
                 int n_units, const uint32_t* words, const float* dens, const uint32_t* flags, WordScratch ws,
                 MeshOut out, const int64_t* d_counts, cudaStream_t st);
 
+// One sweep (a dual and a primal step) of MeshProcessor.cpp:130-306.
+// normals: 0 none, 1 face normals, 2 sums of vertex normals.  The face normals
+// of a sweep only set the vertex normals, which the next face sweep sets
+// anew, so with at most three face sweeps they are computed in the last of
+// them alone.  A vertex keeps its older normal when its new one has n.y == 0
+// (MeshProcessor.cpp:287): the positions before the left-out sweeps are kept,
+// x[0] before the first, x[1] before the second, x[2] (src) before the last,
+// and primal_older_normal takes the normal of such a vertex from them.  Left out: the square roots and divisions of two of three
+// sweeps, a float2 gather per list entry and a normal written per vertex.
+struct SweepBufs {
+  float* x[3] = {nullptr, nullptr, nullptr};  // positions before the left-out sweeps and the last face sweep (null: none left out, in place)
+  float* pos = nullptr;                       // positions out
+  float* nrm = nullptr;                       // normals out (null: none)
+  __host__ __device__ bool keep() const { return x[0] != nullptr; }
+};
+struct SweepStep {
+  int normals, set_colors;
+  const float* src;  // positions read, and written (dst may be src)
+  float* dst;
+  int skipped;  // face sweeps left out before this one (the last face sweep), which sets every vertex's first normal
+};
+// Face sweeps of iters sweeps (MeshProcessor.cpp:149-163) and those left out.
+__host__ __device__ inline int sweep_face_count(int iters) {
+  const int mx = iters / 2 - 3 < 10 ? iters / 2 - 3 : 10, f = mx > 3 ? mx : 3;
+  return f < iters ? f : iters;
+}
+__host__ __device__ inline int sweep_skipped(int iters, int sn) {
+  const int f = sweep_face_count(iters) - 1;
+  return !sn || f < 0 || f > 2 ? 0 : f;
+}
+__host__ __device__ inline int sweep_colors(int m, int iters) {
+  return (m < iters - 1) ? ((m == 3) || (m == 0 && iters <= 3)) : 0;
+}
+// keep: b.x are there
+__host__ __device__ inline SweepStep sweep_step(int m, int iters, int sn, bool keep, const SweepBufs& b) {
+  const int last = sweep_face_count(iters) - 1, k = keep ? sweep_skipped(iters, sn) : 0;
+  SweepStep s;
+  s.normals = !sn ? 0 : (m > last ? 2 : (m < k ? 0 : 1));
+  s.set_colors = m < k ? 0 : sweep_colors(m, iters);
+  s.src = k == 0 || m > k ? b.pos : (m == 0 ? b.x[0] : (m == 1 ? b.x[1] : b.x[2]));
+  s.dst = k == 0 || m >= k ? b.pos : (m == 0 ? b.x[1] : b.x[2]);
+  s.skipped = m == k ? k : 0;
+  return s;
+}
+
 // MeshProcessor: operates on one flat mesh (vertices [0, nv), prims of N).
 struct ProcessScratch {
   uint32_t* off;      // nv + 1 CSR offsets
   uint32_t* cursor;   // nv fill cursors
   uint32_t* adj;      // sum of valences
-  float* dual_p;      // 3 * n_prims
-  float* dual_n;      // 3 * n_prims
+  float* dual_p;      // 4 * n_prims: dual point, normal x
+  float* dual_n;      // 2 * n_prims: normal y, z (unused without normals)
+  // positions before the left-out face sweeps (3 * nv each; null: none are left
+  // out): x[0] is where the emit put the mesh
+  float* x[3] = {nullptr, nullptr, nullptr};
   uint32_t* tmp;      // scan scratch (block totals)
   int block;          // threads per CTA of the dual / primal sweeps (0 = 256)
 };
 // nv / n_prims size the grids; when d_counts is given the actual vertex and
 // index counts are read from d_counts[0] / d_counts[1] on the device (so the
 // sequence can be captured in a CUDA graph before the counts are known).
-// Scratch sizes: off nv+1, cursor nv, adj N*n_prims, dual_p/dual_n 3*n_prims,
-// tmp ceil(nv / 4096) + 1.
+// Scratch sizes: off nv+1, cursor nv, adj N*n_prims, dual_p 4*n_prims, dual_n
+// 2*n_prims, tmp ceil(nv / 4096) + 1.
 // Where the vertex->primitive lists come from: a mesh this library extracted
 // (grid structure known: built analytically per vertex) or any mesh (atomic
 // scatter + per-vertex sort).
@@ -182,11 +253,12 @@ struct StructuredAdj {
   const uint32_t* words;
   WordScratch ws;            // scanned counts + per-word bit-planes
   const uint32_t* vkey;      // per-vertex keys written by the emit kernel
-  // optional (all three or none): the sweeps run chunk by chunk, one CTA per
-  // chunk, taking chunks from queue in the given order
+  // optional (tot and lists.order, or neither): the sweeps run chunk by chunk
   const uint32_t* tot = nullptr;  // per chunk {vertices, indices}
-  const int* order = nullptr;     // chunk indices, largest first
-  int* queue = nullptr;           // one int, reset by launch_process
+  SweepLists lists;               // filled by launch_chunk_scan
+  TeamSync* team = nullptr;       // or (whole mesh, one cooperative launch): the team's barrier, and
+  unsigned* team_failed = nullptr;  // where it tells the host of a wait that ran out (pinned)
+  int* bwd_queue = nullptr;       // the adjoint sweeps' queue over lists.order (one int, reset by launch_process_bwd)
   // the chunk-by-chunk sweeps keep 16-bit chunk-relative adjacency lists for
   // chunks of at most 65535 primitives unless a later pass reads the
   // adjacency (the fit's adjoint sweeps want 32-bit mesh-wide ids)
@@ -195,12 +267,16 @@ struct StructuredAdj {
 void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, WordScratch ws,
                       const uint32_t* vkey, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
                       uint32_t* adj, cudaStream_t st);
-// The chunk-by-chunk form of launch_process for StructuredAdj with tot /
-// order / queue set: CSR offsets, adjacency and all sweeps in one launch.
+// The chunk-by-chunk form of launch_process for StructuredAdj with tot and
+// lists set: CSR offsets, adjacency and all sweeps in one launch.
 void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st);
+// The whole-mesh form of launch_process in one cooperative launch (sa.team set).
+void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,
+                       float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
+                       int iters, int process_boundary, int smooth_normals, const ProcessScratch& s, cudaStream_t st);
 // Returns the number of kernels launched.
 int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, float* pos, float* nrm,
                    const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx, int iters,

@@ -136,23 +136,46 @@ __global__ void k_sort_adj(int64_t nv, int64_t adj_cap, const int64_t* __restric
 template <int N>
 __global__ void k_dual(int64_t n_prims, int64_t nv, const int64_t* __restrict__ d_counts,
                        const uint32_t* __restrict__ idx, const float* __restrict__ pos, const float* __restrict__ nrm,
-                       float* __restrict__ dual_p, float* __restrict__ dual_n, int normal_mode) {
+                       float* __restrict__ dual_p, float* __restrict__ dual_n, int normals) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (d_counts ? min(n_prims, d_counts[1] / N) : n_prims)) return;
-  dual_prim<N>(t, d_counts ? min(nv, d_counts[0]) : nv, idx, pos, nrm, dual_p, dual_n, normal_mode);
+  dual_prim<N>(t, d_counts ? min(nv, d_counts[0]) : nv, idx, pos, nrm, dual_p, dual_n, normals);
 }
 
-// optimize_primal_grid (MeshProcessor.cpp:238-306).
-__global__ void k_primal(int64_t nv, int64_t np_lim, int64_t adj_cap, const int64_t* __restrict__ d_counts,
+// optimize_primal_grid (MeshProcessor.cpp:238-306).  cursor (nullable): list
+// lengths where the lists were filled from the indices.
+template <int N>
+__global__ void k_primal(int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts,
                          const uint32_t* __restrict__ off, const uint32_t* __restrict__ cursor,
                          const uint8_t* __restrict__ valence, const uint32_t* __restrict__ adj,
                          const uint8_t* __restrict__ boundary, const float* __restrict__ dual_p,
-                         const float* __restrict__ dual_n, float* __restrict__ pos, float* __restrict__ nrm,
-                         int process_boundary, int smooth_normals, int set_colors) {
+                         const float* __restrict__ dual_n, const uint32_t* __restrict__ idx, SweepStep st, SweepBufs b,
+                         int iters, int process_boundary) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= (d_counts ? min(nv, d_counts[0]) : nv)) return;
-  primal_vertex(v, np_lim, adj_cap, off, cursor, valence, adj, boundary, dual_p, dual_n, pos, nrm, process_boundary,
-                smooth_normals, set_colors);
+  const int64_t nvb = d_counts ? min(nv, d_counts[0]) : nv;
+  uint32_t o = 0u, n = 0u;
+  if (v < nvb) {
+    // list length: adj_next (MeshProcessor.cpp:247); with a prebuilt adjacency it equals init_valence
+    const uint32_t val = valence[v];
+    const bool frozen = !process_boundary && boundary[v];
+    o = __ldg(off + v);
+    n = (uint32_t)max((int64_t)0, min((int64_t)(cursor ? min(cursor[v], val) : val), adj_cap - (int64_t)o));
+    if (frozen) n = 0u;
+  }
+  const uint32_t np_lim = (uint32_t)min(n_prims, (int64_t)UINT32_MAX);
+  float p[3], nn[3];
+  if (st.normals == 0)
+    primal_sums<4, false, false>(adj + o, n, np_lim, 0u, dual_p, dual_n, p, nn);
+  else
+    primal_sums<4, true, false>(adj + o, n, np_lim, 0u, dual_p, dual_n, p, nn);
+  if (n == 0u) {
+    if (v < nvb) primal_frozen<false>((uint32_t)v, st, b.nrm);
+  } else if (st.normals == 0) {
+    primal_store<false>((uint32_t)v, n, p, nn, st.dst, b.nrm, st.set_colors, 0);
+  } else if (primal_store<true>((uint32_t)v, n, p, nn, st.dst, b.nrm, st.set_colors, st.skipped)) {
+    primal_older_normal<N, false>(v, adj + o, n, np_lim, 0u, idx, 0u, (uint32_t)min(nvb, (int64_t)UINT32_MAX),
+                                  st.skipped, b.x[0], b.x[1], iters, b.nrm);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -338,7 +361,7 @@ constexpr int kBwdChunkThreads = 512;
 template <int N>
 __global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(
     const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, const int* __restrict__ order,
-    int n_chunks, int* __restrict__ queue, int64_t nv, int64_t n_prims, int64_t adj_cap,
+    const int* __restrict__ head, int* __restrict__ queue, int64_t nv, int64_t n_prims, int64_t adj_cap,
     const int64_t* __restrict__ d_counts, const uint32_t* __restrict__ off, const uint8_t* __restrict__ valence,
     const uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary, int process_boundary,
     const uint32_t* __restrict__ idx, float* __restrict__ g, float* __restrict__ g_dual, int iters) {
@@ -346,12 +369,13 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(
   const int64_t nvb = d_counts ? min(nv, d_counts[0]) : nv;
   const int64_t npb = d_counts ? min(n_prims, d_counts[1] / N) : n_prims;
   const float invN = 1.0f / (float)N;
+  const int n_list = head[1];
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
     __syncthreads();
     const int it = s_item;
     __syncthreads();  // everyone has read s_item before thread 0 takes the next
-    if (it >= n_chunks) break;
+    if (it >= n_list) break;
     const int c = order[it];
     const int64_t v0 = chunks[c].vout, v1 = min(v0 + (int64_t)tot[2 * c], nvb);
     const int64_t p0 = chunks[c].iout / N, p1 = min((chunks[c].iout + (int64_t)tot[2 * c + 1]) / N, npb);
@@ -396,7 +420,7 @@ int launch_process_bwd(int N, int64_t nv, int64_t n_prims, const int64_t* d_coun
                        const uint8_t* valence, const uint32_t* idx, int iters, int process_boundary,
                        const ProcessScratch& s, float* g, const StructuredAdj* sa, cudaStream_t st) {
   if (nv == 0 || n_prims == 0 || iters <= 0) return 0;
-  if (sa && sa->tot && sa->order && sa->queue) {
+  if (sa && sa->tot && sa->lists.order && sa->bwd_queue) {
     // one slot array per primitive size: the two kernels' occupancies may differ
     static std::atomic<int> grid3[64] = {}, grid4[64] = {};
     const int grid = per_device_once(N == 3 ? grid3 : grid4, [N](int dev) {
@@ -408,14 +432,14 @@ int launch_process_bwd(int N, int64_t nv, int64_t n_prims, const int64_t* d_coun
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_bwd_chunks<4>, kBwdChunkThreads, 0);
       return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
     });
-    cudaMemsetAsync(sa->queue, 0, sizeof(int), st);
+    cudaMemsetAsync(sa->bwd_queue, 0, sizeof(int), st);
     if (N == 3)
       k_sweep_bwd_chunks<3><<<grid, kBwdChunkThreads, 0, st>>>(
-          sa->chunks, sa->tot, sa->order, sa->n_chunks, sa->queue, nv, n_prims, n_prims * N, d_counts, s.off,
+          sa->chunks, sa->tot, sa->lists.order, sa->lists.head, sa->bwd_queue, nv, n_prims, n_prims * N, d_counts, s.off,
           valence, s.adj, boundary, process_boundary, idx, g, s.dual_p, iters);
     else
       k_sweep_bwd_chunks<4><<<grid, kBwdChunkThreads, 0, st>>>(
-          sa->chunks, sa->tot, sa->order, sa->n_chunks, sa->queue, nv, n_prims, n_prims * N, d_counts, s.off,
+          sa->chunks, sa->tot, sa->lists.order, sa->lists.head, sa->bwd_queue, nv, n_prims, n_prims * N, d_counts, s.off,
           valence, s.adj, boundary, process_boundary, idx, g, s.dual_p, iters);
     return 1;
   }
@@ -435,12 +459,17 @@ int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, 
                    const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx, int iters,
                    int process_boundary, int smooth_normals, ProcessScratch s, const StructuredAdj* sa,
                    cudaStream_t st) {
-  if (nv == 0 || n_prims == 0 || iters <= 0) return 0;
+  if (nv == 0 || iters <= 0 || (n_prims == 0 && !s.x[0])) return 0;
   const int64_t n_slots = n_prims * N;
   const bool sn = smooth_normals != 0 && nrm != nullptr;
-  if (sa && sa->tot && sa->order && sa->queue) {
+  if (sa && sa->tot && sa->lists.order) {
     launch_sweep_chunks(*sa, N, nv, n_prims, d_counts, pos, nrm, boundary, valence, idx, iters, process_boundary,
                         sn ? 1 : 0, s, st);
+    return 1;
+  }
+  if (sa && sa->team) {
+    launch_sweep_team(*sa, N, nv, n_prims, d_counts, pos, nrm, boundary, valence, idx, iters, process_boundary,
+                      sn ? 1 : 0, s, st);
     return 1;
   }
   int launched = 3;
@@ -461,19 +490,23 @@ int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, 
     cursor = s.cursor;
     launched += 2;
   }
-  const int hard_norm_max = 10;
-  const int max_norms = (iters / 2 - 3 < hard_norm_max ? iters / 2 - 3 : hard_norm_max);
+  const SweepBufs b{{s.x[0], s.x[1], s.x[2]}, pos, nrm};
   for (int m = 0; m < iters; ++m) {
-    const int normal_mode = !sn ? 0 : ((m == 0 || m < max_norms || m < 3) ? 1 : 2);
-    if (N == 3)
-      k_dual<3><<<pbt, tb, 0, st>>>(n_prims, nv, d_counts, idx, pos, nrm, s.dual_p, s.dual_n, normal_mode);
+    const SweepStep step = sweep_step(m, iters, sn ? 1 : 0, b.keep(), b);
+    if (pbt == 0) {
+      // no primitives: nothing but kept positions to hand on
+    } else if (N == 3)
+      k_dual<3><<<pbt, tb, 0, st>>>(n_prims, nv, d_counts, idx, step.src, nrm, s.dual_p, s.dual_n, step.normals);
     else
-      k_dual<4><<<pbt, tb, 0, st>>>(n_prims, nv, d_counts, idx, pos, nrm, s.dual_p, s.dual_n, normal_mode);
+      k_dual<4><<<pbt, tb, 0, st>>>(n_prims, nv, d_counts, idx, step.src, nrm, s.dual_p, s.dual_n, step.normals);
     // primal after every dual step but the last (MeshProcessor.cpp:229-232),
     // and once more after the loop with set_colors false (ChunkGenerator.cpp:120)
-    const int set_colors = (m < iters - 1) ? ((m == 3) || (m == 0 && iters <= 3)) : 0;
-    k_primal<<<vbt, tb, 0, st>>>(nv, n_prims, n_slots, d_counts, s.off, cursor, valence, s.adj, boundary, s.dual_p,
-                                 s.dual_n, pos, nrm, process_boundary, sn ? 1 : 0, set_colors);
+    if (N == 3)
+      k_primal<3><<<vbt, tb, 0, st>>>(nv, n_prims, n_slots, d_counts, s.off, cursor, valence, s.adj, boundary, s.dual_p,
+                                      s.dual_n, idx, step, b, iters, process_boundary);
+    else
+      k_primal<4><<<vbt, tb, 0, st>>>(nv, n_prims, n_slots, d_counts, s.off, cursor, valence, s.adj, boundary, s.dual_p,
+                                      s.dual_n, idx, step, b, iters, process_boundary);
     launched += 2;
   }
   return launched;
