@@ -19,11 +19,12 @@ using namespace bmf;
 namespace {
 
 enum Slot {
-  S_CHUNKS, S_UNITS, S_FLAGS, S_TOT, S_INFO, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
+  S_CHUNKS, S_TOT, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
   S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_NUM
 };
 
 constexpr int kMaxDim = 512;
+constexpr int kCounters = 3;  // list counters behind a plan's chunk flags
 // fit plans: the adjoint sweeps run chunk by chunk from this many chunks (one
 // 512-thread CTA per chunk, four per SM)
 constexpr int kChunkSweepBwdMinChunks = 256;
@@ -55,7 +56,7 @@ struct bmf_batch {
   std::vector<ChunkDev> h_chunks;
   ChunkDev* d_chunks = nullptr;
   int* d_units = nullptr;
-  uint32_t* d_flags = nullptr;
+  uint32_t* d_flags = nullptr;  // n flags, then the counters: work list, fix-up list, fill queue (one memset per run)
   uint32_t* d_tot = nullptr;
   int64_t* d_totals = nullptr;
   int* d_ticket = nullptr;  // launch_chunk_scan's
@@ -78,7 +79,6 @@ struct bmf_batch {
   cudaEvent_t stage_done = nullptr;  // the last staging copy has been consumed
   cudaEvent_t run_done = nullptr;    // recorded after every bmf_batch_run (bmf_batch_wait polls it)
   cudaEvent_t extract_done = nullptr;  // recorded inside every run after the emit (bmf_batch_wait_extraction)
-  cudaStream_t aux = nullptr;        // private stream for bmf_batch_wait's read of the totals
   bool ran = false;
   // terrain fill: line items {chunk, first line}, largest chunks first, and
   // the work queue of the persistent form; fill_mode 0 = x-plane kernel,
@@ -215,25 +215,43 @@ ChunkDev chunk_of(const bmf_chunk_desc* d) {
   return c;
 }
 
-// Uploads a single chunk record and its unit range [0, dim).
-bmf_status upload_single(bmf_ctx* ctx, const ChunkDev& c, cudaStream_t st, ChunkDev** d_c, int** d_u) {
+// Device state of a single chunk: its record, unit range [0, dim), flags and
+// work-list counter, set up by one launch.
+struct SingleChunk {
+  ChunkDev* c = nullptr;
+  int* units = nullptr;
+  uint32_t* flags = nullptr;
+  uint32_t* ccount = nullptr;
+};
+bmf_status setup_single(bmf_ctx* ctx, const ChunkDev& c, cudaStream_t st, SingleChunk* o) {
+  char* p;
   bmf_status s;
-  if ((s = scratch(ctx, S_CHUNKS, 1, d_c)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_UNITS, 2, d_u)) != BMF_OK) return s;
-  const int units[2] = {0, c.dim};
-  BMF_CUDA(ctx, cudaMemcpyAsync(*d_c, &c, sizeof(ChunkDev), cudaMemcpyHostToDevice, st));
-  BMF_CUDA(ctx, cudaMemcpyAsync(*d_u, units, sizeof(units), cudaMemcpyHostToDevice, st));
+  if ((s = scratch(ctx, S_CHUNKS, sizeof(ChunkDev) + 16, &p)) != BMF_OK) return s;
+  o->c = (ChunkDev*)p;
+  o->units = (int*)(p + sizeof(ChunkDev));
+  o->flags = (uint32_t*)(o->units + 2);
+  o->ccount = o->flags + 1;
+  launch_setup_chunk(c, o->c, o->units, o->flags, o->ccount, st);
+  BMF_LAUNCHED(ctx, 1);
   return BMF_OK;
 }
 
+// The most vertices and indices a chunk can have, whatever a caller's
+// capacities: three crossings per sample, five triangles per cell (Mode R);
+// four vertices per cell, three quads per sample (Mode Q).
+int64_t chunk_max_verts(int dim, int mode) { return (mode == BMF_MODE_R ? 3ll : 4ll) * dim * dim * dim; }
+int64_t chunk_max_idx(int dim, int mode) { return (mode == BMF_MODE_R ? 15ll : 12ll) * dim * dim * dim; }
+
 // Count -> chunk scan -> emit for one labelled chunk.  Totals land in
-// d_totals (kTotals entries).  flags_ready: the fill set d_flags; else they
-// are cleared here and the count sets them.
-bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunks, const int* d_units, int n_units,
-                        const uint32_t* d_words, const float* d_dens, uint32_t* d_flags, bool flags_ready,
-                        int64_t words_total, const MeshOut& mo, int64_t* d_totals, cudaStream_t st,
-                        StructuredAdj* sa = nullptr) {
+// d_totals (kTotals entries) and ctx->h_pinned.  flags_ready: the fill set the
+// chunk's flags; else the count sets them.
+bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk& c, int n_units,
+                        const uint32_t* d_words, const float* d_dens, bool flags_ready, int64_t words_total,
+                        const MeshOut& mo, int64_t* d_totals, cudaStream_t st, StructuredAdj* sa = nullptr) {
   constexpr int n_chunks = 1;
+  ChunkDev* d_chunks = c.c;
+  const int* d_units = c.units;
+  uint32_t* d_flags = c.flags;
   WordScratch ws{};
   uint32_t* tot = nullptr;
   bmf_status s;
@@ -245,10 +263,8 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunk
   {
     // work list of active cells: each one owns a vertex or emits a primitive
     ws.clist_cap = mo.vcap + mo.icap / (mode == BMF_MODE_R ? 3 : 4) + 1;
-    uint2* list;
-    if ((s = scratch(ctx, S_CLIST, (size_t)ws.clist_cap + 1, &list)) != BMF_OK) return s;
-    ws.clist = list;
-    ws.ccount = (uint32_t*)(list + ws.clist_cap);
+    if ((s = scratch(ctx, S_CLIST, (size_t)ws.clist_cap, &ws.clist)) != BMF_OK) return s;
+    ws.ccount = c.ccount;
   }
   if (sa) {
     *sa = StructuredAdj{mode, d_chunks, n_chunks, d_words, ws, mo.vkey};
@@ -257,11 +273,11 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, ChunkDev* d_chunk
       sa->team_failed = ctx->team_failed();
     }
   }
-  if (!flags_ready) BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
   launch_count(mode, d_chunks, n_chunks, d_units, n_units, d_words, flags_ready ? d_flags : nullptr, ws, st,
                flags_ready ? nullptr : d_flags);
   BMF_LAUNCHED(ctx, 1);
-  launch_chunk_scan(d_chunks, n_chunks, ws, tot, d_flags, mo.vcap, mo.icap, nullptr, d_totals, nullptr, st);
+  launch_chunk_scan(d_chunks, n_chunks, ws, tot, d_flags, mo.vcap, mo.icap, nullptr, d_totals, ctx->h_pinned,
+                    nullptr, st);
   BMF_LAUNCHED(ctx, 1);
   BMF_LAUNCHED(ctx, launch_emit(mode, placement, d_chunks, n_chunks, d_units, n_units, d_words, d_dens, d_flags, ws,
                                 mo, d_totals, st));
@@ -281,6 +297,23 @@ bmf_status mesh_valid(bmf_ctx* ctx, const bmf_mesh* m) {
   return BMF_OK;
 }
 
+// Runs launch (returns the kernels it launched) with the sweeps' scratch for nv
+// vertices and n_prims primitives.
+template <class F>
+bmf_status process_scratch(bmf_ctx* ctx, int N, int64_t nv, int64_t n_prims, float* const* x, F launch) {
+  ProcessScratch ps{};
+  bmf_status s;
+  if ((s = scratch(ctx, S_OFF, (size_t)nv + 1, &ps.off)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_CURSOR, (size_t)nv, &ps.cursor)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_ADJ, (size_t)n_prims * N, &ps.adj)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_DUALP, (size_t)n_prims * 4, &ps.dual_p)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_DUALN, (size_t)n_prims * 2, &ps.dual_n)) != BMF_OK) return s;
+  for (int k = 0; x && k < 3; ++k) ps.x[k] = x[k];
+  if ((s = scratch(ctx, S_SCANTMP, (size_t)(nv / 4096 + 2), &ps.tmp)) != BMF_OK) return s;
+  BMF_LAUNCHED(ctx, launch(ps));
+  return BMF_OK;
+}
+
 // x: the positions before the left-out face sweeps (x[0] the emitted mesh), or null
 bmf_status process_mesh(bmf_ctx* ctx, bmf_mesh* mesh, int iters, int pb, int sn, cudaStream_t st,
                         const StructuredAdj* sa = nullptr, float* const* x = nullptr) {
@@ -292,19 +325,10 @@ bmf_status process_mesh(bmf_ctx* ctx, bmf_mesh* mesh, int iters, int pb, int sn,
   // MeshProcessor::init returns early without work on an empty mesh (MeshProcessor.cpp:28-29)
   // (kept positions have to reach the output even then)
   if (iters <= 0 || nv == 0 || (mesh->n_idx < N && !x)) return BMF_OK;
-  ProcessScratch ps{};
-  bmf_status s;
-  if ((s = scratch(ctx, S_OFF, (size_t)nv + 1, &ps.off)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_CURSOR, (size_t)nv, &ps.cursor)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_ADJ, (size_t)n_prims * N, &ps.adj)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_DUALP, (size_t)n_prims * 4, &ps.dual_p)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_DUALN, (size_t)n_prims * 2, &ps.dual_n)) != BMF_OK) return s;
-  for (int k = 0; x && k < 3; ++k) ps.x[k] = x[k];
-  if ((s = scratch(ctx, S_SCANTMP, (size_t)(nv / 4096 + 2), &ps.tmp)) != BMF_OK) return s;
-  const int k = launch_process(N, nv, n_prims, nullptr, mesh->d_pos, mesh->d_nrm, mesh->d_boundary,
-                               mesh->d_valence, mesh->d_idx, iters, pb, sn, ps, sa, st);
-  BMF_LAUNCHED(ctx, k);
-  return BMF_OK;
+  return process_scratch(ctx, N, nv, n_prims, x, [&](const ProcessScratch& ps) {
+    return launch_process(N, nv, n_prims, nullptr, mesh->d_pos, mesh->d_nrm, mesh->d_boundary, mesh->d_valence,
+                          mesh->d_idx, iters, pb, sn, ps, sa, st);
+  });
 }
 
 }  // namespace
@@ -373,21 +397,17 @@ bmf_status bmf_sample_label(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf_
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "BMF_FIELD_GRID reads d_density, which must be given");
   cudaStream_t st = (cudaStream_t)stream;
   ChunkDev c = chunk_of(desc);
-  ChunkDev* d_c;
-  int* d_u;
-  uint32_t* d_flags;
+  SingleChunk sc;
   bmf_status s;
-  if ((s = upload_single(ctx, c, st, &d_c, &d_u)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_FLAGS, 1, &d_flags)) != BMF_OK) return s;
-  BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
+  if ((s = setup_single(ctx, c, st, &sc)) != BMF_OK) return s;
   const FieldDev fd = make_field(field);
-  launch_sample_label(d_c, 1, d_u, c.dim, c.dim, fd, d_density, field->kind == BMF_FIELD_GRID ? nullptr : d_density,
-                      d_words, d_flags, st);
+  launch_sample_label(sc.c, 1, sc.units, c.dim, c.dim, fd, d_density,
+                      field->kind == BMF_FIELD_GRID ? nullptr : d_density, d_words, sc.flags, st);
   BMF_LAUNCHED(ctx, 1);
   if (h_contains_mesh) {
-    uint32_t f = 0;
-    BMF_CUDA(ctx, cudaMemcpyAsync(&f, d_flags, sizeof(f), cudaMemcpyDeviceToHost, st));
+    BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, sc.flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
+    const uint32_t f = *(const uint32_t*)ctx->h_pinned;
     *h_contains_mesh = ((f & 1u) || ((f & 6u) == 6u)) ? 1 : 0;
   }
   return BMF_OK;
@@ -442,21 +462,17 @@ bmf_status bmf_polygonize(bmf_ctx* ctx, int32_t dim, const float* d_density, con
   c.scale = 1.0f;
   c.dim = dim;
   c.zc = (dim + 31) / 32;
-  ChunkDev* d_c;
-  int* d_u;
-  uint32_t* d_flags;
+  SingleChunk sc;
   int64_t* d_totals;
-  if ((s = upload_single(ctx, c, st, &d_c, &d_u)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_FLAGS, 1, &d_flags)) != BMF_OK) return s;
+  if ((s = setup_single(ctx, c, st, &sc)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_TOTALS, kTotals, &d_totals)) != BMF_OK) return s;
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   if (mode == BMF_MODE_Q && placement == BMF_PLACE_QEF &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
-  if ((s = extract_core(ctx, mode, placement, d_c, d_u, dim, d_words, d_density, d_flags, false,
-                        (int64_t)dim * dim * c.zc, mo, d_totals, st)) != BMF_OK)
+  if ((s = extract_core(ctx, mode, placement, sc, dim, d_words, d_density, false, (int64_t)dim * dim * c.zc, mo,
+                        d_totals, st)) != BMF_OK)
     return s;
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, kTotals * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   BMF_CUDA(ctx, cudaStreamSynchronize(st));
   out->n_verts = ctx->h_pinned[0];
   out->n_idx = ctx->h_pinned[1];
@@ -532,47 +548,58 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_extract_chunk: smoothing needs d_valence and d_boundary");
   cudaStream_t st = (cudaStream_t)stream;
   const ChunkDev c = chunk_of(desc);
-  const int dim = c.dim;
-  ChunkDev* d_c;
-  int* d_u;
-  uint32_t* d_flags;
+  const int dim = c.dim, N = opts->mode == BMF_MODE_R ? 3 : 4;
+  SingleChunk sc;
   int64_t* d_totals;
   float* d_dens;
   uint32_t* d_words;
-  if ((s = upload_single(ctx, c, st, &d_c, &d_u)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_FLAGS, 1, &d_flags)) != BMF_OK) return s;
+  if ((s = setup_single(ctx, c, st, &sc)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_TOTALS, kTotals, &d_totals)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_DENS, (size_t)dim * dim * dim, &d_dens)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_WORDS, (size_t)dim * dim * c.zc, &d_words)) != BMF_OK) return s;
-  BMF_CUDA(ctx, cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st));
   const FieldDev fd = make_field(field);
-  launch_sample_label(d_c, 1, d_u, dim, dim, fd, nullptr, d_dens, d_words, d_flags, st);
+  launch_sample_label(sc.c, 1, sc.units, dim, dim, fd, nullptr, d_dens, d_words, sc.flags, st);
   BMF_LAUNCHED(ctx, 1);
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   if ((opts->iters > 0 || (opts->mode == BMF_MODE_Q && opts->placement == BMF_PLACE_QEF)) &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
+  // What the capacities, bounded by the chunk's size, ask of the sweeps'
+  // scratch: within kOneSyncBytes the sweeps are enqueued behind the emit with
+  // the counts on the device, and positions are kept for left-out face
+  // sweeps; beyond (large chunks) they wait for the counts and are sized by them.
+  constexpr int64_t kOneSyncBytes = 256ll << 20;
+  const int64_t vb = std::min(out->vcap, chunk_max_verts(dim, opts->mode));
+  const int64_t ib = std::min(out->icap, chunk_max_idx(dim, opts->mode));
+  const bool bounded = 40 * vb + 4 * ib + 24 * (ib / N) <= kOneSyncBytes;
   // sweeps that leave steps out read the mesh from x[0] and write out->d_pos
   float* x[3] = {};
-  const int skip = field_skipped(field->kind, opts->iters, opts->smooth_normals && out->d_nrm);
+  const int skip = bounded ? field_skipped(field->kind, opts->iters, opts->smooth_normals && out->d_nrm) : 0;
   for (int k = 0; skip && k <= skip; ++k)
-    if ((s = scratch(ctx, (Slot)(S_X0 + k), (size_t)out->vcap * 3, &x[k])) != BMF_OK) return s;
+    if ((s = scratch(ctx, (Slot)(S_X0 + k), (size_t)vb * 3, &x[k])) != BMF_OK) return s;
   if (skip) {
     mo.pos = x[0];
     mo.nrm = nullptr;
+    mo.vcap = vb;
   }
   StructuredAdj sa{};
-  if ((s = extract_core(ctx, opts->mode, opts->placement, d_c, d_u, dim, d_words, d_dens, d_flags, true,
-                        (int64_t)dim * dim * c.zc, mo, d_totals, st, opts->iters > 0 ? &sa : nullptr)) != BMF_OK)
+  if ((s = extract_core(ctx, opts->mode, opts->placement, sc, dim, d_words, d_dens, true, (int64_t)dim * dim * c.zc, mo,
+                        d_totals, st, opts->iters > 0 ? &sa : nullptr)) != BMF_OK)
     return s;
-  BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, d_totals, kTotals * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  const bool one_sync = bounded && sa.team;
+  if (one_sync && (s = process_scratch(ctx, N, vb, ib / N, x, [&](const ProcessScratch& ps) {
+        return launch_process(N, vb, ib / N, d_totals, out->d_pos, out->d_nrm, out->d_boundary, out->d_valence,
+                              out->d_idx, opts->iters, opts->process_boundary, opts->smooth_normals, ps, &sa, st);
+      })) != BMF_OK)
+    return s;
   BMF_CUDA(ctx, cudaStreamSynchronize(st));
   out->n_verts = ctx->h_pinned[0];
   out->n_idx = ctx->h_pinned[1];
   out->contains_mesh = (int32_t)ctx->h_pinned[2];
-  out->prim_size = opts->mode == BMF_MODE_R ? 3 : 4;
+  out->prim_size = N;
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_extract_chunk: output capacity exceeded (needed counts reported)");
+  if (one_sync) return team_check(ctx, sa.team);
   // ChunkGenerator.cpp:112: processing only when the chunk has a mesh
   if (opts->iters > 0 && out->contains_mesh && out->n_verts && (out->n_idx || skip)) {
     if ((s = process_mesh(ctx, out, opts->iters, opts->process_boundary, opts->smooth_normals, st, &sa,
@@ -634,7 +661,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   bmf_status s;
   if ((s = bail(cudaMalloc(&b->d_chunks, sizeof(ChunkDev) * n_chunks), "chunks")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_units, sizeof(int) * (n_chunks + 1)), "units")) != BMF_OK) return s;
-  if ((s = bail(cudaMalloc(&b->d_flags, sizeof(uint32_t) * n_chunks), "flags")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->d_flags, sizeof(uint32_t) * (n_chunks + kCounters)), "flags")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_tot, sizeof(uint32_t) * 2 * n_chunks), "tot")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_totals, sizeof(int64_t) * kTotals), "totals")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_ticket, sizeof(int)), "scan ticket")) != BMF_OK) return s;
@@ -679,7 +706,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
     }
     b->n_fill_items = (int)items.size();
     if ((s = bail(cudaMalloc(&b->d_fill_items, sizeof(int2) * items.size()), "fill items")) != BMF_OK) return s;
-    if ((s = bail(cudaMalloc(&b->d_queue, sizeof(int)), "fill queue")) != BMF_OK) return s;
+    b->d_queue = (int*)(b->d_flags + n_chunks + 2);
     if ((s = bail(cudaMemcpy(b->d_fill_items, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice),
                   "upload fill items")) != BMF_OK)
       return s;
@@ -729,11 +756,11 @@ bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
     if (b->d_clist) cudaFree(b->d_clist);
     b->d_clist = nullptr;
     b->clist_cap = 0;
-    BMF_CUDA(b->ctx, cudaMalloc(&b->d_clist, sizeof(uint2) * (cap + 1)));
+    BMF_CUDA(b->ctx, cudaMalloc(&b->d_clist, sizeof(uint2) * cap));
     b->clist_cap = cap;
   }
   b->ws.clist = b->d_clist;
-  b->ws.ccount = (uint32_t*)(b->d_clist + b->clist_cap);
+  b->ws.ccount = b->d_flags + b->n;
   b->ws.clist_cap = b->clist_cap;
   if (b->d_exact) {
     // band fill: every crossing (one vertex each in Mode R) lists at most its two ends
@@ -742,11 +769,11 @@ bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
       if (b->d_fix) cudaFree(b->d_fix);
       b->d_fix = nullptr;
       b->fix_cap = 0;
-      BMF_CUDA(b->ctx, cudaMalloc(&b->d_fix, sizeof(uint2) * (fcap + 1)));
+      BMF_CUDA(b->ctx, cudaMalloc(&b->d_fix, sizeof(uint2) * fcap));
       b->fix_cap = fcap;
     }
     b->ws.fix = b->d_fix;
-    b->ws.fcount = (uint32_t*)(b->d_fix + b->fix_cap);
+    b->ws.fcount = b->d_flags + b->n + 1;
     b->ws.fix_cap = b->fix_cap;
   }
   const bool band = batch_band(b);
@@ -863,13 +890,13 @@ int batch_sweeps(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st) {
 bmf_status batch_record(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st, int64_t* kernels) {
   bmf_ctx* ctx = b->ctx;
   const bool proc = b->opts.iters > 0;
-  BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * b->n, st));
+  BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * (b->n + kCounters), st));
   batch_fill(b, st);
   launch_count(b->opts.mode, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_flags, b->ws, st);
   const bool band = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;  // the 2D column fill needs no fix-up
   if (band) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                    b->d_totals, b->d_ticket, st, &b->sweep);
+                    b->d_totals, b->h_pinned, b->d_ticket, st, &b->sweep);
   const MeshOut mo = batch_mesh_out(b, out);
   int64_t k = (band ? 4 : 3) + (b->d_cols ? 1 : 0);
   k += launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_dens,
@@ -941,7 +968,6 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
   BMF_CUDA(ctx, cudaEventRecord(b->run_done, st));
   b->ran = true;
   if (sync) {
-    BMF_CUDA(ctx, cudaMemcpyAsync(b->h_pinned, b->d_totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
     out->n_verts = b->h_pinned[0];
     out->n_idx = b->h_pinned[1];
@@ -969,9 +995,6 @@ bmf_status bmf_batch_wait(bmf_batch* b, bmf_batch_out* out, int32_t timeout_ms) 
                       " ms (nothing was cancelled; wait again)");
     std::this_thread::sleep_for(std::chrono::microseconds(50));
   }
-  if (!b->aux) BMF_CUDA(ctx, cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking));
-  BMF_CUDA(ctx, cudaMemcpyAsync(b->h_pinned, b->d_totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, b->aux));
-  BMF_CUDA(ctx, cudaStreamSynchronize(b->aux));
   out->n_verts = b->h_pinned[0];
   out->n_idx = b->h_pinned[1];
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
@@ -1033,7 +1056,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   cudaEvent_t ev[8];
   for (auto& e : ev) BMF_CUDA(ctx, cudaEventCreate(&e));
   BMF_CUDA(ctx, cudaEventRecord(ev[0], st));
-  BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * b->n, st));
+  BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * (b->n + kCounters), st));
   batch_fill(b, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[1], st));
   launch_count(b->opts.mode, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_flags, b->ws, st);
@@ -1044,7 +1067,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaEventRecord(ev[7], st));
   BMF_CUDA(ctx, cudaEventRecord(ev[3], st));  // the word scan is part of the count
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
-                    b->d_totals, b->d_ticket, st, &b->sweep);
+                    b->d_totals, b->h_pinned, b->d_ticket, st, &b->sweep);
   BMF_CUDA(ctx, cudaEventRecord(ev[4], st));
   const MeshOut mo = batch_mesh_out(b, out);
   const int ek = launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words,
@@ -1168,7 +1191,7 @@ bmf_status bmf_batch_autotune(bmf_batch* b, bmf_batch_out* out, int32_t reps, vo
       if ((s = bmf_batch_set_tuning(b, &t)) != BMF_OK) return s;
       float ms = 0.0f;
       s = time_it([&] {
-        cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * b->n, st);
+        cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * (b->n + kCounters), st);
         batch_fill(b, st);
       }, &ms);
       if (s != BMF_OK) return s;
@@ -1295,7 +1318,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
   const int64_t np = icap / 4;
   bool ok = cudaMalloc(&f->d_chunks, sizeof(ChunkDev) * n_chunks) == cudaSuccess &&
             cudaMalloc(&f->d_units, sizeof(int) * (n_chunks + 1)) == cudaSuccess &&
-            cudaMalloc(&f->d_flags, sizeof(uint32_t) * n_chunks) == cudaSuccess &&
+            cudaMalloc(&f->d_flags, sizeof(uint32_t) * (n_chunks + kCounters)) == cudaSuccess &&
             cudaMalloc(&f->d_tot, sizeof(uint32_t) * 2 * n_chunks) == cudaSuccess &&
             cudaMalloc(&f->d_words, sizeof(uint32_t) * words) == cudaSuccess &&
             cudaMalloc(&f->d_totals, sizeof(int64_t) * kTotals) == cudaSuccess &&
@@ -1334,7 +1357,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
   }
   f->ws.clist = f->d_clist;
   f->ws.clist_cap = vcap + icap / 4 + 1;
-  f->ws.ccount = (uint32_t*)(f->d_clist + f->ws.clist_cap);
+  f->ws.ccount = f->d_flags + n_chunks;
   *out = f;
   return BMF_OK;
 }
@@ -1348,12 +1371,12 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   cudaStream_t st = (cudaStream_t)stream;
   FieldDev fd{};
   fd.kind = BMF_FIELD_GRID;
-  BMF_CUDA(ctx, cudaMemsetAsync(f->d_flags, 0, sizeof(uint32_t) * f->n, st));
+  BMF_CUDA(ctx, cudaMemsetAsync(f->d_flags, 0, sizeof(uint32_t) * (f->n + kCounters), st));
   launch_sample_label(f->d_chunks, f->n, f->d_units, f->n * f->dim, f->dim, fd, d_density, nullptr, f->d_words,
                       f->d_flags, st);
   launch_count(BMF_MODE_Q, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words, f->d_flags, f->ws, st);
   launch_chunk_scan(f->d_chunks, f->n, f->ws, f->d_tot, f->d_flags, f->vcap, f->icap, d_chunk_info, f->d_totals,
-                    f->d_ticket, st, &f->sweep);
+                    f->h_pinned, f->d_ticket, st, &f->sweep);
   MeshOut mo{d_pos, nullptr, f->d_boundary, f->d_valence, d_idx, f->d_idxg, f->vcap, f->icap, f->d_vkey};
   if (f->d_qflag && f->placement == BMF_PLACE_QEF) {  // the wide adjoint reads the forward's QEF branches
     mo.qflag = f->d_qflag;
@@ -1379,7 +1402,6 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   BMF_LAUNCHED(ctx, k);
   f->last_density = d_density;
   if (h_counts) {
-    BMF_CUDA(ctx, cudaMemcpyAsync(f->h_pinned, f->d_totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
     h_counts[0] = f->h_pinned[0];
     h_counts[1] = f->h_pinned[1];
@@ -1452,7 +1474,7 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
   void* ptrs[] = {b->d_chunks, b->d_units, b->d_flags, b->d_tot, b->d_totals, b->d_dens, b->d_words,
                   b->ws.vcnt, b->ws.icnt, b->ws.gpl, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
-                  b->d_fill_items, b->d_queue, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
+                  b->d_fill_items, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
                   b->d_cols, b->d_ticket, b->ws.pb, b->team, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1461,7 +1483,6 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
   if (b->stage_done) cudaEventDestroy(b->stage_done);
   if (b->run_done) cudaEventDestroy(b->run_done);
   if (b->extract_done) cudaEventDestroy(b->extract_done);
-  if (b->aux) cudaStreamDestroy(b->aux);
   delete b;
   return BMF_OK;
 }

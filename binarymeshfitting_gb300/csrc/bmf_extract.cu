@@ -413,7 +413,8 @@ __device__ __forceinline__ int size_bin(uint32_t v) {
 __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restrict__ chunks, int n, uint2* __restrict__ pb,
                                                              uint32_t* tot, const uint32_t* __restrict__ flags,
                                                              int64_t vcap, int64_t icap, int64_t* __restrict__ info,
-                                                             int64_t* __restrict__ totals, int* __restrict__ ticket,
+                                                             int64_t* __restrict__ totals,
+                                                             int64_t* __restrict__ h_totals, int* __restrict__ ticket,
                                                              SweepLists sweep) {
   __shared__ int64_t s_v[kScanWarps], s_i[kScanWarps];
   __shared__ bool s_last;
@@ -479,6 +480,8 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
     totals[0] = carry_v;
     totals[1] = carry_i;
     totals[2] = contains_mesh(flags[0]) ? 1 : 0;
+    if (h_totals)
+      for (int k = 0; k < kTotals; ++k) h_totals[k] = totals[k];
     if (gridDim.x > 1) *ticket = 0;
   }
   if (!sweep.order) return;
@@ -1506,11 +1509,22 @@ SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s) {
   return kSweepLaunches;
 }
 
+__global__ void k_setup_chunk(const ChunkDev c, ChunkDev* d_c, int* units, uint32_t* flags, uint32_t* ccount) {
+  *d_c = c;
+  units[0] = 0;
+  units[1] = c.dim;
+  *flags = 0u;
+  if (ccount) *ccount = 0u;
+}
+
+void launch_setup_chunk(const ChunkDev& c, ChunkDev* d_c, int* d_units, uint32_t* d_flags, uint32_t* d_ccount,
+                        cudaStream_t st) {
+  k_setup_chunk<<<1, 1, 0, st>>>(c, d_c, d_units, d_flags, d_ccount);
+}
+
 void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
                   const uint32_t* words, const uint32_t* flags, WordScratch ws, cudaStream_t st,
                   uint32_t* flags_out) {
-  if (ws.clist) cudaMemsetAsync(ws.ccount, 0, sizeof(uint32_t), st);
-  if (ws.exact) cudaMemsetAsync(ws.fcount, 0, sizeof(uint32_t), st);
 #define BMF_COUNT(M, T) \
   k_count<M, T><<<n_units, T, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, flags, flags_out, ws)
   if (n_units < kCountFewUnits) {
@@ -1522,10 +1536,11 @@ void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d
 }
 
 void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
-                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
+                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int64_t* h_totals, int* d_ticket,
                        cudaStream_t st, const SweepLists* sweep) {
   k_chunk_scan<<<(n_chunks + kScanWarps - 1) / kScanWarps, kScanThreads, 0, st>>>(
-      d_chunks, n_chunks, ws.pb, d_tot, flags, vcap, icap, d_info, d_totals, d_ticket, sweep ? *sweep : SweepLists{});
+      d_chunks, n_chunks, ws.pb, d_tot, flags, vcap, icap, d_info, d_totals, h_totals, d_ticket,
+      sweep ? *sweep : SweepLists{});
 }
 
 // k-th set bit (from 0) of m; m must have more than k set bits.

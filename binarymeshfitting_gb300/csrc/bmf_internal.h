@@ -108,7 +108,8 @@ void launch_words2d(const ChunkDev* d_chunks, int n_chunks, const int* d_unit_st
                     const FieldDev& field, const float* cols, uint32_t* words, uint32_t* flags, cudaStream_t st);
 // Terrain FBM fill over line items {chunk, first line} (kFillLines lines
 // each; d_items null = chunk 0's items in order).  d_queue non-null: grid
-// persistent CTAs take items from the queue (reset here); else one CTA per item.
+// persistent CTAs take items from the queue (zeroed by the caller); else one CTA
+// per item.
 // run = z-samples per step (4, 8, 16 or 32).
 // exact (nullable): the band fill's exactness mask (words layout); with it
 // the fill may leave decided samples inexact (see k_fill_terrain<RUN, true>)
@@ -136,7 +137,13 @@ int fill_terrain_items(int dim);          // items of one chunk
 int fill_terrain_lines();                 // lines per item
 int fill_terrain_resident_ctas(int run, int octaves, bool band);  // persistent grid: SMs x resident CTAs per SM
 void launch_cell_masks(int dim, const uint32_t* W, uint8_t* masks, cudaStream_t st);
-// Extraction: count -> chunk scan -> emit.  flags: the contains_mesh flags the
+// The record and unit range of a single chunk, its flags and (nullable) its
+// work-list counter zeroed: one small launch instead of two copies and two
+// memsets.
+void launch_setup_chunk(const ChunkDev& c, ChunkDev* d_c, int* d_units, uint32_t* d_flags, uint32_t* d_ccount,
+                        cudaStream_t st);
+// Extraction: count -> chunk scan -> emit.  The list counters in ws are zeroed
+// by the caller.  flags: the contains_mesh flags the
 // fill wrote; flags_out (instead, with flags null): words produced elsewhere,
 // whose flags the count kernel adds up here (cleared by the caller).
 void launch_count(int mode, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
@@ -166,8 +173,10 @@ struct TeamSync {
   unsigned arrived, left, failed, pad;
   uint32_t seg[kTeamMax];
 };
+// h_totals (nullable): the same totals in pinned host memory, so that the host
+// needs a synchronisation but no copy to read them.
 void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_t* d_tot, const uint32_t* flags,
-                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int* d_ticket,
+                       int64_t vcap, int64_t icap, int64_t* d_info, int64_t* d_totals, int64_t* h_totals, int* d_ticket,
                        cudaStream_t st, const SweepLists* sweep = nullptr);
 // How the sweeps of n_chunks chunks with `columns` (sum of dim^2) columns in all
 // run: one launch per step, one cooperative launch over the whole mesh, or

@@ -53,13 +53,6 @@ constexpr int kMaxDevices = 64;
 std::mutex g_lookup_mutex;
 uint32_t* g_scratch_ptr[kMaxDevices] = {};
 
-// Writes the single chunk record and its unit range into the scratch header.
-__global__ void k_noalloc_header(ChunkDev c, ChunkDev* dst, int* units) {
-  *dst = c;
-  units[0] = 0;
-  units[1] = c.dim;
-}
-
 // Device address of the scratch array for the current device (looked up once).
 bmf_status scratch_for_current_device(uint32_t** out) {
   int dev = -1;
@@ -105,10 +98,9 @@ extern "C" bmf_status bmf_polygonize_noalloc(int32_t dim, const float* d_density
   c.scale = 1.0f;
   c.dim = dim;
   c.zc = zc;
-  k_noalloc_header<<<1, 1, 0, st>>>(c, d_c, d_u);
-  cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), st);
+  launch_setup_chunk(c, d_c, d_u, d_flags, nullptr, st);
   launch_count(mode, d_c, 1, d_u, dim, d_words, nullptr, ws, st, d_flags);  // sets the flags
-  launch_chunk_scan(d_c, 1, ws, d_tot, d_flags, out->vcap, out->icap, nullptr, d_totals, nullptr, st);
+  launch_chunk_scan(d_c, 1, ws, d_tot, d_flags, out->vcap, out->icap, nullptr, d_totals, nullptr, nullptr, st);
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   launch_emit(mode, placement, d_c, 1, d_u, dim, d_words, d_density, d_flags, ws, mo, nullptr, st);
   if (cudaPeekAtLastError() != cudaSuccess) return BMF_ERR_CUDA;

@@ -555,7 +555,6 @@ void launch_fill_terrain(int run, const ChunkDev* d_chunks, const int2* d_items,
                          int grid, const FieldDev& field, float* dens_out, uint32_t* words, uint32_t* flags,
                          uint32_t* exact, cudaStream_t st) {
   if (n_items <= 0) return;
-  if (d_queue) cudaMemsetAsync(d_queue, 0, sizeof(int), st);
   const int g = d_queue ? grid : n_items;
   fill_terrain_smem_optin();
   const bool band = exact && dens_out;

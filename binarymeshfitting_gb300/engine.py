@@ -20,6 +20,27 @@ def _stream(stream=None):
     return ctypes.c_void_p(s.cuda_stream)
 
 
+# bmf_chunk_desc as a numpy record (the fields of _lib.ChunkDesc)
+DESC_DTYPE = np.dtype([("origin", np.float32, 3), ("scale", np.float32), ("dim", np.int32), ("level", np.int32)])
+_DESC_ONLY = {L.ChunkDesc}
+
+
+def _desc_array(descs, n):
+    """(object to keep alive, pointer) of n chunk descriptors given as a list of
+    ChunkDesc, a ctypes array of them or a DESC_DTYPE array.  A list is joined
+    as bytes: constructing a ctypes array of 4096 elements takes 1 ms, during
+    which the GPU has nothing to do."""
+    if isinstance(descs, np.ndarray) and descs.dtype == DESC_DTYPE and descs.shape == (n,):
+        a = np.ascontiguousarray(descs)
+        return a, ctypes.cast(a.ctypes.data, ctypes.POINTER(L.ChunkDesc))
+    if isinstance(descs, (list, tuple)) and len(descs) == n and set(map(type, descs)) == _DESC_ONLY:
+        raw = b"".join(descs)
+        return raw, ctypes.cast(ctypes.c_char_p(raw), ctypes.POINTER(L.ChunkDesc))
+    if not (isinstance(descs, ctypes.Array) and descs._type_ is L.ChunkDesc and len(descs) == n):
+        descs = (L.ChunkDesc * n)(*descs)
+    return descs, descs
+
+
 def zpad(dim):
     return 32 * ((dim + 31) // 32)
 
@@ -218,8 +239,8 @@ class Batch:
                  process_boundary=False, smooth_normals=False):
         self.ctx = ctx
         self.n = len(descs)
-        arr = (L.ChunkDesc * self.n)(*descs)
-        self.descs = arr
+        keep, arr = _desc_array(descs, self.n)
+        self.descs = (L.ChunkDesc * self.n).from_buffer_copy(ctypes.string_at(arr, self.n * ctypes.sizeof(L.ChunkDesc)))
         self.opts = L.ExtractOpts(mode, placement, iters, int(process_boundary), int(smooth_normals), 0)
         self.field = field
         self.mode = mode
@@ -262,8 +283,8 @@ class Batch:
         self.ctx._check(self.ctx.lib.bmf_batch_wait_extraction(self.h, _stream(stream)))
 
     def set_descs(self, descs, stream=None):
-        arr = (L.ChunkDesc * self.n)(*descs)
-        self.ctx._check(self.ctx.lib.bmf_batch_set_descs(self.h, arr, self.n, _stream(stream)))
+        keep, p = _desc_array(descs, self.n)  # copied into pinned staging by the call
+        self.ctx._check(self.ctx.lib.bmf_batch_set_descs(self.h, p, self.n, _stream(stream)))
 
     def profile(self, stream=None):
         """Stage times (ms) of one update: fill+label, count, scan, offsets, emit, processing."""
@@ -317,6 +338,21 @@ class Batch:
         return dict(pos=b["pos"][vo:vo + vc], nrm=b["nrm"][vo:vo + vc] if b["nrm"] is not None else None,
                     boundary=b["boundary"][vo:vo + vc] if b["boundary"] is not None else None,
                     idx=b["idx"][io:io + ic], contains_mesh=bool(info[4]), status=int(info[5]))
+
+    def chunk_meshes(self, n_verts, n_idx):
+        """chunk_mesh of every chunk of the last run, over one copy of its n_verts
+        vertices and n_idx indices (the arena may be overwritten): one read of
+        the chunk table and one copy per attribute, whatever the chunk count."""
+        info = self.bufs["info"].cpu().tolist()
+        vc, ic = [r[1] for r in info], [r[3] for r in info]
+        b = self.bufs
+
+        def parts(t, n, sizes):
+            return t[:n].clone().split(sizes) if t is not None else [None] * len(sizes)
+
+        return [dict(pos=p, nrm=q, boundary=f, idx=i, contains_mesh=bool(r[4]), status=int(r[5]))
+                for r, p, q, f, i in zip(info, parts(b["pos"], n_verts, vc), parts(b["nrm"], n_verts, vc),
+                                         parts(b["boundary"], n_verts, vc), parts(b["idx"], n_idx, ic))]
 
     def close(self):
         if self.h:

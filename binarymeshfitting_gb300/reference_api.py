@@ -16,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib as L
-from .engine import Batch, ChunkMesh, Context
+from .engine import DESC_DTYPE, Batch, ChunkMesh, Context
 
 RESOLUTION = 32  # DMCChunk.cpp:34 (samples per axis of a world chunk)
 
@@ -40,6 +40,15 @@ def chunk_frame(pos, size, overlap, dim):
     delta = f(f(s * f(f(1.0) + f(o * f(2.0)))) / f(dim - 1))
     shift = f(s * o)
     return float(delta), tuple(float(f(f(p) - shift)) for p in pos)
+
+
+def chunk_frames(pos, size, overlap, dim):
+    """chunk_frame of many chunks at once (the same single-precision operations,
+    elementwise): (delta (n,), overlap_pos (n, 3)) as float32 arrays."""
+    f = np.float32
+    p, s, o = (np.asarray(v, np.float64).astype(f) for v in (pos, size, overlap))
+    delta = s * (f(1.0) + o * f(2.0)) / f(dim - 1)
+    return delta, p - (s * o)[:, None]
 
 
 class Sampler:
@@ -202,10 +211,11 @@ class ChunkGenerator:
         return p.overlap + 0.005 * float(p.process_iters)
 
     def _descs(self, batch):
-        out = []
-        for n in batch:
-            delta, org = chunk_frame(n.pos, n.size, self.overlap_for(n), self.dim)
-            out.append(L.ChunkDesc.make(org, delta, self.dim, n.level))
+        out = np.empty(len(batch), DESC_DTYPE)
+        out["scale"], out["origin"] = chunk_frames([n.pos for n in batch], [n.size for n in batch],
+                                                   [self.overlap_for(n) for n in batch], self.dim)
+        out["dim"] = self.dim
+        out["level"] = [n.level for n in batch]
         return out
 
     def process_queue(self, batch: List[WorldOctreeNode]):
@@ -225,17 +235,18 @@ class ChunkGenerator:
             self._plan = b
             vcap, icap = max(4096, len(batch) * self.dim ** 2 * 4), max(16384, len(batch) * self.dim ** 2 * 24)
             b.allocate(vcap, icap, normals=p.smooth_normals)
+        nv = ni = 0
         for _ in range(3):
             try:
-                b.run(use_graph=True, sync=True)
+                nv, ni = b.run(use_graph=True, sync=True)
                 break
             except L.BmfError as e:
                 if e.status != L.ERR_CAPACITY:
                     raise
                 b.allocate(int(b.out.n_verts) + 1024, int(b.out.n_idx) + 1024, normals=p.smooth_normals)
-        for i, n in enumerate(batch):
-            # copies: the arena is overwritten by the next queue
-            n.vi = {k: (v.clone() if isinstance(v, torch.Tensor) else v) for k, v in b.chunk_mesh(i).items()}
+        # copies: the arena is overwritten by the next queue
+        for n, vi in zip(batch, b.chunk_meshes(nv, ni)):
+            n.vi = vi
         return batch
 
     def close(self):
