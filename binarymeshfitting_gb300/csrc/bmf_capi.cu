@@ -20,7 +20,7 @@ namespace {
 
 enum Slot {
   S_CHUNKS, S_TOT, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
-  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_NUM
+  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_COLS, S_NUM
 };
 
 constexpr int kMaxDim = 512;
@@ -236,6 +236,21 @@ bmf_status setup_single(bmf_ctx* ctx, const ChunkDev& c, cudaStream_t st, Single
   return BMF_OK;
 }
 
+// Fill + label of a single chunk (the 2D heightmap's column heights first).
+bmf_status fill_single(bmf_ctx* ctx, const SingleChunk& sc, int dim, const FieldDev& fd, const float* dens_in,
+                       float* dens_out, uint32_t* d_words, cudaStream_t st) {
+  float* cols = nullptr;
+  if (fd.kind == BMF_FIELD_TERRAIN_2D) {
+    bmf_status s = scratch(ctx, S_COLS, (size_t)dim * dim, &cols);
+    if (s != BMF_OK) return s;
+    launch_columns2d(sc.c, nullptr, (dim * dim + columns2d_item() - 1) / columns2d_item(), fd, cols, st);
+    BMF_LAUNCHED(ctx, 1);
+  }
+  launch_sample_label(sc.c, 1, sc.units, dim, dim, fd, dens_in, dens_out, d_words, sc.flags, st, cols);
+  BMF_LAUNCHED(ctx, 1);
+  return BMF_OK;
+}
+
 // The most vertices and indices a chunk can have, whatever a caller's
 // capacities: three crossings per sample, five triangles per cell (Mode R);
 // four vertices per cell, three quads per sample (Mode Q).
@@ -401,9 +416,9 @@ bmf_status bmf_sample_label(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf_
   bmf_status s;
   if ((s = setup_single(ctx, c, st, &sc)) != BMF_OK) return s;
   const FieldDev fd = make_field(field);
-  launch_sample_label(sc.c, 1, sc.units, c.dim, c.dim, fd, d_density,
-                      field->kind == BMF_FIELD_GRID ? nullptr : d_density, d_words, sc.flags, st);
-  BMF_LAUNCHED(ctx, 1);
+  if ((s = fill_single(ctx, sc, c.dim, fd, d_density, field->kind == BMF_FIELD_GRID ? nullptr : d_density, d_words,
+                       st)) != BMF_OK)
+    return s;
   if (h_contains_mesh) {
     BMF_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned, sc.flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
@@ -558,8 +573,7 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   if ((s = scratch(ctx, S_DENS, (size_t)dim * dim * dim, &d_dens)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_WORDS, (size_t)dim * dim * c.zc, &d_words)) != BMF_OK) return s;
   const FieldDev fd = make_field(field);
-  launch_sample_label(sc.c, 1, sc.units, dim, dim, fd, nullptr, d_dens, d_words, sc.flags, st);
-  BMF_LAUNCHED(ctx, 1);
+  if ((s = fill_single(ctx, sc, dim, fd, nullptr, d_dens, d_words, st)) != BMF_OK) return s;
   MeshOut mo{out->d_pos, out->d_nrm, out->d_boundary, out->d_valence, out->d_idx, nullptr, out->vcap, out->icap};
   if ((opts->iters > 0 || (opts->mode == BMF_MODE_Q && opts->placement == BMF_PLACE_QEF)) &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
@@ -717,7 +731,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
     }
     b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], b->fill_band != 0);
   }
-  if (b->field.kind == BMF_FIELD_TERRAIN_2D && b->opts.mode == BMF_MODE_R && fill_band_supported(b->field)) {
+  if (b->field.kind == BMF_FIELD_TERRAIN_2D) {
     // column items {chunk, first column}, largest chunks first
     std::vector<int2> items;
     const int per = columns2d_item();
@@ -731,7 +745,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
                   "upload column items")) != BMF_OK)
       return s;
     if ((s = bail(cudaMalloc(&b->d_cols, sizeof(float) * words), "column heights")) != BMF_OK) return s;
-    b->fill_band = 1;
+    b->fill_band = b->opts.mode == BMF_MODE_R && fill_band_supported(b->field);
   }
   if ((s = bail(cudaEventCreateWithFlags(&b->extract_done, cudaEventDisableTiming), "extraction event")) != BMF_OK)
     return s;
@@ -1124,7 +1138,7 @@ bmf_status bmf_batch_set_tuning(bmf_batch* b, const bmf_batch_tuning* t) {
   if (t->fill_mode < 0 || t->fill_mode > 2 || (!terrain && t->fill_mode != 0) ||
       (t->fill_run != 4 && t->fill_run != 8 && t->fill_run != 16) ||
       (t->sweep_block != 128 && t->sweep_block != 256 && t->sweep_block != 512) ||
-      (t->fill_band != 0 && t->fill_band != 1) || (t->fill_band && !b->d_exact && !b->d_cols))
+      (t->fill_band != 0 && t->fill_band != 1) || (t->fill_band && !b->d_exact && !(b->d_cols && b->opts.mode == BMF_MODE_R)))
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT,
                 "bmf_batch_set_tuning: fill_mode 0..2 (1, 2 for terrain fields only), fill_run 4/8/16, "
                 "sweep_block 128/256/512, fill_band 0/1 (1 for Mode R terrain and 2D heightmap plans only)");

@@ -305,16 +305,20 @@ __device__ __forceinline__ float terrain2d_density(const FieldDev& f, float py, 
   return -dy - n * f.p[1];
 }
 
+// The sphere-wave field with its x and z sines given.
+__device__ __forceinline__ float sphere_wave(const FieldDev& f, float px, float py, float pz, float sx, float sz) {
+  const float l = len3(px - f.p[0], py - f.p[1], pz - f.p[2]);
+  float s = sx * det_sin(f.p[5] * py);
+  s = s * sz;
+  return (l - f.p[3]) + f.p[4] * s;
+}
+
 __device__ __forceinline__ float eval_field(const FieldDev& f, const int* __restrict__ perm,
                                             const float4* __restrict__ gtab, float px, float py,
                                             float pz) {
   switch (f.kind) {
-    case BMF_FIELD_SPHERE_WAVE: {
-      const float l = len3(px - f.p[0], py - f.p[1], pz - f.p[2]);
-      float s = det_sin(f.p[5] * px) * det_sin(f.p[5] * py);
-      s = s * det_sin(f.p[5] * pz);
-      return (l - f.p[3]) + f.p[4] * s;
-    }
+    case BMF_FIELD_SPHERE_WAVE:
+      return sphere_wave(f, px, py, pz, det_sin(f.p[5] * px), det_sin(f.p[5] * pz));
     case BMF_FIELD_TERRAIN_FBM: {
       const int oct = (int)f.p[5];
       float sum = 0.0f, amp = 1.0f, fr = f.p[2];

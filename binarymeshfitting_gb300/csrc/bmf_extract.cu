@@ -1660,17 +1660,24 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
                                                                  MeshOut out) {
   __shared__ uint64_t s_tri[256], s_uses[256];
   __shared__ RTile s_tiles[kEmitWarps];
+  const int64_t n = min((int64_t)*ws.ccount, ws.clist_cap);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  RTile& R = s_tiles[warp];
+  const int64_t nwarps = (int64_t)gridDim.x * kEmitWarps;
+  // A short list (a chunk) is spread over the whole grid, few words per warp:
+  // a tile's time is the chain of its phases and rounds, whatever its size
+  // (33^3 chunk, ~300 busy words: 16 us as 16-word tiles on 19 warps).
+  const bool spread = n <= nwarps * (kTileWords / 2);
+  const int64_t tw = spread ? (n + nwarps - 1) / nwarps : kTileWords;
+  const int64_t w0 = spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * kEmitWarps + warp;
+  if ((spread ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kEmitWarps) * tw >= n) return;  // no warp has a tile
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
     s_tri[i] = __ldg(g_tri_cases + i);
     s_uses[i] = __ldg(g_edge_uses + i);
   }
   __syncthreads();
-  const int64_t n = min((int64_t)*ws.ccount, ws.clist_cap);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  RTile& R = s_tiles[warp];
-  const int64_t nwarps = (int64_t)gridDim.x * kEmitWarps;
-  for (int64_t t0 = ((int64_t)blockIdx.x * kEmitWarps + warp) * kTileWords; t0 < n; t0 += nwarps * kTileWords) {
-    const int nt = (int)min((int64_t)kTileWords, n - t0);
+  for (int64_t t0 = w0 * tw; t0 < n; t0 += nwarps * tw) {
+    const int nt = (int)min(tw, n - t0);
     // 1. the tile's words
     uint2 pb0 = make_uint2(0u, 0u);  // this lane's word: its plane's bases, the next plane's vertex base
     uint32_t pv1 = 0u;

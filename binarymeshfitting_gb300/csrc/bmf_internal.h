@@ -88,17 +88,18 @@ struct WordScratch {
   float c2d_g = 0.0f, c2d_height = 0.0f;
 };
 
-// Fill + label.  A terrain field of a single chunk goes through the line
-// kernel (k_fill_terrain) directly; batches pass their own item queue to
+// Fill + label.  A terrain field of a single chunk goes through the block or the
+// line kernel directly; batches pass their own item queue to
 // launch_fill_terrain.
-// cols (nullable, BMF_FIELD_TERRAIN_2D): the (x, z) column heights from
+// cols (BMF_FIELD_TERRAIN_2D needs it): the (x, z) column heights from
 // launch_columns2d, stored at chunk.words + x * dim + z (a chunk's dim^2
-// columns fit its words' span); without it the x-plane CTAs evaluate them.
+// columns fit its words' span).
 void launch_sample_label(const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units, int max_dim,
                          const FieldDev& field, const float* dens_in, float* dens_out, uint32_t* words,
                          uint32_t* flags, cudaStream_t st, const float* cols = nullptr);
 // The 2D heightmap's column heights of a batch into cols (layout above), over
-// items {chunk, first column} of columns2d_item() columns each.
+// items {chunk, first column} of columns2d_item() columns each (null: chunk 0's
+// columns in order).
 void launch_columns2d(const ChunkDev* d_chunks, const int2* d_items, int n_items, const FieldDev& field, float* cols,
                       cudaStream_t st);
 int columns2d_item();

@@ -28,40 +28,121 @@ constexpr int kColumnItem = 256;  // columns per k_columns2d CTA
 // flags bits: 1 = a word that is neither empty nor full, 2 = a full word,
 // 4 = an empty word.  contains_mesh = (f & 1) || ((f & 6) == 6), the
 // reference's mesh / negative / positive logic (DMCChunk.cpp:141-162).
+__device__ __forceinline__ uint32_t word_class(uint32_t w) { return (w != 0u && w != kFull) ? 1u : (w == kFull ? 2u : 4u); }
+
+// Fill + label of every field but the terrain FBM, and of a caller's grid (GRID:
+// densities read, not written): a CTA takes `lines` whole lines of an x-plane,
+// which are contiguous in memory.  Lanes take consecutive samples, so loads
+// and stores are whole 128-byte rows whatever the dim; a ballot gives 32
+// consecutive inside bits, the CTA's bit stream stays in shared memory, and each
+// occupancy word is cut out of it with a funnel shift (a line of 65 samples
+// is three words, the last of one bit).  Bound by HBM: 4 bytes per sample.
+// Runs of four samples per thread with a shared atomicOr each reached 1.5 TB/s
+// on a grid (512 x 65^3: 380 us).
+constexpr int kPlaneThreads = 256;
+constexpr int kPlaneUnroll = 8;  // rows in flight per warp
+
+template <bool GRID>
+__global__ void __launch_bounds__(kPlaneThreads) k_sample_plane(const ChunkDev* __restrict__ chunks, int n_chunks,
+                                                               const int* __restrict__ unit_start, FieldDev field,
+                                                               const float* __restrict__ dens_in,
+                                                               float* __restrict__ dens_out,
+                                                               uint32_t* __restrict__ words,
+                                                               uint32_t* __restrict__ flags,
+                                                               const float* __restrict__ cols, int lines) {
+  extern __shared__ uint32_t s_bits[];
+  // per z: the 2D heightmap's column height, or the sphere wave's sin(k z)
+  __shared__ float s_z[GRID ? 1 : kMaxColumn];
+  const int u = blockIdx.x;
+  const int c = find_chunk(unit_start, n_chunks, u);
+  const ChunkDev ch = chunks[c];
+  const int x = u - __ldg(unit_start + c), dim = ch.dim, zc = ch.zc;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float px = ch.ox + (float)x * ch.scale;
+  float sx = 0.0f;
+  if (!GRID) {
+    if (field.kind == BMF_FIELD_TERRAIN_2D) {
+      for (int z = threadIdx.x; z < dim; z += kPlaneThreads) s_z[z] = __ldg(cols + ch.words + (int64_t)x * dim + z);
+    } else if (field.kind == BMF_FIELD_SPHERE_WAVE) {
+      sx = det_sin(field.p[5] * px);
+      for (int z = threadIdx.x; z < dim; z += kPlaneThreads) s_z[z] = det_sin(field.p[5] * (ch.oz + (float)z * ch.scale));
+    }
+    __syncthreads();
+  }
+  // a sample's line from a multiply-high: exact while i * dim < 2^32
+  const uint64_t dmagic = ((1ull << 32) + (uint64_t)dim - 1u) / (uint64_t)dim;
+  uint32_t fl = 0u;
+  for (int y0 = blockIdx.y * lines; y0 < dim; y0 += gridDim.y * lines) {
+    const int nl = min(lines, dim - y0), ns = nl * dim, rows = (ns + 31) >> 5;
+    const int64_t base = ch.dens + ((int64_t)x * dim + y0) * dim;
+    for (int r0 = warp; r0 < rows; r0 += (kPlaneThreads / 32) * kPlaneUnroll) {
+      float v[kPlaneUnroll];
+#pragma unroll
+      for (int k = 0; k < kPlaneUnroll; ++k) {
+        const int i = (r0 + k * (kPlaneThreads / 32)) * 32 + lane;
+        v[k] = 0.0f;
+        if (i < ns) {
+          if (GRID) {
+            v[k] = __ldg(dens_in + base + i);
+          } else {
+            const int yl = (int)(((uint64_t)(uint32_t)i * dmagic) >> 32), z = i - yl * dim;
+            const float py = ch.oy + (float)(y0 + yl) * ch.scale;
+            if (field.kind == BMF_FIELD_TERRAIN_2D) {
+              v[k] = terrain2d_density(field, py, s_z[z]);
+            } else {
+              const float pz = ch.oz + (float)z * ch.scale;
+              if (field.kind == BMF_FIELD_SPHERE_WAVE)
+                v[k] = sphere_wave(field, px, py, pz, sx, s_z[z]);
+              else
+                v[k] = eval_field(field, nullptr, nullptr, px, py, pz);
+            }
+            if (dens_out) dens_out[base + i] = v[k];
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kPlaneUnroll; ++k) {
+        const int row = r0 + k * (kPlaneThreads / 32);
+        const uint32_t b = __ballot_sync(kFull, v[k] < 0.0f);
+        if (lane == 0 && row < rows) s_bits[row] = b;
+      }
+    }
+    if (threadIdx.x == 0) s_bits[rows] = 0u;  // the funnel shift may look one row further
+    __syncthreads();
+    uint32_t* wout = words + ch.words + ((int64_t)x * dim + y0) * zc;
+    for (int i = threadIdx.x; i < nl * zc; i += kPlaneThreads) {
+      const int yl = i / zc, z = 32 * (i - yl * zc), at = yl * dim + z, n = min(32, dim - z);
+      uint32_t w = __funnelshift_r(s_bits[at >> 5], s_bits[(at >> 5) + 1], at & 31);
+      if (n < 32) w &= (1u << n) - 1u;
+      wout[i] = w;
+      fl |= word_class(w);
+    }
+    __syncthreads();  // the next lines overwrite the stream
+  }
+  fl = __reduce_or_sync(kFull, fl);
+  if (lane == 0 && fl) atomicOr(flags + c, fl);
+}
+
+// The terrain FBM's x-plane fill (fill_mode 0 of a plan).
 __global__ void __launch_bounds__(256) k_sample_label(const ChunkDev* __restrict__ chunks, int n_chunks,
                                                       const int* __restrict__ unit_start, FieldDev field,
-                                                      const float* __restrict__ dens_in, float* __restrict__ dens_out,
-                                                      uint32_t* __restrict__ words, uint32_t* __restrict__ flags,
-                                                      const float* __restrict__ cols) {
+                                                      float* __restrict__ dens_out, uint32_t* __restrict__ words,
+                                                      uint32_t* __restrict__ flags) {
   extern __shared__ uint32_t sw[];
   __shared__ int perm2[512];
   __shared__ float4 gtab[512];
-  // BMF_FIELD_TERRAIN_2D: the height noise of the plane's (x, z) columns,
-  // evaluated here or (cols non-null) read from k_columns2d's output
-  __shared__ float s_col[kMaxColumn];
   const int u = blockIdx.x;
   const int c = find_chunk(unit_start, n_chunks, u);
   const ChunkDev ch = chunks[c];
   const int x = u - __ldg(unit_start + c);
   const int dim = ch.dim, zc = ch.zc;
   const int nw = dim * zc;
-  if (field.kind == BMF_FIELD_TERRAIN_FBM || field.kind == BMF_FIELD_TERRAIN_2D) {  // the noise tables
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-      perm2[i] = field.perm[i & 255];
-      gtab[i] = grad_coeffs(field.perm[i & 255]);
-    }
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {  // the noise tables
+    perm2[i] = field.perm[i & 255];
+    gtab[i] = grad_coeffs(field.perm[i & 255]);
   }
   for (int i = threadIdx.x; i < nw; i += blockDim.x) sw[i] = 0u;
   __syncthreads();
-  const bool col2d = field.kind == BMF_FIELD_TERRAIN_2D && dim <= kMaxColumn;
-  if (col2d) {  // one height evaluation per column, shared by the plane's dim samples of it
-    const float pxc = ch.ox + (float)x * ch.scale;
-    for (int z = threadIdx.x; z < dim; z += blockDim.x)
-      s_col[z] = cols ? __ldg(cols + ch.words + (int64_t)x * dim + z)
-                      : terrain2d_height(field, perm2, pxc, ch.oz + (float)z * ch.scale);
-    __syncthreads();
-  }
-
   // Work item = a run of kRun consecutive z-samples of one (x, y) line; runs
   // start at multiples of kRun (which divides 32), so a run's inside bits land
   // in a single occupancy word.
@@ -75,31 +156,15 @@ __global__ void __launch_bounds__(256) k_sample_label(const ChunkDev* __restrict
     const int n = min(kRun, dim - z0);
     const int64_t o = dbase + (int64_t)y * dim + z0;
     float v[kRun];
-    if (field.kind == BMF_FIELD_GRID) {
+    const float py = ch.oy + (float)y * ch.scale;
+    float pz[kRun];
+#pragma unroll
+    for (int k = 0; k < kRun; ++k) pz[k] = ch.oz + (float)(z0 + k) * ch.scale;
+    terrain_run(field, perm2, gtab, px, py, pz, n, v);
+    if (dens_out) {
 #pragma unroll
       for (int k = 0; k < kRun; ++k)
-        if (k < n) v[k] = __ldg(dens_in + o + k);
-    } else {
-      const float py = ch.oy + (float)y * ch.scale;
-      float pz[kRun];
-#pragma unroll
-      for (int k = 0; k < kRun; ++k) pz[k] = ch.oz + (float)(z0 + k) * ch.scale;
-      if (field.kind == BMF_FIELD_TERRAIN_FBM) {
-        terrain_run(field, perm2, gtab, px, py, pz, n, v);
-      } else if (col2d) {
-#pragma unroll
-        for (int k = 0; k < kRun; ++k)
-          if (k < n) v[k] = terrain2d_density(field, py, s_col[z0 + k]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < kRun; ++k)
-          if (k < n) v[k] = eval_field(field, perm2, gtab, px, py, pz[k]);
-      }
-      if (dens_out) {
-#pragma unroll
-        for (int k = 0; k < kRun; ++k)
-          if (k < n) dens_out[o + k] = v[k];
-      }
+        if (k < n) dens_out[o + k] = v[k];
     }
     uint32_t bits = 0u;
 #pragma unroll
@@ -108,20 +173,15 @@ __global__ void __launch_bounds__(256) k_sample_label(const ChunkDev* __restrict
     if (bits) atomicOr(&sw[y * zc + (z0 >> 5)], bits << (z0 & 31));
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
   uint32_t f = 0;
   uint32_t* wout = words + ch.words + (int64_t)x * nw;
   for (int i = threadIdx.x; i < nw; i += blockDim.x) {
     const uint32_t w = sw[i];
     wout[i] = w;
-    f |= (w != 0u && w != kFull) ? 1u : (w == kFull ? 2u : 4u);
+    f |= word_class(w);
   }
-  f |= __shfl_xor_sync(kFull, f, 16);
-  f |= __shfl_xor_sync(kFull, f, 8);
-  f |= __shfl_xor_sync(kFull, f, 4);
-  f |= __shfl_xor_sync(kFull, f, 2);
-  f |= __shfl_xor_sync(kFull, f, 1);
-  if (lane == 0 && f) atomicOr(flags + c, f);
+  f = __reduce_or_sync(kFull, f);
+  if ((threadIdx.x & 31) == 0 && f) atomicOr(flags + c, f);
 }
 
 // ---------------------------------------------------------------------------
@@ -675,7 +735,7 @@ __global__ void k_cell_masks(int dim, int zc, const uint32_t* __restrict__ W, ui
 
 // The 2D heightmap's (x, z) column heights of a batch, one thread per column
 // over items of kColumnItem consecutive columns of one chunk ({chunk, first
-// column}, column = x * dim + z), stored at chunk.words + column: every
+// column}, column = x * dim + z; items null: chunk 0's in order), stored at chunk.words + column: every
 // column is evaluated once, by a full CTA, instead of by the dim threads of
 // an x-plane's CTA while the rest wait.
 __global__ void __launch_bounds__(kColumnItem) k_columns2d(const ChunkDev* __restrict__ chunks,
@@ -684,7 +744,7 @@ __global__ void __launch_bounds__(kColumnItem) k_columns2d(const ChunkDev* __res
   __shared__ int perm2[512];
   for (int i = threadIdx.x; i < 512; i += blockDim.x) perm2[i] = field.perm[i & 255];
   __syncthreads();
-  const int2 it = items[blockIdx.x];
+  const int2 it = items ? items[blockIdx.x] : make_int2(0, (int)blockIdx.x * kColumnItem);
   const ChunkDev& ch = chunks[it.x];
   const int dim = ch.dim, col = it.y + (int)threadIdx.x;
   if (col >= dim * dim) return;
@@ -767,18 +827,130 @@ void launch_words2d(const ChunkDev* d_chunks, int n_chunks, const int* d_unit_st
                                                        flags);
 }
 
+// The fill of one terrain chunk (k_fill_block): a thread takes one run of a
+// line, so that a chunk gives enough threads for the whole GPU; the line kernel
+// (a thread walks its line) keeps lattice-cell state from run to run but has
+// 5 CTAs for a 33^3 chunk and 66 for a 129^3 one.  Up to kFillBlockMax samples
+// per axis the block form is the faster (whole call without sweeps, block / line:
+// 65^3 50 / 66 us, 97^3 64 / 77, 129^3 76 / 87, 161^3 98 / 100, 193^3 127 / 114;
+// runs of 16 per thread: 33^3 52 against 48).
+constexpr int kBlockRun = 8;                       // z-samples per thread
+constexpr int kBlockRuns = 32 / kBlockRun;         // runs of a word
+constexpr int kBlockThreads = 128, kBlockLines = kBlockThreads / kBlockRuns;
+constexpr int kFillBlockMax = 160;
+
+__global__ void __launch_bounds__(kBlockThreads) k_fill_block(const ChunkDev* __restrict__ chunks, FieldDev field,
+                                                             float* __restrict__ dens_out,
+                                                             uint32_t* __restrict__ words,
+                                                             uint32_t* __restrict__ flags) {
+  __shared__ int perm2[512];
+  __shared__ float4 gtab[512];
+  __shared__ float4 zt[kMaxOctaves * 32];  // {zf, zf - 1, fade(zf), Z} per octave and sample of the word
+  __shared__ uint32_t s_run[kBlockThreads];
+  for (int i = threadIdx.x; i < 512; i += kBlockThreads) {
+    perm2[i] = field.perm[i & 255];
+    gtab[i] = grad_coeffs(field.perm[i & 255]);
+  }
+  const ChunkDev ch = chunks[0];
+  const int dim = ch.dim, zc = ch.zc, zb = blockIdx.y;
+  const int oct = min((int)field.p[5], kMaxOctaves);
+  const float h0 = field.p[0], ampl = field.p[1], freq = field.p[2], lac = field.p[3], gain = field.p[4];
+  for (int e = threadIdx.x; e < oct * 32; e += kBlockThreads) {
+    float fr = freq;
+    for (int i = 0; i < e >> 5; ++i) fr = fr * lac;
+    const float pz = ch.oz + (float)(32 * zb + (e & 31)) * ch.scale;
+    const float zs = pz * fr;
+    const float fz = floorf(zs);
+    const float zf = zs - fz;
+    zt[e] = make_float4(zf, zf - 1.0f, fade(zf), __int_as_float(((int)fz) & 255));
+  }
+  __syncthreads();
+  // a warp's lanes are 32 lines of one run: z terms and lattice cells are
+  // the same for all of them
+  const int run = threadIdx.x / kBlockLines, l = threadIdx.x % kBlockLines;
+  const int line = blockIdx.x * kBlockLines + l, z0 = 32 * zb + run * kBlockRun, n = min(kBlockRun, dim - z0);
+  uint32_t bits = 0u;
+  if (line < dim * dim && n > 0) {
+    const int x = line / dim, y = line - x * dim;
+    const float px = ch.ox + (float)x * ch.scale, py = ch.oy + (float)y * ch.scale;
+    float sum[kBlockRun];
+#pragma unroll
+    for (int k = 0; k < kBlockRun; ++k) sum[k] = 0.0f;
+    float amp = 1.0f, fr = freq;
+#pragma unroll 1
+    for (int o = 0; o < oct; ++o) {
+      OctLine L;
+      oct_line_init(L, px, py, fr, perm2);
+      const float4* zo = zt + o * 32 + run * kBlockRun;
+#pragma unroll
+      for (int k = 0; k < kBlockRun; ++k) {  // (samples past the line's end are evaluated and dropped)
+        const float4 t = zo[k];
+        const int Z = __float_as_int(t.w);
+        if (Z != L.Zp) oct_line_cell(L, Z, gtab);
+        const float l0 = __fmaf_rn(L.b0, t.x, L.a0);
+        const float l1 = __fmaf_rn(L.b1, t.y, L.a1);
+        sum[k] = __fmaf_rn(amp, __fmaf_rn(t.z, l1 - l0, l0), sum[k]);
+      }
+      fr = fr * lac;
+      amp = amp * gain;
+    }
+    float* out = dens_out ? dens_out + ch.dens + (int64_t)line * dim + z0 : nullptr;
+#pragma unroll
+    for (int k = 0; k < kBlockRun; ++k) {
+      const float d = __fmaf_rn(-ampl, sum[k], py - h0);
+      if (k < n) {
+        if (out) out[k] = d;
+        if (d < 0.0f) bits |= 1u << k;
+      }
+    }
+  }
+  s_run[threadIdx.x] = bits << (run * kBlockRun);
+  __syncthreads();
+  uint32_t fl = 0u;
+  const int wline = blockIdx.x * kBlockLines + (int)threadIdx.x;
+  if (threadIdx.x < kBlockLines && wline < dim * dim) {
+    uint32_t w = 0u;
+#pragma unroll
+    for (int k = 0; k < kBlockRuns; ++k) w |= s_run[k * kBlockLines + threadIdx.x];
+    words[ch.words + (int64_t)wline * zc + zb] = w;
+    fl = word_class(w);
+  }
+  fl = __reduce_or_sync(kFull, fl);
+  if ((threadIdx.x & 31) == 0 && fl) atomicOr(flags, fl);
+}
+
 void launch_sample_label(const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units, int max_dim,
                          const FieldDev& field, const float* dens_in, float* dens_out, uint32_t* words,
                          uint32_t* flags, cudaStream_t st, const float* cols) {
-  if (field.kind == BMF_FIELD_TERRAIN_FBM && n_chunks == 1) {
-    launch_fill_terrain(16, d_chunks, nullptr, fill_terrain_items(max_dim), nullptr, 0, field, dens_out, words, flags,
-                        nullptr, st);
+  const int max_zc = (max_dim + 31) / 32;
+  if (field.kind == BMF_FIELD_TERRAIN_FBM) {
+    if (n_chunks == 1 && max_dim <= kFillBlockMax) {
+      const dim3 grid((max_dim * max_dim + kBlockLines - 1) / kBlockLines, max_zc);
+      k_fill_block<<<grid, kBlockThreads, 0, st>>>(d_chunks, field, dens_out, words, flags);
+    } else if (n_chunks == 1) {
+      launch_fill_terrain(16, d_chunks, nullptr, fill_terrain_items(max_dim), nullptr, 0, field, dens_out, words, flags,
+                          nullptr, st);
+    } else {
+      const size_t smem = (size_t)max_dim * max_zc * sizeof(uint32_t);
+      k_sample_label<<<n_units, 256, smem, st>>>(d_chunks, n_chunks, d_unit_start, field, dens_out, words, flags);
+    }
     return;
   }
-  const int max_zc = (max_dim + 31) / 32;
-  const size_t smem = (size_t)max_dim * max_zc * sizeof(uint32_t);
-  k_sample_label<<<n_units, 256, smem, st>>>(d_chunks, n_chunks, d_unit_start, field, dens_in, dens_out, words,
-                                             flags, field.kind == BMF_FIELD_TERRAIN_2D ? cols : nullptr);
+  // lines per CTA step: at most 16384 samples of bits, and parts of a plane
+  // where there are few planes
+  const int parts = n_units < 1024 ? min(8, (1024 + n_units - 1) / n_units) : 1;
+  int lines = (max_dim + parts - 1) / parts;
+  lines = max(1, min(lines, 16384 / max_dim));
+  const int steps = (max_dim + lines - 1) / lines;
+  lines = (max_dim + steps - 1) / steps;  // even steps
+  const size_t smem = sizeof(uint32_t) * (((size_t)lines * max_dim + 31) / 32 + 2);
+  const dim3 grid(n_units, parts);
+  if (field.kind == BMF_FIELD_GRID)
+    k_sample_plane<true><<<grid, kPlaneThreads, smem, st>>>(d_chunks, n_chunks, d_unit_start, field, dens_in, dens_out,
+                                                           words, flags, nullptr, lines);
+  else
+    k_sample_plane<false><<<grid, kPlaneThreads, smem, st>>>(d_chunks, n_chunks, d_unit_start, field, dens_in,
+                                                            dens_out, words, flags, cols, lines);
 }
 
 void launch_cell_masks(int dim, const uint32_t* W, uint8_t* masks, cudaStream_t st) {
