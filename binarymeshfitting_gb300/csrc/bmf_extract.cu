@@ -352,30 +352,13 @@ __global__ void __launch_bounds__(THREADS) k_count(const ChunkDev* __restrict__ 
       }
     }
     if (listing && __any_sync(kFull, act != 0u)) {
-      // one global reservation per warp; Mode R lists busy words, Mode Q
-      // each word's active cells in bit order
-      const int na = MODE == 0 ? (act != 0u ? 1 : 0) : __popc(act);
-      int incl = na;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl += v;
-      }
-      const int tot = __shfl_sync(kFull, incl, 31);
+      // one global reservation per warp for its busy words
+      const uint32_t busy = __ballot_sync(kFull, act != 0u);
       uint32_t wbase = 0u;
-      if (lane == 31 && tot) wbase = atomicAdd(ws.ccount, (uint32_t)tot);
-      wbase = __shfl_sync(kFull, wbase, 31);
-      if (act) {
-        int64_t slot = (int64_t)wbase + incl - na;
-        if (MODE == 0) {
-          if (slot < ws.clist_cap) ws.clist[slot] = make_uint2((uint32_t)c, (uint32_t)(x * nw + wi));
-        } else {
-          const uint32_t key0 = vertex_key(x, y, 32 * zb, 0);  // the cell as a vertex key (k = 0)
-          for (uint32_t m = act; m; m &= m - 1u, ++slot)
-            if (slot < ws.clist_cap)
-              ws.clist[slot] = make_uint2((uint32_t)c, key0 + ((uint32_t)(__ffs(m) - 1) << 2));
-        }
-      }
+      if (lane == 0) wbase = atomicAdd(ws.ccount, (uint32_t)__popc(busy));
+      wbase = __shfl_sync(kFull, wbase, 0);
+      const int64_t slot = (int64_t)wbase + __popc(busy & lane_lt(lane));
+      if (act && slot < ws.clist_cap) ws.clist[slot] = make_uint2((uint32_t)c, (uint32_t)(x * nw + wi));
     }
   }
   if (threadIdx.x == 0) ws.pb[u] = make_uint2(carry_v, carry_i);
@@ -712,7 +695,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
           // otherwise
           if (PLACE != 2 || !out.vkey) {
             float P[3];
-            q_place<PLACE>(D, dim, x, y, z, mask, g, P);
+            q_place<PLACE, false>(D, dim, x, y, z, group_edges(mask, g), P);
             out.pos[3 * gv] = P[0];
             out.pos[3 * gv + 1] = P[1];
             out.pos[3 * gv + 2] = P[2];
@@ -1919,109 +1902,266 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
   }
 }
 
-// Mode Q emission over the work list, one thread per active cell: the cell's
-// group vertices (ids from the word base and the group-count planes; mass
-// point / centre placed here, QEF by k_place_qef when keys are kept) and the
-// quads of the interior crossing edges its sample owns (slot from the word's
-// index base and the popcounts of the owned crossings below it) -- exactly
-// what k_emit<1,P> writes for the cell's lane.
+// Mode Q emission over the busy-word list, in the form of k_emit_words_r: a
+// warp stages the neighbourhoods of its words (the occupancy words of lines
+// (x-1..x+1, y-1..y+1) in blocks zb-1..zb+1, and the vertex base and group-count
+// planes of the cell lines (x-1..x, y-1..y) in blocks zb-1, zb), then writes one
+// lane per vertex (the k-th vertex group of a word, from its group-count
+// planes) and one lane per quad (the k-th interior crossing edge; its four
+// cells' masks, groups and vertex ids from the staged lines).  Issue-bound: 512 x
+// 65^3 fitting grids (3.9 M vertices) 352 us, 512 mixed terrain chunks 180 us; the
+// thread-per-cell form it replaces read each quad's four cells from global
+// memory behind bounds checks (512 x 65^3 fitting grids: 607 us).
+struct QTile {
+  uint32_t w[kTileWords][27];      // [i][j][b]: line (x-1+i, y-1+j), block zb-1+b
+  uint32_t cv[kTileWords][8][4];   // [2i+j][b]: cell line (x-1+i, y-1+j), block zb-1+b: vertex base, planes
+  uint32_t ib[kTileWords], X[kTileWords], Y[kTileWords], Z[kTileWords];
+  int x[kTileWords], y[kTileWords], zb[kTileWords], dim[kTileWords], zc[kTileWords];
+  int64_t cw[kTileWords], dens[kTileWords], vout[kTileWords], iout[kTileWords];
+  int voff[kTileWords + 1], qoff[kTileWords + 1];  // exclusive vertex / quad offsets of the tile's words
+};
+
+// Corner mask of the cell of line (x-1+i, y-1+j), i, j in {0, 1}, at bit zr in
+// [0, 64) of blocks zb-1, zb.
+__device__ __forceinline__ int qtile_mask(const uint32_t* w, int i, int j, int zr) {
+  int m = 0;
+  const int b = zr >> 5, l = zr & 31;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) {
+    const uint32_t* q = w + ((i + (d >> 1)) * 3 + j + (d & 1)) * 3 + b;
+    m |= (int)(__funnelshift_r(q[0], q[1], l) & 3u) << (2 * d);
+  }
+  return m;
+}
+
 template <int PLACE>
-__global__ void __launch_bounds__(256, 3) k_emit_cells_q(const ChunkDev* __restrict__ chunks,
-                                                         const uint32_t* __restrict__ words,
-                                                         const float* __restrict__ dens, WordScratch ws, MeshOut out) {
-  __shared__ SmemTabs T;
-  load_tabs(T);
+__global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const ChunkDev* __restrict__ chunks,
+                                                                 const uint32_t* __restrict__ words,
+                                                                 const float* __restrict__ dens, WordScratch ws,
+                                                                 MeshOut out) {
+  __shared__ uint64_t s_grp[256];
+  __shared__ QTile s_tiles[kEmitWarps];
   const int64_t n = min((int64_t)*ws.ccount, ws.clist_cap);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint2 ent = ws.clist[i];
-    const ChunkDev ch = chunks[ent.x];
-    const int dim = ch.dim, zc = ch.zc;
-    int x, y, z, k0;
-    vertex_key_decode(ent.y, x, y, z, k0);
-    const int zb = z >> 5, lane = z & 31;
-    const uint32_t lt = lane_lt(lane);
-    const uint32_t* W = words + ch.words;
-    const uint32_t* vbase = ws.vcnt + ch.words;
-    const uint2* pb = ws.pb + ch.unit0;
-    const float* D = dens + ch.dens;
-    const int64_t wo = ((int64_t)x * dim + y) * zc + zb;
-    const bool interior = x <= dim - 2 && y <= dim - 2 && z <= dim - 2;
-    const int mask = interior ? cell_mask_at(W, dim, zc, x, y, z) : 0;
-    const uint64_t gw = T.grp[mask];
-    const int ng = (int)((gw >> 48) & 0xF);
-    if (ng) {
-      const uint32_t* pl = ws.gpl + 3 * (ch.words + wo);
-      uint32_t vid = __ldg(&pb[x].x) + __ldg(vbase + wo) + __popc(__ldg(pl) & lt) +
-                     2 * __popc(__ldg(pl + 1) & lt) + 4 * __popc(__ldg(pl + 2) & lt);
-      const int nc = dim - 1;
-      const uint8_t bnd = (x == 0 || y == 0 || z == 0 || x == nc - 1 || y == nc - 1 || z == nc - 1);
-      for (int g = 0; g < ng; ++g, ++vid) {
-        const int64_t gv = ch.vout + vid;
-        if (gv >= out.vcap) continue;
-        if (PLACE != 2 || !out.vkey) {
-          float P[3];
-          q_place<PLACE>(D, dim, x, y, z, mask, g, P);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  QTile& R = s_tiles[warp];
+  const int64_t nwarps = (int64_t)gridDim.x * kEmitWarps;
+  const bool spread = n <= nwarps * (kTileWords / 2);  // (as k_emit_words_r)
+  const int64_t tw = spread ? (n + nwarps - 1) / nwarps : kTileWords;
+  const int64_t w0 = spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * kEmitWarps + warp;
+  if ((spread ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kEmitWarps) * tw >= n) return;  // no warp has a tile
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) s_grp[i] = __ldg(g_group_cases + i);
+  __syncthreads();
+  const bool idx16 = (((uintptr_t)out.idx | (uintptr_t)out.idx_global) & 15) == 0;  // quads as 16-byte stores
+  for (int64_t t0 = w0 * tw; t0 < n; t0 += nwarps * tw) {
+    const int nt = (int)min(tw, n - t0);
+    // 1. the tile's words
+    uint2 pb1 = make_uint2(0u, 0u);  // this lane's word: its plane's bases, and the previous plane's vertex base
+    uint32_t pv0 = 0u;
+    if (lane < nt) {
+      const uint2 e = ws.clist[t0 + lane];
+      const ChunkDev& ch = chunks[e.x];
+      const int dim = ch.dim, zc = ch.zc, wi = (int)e.y;
+      const int xy = wi / zc;
+      R.zb[lane] = wi - xy * zc;
+      R.y[lane] = xy % dim;
+      R.x[lane] = xy / dim;
+      R.dim[lane] = dim;
+      R.zc[lane] = zc;
+      const uint2* pb = ws.pb + ch.unit0 + R.x[lane];
+      pb1 = __ldg(pb);
+      if (R.x[lane] > 0) pv0 = __ldg(&pb[-1].x);
+      R.cw[lane] = ch.words;
+      R.dens[lane] = ch.dens;
+      R.vout[lane] = ch.vout;
+      R.iout[lane] = ch.iout;
+    }
+    __syncwarp();
+    // 2. stage the neighbourhoods (zeros outside the chunk)
+    for (int k = lane; k < nt * 9; k += 32) {
+      const int t = k / 9, l = k - 9 * t, i = l / 3, j = l - 3 * i;
+      const int dim = R.dim[t], zc = R.zc[t], zb = R.zb[t];
+      const int xx = R.x[t] - 1 + i, yy = R.y[t] - 1 + j;
+      uint32_t* dst = R.w[t] + l * 3;
+      if (xx < 0 || yy < 0 || xx >= dim || yy >= dim) {
+        dst[0] = dst[1] = dst[2] = 0u;
+      } else {
+        const uint32_t* L = words + R.cw[t] + (xx * dim + yy) * zc + zb;
+        if (zb > 0) stage_async(dst, L - 1); else dst[0] = 0u;
+        stage_async(dst + 1, L);
+        if (zb + 1 < zc) stage_async(dst + 2, L + 1); else dst[2] = 0u;
+      }
+    }
+    for (int k = lane; k < nt * 8; k += 32) {
+      const int t = k >> 3, l = k & 7, b = l & 1;
+      const int dim = R.dim[t], zc = R.zc[t], zb = R.zb[t] - 1 + b;
+      const int xx = R.x[t] - 1 + (l >> 2), yy = R.y[t] - 1 + ((l >> 1) & 1);
+      if (xx < 0 || yy < 0 || zb < 0) continue;  // no cell there: never read
+      const int64_t wi = R.cw[t] + (xx * dim + yy) * zc + zb;
+      uint32_t* dst = R.cv[t][l];
+      stage_async(dst, ws.vcnt + wi);
+      stage_async(dst + 1, ws.gpl + 3 * wi);
+      stage_async(dst + 2, ws.gpl + 3 * wi + 1);
+      stage_async(dst + 3, ws.gpl + 3 * wi + 2);
+    }
+    if (lane < nt) {
+      const int64_t wi = R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane];
+      stage_async(&R.ib[lane], ws.icnt + wi);
+    }
+    stage_wait();
+    __syncwarp();
+    // 3. per word: its interior crossings (quads), vertex and quad counts,
+    // scanned over the tile in one word (vertices low, quads high)
+    {
+      uint32_t packed = 0u;
+      if (lane < nt) {
+        const uint32_t* w = R.w[lane];
+        const int dim = R.dim[lane], x = R.x[lane], y = R.y[lane], zb = R.zb[lane];
+        const uint32_t wc = w[13];  // line (x, y), block zb
+        const bool xi = x >= 1 && x <= dim - 2, yi = y >= 1 && y <= dim - 2;
+        const uint32_t zu = zbits_upto(dim - 2, zb), zi = zb == 0 ? zu & ~1u : zu;
+        const uint32_t X = (yi && x + 1 < dim) ? (wc ^ w[22]) & zi : 0u;
+        const uint32_t Y = (xi && y + 1 < dim) ? (wc ^ w[16]) & zi : 0u;
+        const uint32_t Z = (xi && yi) ? (wc ^ ((wc >> 1) | (w[14] << 31))) & zu : 0u;
+        R.X[lane] = X;
+        R.Y[lane] = Y;
+        R.Z[lane] = Z;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          R.cv[lane][b][0] += pv0;
+          R.cv[lane][4 + b][0] += pb1.x;
+        }
+        R.ib[lane] += pb1.y;
+        const uint32_t* own = R.cv[lane][7];
+        const uint32_t nv = __popc(own[1]) + 2u * __popc(own[2]) + 4u * __popc(own[3]);
+        packed = nv | ((__popc(X) + __popc(Y) + __popc(Z)) << 16);  // at most 128 and 96 per word
+      }
+      uint32_t incl = packed;
+#pragma unroll
+      for (int o = 1; o < kTileWords; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane < kTileWords) {
+        R.voff[lane + 1] = (int)(incl & 0xFFFFu);
+        R.qoff[lane + 1] = (int)(incl >> 16);
+      }
+      if (lane == 0) R.voff[0] = R.qoff[0] = 0;
+    }
+    __syncwarp();
+    // 4. one lane per vertex: the k-th vertex of word t is in the cell l whose
+    // preceding cells hold k or fewer (count planes), its (k - that)-th group
+    const int nvt = R.voff[nt];
+    for (int jb = 0; jb < nvt; jb += 32) {
+      const int j = jb + lane;
+      bool in = j < nvt;
+      const int t = tile_word(R.voff, nt, in ? j : 0);
+      const int k = in ? j - R.voff[t] : 0;
+      const uint32_t* own = R.cv[t][7];
+      const uint32_t c0 = own[1], c1 = own[2], c2 = own[3];
+      int l = 0;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t m = lane_lt(l + s);
+        if ((int)(__popc(c0 & m) + 2 * __popc(c1 & m) + 4 * __popc(c2 & m)) <= k) l += s;
+      }
+      const uint32_t lt = lane_lt(l);
+      const int g = k - (int)(__popc(c0 & lt) + 2 * __popc(c1 & lt) + 4 * __popc(c2 & lt));
+      const int64_t gv = R.vout[t] + (int64_t)own[0] + k;
+      in = in && gv < out.vcap;
+      const int dim = R.dim[t], x = R.x[t], y = R.y[t], z = 32 * R.zb[t] + l;
+      const uint32_t edges = in ? group_edges(qtile_mask(R.w[t], 1, 1, 32 + l), g & 3) : 0u;
+      if (PLACE != 2 || !out.vkey) {
+        float P[3];
+        q_place<PLACE, true>(dens + R.dens[t], dim, x, y, z, edges, P);
+        if (in) {
           out.pos[3 * gv] = P[0];
           out.pos[3 * gv + 1] = P[1];
           out.pos[3 * gv + 2] = P[2];
         }
+      }
+      if (in) {
         if (out.nrm) { out.nrm[3 * gv] = 0.0f; out.nrm[3 * gv + 1] = 0.0f; out.nrm[3 * gv + 2] = 0.0f; }
-        if (out.boundary) out.boundary[gv] = bnd;
+        // cells run to dim - 2
+        if (out.boundary)
+          out.boundary[gv] = (x == 0 || y == 0 || z == 0 || x == dim - 2 || y == dim - 2 || z == dim - 2);
         if (out.vkey) out.vkey[gv] = vertex_key(x, y, z, g);
         if (out.valence) {
-          int val = 0;
-          for (int e = 0; e < 12; ++e) {
-            if ((int)((gw >> (4 * e)) & 0xF) != g) continue;
-            const int c0 = edge_c0(e);
-            val += q_edge_interior(dim, x + ((c0 >> 2) & 1), y + ((c0 >> 1) & 1), z + (c0 & 1), e >> 2);
-          }
-          out.valence[gv] = (uint8_t)val;
+          // the group's edges whose four cells exist (q_edge_interior)
+          uint32_t in12 = 0xFFFu;
+          const auto cut = [&](bool has, uint32_t m) { if (!has) in12 &= ~m; };
+          cut(x > 0, 0x330u);          // y-edges 4, 5 and z-edges 8, 9 at dx = 0
+          cut(x + 1 <= dim - 2, 0xCC0u);  // 6, 7, 10, 11 at dx = 1
+          cut(y > 0, 0x503u);          // x-edges 0, 1 and z-edges 8, 10 at dy = 0
+          cut(y + 1 <= dim - 2, 0xA0Cu);  // 2, 3, 9, 11 at dy = 1
+          cut(z > 0, 0x055u);          // x-edges 0, 2 and y-edges 4, 6 at dz = 0
+          cut(z + 1 <= dim - 2, 0x0AAu);  // 1, 3, 5, 7 at dz = 1
+          out.valence[gv] = (uint8_t)__popc(edges & in12);
         }
       }
+      __syncwarp();
     }
-    uint32_t Xi, Yi, Zi;
-    q_quad_words(W, dim, zc, x, y, zb, Xi, Yi, Zi);
-    const int own = (int)(((Xi >> lane) & 1u) | (((Yi >> lane) & 1u) << 1) | (((Zi >> lane) & 1u) << 2));
-    if (!own) continue;
-    int64_t gi = ch.iout + (int64_t)(__ldg(&pb[x].y) + __ldg(ws.icnt + ch.words + wo)) +
-                 4 * (int64_t)(__popc(Xi & lt) + __popc(Yi & lt) + __popc(Zi & lt));
-    const bool in0 = ((word_at(W, dim, zc, x, y, zb) >> lane) & 1u) != 0u;
-    for (int a = 0; a < 3; ++a) {
-      if (!((own >> a) & 1)) continue;
-      const int b = (a + 1) % 3, cax = (a + 2) % 3;
+    // 5. one lane per quad: the k-th interior crossing of word t
+    const int nqt = R.qoff[nt];
+    for (int j = lane; j < nqt; j += 32) {
+      const int t = tile_word(R.qoff, nt, j);
+      const int k = j - R.qoff[t];
+      const uint32_t X = R.X[t], Y = R.Y[t], Z = R.Z[t];
+      int l = 0;
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t m = lane_lt(l + s);
+        if ((int)(__popc(X & m) + __popc(Y & m) + __popc(Z & m)) <= k) l += s;
+      }
+      const uint32_t lt = lane_lt(l);
+      const int r = k - (int)(__popc(X & lt) + __popc(Y & lt) + __popc(Z & lt));
+      uint32_t ownb = ((X >> l) & 1u) | (((Y >> l) & 1u) << 1) | (((Z >> l) & 1u) << 2);
+      if (r >= 1) ownb &= ownb - 1u;
+      if (r >= 2) ownb &= ownb - 1u;
+      const int a = __ffs(ownb) - 1;
+      const uint32_t* w = R.w[t];
       uint32_t q[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int ob = (k == 0 || k == 3) ? -1 : 0, oc = (k < 2) ? -1 : 0;
-        int cc[3] = {x, y, z};
-        cc[b] += ob;
-        cc[cax] += oc;
-        int lo[3] = {0, 0, 0};
-        lo[b] = -ob;
-        lo[cax] = -oc;
-        const int e = a == 0 ? 2 * lo[1] + lo[2] : (a == 1 ? 4 + 2 * lo[0] + lo[2] : 8 + 2 * lo[0] + lo[1]);
-        const int cm = cell_mask_at(W, dim, zc, cc[0], cc[1], cc[2]);
-        q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, pb, dim, zc, cc[0], cc[1], cc[2]) +
-               (uint32_t)((T.grp[cm] >> (4 * e)) & 0xF);
+      for (int c = 0; c < 4; ++c) {
+        // cell at (b, c) offsets (-1,-1), (0,-1), (0,0), (-1,0) of axes a + 1, a + 2; lb, lc: the edge's place in it
+        const int lb = (c == 0 || c == 3) ? 1 : 0, lc = c < 2 ? 1 : 0;
+        const int dx = a == 0 ? 0 : (a == 1 ? lc : lb), dy = a == 0 ? lb : (a == 1 ? 0 : lc);
+        const int dz = a == 0 ? lc : (a == 1 ? lb : 0);
+        const int e = a == 0 ? 2 * dy + dz : (a == 1 ? 4 + 2 * dx + dz : 8 + 2 * dx + dy);
+        const int i = 1 - dx, jj = 1 - dy, zr = 32 + l - dz;
+        const int m = qtile_mask(w, i, jj, zr);
+        const uint32_t* cv = R.cv[t][(i * 2 + jj) * 2 + (zr >> 5)];
+        const uint32_t ct = lane_lt(zr & 31);
+        q[c] = cv[0] + __popc(cv[1] & ct) + 2 * __popc(cv[2] & ct) + 4 * __popc(cv[3] & ct) +
+               (uint32_t)((s_grp[m] >> (4 * e)) & 0xF);
       }
-      if (!in0) {
-        const uint32_t t = q[1];
+      if (!((w[13] >> l) & 1u)) {  // lower sample outside: reversed
+        const uint32_t v = q[1];
         q[1] = q[3];
-        q[3] = t;
+        q[3] = v;
       }
+      const int64_t gi = R.iout[t] + (int64_t)R.ib[t] + 4 * (int64_t)k;
+      const uint32_t vo = (uint32_t)R.vout[t];
+      if (idx16 && gi + 4 <= out.icap) {
+        *reinterpret_cast<uint4*>(out.idx + gi) = make_uint4(q[0], q[1], q[2], q[3]);
+        if (out.idx_global)
+          *reinterpret_cast<uint4*>(out.idx_global + gi) = make_uint4(q[0] + vo, q[1] + vo, q[2] + vo, q[3] + vo);
+      } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k, ++gi)
-        if (gi < out.icap) {
-          out.idx[gi] = q[k];
-          if (out.idx_global) out.idx_global[gi] = (uint32_t)(ch.vout + q[k]);
-        }
+        for (int c = 0; c < 4; ++c)
+          if (gi + c < out.icap) {
+            out.idx[gi + c] = q[c];
+            if (out.idx_global) out.idx_global[gi + c] = q[c] + vo;
+          }
+      }
     }
+    __syncwarp();  // the next tile overwrites the stage
   }
 }
 
 // Mode Q QEF placement, one thread per vertex (dense lanes, unlike the
 // warp-per-word emit where only surface cells' lanes work): the same
 // q_place<2> on the vertex's cell and group, decoded from its key.
+template <bool RECORD>
 __global__ void __launch_bounds__(128) k_place_qef(const ChunkDev* __restrict__ chunks, int n_chunks,
                                                    const uint32_t* __restrict__ words, const float* __restrict__ dens,
                                                    const uint32_t* __restrict__ vkey,
@@ -2029,37 +2169,68 @@ __global__ void __launch_bounds__(128) k_place_qef(const ChunkDev* __restrict__ 
                                                    float* __restrict__ pos, uint8_t* __restrict__ qflag,
                                                    uint32_t* __restrict__ qlist, uint32_t* __restrict__ qcount,
                                                    float* __restrict__ qseed) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= min(vcap, d_counts[0])) return;
-  const int c = find_chunk_by_vertex(chunks, n_chunks, v);
-  const ChunkDev ch = chunks[c];
-  const int dim = ch.dim;
-  int x, y, z, g;
-  vertex_key_decode(vkey[v], x, y, z, g);
-  const int mask = cell_mask_at(words + ch.words, dim, ch.zc, x, y, z);
-  float P[3];
-  if (qflag) {
-    // record the branch, and for a QEF-placed vertex its FP32 eigenvectors
-    // (the seeds of the wide adjoint), in the list of QEF-placed vertices
+  const int64_t nv = min(vcap, d_counts[0]);
+  for (int64_t v0 = (int64_t)blockIdx.x * blockDim.x; v0 < nv; v0 += (int64_t)gridDim.x * blockDim.x) {
+    const bool in = v0 + threadIdx.x < nv;
+    const int64_t v = in ? v0 + threadIdx.x : nv - 1;
+    const ChunkDev& ch = chunks[find_chunk_by_vertex(chunks, n_chunks, v)];
+    const int dim = ch.dim;
+    int x, y, z, g;
+    vertex_key_decode(vkey[v], x, y, z, g);
+    const uint32_t edges = in ? group_edges(cell_mask_at(words + ch.words, dim, ch.zc, x, y, z), g) : 0u;
+    float P[3];
     QefSolveInfo info;
     bool used = false;
-    q_place<2>(dens + ch.dens, dim, x, y, z, mask, g, P, &info, &used);
-    qflag[v] = used ? 1 : 0;
-    if (used) {
-      const uint32_t k = atomicAdd(qcount, 1u);
-      qlist[k] = (uint32_t)v;
+    q_place<2, true>(dens + ch.dens, dim, x, y, z, edges, P, RECORD ? &info : nullptr, RECORD ? &used : nullptr);
+    if (RECORD) {
+      // record the branch, and for a QEF-placed vertex its FP32 eigenvectors
+      // (the seeds of the wide adjoint), in the list of QEF-placed vertices:
+      // one reservation per warp
+      __syncwarp();
+      const uint32_t take = __ballot_sync(kFull, used);
+      uint32_t base = 0u;
+      if ((threadIdx.x & 31) == 0 && take) base = atomicAdd(qcount, (uint32_t)__popc(take));
+      base = __shfl_sync(kFull, base, 0);
+      if (in) qflag[v] = used ? 1 : 0;
+      if (used) {
+        const uint32_t k = base + __popc(take & lane_lt(threadIdx.x & 31));
+        qlist[k] = (uint32_t)v;
 #pragma unroll
-      for (int r = 0; r < 3; ++r) {
+        for (int r = 0; r < 3; ++r) {
 #pragma unroll
-        for (int c3 = 0; c3 < 3; ++c3) qseed[9 * (int64_t)k + 3 * r + c3] = info.V[r][c3];
+          for (int c3 = 0; c3 < 3; ++c3) qseed[9 * (int64_t)k + 3 * r + c3] = info.V[r][c3];
+        }
       }
     }
-  } else {
-    q_place<2>(dens + ch.dens, dim, x, y, z, mask, g, P);
+    if (in) {
+      pos[3 * v] = P[0];
+      pos[3 * v + 1] = P[1];
+      pos[3 * v + 2] = P[2];
+    }
+    __syncwarp();
   }
-  pos[3 * v] = P[0];
-  pos[3 * v + 1] = P[1];
-  pos[3 * v + 2] = P[2];
+}
+
+static void launch_place_qef(const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, const float* dens,
+                             const MeshOut& out, const int64_t* d_counts, cudaStream_t st) {
+  // persistent: as many CTAs as are resident, whatever the arena's capacity
+  static std::atomic<int> grid[64] = {};
+  const int g = per_device_once(grid, [](int dev) {
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_place_qef<true>, 128, 0);
+    return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+  });
+  const int64_t need = (out.vcap + 127) / 128;
+  const int blocks = (int)(need < g ? need : g);
+  if (out.qflag) {
+    cudaMemsetAsync(out.qcount, 0, sizeof(uint32_t), st);
+    k_place_qef<true><<<blocks, 128, 0, st>>>(d_chunks, n_chunks, words, dens, out.vkey, d_counts, out.vcap, out.pos,
+                                              out.qflag, out.qlist, out.qcount, out.qseed);
+  } else {
+    k_place_qef<false><<<blocks, 128, 0, st>>>(d_chunks, n_chunks, words, dens, out.vkey, d_counts, out.vcap, out.pos,
+                                               nullptr, nullptr, nullptr, nullptr);
+  }
 }
 
 int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start,
@@ -2078,18 +2249,19 @@ int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks,
   } else if (mode == 0) {
     k_emit<0, 0><<<n_units, 256, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, dens, flags, ws, out);
   } else if (ws.clist) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static std::atomic<int> grid[64] = {};  // persistent: one wave of resident CTAs
+    const int g = per_device_once(grid, [](int dev) {
+      int sms = 0, per_sm = 0;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_emit_words_q<1>, 32 * kEmitWarps, 0);
+      return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+    });
     if (placement == 2 && (!out.vkey || !d_counts)) out.vkey = nullptr;
-    if (placement == 0) k_emit_cells_q<0><<<sms * 8, 256, 0, st>>>(d_chunks, words, dens, ws, out);
-    else if (placement == 1) k_emit_cells_q<1><<<sms * 8, 256, 0, st>>>(d_chunks, words, dens, ws, out);
-    else k_emit_cells_q<2><<<sms * 8, 256, 0, st>>>(d_chunks, words, dens, ws, out);
+    if (placement == 0) k_emit_words_q<0><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
+    else if (placement == 1) k_emit_words_q<1><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
+    else k_emit_words_q<2><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
     if (placement == 2 && out.vkey && out.vcap > 0) {
-      if (out.qflag) cudaMemsetAsync(out.qcount, 0, sizeof(uint32_t), st);
-      k_place_qef<<<(int)((out.vcap + 127) / 128), 128, 0, st>>>(d_chunks, n_chunks, words, dens, out.vkey, d_counts,
-                                                                out.vcap, out.pos, out.qflag, out.qlist, out.qcount,
-                                                                out.qseed);
+      launch_place_qef(d_chunks, n_chunks, words, dens, out, d_counts, st);
       return 2;
     }
   } else if (placement == 0) {
@@ -2100,10 +2272,7 @@ int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks,
     if (!out.vkey || !d_counts) out.vkey = nullptr;  // no keys: the emit places in place
     k_emit<1, 2><<<n_units, 256, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, dens, flags, ws, out);
     if (out.vkey && out.vcap > 0) {
-      if (out.qflag) cudaMemsetAsync(out.qcount, 0, sizeof(uint32_t), st);
-      k_place_qef<<<(int)((out.vcap + 127) / 128), 128, 0, st>>>(d_chunks, n_chunks, words, dens, out.vkey, d_counts,
-                                                                out.vcap, out.pos, out.qflag, out.qlist, out.qcount,
-                                                                out.qseed);
+      launch_place_qef(d_chunks, n_chunks, words, dens, out, d_counts, st);
       return 2;
     }
   }

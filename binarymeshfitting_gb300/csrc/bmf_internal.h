@@ -59,12 +59,10 @@ struct WordScratch {
   uint32_t* icnt;   // indices of the x-plane's words before this one; Mode R's emit replaces it by the word's
                     // chunk-local primitive base, which the adjacency reads
   uint32_t* gpl;    // 3 bit-planes of the per-cell triangle (Mode R) / vertex-group (Mode Q) count
-  // Work list (nullable), in no particular order; *ccount (zeroed before the
-  // count kernel) entries, at most clist_cap kept.  Mode R: every busy word
-  // (one whose cells own a crossing or emit triangles) as {chunk, word index
-  // in the chunk}; Mode Q: every cell that holds vertex groups or owns an
-  // interior crossing, as {chunk, vertex_key(x, y, z, 0)}.  Either way its size
-  // bound is vcap + icap / prim_size + 1.
+  // Work list (nullable) of the busy words (those that own a vertex or emit a
+  // primitive) as {chunk, word index in the chunk}, in no particular order;
+  // *ccount (zeroed before the count kernel) entries, at most clist_cap kept:
+  // vcap + icap / prim_size + 1 suffice.
   uint2* clist;
   uint32_t* ccount;
   int64_t clist_cap;

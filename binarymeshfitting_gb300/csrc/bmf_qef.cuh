@@ -25,18 +25,36 @@ __device__ __forceinline__ float dens_at(const float* D, int dim, int x, int y, 
   return __ldg(D + ((int64_t)x * dim + y) * dim + z);
 }
 
-// Central-difference grid gradient, one-sided at the chunk faces.
-__device__ __forceinline__ void grid_gradient(const float* D, int dim, int x, int y, int z, float g[3]) {
-  const int c[3] = {x, y, z};
+// Central-difference grid gradient at sample (x, y, z), at offset o of the
+// chunk's densities (at most 2^27 of them), one-sided at the chunk faces.
+__device__ __forceinline__ void grid_gradient(const float* __restrict__ D, int dim, int x, int y, int z, int o,
+                                              float g[3]) {
+  const int c[3] = {x, y, z}, st[3] = {dim * dim, dim, 1};
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    int lo[3] = {x, y, z}, hi[3] = {x, y, z};
-    float h = 0.5f;
-    if (c[a] > 0) lo[a]--; else h = 1.0f;
-    if (c[a] < dim - 1) hi[a]++; else h = 1.0f;
-    g[a] = (dens_at(D, dim, hi[0], hi[1], hi[2]) - dens_at(D, dim, lo[0], lo[1], lo[2])) * h;
+    const bool lo = c[a] > 0, hi = c[a] < dim - 1;
+    const float h = lo && hi ? 0.5f : 1.0f;
+    g[a] = (__ldg(D + (o + (hi ? st[a] : 0))) - __ldg(D + (o - (lo ? st[a] : 0)))) * h;
   }
 }
+
+// Per corner mask and vertex group (four per mask): the group's edges as a
+// 12-bit set.
+struct GroupEdges {
+  uint16_t w[1024];
+};
+constexpr GroupEdges make_group_edges() {
+  constexpr uint64_t grp[256] = BMF_GROUP_CASES_INIT;
+  GroupEdges r{};
+  for (int m = 0; m < 256; ++m)
+    for (int e = 0; e < 12; ++e) {
+      const int g = (int)((grp[m] >> (4 * e)) & 0xFu);
+      if (g < 4) r.w[4 * m + g] |= (uint16_t)(1u << e);
+    }
+  return r;
+}
+static __device__ const GroupEdges g_group_edges = make_group_edges();
+__device__ __forceinline__ uint32_t group_edges(int mask, int g) { return __ldg(&g_group_edges.w[4 * mask + g]); }
 
 // QEF solve, restating qef_simd.h:150-579 lane by lane in FP32 with the exact
 // 1/sqrt in place of _mm_rsqrt_ps.
@@ -194,12 +212,18 @@ struct QefAccum {
 };
 
 // Crossing point (and hermite normal) of edge e of cell (x, y, z).
-__device__ __forceinline__ void hermite(const float* D, int dim, int x, int y, int z, int e, bool want_n, float p[3],
-                                        float n[3]) {
-  const int ca = edge_c0(e), cb = edge_c1(e);
+__device__ __forceinline__ void hermite(const float* __restrict__ D, int dim, int x, int y, int z, int e, bool want_n,
+                                        float p[3], float n[3]) {
+  const int ca = edge_c0(e), ax = e >> 2;
   const int a0[3] = {x + ((ca >> 2) & 1), y + ((ca >> 1) & 1), z + (ca & 1)};
-  const int a1[3] = {x + ((cb >> 2) & 1), y + ((cb >> 1) & 1), z + (cb & 1)};
-  const float s0 = dens_at(D, dim, a0[0], a0[1], a0[2]), s1 = dens_at(D, dim, a1[0], a1[1], a1[2]);
+  const int a1[3] = {a0[0] + (ax == 0), a0[1] + (ax == 1), a0[2] + (ax == 2)};
+  const int o0 = (a0[0] * dim + a0[1]) * dim + a0[2], o1 = o0 + (ax == 0 ? dim * dim : (ax == 1 ? dim : 1));
+  const float s0 = __ldg(D + o0), s1 = __ldg(D + o1);
+  float g0[3], g1[3];
+  if (want_n) {  // (loads in flight together with the samples')
+    grid_gradient(D, dim, a0[0], a0[1], a0[2], o0, g0);
+    grid_gradient(D, dim, a1[0], a1[1], a1[2], o1, g1);
+  }
   const float mu = (0.0f - s0) / (s1 - s0);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -207,9 +231,7 @@ __device__ __forceinline__ void hermite(const float* D, int dim, int x, int y, i
     p[k] = dv + (float)a0[k];
   }
   if (want_n) {
-    float g0[3], g1[3], g[3];
-    grid_gradient(D, dim, a0[0], a0[1], a0[2], g0);
-    grid_gradient(D, dim, a1[0], a1[1], a1[2], g1);
+    float g[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) g[k] = g0[k] + (g1[k] - g0[k]) * mu;
     const float l2 = (g[0] * g[0] + g[1] * g[1]) + g[2] * g[2];
@@ -219,12 +241,17 @@ __device__ __forceinline__ void hermite(const float* D, int dim, int x, int y, i
   }
 }
 
+// Position of the vertex of the cell's edges `edges` (group_edges), taken in
+// ascending order: each lane walks its own set, so that a warp runs as many
+// rounds as its longest list, not the union of the lists over twelve edges.
+// WARP: all lanes of the warp call it (edges = 0: nothing is placed) and leave
+// the walk together.
 // info / qef_used (optional, QEF placement): the solve's eigen data and
 // whether the vertex took the QEF branch (a successful solve inside the cell)
 // -- what the QEF adjoint needs from the forward.
-template <int PLACE>
-__device__ __forceinline__ void q_place(const float* D, int dim, int x, int y, int z, int mask, int g, float out[3],
-                                        QefSolveInfo* info = nullptr, bool* qef_used = nullptr) {
+template <int PLACE, bool WARP>
+__device__ __forceinline__ void q_place(const float* __restrict__ D, int dim, int x, int y, int z, uint32_t edges,
+                                        float out[3], QefSolveInfo* info = nullptr, bool* qef_used = nullptr) {
   if (PLACE == 0) {
     out[0] = (float)x + 0.5f;
     out[1] = (float)y + 0.5f;
@@ -232,17 +259,20 @@ __device__ __forceinline__ void q_place(const float* D, int dim, int x, int y, i
     return;
   }
   float mp[3] = {0.0f, 0.0f, 0.0f};
-  int cnt = 0;
+  const int cnt = __popc(edges);
   QefAccum q;
   if (PLACE == 2) q.init();
-  for (int e = 0; e < 12; ++e) {
-    if (group_of(mask, e) != g) continue;
+#pragma unroll 1
+  for (uint32_t em = edges; em; em &= em - 1u) {
     float p[3], n[3];
-    hermite(D, dim, x, y, z, e, PLACE == 2, p, n);
+    hermite(D, dim, x, y, z, __ffs(em) - 1, PLACE == 2, p, n);
 #pragma unroll
     for (int k = 0; k < 3; ++k) mp[k] = mp[k] + p[k];
-    ++cnt;
     if (PLACE == 2) q.add(p, n);
+  }
+  if (WARP) {
+    __syncwarp();
+    if (!edges) return;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) mp[k] = mp[k] / (float)cnt;
@@ -425,16 +455,6 @@ __device__ void eig3_refine(const R A[3][3], const float V0[3][3], R w[3], R V[3
   }
 #pragma unroll
   for (int i = 0; i < 3; ++i) w[i] = B[i][i];
-}
-
-// The edges of cell-mask group g as a 12-bit set.  The adjoint loops walk
-// it in ascending edge order (the order of the forward's accumulation): each
-// lane runs only its own vertex's edges, not the union of the warp's.
-__device__ __forceinline__ uint32_t group_edges(int mask, int g) {
-  uint32_t m = 0u;
-#pragma unroll
-  for (int e = 0; e < 12; ++e) m |= (group_of(mask, e) == g ? 1u : 0u) << e;
-  return m;
 }
 
 // LIST = 0: every vertex; 1: every vertex, but QEF-placed ones are only
