@@ -1476,9 +1476,9 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
                              0, f->ps, f->d_g, &sa, st);
   BMF_CUDA(ctx, cudaMemsetAsync(d_grad_density, 0, sizeof(float) * (size_t)f->n * f->dim * f->dim * f->dim, st));
   const int wide = (f->flags & BMF_FIT_ADJOINT_F64) ? 1 : ((f->flags & BMF_FIT_ADJOINT_DF) ? 2 : 0);
-  launch_place_bwd(f->placement, wide, f->d_chunks, f->n, f->d_words, f->last_density, f->d_vkey, f->d_totals,
+  k += launch_place_bwd(f->placement, wide, f->d_chunks, f->n, f->d_words, f->last_density, f->d_vkey, f->d_totals,
                    f->vcap, f->d_g, d_grad_density, f->d_qlist, f->d_qlist + f->vcap, f->d_qseed, f->d_qflag, st);
-  BMF_LAUNCHED(ctx, k + (wide && f->placement == BMF_PLACE_QEF ? 2 : 1));
+  BMF_LAUNCHED(ctx, k);
   return BMF_OK;
 }
 

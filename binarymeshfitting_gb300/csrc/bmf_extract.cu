@@ -759,35 +759,25 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
   }
 }
 
-void launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words,
-                      const float* dens, const uint32_t* vkey, const int64_t* d_counts, int64_t vcap,
-                      const float* grad_pos, float* grad_dens, uint32_t* qlist, uint32_t* qcount, float* qseed,
-                      const uint8_t* qflag, cudaStream_t st) {
+int launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words,
+                     const float* dens, const uint32_t* vkey, const int64_t* d_counts, int64_t vcap,
+                     const float* grad_pos, float* grad_dens, const uint32_t* qlist, const uint32_t* qcount,
+                     const float* qseed, const uint8_t* qflag, cudaStream_t st) {
   const int blocks = (int)((vcap + 127) / 128);
-  if (blocks == 0) return;
-#define BMF_PLACE_BWD(P, T, L)                                                                                     \
-  k_place_bwd<P, T, L><<<blocks, 128, 0, st>>>(d_chunks, n_chunks, words, dens, vkey, d_counts, vcap, grad_pos, \
-                                               grad_dens, qlist, qcount, qseed, qflag)
-  if (placement == 2 && wide && qlist && qcount && qseed && qflag) {
+  if (blocks == 0) return 0;
+#define BMF_PLACE_BWD(P, A)                                                                                        \
+  k_place_bwd<P, A><<<blocks, 128, 0, st>>>(d_chunks, n_chunks, words, dens, vkey, d_counts, vcap, grad_pos,        \
+                                            grad_dens, qflag)
+  if (placement == 2 && wide) {
     // the forward recorded the branch and built the list: float pass over the
     // mass-point vertices, then the wide QEF adjoint over the list
-    BMF_PLACE_BWD(2, float, 3);
-    launch_place_bwd_wide_list(wide, d_chunks, n_chunks, words, dens, vkey, d_counts, vcap, grad_pos, grad_dens,
-                               qlist, qcount, qseed, st);
-  } else if (placement == 2 && wide && qlist && qcount && qseed) {
-    // float pass for the mass-point vertices, then the wide QEF adjoint over
-    // the compacted list of QEF-placed ones (no idle lanes in the wide code;
-    // its own translation unit, compiled with FMA contraction)
-    cudaMemsetAsync(qcount, 0, sizeof(uint32_t), st);
-    BMF_PLACE_BWD(2, float, 1);
-    launch_place_bwd_wide_list(wide, d_chunks, n_chunks, words, dens, vkey, d_counts, vcap, grad_pos, grad_dens,
-                               qlist, qcount, qseed, st);
-  } else if (placement == 2) {
-    if (wide) BMF_PLACE_BWD(2, double, 0); else BMF_PLACE_BWD(2, float, 0);
-  } else {
-    BMF_PLACE_BWD(1, float, 0);
+    BMF_PLACE_BWD(2, false);
+    launch_qef_bwd(wide, d_chunks, n_chunks, words, dens, vkey, vcap, grad_pos, grad_dens, qlist, qcount, qseed, st);
+    return 2;
   }
+  if (placement == 2) BMF_PLACE_BWD(2, true); else BMF_PLACE_BWD(1, true);
 #undef BMF_PLACE_BWD
+  return 1;
 }
 
 // ---------------------------------------------------------------------------

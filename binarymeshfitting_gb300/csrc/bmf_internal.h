@@ -307,23 +307,19 @@ int launch_format(const ChunkDev* d_chunks, int n_chunks, int64_t nv, int64_t ni
 int launch_process_bwd(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,
                        const uint8_t* valence, const uint32_t* idx, int iters, int process_boundary,
                        const ProcessScratch& s, float* g, const StructuredAdj* sa, cudaStream_t st);
-// Adjoint of Mode Q placement (placement 1 mass point, 2 QEF; f64: the QEF
-// derivative from an FP64 re-solve); accumulates into grad_dens (the caller
-// clears it).
-// The wide list pass of launch_place_bwd (bmf_adjoint64.cu): wide 1 = FP64,
-// 2 = double-float.
-void launch_place_bwd_wide_list(int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words,
-                                const float* dens, const uint32_t* vkey, const int64_t* d_counts, int64_t vcap,
-                                const float* grad_pos, float* grad_dens, uint32_t* qlist, uint32_t* qcount,
-                                float* qseed, cudaStream_t st);
-// qlist (vcap entries) + qcount + qseed (9 floats per entry: the first pass's
-// FP32 eigenvectors of the listed vertex): scratch of the two-pass wide form
-// (nullable: one pass, idle lanes in the wide code).  wide: 0 FP32 adjoint, 1 the QEF
-// derivative from an FP64 re-solve, 2 from a double-float re-solve.
-void launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words,
-                      const float* dens, const uint32_t* vkey, const int64_t* d_counts, int64_t vcap,
-                      const float* grad_pos, float* grad_dens, uint32_t* qlist, uint32_t* qcount, float* qseed,
-                      const uint8_t* qflag, cudaStream_t st);
+// Adjoint of Mode Q placement (placement 1 mass point, 2 QEF); accumulates into
+// grad_dens (the caller clears it).  wide (QEF): 0 FP32 adjoint, 1 the QEF
+// derivative from an FP64 re-solve, 2 from a double-float re-solve; these read
+// the forward's record (MeshOut::qflag, qlist, qcount, qseed).  Returns the
+// kernels launched.
+int launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words,
+                     const float* dens, const uint32_t* vkey, const int64_t* d_counts, int64_t vcap,
+                     const float* grad_pos, float* grad_dens, const uint32_t* qlist, const uint32_t* qcount,
+                     const float* qseed, const uint8_t* qflag, cudaStream_t st);
+// Its wide pass over the list (bmf_adjoint64.cu).
+void launch_qef_bwd(int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, const float* dens,
+                    const uint32_t* vkey, int64_t vcap, const float* grad_pos, float* grad_dens, const uint32_t* qlist,
+                    const uint32_t* qcount, const float* qseed, cudaStream_t st);
 void launch_exclusive_scan_u8_to_u32(const uint8_t* in, uint32_t* out, int64_t n, const int64_t* d_n,
                                      uint32_t* block_tmp, cudaStream_t st);
 
