@@ -92,10 +92,11 @@ struct bmf_batch {
   int fill_grid = 0;
   int fill_mode = 0;
   int fill_run = 16;  // the tile height the autotuner picks on the mixed-LOD update
-  // band fill (Mode R, terrain): exact densities only where the mesh reads
+  // band fill (terrain FBM): exact densities only where the mesh reads
   // them; d_exact is its per-sample exactness mask (words layout)
   int fill_band = 0;
   uint32_t* d_exact = nullptr;
+  uint32_t* d_ends = nullptr;  // Mode Q's samples at the crossings' ends (part of d_exact's allocation)
   // the 2D heightmap's band form (the column fill): the fill stores each
   // (x, z) column height (words layout: chunk.words + x * dim + z) and the
   // occupancy words, no densities; the emit computes a crossing end's
@@ -108,6 +109,32 @@ struct bmf_batch {
   uint2* d_clist = nullptr;
   int64_t clist_cap = 0;
 };
+
+namespace {
+
+// The band form of the fill is on: the terrain FBM's band fill (the knob switches
+// it in Mode R plans; a Mode Q plan's is on whenever its line kernel runs), or
+// the 2D heightmap's column fill.
+bool batch_band(const bmf_batch* b) {
+  if (b->field.kind == BMF_FIELD_TERRAIN_FBM)
+    return b->d_exact && b->fill_mode != 0 && (b->fill_band || b->opts.mode == BMF_MODE_Q);
+  return b->fill_band && b->field.kind == BMF_FIELD_TERRAIN_2D && b->d_cols;
+}
+
+// The exact densities that the mesh of a band-filled update reads; returns the kernels launched.
+int batch_fixup(bmf_batch* b, cudaStream_t st) {
+  if (!batch_band(b) || b->field.kind != BMF_FIELD_TERRAIN_FBM) return 0;  // the 2D column fill needs none
+  if (b->opts.mode == BMF_MODE_R)
+    launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
+  else if (b->opts.placement == BMF_PLACE_CENTER)
+    return 0;  // reads no density
+  else
+    launch_fill_need(b->opts.placement == BMF_PLACE_QEF, b->d_chunks, b->n, b->d_units, b->n_units, b->d_flags, b->ws,
+                     b->field, b->d_dens, st);
+  return 1;
+}
+
+}  // namespace
 
 namespace {
 
@@ -725,11 +752,14 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
                   "upload fill items")) != BMF_OK)
       return s;
     b->fill_mode = 2;
-    if (b->opts.mode == BMF_MODE_R && fill_band_supported(b->field)) {
-      if ((s = bail(cudaMalloc(&b->d_exact, sizeof(uint32_t) * words), "exactness mask")) != BMF_OK) return s;
-      b->fill_band = 1;
+    if (fill_band_supported(b->field)) {
+      // Mode Q: the samples at the crossings' ends behind the exactness mask
+      const size_t masks = b->opts.mode == BMF_MODE_R ? 1 : 2;
+      if ((s = bail(cudaMalloc(&b->d_exact, sizeof(uint32_t) * words * masks), "exactness mask")) != BMF_OK) return s;
+      if (masks == 2) b->d_ends = b->d_exact + words;
+      b->fill_band = b->opts.mode == BMF_MODE_R;
     }
-    b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], b->fill_band != 0);
+    b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], batch_band(b));
   }
   if (b->field.kind == BMF_FIELD_TERRAIN_2D) {
     // column items {chunk, first column}, largest chunks first
@@ -755,14 +785,6 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
 
 namespace {
 
-// The band form of the fill is on: the terrain FBM's band fill, or the 2D
-// heightmap's column fill.
-bool batch_band(const bmf_batch* b) {
-  if (!b->fill_band) return false;
-  if (b->field.kind == BMF_FIELD_TERRAIN_FBM) return b->d_exact && b->fill_mode != 0;
-  return b->field.kind == BMF_FIELD_TERRAIN_2D && b->d_cols;
-}
-
 // The work list of active cells for an output arena of (vcap, icap) (+ its counter).
 bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   const int64_t cap = vcap + icap / (b->opts.mode == BMF_MODE_R ? 3 : 4) + 1;
@@ -776,7 +798,7 @@ bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   b->ws.clist = b->d_clist;
   b->ws.ccount = b->d_flags + b->n;
   b->ws.clist_cap = b->clist_cap;
-  if (b->d_exact) {
+  if (b->d_exact && b->opts.mode == BMF_MODE_R) {
     // band fill: every crossing (one vertex each in Mode R) lists at most its two ends
     const int64_t fcap = 2 * vcap + 1;
     if (fcap > b->fix_cap) {
@@ -792,6 +814,7 @@ bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   }
   const bool band = batch_band(b);
   b->ws.exact = band && b->field.kind == BMF_FIELD_TERRAIN_FBM ? b->d_exact : nullptr;
+  b->ws.ends = b->ws.exact && b->opts.placement != BMF_PLACE_CENTER ? b->d_ends : nullptr;
   const bool col2d = band && b->field.kind == BMF_FIELD_TERRAIN_2D;
   b->ws.cols2d = col2d ? b->d_cols : nullptr;
   b->ws.c2d_g = b->field.p[0];
@@ -907,12 +930,11 @@ bmf_status batch_record(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st,
   BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * (b->n + kCounters), st));
   batch_fill(b, st);
   launch_count(b->opts.mode, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_flags, b->ws, st);
-  const bool band = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;  // the 2D column fill needs no fix-up
-  if (band) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
+  const int fixups = batch_fixup(b, st);
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
                     b->d_totals, b->h_pinned, b->d_ticket, st, &b->sweep);
   const MeshOut mo = batch_mesh_out(b, out);
-  int64_t k = (band ? 4 : 3) + (b->d_cols ? 1 : 0);
+  int64_t k = 3 + fixups + (b->d_cols ? 1 : 0);
   k += launch_emit(b->opts.mode, b->opts.placement, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_dens,
                    b->d_flags, b->ws, mo, b->d_totals, st);
   // indices and chunk table are final here (bmf_batch_wait_extraction); an
@@ -1076,8 +1098,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   launch_count(b->opts.mode, b->d_chunks, b->n, b->d_units, b->n_units, b->d_words, b->d_flags, b->ws, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[2], st));
   // the band fill's exact-density fix-up belongs to the fill stage
-  const bool fixup = batch_band(b) && b->field.kind == BMF_FIELD_TERRAIN_FBM;
-  if (fixup) launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
+  const int fixups = batch_fixup(b, st);
   BMF_CUDA(ctx, cudaEventRecord(ev[7], st));
   BMF_CUDA(ctx, cudaEventRecord(ev[3], st));  // the word scan is part of the count
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
@@ -1100,7 +1121,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[2], ev[7], ev[3]));
   for (int k = 3; k < 6; ++k) BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[k], ev[k], ev[k + 1]));
   for (auto& e : ev) cudaEventDestroy(e);
-  ctx->launches += (fixup ? 4 : 3) + (b->d_cols ? 1 : 0) + ek + pk;
+  ctx->launches += 3 + fixups + (b->d_cols ? 1 : 0) + ek + pk;
   return BMF_OK;
 }
 
@@ -1138,16 +1159,14 @@ bmf_status bmf_batch_set_tuning(bmf_batch* b, const bmf_batch_tuning* t) {
   if (t->fill_mode < 0 || t->fill_mode > 2 || (!terrain && t->fill_mode != 0) ||
       (t->fill_run != 4 && t->fill_run != 8 && t->fill_run != 16) ||
       (t->sweep_block != 128 && t->sweep_block != 256 && t->sweep_block != 512) ||
-      (t->fill_band != 0 && t->fill_band != 1) || (t->fill_band && !b->d_exact && !(b->d_cols && b->opts.mode == BMF_MODE_R)))
+      (t->fill_band != 0 && t->fill_band != 1) || (t->fill_band && !((b->d_exact || b->d_cols) && b->opts.mode == BMF_MODE_R)))
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT,
                 "bmf_batch_set_tuning: fill_mode 0..2 (1, 2 for terrain fields only), fill_run 4/8/16, "
                 "sweep_block 128/256/512, fill_band 0/1 (1 for Mode R terrain and 2D heightmap plans only)");
   b->fill_mode = t->fill_mode;
-  if (t->fill_run != b->fill_run || t->fill_band != b->fill_band) {
-    b->fill_run = t->fill_run;
-    b->fill_band = t->fill_band;
-    if (terrain) b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], b->fill_band != 0);
-  }
+  b->fill_run = t->fill_run;
+  b->fill_band = t->fill_band;
+  if (terrain) b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], batch_band(b));
   b->ps.block = t->sweep_block;
   if (b->exec) {
     cudaGraphExecDestroy(b->exec);

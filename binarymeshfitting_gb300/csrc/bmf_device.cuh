@@ -56,6 +56,14 @@ struct ChunkDev {
   int64_t iout;   // offset of the chunk's indices in the output arena
 };
 
+// A chunk's flags: 1 = a word neither empty nor full, 2 = a full word, 4 = an empty one.
+__device__ __forceinline__ bool contains_mesh(uint32_t f) { return (f & 1u) || ((f & 6u) == 6u); }
+// Cells z of block zb with z <= hi (bits [0, hi - 32 zb]).
+__device__ __forceinline__ uint32_t zbits_upto(int hi, int zb) {
+  const int n = hi - 32 * zb + 1;
+  return n >= 32 ? kFull : (n <= 0 ? 0u : ((1u << n) - 1u));
+}
+
 // Field parameters passed by value.  perm is the noise permutation.
 struct FieldDev {
   int kind;

@@ -39,8 +39,6 @@ __device__ __forceinline__ int find_chunk_e(const int* __restrict__ unit_start, 
   return lo;
 }
 
-__device__ __forceinline__ bool contains_mesh(uint32_t f) { return (f & 1u) || ((f & 6u) == 6u); }
-
 // EDGE_V offsets (DMCChunk.cpp:32, 543-565): edge e of a cell is the axis-a
 // crossing owned by the cell at offset (ox, oy, oz).
 static __constant__ int8_t c_edge_owner[12][4] = {{0, 0, 0, 0}, {0, 0, 1, 0}, {0, 1, 0, 0}, {0, 1, 1, 0},
@@ -193,12 +191,6 @@ static __device__ const EdgeTris g_edge_tris = make_edge_tris();
 constexpr int kCountThreads = 64, kCountThreadsFew = 256;
 constexpr int kCountFewUnits = 2048;
 
-// Cells z of block zb with z <= hi (bits [0, hi - 32 zb]).
-__device__ __forceinline__ uint32_t zbits_upto(int hi, int zb) {
-  const int n = hi - 32 * zb + 1;
-  return n >= 32 ? kFull : (n <= 0 ? 0u : ((1u << n) - 1u));
-}
-
 template <int MODE, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_count(const ChunkDev* __restrict__ chunks, int n_chunks,
                                                    const int* __restrict__ unit_start,
@@ -290,6 +282,15 @@ __global__ void __launch_bounds__(THREADS) k_count(const ChunkDev* __restrict__ 
         vc = t;
         ic = 4u * (__popc(Xi) + __popc(Yi) + __popc(Zi));
         act = p0 | p1 | p2 | Xi | Yi | Zi;
+        if (ws.ends) {
+          // samples with a neighbour of the other sign, along each axis and way
+          const uint32_t Z = (w00 ^ a1) & zint;
+          uint32_t e = Z | (Z << 1) | (xin ? w00 ^ w10 : 0u) | (yin ? w00 ^ w01 : 0u);
+          if (zb > 0) e |= (w00 ^ (__ldg(L00 - 1) >> 31)) & 1u;
+          if (x > 0) e |= w00 ^ __ldg(L00 - nw);
+          if (y > 0) e |= w00 ^ __ldg(L00 - zc);
+          ws.ends[ch.words + (int64_t)x * nw + wi] = e;
+        }
       }
     }
     {

@@ -69,7 +69,7 @@ struct WordScratch {
   // Per x-plane (ChunkDev::unit0 + x): its {vertex, index} totals (count
   // kernel), then their exclusive sums over the chunk's planes (k_chunk_scan)
   uint2* pb;
-  // Band fill (Mode R, nullable): its exactness mask, and the list of samples
+  // Band fill (nullable): its exactness mask, and (Mode R) the list of samples
   // the count kernel finds at an end of a crossing with an inexact density,
   // as {chunk, sample index in the chunk}; *fcount (zeroed before the count
   // kernel) entries, at most fix_cap kept.  A crossing has two ends, so the
@@ -78,6 +78,9 @@ struct WordScratch {
   uint2* fix = nullptr;
   uint32_t* fcount = nullptr;
   int64_t fix_cap = 0;
+  // Mode Q's band fill (nullable): per word the samples at an end of a crossing,
+  // for launch_fill_need (words layout; only of chunks with a mesh).
+  uint32_t* ends = nullptr;
   // The 2D heightmap's column fill (Mode R batches, nullable): no densities
   // are stored; the emit computes a crossing end's density from its (x, z)
   // column height (at chunk.words + x * dim + z) as the full fill does,
@@ -132,6 +135,11 @@ int launch_adam(float* p, const float* g, float* m, float* v, int64_t n, int* st
 // inexact ends of crossings; after launch_count, before launch_emit)
 void launch_fill_fixup(const ChunkDev* d_chunks, const WordScratch& ws, const FieldDev& field, float* dens,
                        cudaStream_t st);
+// the same for a Mode Q mesh: the ends of all crossings, with grad also their
+// neighbours along the axes (what the QEF's central differences read)
+void launch_fill_need(bool grad, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
+                      const uint32_t* flags, const WordScratch& ws, const FieldDev& field, float* dens,
+                      cudaStream_t st);
 int fill_terrain_items(int dim);          // items of one chunk
 int fill_terrain_lines();                 // lines per item
 int fill_terrain_resident_ctas(int run, int octaves, bool band);  // persistent grid: SMs x resident CTAs per SM

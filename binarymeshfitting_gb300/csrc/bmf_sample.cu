@@ -272,7 +272,7 @@ __device__ __forceinline__ void oct_line_cell(OctLine& s, int Z, const float4* _
 // Its samples then hold the partial density (right sign, inexact value) and
 // clear their bits in the `exact` mask (laid out like the words); the mesh
 // only reads densities at the ends of sign-changing edges, and
-// k_fill_fixup recomputes those that are inexact before the emit runs, with
+// k_fill_fixup (Mode Q: k_fill_need) recomputes those that are inexact before the emit runs, with
 // the same operations, so the output is bit-identical to a full fill.
 // Lanes take the lines of an item y-major (x fastest), so a warp's lanes
 // share py and mostly stop at the same octave.
@@ -693,6 +693,100 @@ void launch_fill_fixup(const ChunkDev* d_chunks, const WordScratch& ws, const Fi
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   });
   k_fill_fixup<<<g, 256, 0, st>>>(d_chunks, ws.fix, ws.fcount, ws.fix_cap, field, dens);
+}
+
+// ---------------------------------------------------------------------------
+// The same for the samples a Mode Q mesh reads: the ends of its crossings (mass
+// point; the count kernel's ws.ends) and, with GRAD (QEF placement: central
+// differences at the ends), their neighbours along the axes.  A sample is in reach
+// of several crossings, so the set is formed per word, without a list or a
+// capacity: a warp takes 32 words of an x-plane, puts their inexact samples of
+// the set into its list in shared memory and evaluates them lane by lane.
+// Bound by the evaluations: ~0.6k instructions a sample.  512-chunk QEF update:
+// 186 us, with a band fill of 415 us in place of a full one of 1187 us (update 2755
+// -> 2265 us); one list per CTA instead of per warp 200 us, for the barriers.
+// ---------------------------------------------------------------------------
+constexpr int kNeedThreads = 256;
+
+template <bool GRAD>
+__global__ void __launch_bounds__(kNeedThreads) k_fill_need(const ChunkDev* __restrict__ chunks, int n_chunks,
+                                                           const int* __restrict__ unit_start, int n_units,
+                                                           const uint32_t* __restrict__ flags,
+                                                           const uint32_t* __restrict__ exact,
+                                                           const uint32_t* __restrict__ ends, FieldDev field,
+                                                           float* __restrict__ dens) {
+  __shared__ int perm2[512];
+  __shared__ float4 gtab[512];
+  __shared__ uint16_t s_list[kNeedThreads / 32][1024];  // (word of the warp's 32) * 32 + sample of the word
+  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+    perm2[i] = field.perm[i & 255];
+    gtab[i] = grad_coeffs(field.perm[i & 255]);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  uint16_t* list = s_list[threadIdx.x >> 5];
+  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+    const int c = find_chunk(unit_start, n_chunks, u);
+    if (!contains_mesh(__ldg(flags + c))) continue;  // (its words' ends are not set)
+    const ChunkDev ch = chunks[c];
+    const int x = u - __ldg(unit_start + c);
+    const int dim = ch.dim, zc = ch.zc, nw = dim * zc;
+    const uint64_t zmagic = ((1ull << 32) + (uint64_t)zc - 1u) / (uint64_t)zc;  // (as in the count kernel)
+    const uint32_t* E = ends + ch.words + (int64_t)x * nw;
+    const uint32_t* X = exact + ch.words + (int64_t)x * nw;
+    for (int base = (int)(threadIdx.x & ~31u); base < nw; base += kNeedThreads) {
+      const int wi = base + lane;
+      uint32_t need = 0u;
+      if (wi < nw) {
+        need = __ldg(E + wi);
+        if (GRAD) {
+          const int y = (int)(((uint64_t)(uint32_t)wi * zmagic) >> 32), zb = wi - y * zc;
+          need |= (need << 1) | (need >> 1);
+          if (zb > 0) need |= __ldg(E + wi - 1) >> 31;
+          if (zb + 1 < zc) need |= __ldg(E + wi + 1) << 31;
+          if (y > 0) need |= __ldg(E + wi - zc);
+          if (y + 1 < dim) need |= __ldg(E + wi + zc);
+          if (x > 0) need |= __ldg(E + wi - nw);
+          if (x + 1 < dim) need |= __ldg(E + wi + nw);
+          need &= zbits_upto(dim - 1, zb);
+        }
+        if (need) need &= ~__ldg(X + wi);
+      }
+      if (!__any_sync(kFull, need != 0u)) continue;
+      int at = __popc(need);
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(kFull, at, off);
+        if (lane >= off) at += v;
+      }
+      const int total = __shfl_sync(kFull, at, 31);
+      at -= __popc(need);
+      for (uint32_t m = need; m; m &= m - 1u) list[at++] = (uint16_t)((lane << 5) | (__ffs(m) - 1));
+      __syncwarp();
+      for (int e = lane; e < total; e += 32) {
+        const int w = base + (list[e] >> 5);
+        const int y = (int)(((uint64_t)(uint32_t)w * zmagic) >> 32), z = 32 * (w - y * zc) + (list[e] & 31);
+        dens[ch.dens + ((int64_t)x * dim + y) * dim + z] = terrain_exact(field, perm2, gtab, ch, x, y, z);
+      }
+      __syncwarp();
+    }
+  }
+}
+
+void launch_fill_need(bool grad, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,
+                      const uint32_t* flags, const WordScratch& ws, const FieldDev& field, float* dens,
+                      cudaStream_t st) {
+  static std::atomic<int> grid[64] = {};
+  const int g = per_device_once(grid, [](int dev) {
+    int sms = 0, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fill_need<true>, kNeedThreads, 0);
+    return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
+  });
+  if (n_units <= 0) return;
+  const auto kernel = grad ? k_fill_need<true> : k_fill_need<false>;
+  kernel<<<min(g, n_units), kNeedThreads, 0, st>>>(d_chunks, n_chunks, d_unit_start, n_units, flags, ws.exact, ws.ends,
+                                                   field, dens);
 }
 
 int fill_terrain_items(int dim) { return (dim * dim + kFillLines - 1) / kFillLines; }

@@ -292,7 +292,9 @@ typedef struct {
                           BMF_FIELD_TERRAIN_2D the column fill: each (x, z) column height is evaluated once, the
                           occupancy words come from the heights, and the emit computes the densities it reads
                           from them (no density is stored); 0: every sample's density exact.  Both give
-                          bit-identical meshes.  Default 1 where supported. */
+                          bit-identical meshes.  Default 1 where supported.  (A Mode Q terrain plan has no
+                          such knob: its line kernel, fill_mode 1 or 2, always stops early, and the samples
+                          its mesh reads are made exact.) */
   int32_t reserved[4];
 } bmf_batch_tuning;
 BMF_API bmf_status bmf_batch_get_tuning(const bmf_batch* b, bmf_batch_tuning* t);
