@@ -1209,15 +1209,18 @@ struct TeamArgs {
 // Barrier over the team's CTAs (all resident: a cooperative launch).  The wait
 // is bounded: after kTeamSpins polls (a second or so) or once another CTA has
 // given up, the CTA marks the team failed and no longer waits anywhere; the
-// host finds the mark after its synchronisation.
+// host finds the mark after its synchronisation.  Thread 0 releases the CTA's
+// stores with its arrival and acquires the others' with its polls, and the block
+// barriers carry both to the other threads; sequentially consistent fences around
+// a relaxed arrival cost 0.3 us more a meeting (129^3 chunk: 117.8 against 113.8 us).
 constexpr unsigned kTeamSpins = 1u << 22;
 __device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed, unsigned& target, unsigned team,
                                              bool& dead) {
   __syncthreads();
   target += team;
   if (threadIdx.x == 0 && team > 1 && !dead) {
-    __threadfence();  // the CTA's stores (ordered before by the block barrier) before the arrival
-    atomicAdd(&y->arrived, 1u);
+    // release: the CTA's stores (ordered before by the block barrier) come before the arrival
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&y->arrived) : "memory");
     unsigned v = 0;
     for (unsigned spins = 0;; ++spins) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&y->arrived) : "memory");
@@ -1229,7 +1232,6 @@ __device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed,
         break;
       }
     }
-    __threadfence();
   }
   __syncthreads();
 }
