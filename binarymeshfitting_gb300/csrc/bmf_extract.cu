@@ -74,24 +74,6 @@ struct LineWords {
 
 constexpr int kWordBlock = 256;  // threads per CTA of the count / emit kernels
 
-// The case tables staged in shared memory: per-lane lookups with different
-// masks serialise on the constant cache, not on shared memory.
-struct SmemTabs {
-  uint64_t tri[256];
-  uint64_t uses[256];
-  uint64_t grp[256];
-  uint64_t etris[256];  // per case and edge e: bits [5 e, 5 e + 5) mark the triangles that use e
-};
-__device__ __forceinline__ void load_tabs(SmemTabs& t) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    t.tri[i] = __ldg(g_tri_cases + i);
-    t.uses[i] = __ldg(g_edge_uses + i);
-    t.grp[i] = __ldg(g_group_cases + i);
-  }
-  __syncthreads();
-}
-__device__ __forceinline__ int tab_uses(const SmemTabs& t, int mask, int e) { return (int)((t.uses[mask] >> (4 * e)) & 0xF); }
-
 // A word is quiet when its 32 cells can neither own a crossing nor have a
 // mixed corner mask: the four line words around it are identical, so are the
 // four next-block words, and the line has no z-crossing.  Then X = Y = Z = 0
@@ -804,27 +786,27 @@ __device__ __forceinline__ uint32_t line_bits3(const uint32_t* __restrict__ W, i
   return bits & 7u;
 }
 
-// Which case tables a kernel stages in shared memory.
-template <bool TRI, bool USES, bool GRP, bool ETRIS = false>
-__device__ __forceinline__ void load_tabs_some(SmemTabs& t) {
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-    if (TRI) t.tri[i] = __ldg(g_tri_cases + i);
-    if (USES) t.uses[i] = __ldg(g_edge_uses + i);
-    if (GRP) t.grp[i] = __ldg(g_group_cases + i);
-    if (ETRIS) t.etris[i] = g_edge_tris.w[i];
-  }
+// Mode R's adjacency table in shared memory: per case and edge e, bits
+// [5 e, 5 e + 5) mark the triangles that use e.
+struct SmemTabs {
+  uint64_t etris[256];
+};
+template <int MODE>
+__device__ __forceinline__ void load_tabs(SmemTabs& t) {
+  if (MODE != 0) return;
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) t.etris[i] = g_edge_tris.w[i];
   __syncthreads();
 }
 
-// The adjacency list of one vertex (key: its packed grid position) of chunk
-// ch, at most room entries, into out.
+// The adjacency list of one vertex (key: its packed grid position; edges: Mode Q,
+// its edges with a quad) of chunk ch, at most room entries, into out.
 // OUT = uint16_t with rel = the chunk's first primitive: the list holds
 // chunk-relative ids (the chunk-by-chunk sweeps, for chunks of at most 65535
 // primitives: half the bytes in the gathers' working set).
 template <int MODE, typename OUT = uint32_t>
 __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch, const uint32_t* __restrict__ words,
-                                           const WordScratch& ws, uint32_t key, OUT* __restrict__ out,
-                                           int room, int64_t rel = 0) {
+                                           const WordScratch& ws, uint32_t key, uint32_t edges,
+                                           OUT* __restrict__ out, int room, int64_t rel = 0) {
   const int dim = ch.dim, zc = ch.zc;
   const int64_t iout = ch.iout;
   const uint32_t* W = words + ch.words;
@@ -872,29 +854,24 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
       for (; tm && n < room; tm &= tm - 1u) out[n++] = (OUT)(first + __ffs(tm) - 1 - rel);
     }
   } else {
-    const int g = k;
-    const int m = cell_mask_at(W, dim, zc, x, y, z);
-    const uint64_t gw = T.grp[m];
-    // a quad's id grows with its edge's owner sample, then axis: walking the
-    // cell's edges in that order gives the list ascending
-    constexpr uint64_t kEdgeOrder = 0xB7A639251840ull;  // 0, 4, 8, 1, 5, 2, 9, 3, 6, 10, 7, 11 from the low nibble
+    // The vertex's edges with a quad, ascending by the quad's id; a quad's id is its
+    // rank in the owner sample's word, one 16-byte record of the emit.  (Rebuilding
+    // the crossings of the owner's word for each of the 12 edges in turn cost 80% of
+    // the sweeps' instructions at 18 lanes each: k_sweep_chunks on 512 x 65^3, eight
+    // sweeps, 1090 us against 789; a 512-chunk QEF update, four, 750 against 501.)
+    if (x > dim - 2 || y > dim - 2 || z > dim - 2) return;  // a vertex past the work list's capacity has no key
+    constexpr uint64_t kCorner = 0x654432211000ull;  // owner sample 4 dx + 2 dy + dz per edge in quad order
+    constexpr uint32_t kAxis = 0x992124u;            // and axis
+    const uint4* Q = ws.quads + ch.words;
 #pragma unroll 1
-    for (uint64_t eo = kEdgeOrder, i = 0; i < 12; ++i, eo >>= 4) {
-      const int e = (int)(eo & 0xF);
-      if ((int)((gw >> (4 * e)) & 0xF) != g) continue;
-      const int c0 = edge_c0(e), a = e >> 2;
-      const int sx = x + ((c0 >> 2) & 1), sy = y + ((c0 >> 1) & 1), sz = z + (c0 & 1);
-      if (!q_edge_interior(dim, sx, sy, sz, a)) continue;
-      uint32_t Xi, Yi, Zi;
-      q_quad_words(W, dim, zc, sx, sy, sz >> 5, Xi, Yi, Zi);
+    for (uint32_t set = edges; set; set &= set - 1u) {
+      const int i = __ffs(set) - 1, c0 = (int)(kCorner >> (4 * i)) & 7, a = (int)(kAxis >> (2 * i)) & 3;
+      const int sz = z + (c0 & 1);
+      const uint4 q = __ldcg(Q + (((x + (c0 >> 2)) * dim + (y + ((c0 >> 1) & 1))) * zc + (sz >> 5)));
       const int l = sz & 31;
-      const uint32_t lt = lane_lt(l);
-      uint32_t pre = __popc(Xi & lt) + __popc(Yi & lt) + __popc(Zi & lt);
-      if (a >= 1) pre += (Xi >> l) & 1u;
-      if (a >= 2) pre += (Yi >> l) & 1u;
-      const int wi = (sx * dim + sy) * zc + (sz >> 5);
-      const int64_t id = pbase + (__ldg(&ws.pb[ch.unit0 + sx].y) + __ldg(ibase + wi)) / 4u + pre;
-      if (n < room) out[n++] = (OUT)(id - rel);
+      const uint32_t bit = 1u << l, lt = bit - 1u, lx = a >= 1 ? lt | bit : lt, ly = a >= 2 ? lt | bit : lt;
+      const uint32_t pre = __popc(q.x & lx) + __popc(q.y & ly) + __popc(q.z & lt);
+      if (n < room) out[n++] = (OUT)(pbase + q.w + pre - rel);
     }
   }
 }
@@ -902,25 +879,26 @@ __device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch
 template <int MODE>
 __global__ void __launch_bounds__(256) k_adj_build(const ChunkDev* __restrict__ chunks, int n_chunks,
                                                    const uint32_t* __restrict__ words, WordScratch ws,
-                                                   const uint32_t* __restrict__ vkey, const uint32_t* __restrict__ off,
+                                                   const uint32_t* __restrict__ vkey,
+                                                   const uint16_t* __restrict__ vedge, const uint32_t* __restrict__ off,
                                                    const int64_t* __restrict__ d_counts, int64_t vcap,
                                                    uint32_t* __restrict__ adj) {
   __shared__ SmemTabs T;
-  load_tabs_some<false, false, MODE != 0, MODE == 0>(T);
+  load_tabs<MODE>(T);
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= (d_counts ? min(vcap, d_counts[0]) : vcap)) return;
   const int c = find_chunk_by_vertex(chunks, n_chunks, v);
   // the vertex's CSR range (the exclusive scan of init_valence): never write past it
-  adj_vertex<MODE>(T, chunks[c], words, ws, vkey[v], adj + off[v], (int)(off[v + 1] - off[v]));
+  adj_vertex<MODE>(T, chunks[c], words, ws, vkey[v], MODE ? vedge[v] : 0u, adj + off[v], (int)(off[v + 1] - off[v]));
 }
 
 void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, WordScratch ws,
-                      const uint32_t* vkey, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
-                      uint32_t* adj, cudaStream_t st) {
+                      const uint32_t* vkey, const uint16_t* vedge, const uint32_t* off, const int64_t* d_counts,
+                      int64_t vcap, uint32_t* adj, cudaStream_t st) {
   const int blocks = (int)((vcap + 255) / 256);
   if (blocks == 0) return;
-  if (mode == 0) k_adj_build<0><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, off, d_counts, vcap, adj);
-  else k_adj_build<1><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, off, d_counts, vcap, adj);
+  if (mode == 0) k_adj_build<0><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, vedge, off, d_counts, vcap, adj);
+  else k_adj_build<1><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, vedge, off, d_counts, vcap, adj);
 }
 
 // ---------------------------------------------------------------------------
@@ -946,6 +924,7 @@ struct SweepArgs {
   const uint32_t* __restrict__ words;
   WordScratch ws;
   const uint32_t* __restrict__ vkey;
+  const uint16_t* __restrict__ vedge;
   int64_t nv, n_prims, adj_cap;
   const int64_t* __restrict__ d_counts;
   uint32_t* __restrict__ off;
@@ -1034,12 +1013,12 @@ __device__ __forceinline__ void sweep_older(const SweepArgs& A, ChunkPart c, int
 template <int MODE, int N>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
     const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, SweepLists lists,
-    const uint32_t* __restrict__ words, WordScratch ws, const uint32_t* __restrict__ vkey, int64_t nv, int64_t n_prims,
-    int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
+    const uint32_t* __restrict__ words, WordScratch ws, const uint32_t* __restrict__ vkey,
+    const uint16_t* __restrict__ vedge, int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
     const uint8_t* __restrict__ valence, uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary,
     const uint32_t* __restrict__ idx, SweepBufs b_, float* __restrict__ dual_p, float* __restrict__ dual_n, int iters,
     int process_boundary, int sn, int wide_adj) {
-  const SweepArgs A{chunks, tot, lists, words, ws, vkey, nv, n_prims, adj_cap, d_counts, off, valence, adj, boundary,
+  const SweepArgs A{chunks, tot, lists, words, ws, vkey, vedge, nv, n_prims, adj_cap, d_counts, off, valence, adj, boundary,
                     idx, b_, dual_p, dual_n, iters, process_boundary, sn, wide_adj};
   constexpr int kThreads = kSweepThreads, kWarps = kThreads / 32;
   __shared__ SmemTabs T;
@@ -1047,7 +1026,8 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
   __shared__ uint32_t s_total;
   __shared__ uint32_t s_item;
   __shared__ uint32_t s_seg[8];  // valence sum of each CTA's vertices
-  load_tabs_some<false, false, MODE != 0, MODE == 0>(T);
+  load_tabs<MODE>(T);
+  cluster_barrier();  // every CTA of the cluster has started before its shared memory is written
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_big = A.lists.head[0], n_list = A.lists.head[1];
   bool wide = true;  // the cluster's items first, then single CTAs
@@ -1147,10 +1127,10 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
       const uint32_t o = A.off[v];
       const int room = (int)max((int64_t)0, min((int64_t)__ldg(A.valence + v), A.adj_cap - (int64_t)o));
       if (compact)
-        adj_vertex<MODE, uint16_t>(T, ch, A.words, A.ws, __ldg(A.vkey + v),
+        adj_vertex<MODE, uint16_t>(T, ch, A.words, A.ws, __ldg(A.vkey + v), MODE ? __ldg(A.vedge + v) : 0u,
                                    const_cast<uint16_t*>(sweep_list<uint16_t>(A, c, o)), room, (int64_t)c.p0);
       else
-        adj_vertex<MODE>(T, ch, A.words, A.ws, __ldg(A.vkey + v), A.adj + o, room);
+        adj_vertex<MODE>(T, ch, A.words, A.ws, __ldg(A.vkey + v), MODE ? __ldg(A.vedge + v) : 0u, A.adj + o, room);
     }
     for (int m = 0; m < A.iters; ++m) {
       const SweepStep st = sweep_step(m, A.iters, A.sn, A.b.keep(), A.b);
@@ -1192,6 +1172,7 @@ struct TeamArgs {
   const uint32_t* words;
   WordScratch ws;
   const uint32_t* vkey;
+  const uint16_t* vedge;
   int64_t nv, n_prims;
   const int64_t* d_counts;
   uint32_t* off;
@@ -1250,7 +1231,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
     if (threadIdx.x == 0) *(volatile unsigned*)A.host_failed = 1u;
     return;
   }
-  load_tabs_some<false, false, MODE != 0, MODE == 0>(T);
+  load_tabs<MODE>(T);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
   const int iters = A.iters;
   unsigned target = 0;
@@ -1294,7 +1275,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
       A.off[v] = o;
       const int room = o < cap ? (int)min(x, cap - o) : 0;
       adj_vertex<MODE>(T, A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.words, A.ws, __ldg(A.vkey + v),
-                       A.adj + o, room);
+                       MODE ? __ldg(A.vedge + v) : 0u, A.adj + o, room);
     }
     carry += s_total;
     __syncthreads();
@@ -1385,7 +1366,7 @@ void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_pri
                        float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
                        int iters, int process_boundary, int smooth_normals, const ProcessScratch& s,
                        cudaStream_t st) {
-  TeamArgs A{sa.chunks, sa.n_chunks, sa.words, sa.ws, sa.vkey, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
+  TeamArgs A{sa.chunks, sa.n_chunks, sa.words, sa.ws, sa.vkey, sa.vedge, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
              idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
              smooth_normals, sa.team, sa.team_failed};
   cudaLaunchConfig_t cfg{};
@@ -1429,7 +1410,7 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st) {
-  SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.words, sa.ws, sa.vkey, nv, n_prims, n_prims * N, d_counts, s.off,
+  SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.words, sa.ws, sa.vkey, sa.vedge, nv, n_prims, n_prims * N, d_counts, s.off,
               valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters,
               process_boundary, smooth_normals, sa.wide_adj ? 1 : 0};
   cudaLaunchConfig_t cfg{};
@@ -1443,7 +1424,8 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const auto go = [&](auto kernel) {
-    cudaLaunchKernelEx(&cfg, kernel, A.chunks, A.tot, A.lists, A.words, A.ws, A.vkey, A.nv, A.n_prims, A.adj_cap,
+    cudaLaunchKernelEx(&cfg, kernel, A.chunks, A.tot, A.lists, A.words, A.ws, A.vkey, A.vedge, A.nv, A.n_prims,
+                       A.adj_cap,
                        A.d_counts, A.off, A.valence, A.adj, A.boundary, A.idx, A.b, A.dual_p, A.dual_n, A.iters,
                        A.process_boundary, A.sn, A.wide_adj);
   };
@@ -2024,6 +2006,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
           R.cv[lane][4 + b][0] += pb1.x;
         }
         R.ib[lane] += pb1.y;
+        if (ws.quads) ws.quads[R.cw[lane] + (x * dim + R.y[lane]) * R.zc[lane] + zb] = make_uint4(X, Y, Z, R.ib[lane] / 4u);
         const uint32_t* own = R.cv[lane][7];
         const uint32_t nv = __popc(own[1]) + 2u * __popc(own[2]) + 4u * __popc(own[3]);
         packed = nv | ((__popc(X) + __popc(Y) + __popc(Z)) << 16);  // at most 128 and 96 per word
@@ -2062,7 +2045,8 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
       const int64_t gv = R.vout[t] + (int64_t)own[0] + k;
       in = in && gv < out.vcap;
       const int dim = R.dim[t], x = R.x[t], y = R.y[t], z = 32 * R.zb[t] + l;
-      const uint32_t edges = in ? group_edges(qtile_mask(R.w[t], 1, 1, 32 + l), g & 3) : 0u;
+      const int mask = qtile_mask(R.w[t], 1, 1, 32 + l);
+      const uint32_t edges = in && (PLACE != 2 || !out.vkey) ? group_edges(mask, g & 3) : 0u;
       if (PLACE != 2 || !out.vkey) {
         float P[3];
         q_place<PLACE, true>(dens + R.dens[t], dim, x, y, z, edges, P);
@@ -2079,16 +2063,17 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
           out.boundary[gv] = (x == 0 || y == 0 || z == 0 || x == dim - 2 || y == dim - 2 || z == dim - 2);
         if (out.vkey) out.vkey[gv] = vertex_key(x, y, z, g);
         if (out.valence) {
-          // the group's edges whose four cells exist (q_edge_interior)
-          uint32_t in12 = 0xFFFu;
-          const auto cut = [&](bool has, uint32_t m) { if (!has) in12 &= ~m; };
-          cut(x > 0, 0x330u);          // y-edges 4, 5 and z-edges 8, 9 at dx = 0
-          cut(x + 1 <= dim - 2, 0xCC0u);  // 6, 7, 10, 11 at dx = 1
-          cut(y > 0, 0x503u);          // x-edges 0, 1 and z-edges 8, 10 at dy = 0
-          cut(y + 1 <= dim - 2, 0xA0Cu);  // 2, 3, 9, 11 at dy = 1
-          cut(z > 0, 0x055u);          // x-edges 0, 2 and y-edges 4, 6 at dz = 0
-          cut(z + 1 <= dim - 2, 0x0AAu);  // 1, 3, 5, 7 at dz = 1
-          out.valence[gv] = (uint8_t)__popc(edges & in12);
+          // the group's edges whose four cells exist (q_edge_interior), in quad order
+          uint32_t set = group_edges_q(mask, g & 3);
+          const auto cut = [&](bool has, uint32_t m) { if (!has) set &= ~m; };
+          cut(x > 0, kQuadDx0);
+          cut(x + 1 <= dim - 2, kQuadDx1);
+          cut(y > 0, kQuadDy0);
+          cut(y + 1 <= dim - 2, kQuadDy1);
+          cut(z > 0, kQuadDz0);
+          cut(z + 1 <= dim - 2, kQuadDz1);
+          out.valence[gv] = (uint8_t)__popc(set);
+          if (out.vedge) out.vedge[gv] = (uint16_t)set;
         }
       }
       __syncwarp();

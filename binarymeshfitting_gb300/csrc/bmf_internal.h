@@ -41,6 +41,9 @@ struct MeshOut {
   // k = crossing axis (Mode R) or vertex group (Mode Q); the key the analytic
   // adjacency build starts from.
   uint32_t* vkey = nullptr;
+  // optional (Mode Q): per vertex the edges of its group that have a quad, as a
+  // 12-bit set in quad order (valence is its size); the adjacency reads it
+  uint16_t* vedge = nullptr;
   // optional (QEF placement with keys): the record the QEF adjoint reads --
   // per vertex whether it took the QEF branch, the list of those vertices
   // (count in *qcount) and their FP32 eigenvectors (9 floats per entry)
@@ -81,6 +84,9 @@ struct WordScratch {
   // Mode Q's band fill (nullable): per word the samples at an end of a crossing,
   // for launch_fill_need (words layout; only of chunks with a mesh).
   uint32_t* ends = nullptr;
+  // Mode Q with sweeps (nullable): per busy word its interior crossings along x, y, z
+  // and its first quad (of the chunk), which the emit writes and the adjacency reads.
+  uint4* quads = nullptr;
   // The 2D heightmap's column fill (Mode R batches, nullable): no densities
   // are stored; the emit computes a crossing end's density from its (x, z)
   // column height (at chunk.words + x * dim + z) as the full fill does,
@@ -269,6 +275,7 @@ struct StructuredAdj {
   const uint32_t* words;
   WordScratch ws;            // scanned counts + per-word bit-planes
   const uint32_t* vkey;      // per-vertex keys written by the emit kernel
+  const uint16_t* vedge;     // Mode Q: MeshOut::vedge (and ws.quads)
   // optional (tot and lists.order, or neither): the sweeps run chunk by chunk
   const uint32_t* tot = nullptr;  // per chunk {vertices, indices}
   SweepLists lists;               // filled by launch_chunk_scan
@@ -281,7 +288,7 @@ struct StructuredAdj {
   bool wide_adj = false;
 };
 void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, WordScratch ws,
-                      const uint32_t* vkey, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
+                      const uint32_t* vkey, const uint16_t* vedge, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
                       uint32_t* adj, cudaStream_t st);
 // The chunk-by-chunk form of launch_process for StructuredAdj with tot and
 // lists set: CSR offsets, adjacency and all sweeps in one launch.

@@ -36,10 +36,27 @@ __device__ __forceinline__ void grid_gradient(const float* __restrict__ D, int d
   }
 }
 
+// The edges of a cell in the order of their quads' ids (by owner sample, then
+// axis): 0, 4, 8, 1, 5, 2, 9, 3, 6, 10, 7, 11 from the low nibble; and a set of
+// edges with its bits in that order.
+constexpr uint64_t kQuadOrder = 0xB7A639251840ull;
+constexpr uint32_t in_quad_order(uint32_t edges) {
+  uint32_t r = 0u;
+  for (int i = 0; i < 12; ++i)
+    if ((edges >> ((kQuadOrder >> (4 * i)) & 0xF)) & 1u) r |= 1u << i;
+  return r;
+}
+
+// The edges on a side of the cell (each has a quad only if the cell across it
+// exists): y-edges 4, 5 and z-edges 8, 9 at dx = 0, and so on.
+constexpr uint32_t kQuadDx0 = in_quad_order(0x330u), kQuadDx1 = in_quad_order(0xCC0u),
+                   kQuadDy0 = in_quad_order(0x503u), kQuadDy1 = in_quad_order(0xA0Cu),
+                   kQuadDz0 = in_quad_order(0x055u), kQuadDz1 = in_quad_order(0x0AAu);
+
 // Per corner mask and vertex group (four per mask): the group's edges as a
-// 12-bit set.
+// 12-bit set, and the same in quad order.
 struct GroupEdges {
-  uint16_t w[1024];
+  uint16_t w[1024], q[1024];
 };
 constexpr GroupEdges make_group_edges() {
   constexpr uint64_t grp[256] = BMF_GROUP_CASES_INIT;
@@ -49,10 +66,12 @@ constexpr GroupEdges make_group_edges() {
       const int g = (int)((grp[m] >> (4 * e)) & 0xFu);
       if (g < 4) r.w[4 * m + g] |= (uint16_t)(1u << e);
     }
+  for (int i = 0; i < 1024; ++i) r.q[i] = (uint16_t)in_quad_order(r.w[i]);
   return r;
 }
 static __device__ const GroupEdges g_group_edges = make_group_edges();
 __device__ __forceinline__ uint32_t group_edges(int mask, int g) { return __ldg(&g_group_edges.w[4 * mask + g]); }
+__device__ __forceinline__ uint32_t group_edges_q(int mask, int g) { return __ldg(&g_group_edges.q[4 * mask + g]); }
 
 // QEF solve, restating qef_simd.h:150-579 lane by lane in FP32 with the exact
 // 1/sqrt in place of _mm_rsqrt_ps.
