@@ -19,8 +19,8 @@ using namespace bmf;
 namespace {
 
 enum Slot {
-  S_CHUNKS, S_TOT, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_ICNT, S_GPL,
-  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_COLS, S_VEDGE, S_QUADS, S_NUM
+  S_CHUNKS, S_TOT, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_REC,
+  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_COLS, S_VADJ, S_QUADS, S_NUM
 };
 
 constexpr int kMaxDim = 512;
@@ -70,7 +70,7 @@ struct bmf_batch {
   uint8_t* d_valence = nullptr;
   uint8_t* d_boundary = nullptr;
   uint32_t* d_vkey = nullptr;
-  uint16_t* d_vedge = nullptr;
+  uint32_t* d_vadj = nullptr;
   // captured graph and the output it was captured for
   cudaGraphExec_t exec = nullptr;
   bmf_batch_out graph_out{};
@@ -299,8 +299,7 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk
   uint32_t* tot = nullptr;
   bmf_status s;
   if ((s = scratch(ctx, S_VCNT, (size_t)words_total, &ws.vcnt)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_ICNT, (size_t)words_total, &ws.icnt)) != BMF_OK) return s;
-  if ((s = scratch(ctx, S_GPL, (size_t)words_total * 3, &ws.gpl)) != BMF_OK) return s;
+  if ((s = scratch(ctx, S_REC, (size_t)words_total, &ws.rec)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_PB, (size_t)n_units, &ws.pb)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_TOT, (size_t)n_chunks * 2, &tot)) != BMF_OK) return s;
   {
@@ -310,8 +309,8 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk
     ws.ccount = c.ccount;
   }
   if (sa) {
-    if (mo.vedge && (s = scratch(ctx, S_QUADS, (size_t)words_total, &ws.quads)) != BMF_OK) return s;
-    *sa = StructuredAdj{mode, d_chunks, n_chunks, d_words, ws, mo.vkey, mo.vedge};
+    if (mode == BMF_MODE_Q && (s = scratch(ctx, S_QUADS, (size_t)words_total, &ws.quads)) != BMF_OK) return s;
+    *sa = StructuredAdj{mode, d_chunks, n_chunks, ws, mo.vkey, mo.vadj};
     if (sweep_form(mode, 1, (int64_t)n_units * n_units, &sa->lists) == kSweepTeam) {
       sa->team = ctx->team;
       sa->team_failed = ctx->team_failed();
@@ -607,9 +606,7 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   if ((opts->iters > 0 || (opts->mode == BMF_MODE_Q && opts->placement == BMF_PLACE_QEF)) &&
       (s = scratch(ctx, S_VKEY, (size_t)out->vcap + 1, &mo.vkey)) != BMF_OK)
     return s;
-  if (opts->iters > 0 && opts->mode == BMF_MODE_Q &&
-      (s = scratch(ctx, S_VEDGE, (size_t)out->vcap + 1, &mo.vedge)) != BMF_OK)
-    return s;
+  if (opts->iters > 0 && (s = scratch(ctx, S_VADJ, (size_t)out->vcap + 1, &mo.vadj)) != BMF_OK) return s;
   // What the capacities, bounded by the chunk's size, ask of the sweeps'
   // scratch: within kOneSyncBytes the sweeps are enqueued behind the emit with
   // the counts on the device, and positions are kept for left-out face
@@ -716,8 +713,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if ((s = bail(cudaMalloc(&b->d_dens, sizeof(float) * dens), "density")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->d_words, sizeof(uint32_t) * words), "words")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->ws.vcnt, sizeof(uint32_t) * words), "vcnt")) != BMF_OK) return s;
-  if ((s = bail(cudaMalloc(&b->ws.icnt, sizeof(uint32_t) * words), "icnt")) != BMF_OK) return s;
-  if ((s = bail(cudaMalloc(&b->ws.gpl, sizeof(uint32_t) * 3 * words), "gpl")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->ws.rec, sizeof(uint4) * words), "word records")) != BMF_OK) return s;
   if (opts->mode == BMF_MODE_Q && opts->iters > 0 &&
       (s = bail(cudaMalloc(&b->ws.quads, sizeof(uint4) * words), "quads per word")) != BMF_OK)
     return s;
@@ -864,7 +860,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   void** ptrs[] = {(void**)&b->ps.off, (void**)&b->ps.adj, (void**)&b->ps.dual_p, (void**)&b->ps.dual_n,
                    (void**)&b->ps.tmp, (void**)&b->ps.x[0], (void**)&b->ps.x[1], (void**)&b->ps.x[2],
                    (void**)&b->d_idxg, (void**)&b->d_valence, (void**)&b->d_boundary, (void**)&b->d_vkey,
-                   (void**)&b->d_vedge};
+                   (void**)&b->d_vadj};
   for (void** p : ptrs) {
     if (*p) cudaFree(*p);
     *p = nullptr;
@@ -882,7 +878,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   BMF_CUDA(ctx, cudaMalloc(&b->d_valence, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_boundary, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_vkey, sizeof(uint32_t) * (vcap + 1)));
-  if (b->ws.quads) BMF_CUDA(ctx, cudaMalloc(&b->d_vedge, sizeof(uint16_t) * (vcap + 1)));
+  if (b->opts.iters > 0) BMF_CUDA(ctx, cudaMalloc(&b->d_vadj, sizeof(uint32_t) * (vcap + 1)));
   b->proc_vcap = vcap;
   b->proc_icap = icap;
   return BMF_OK;
@@ -890,7 +886,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
 
 // The structured adjacency of a batch.
 StructuredAdj batch_adj(const bmf_batch* b) {
-  StructuredAdj sa{b->opts.mode, b->d_chunks, b->n, b->d_words, b->ws, b->d_vkey, b->d_vedge};
+  StructuredAdj sa{b->opts.mode, b->d_chunks, b->n, b->ws, b->d_vkey, b->d_vadj};
   if (b->form == kSweepChunks) {
     sa.tot = b->d_tot;
     sa.lists = b->sweep;
@@ -920,7 +916,7 @@ MeshOut batch_mesh_out(const bmf_batch* b, const bmf_batch_out* out) {
   return MeshOut{keep ? ps.x[0] : out->d_pos, keep ? nullptr : out->d_nrm,
                  proc && !out->d_boundary ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr, out->d_idx,
                  proc && b->form != kSweepChunks ? b->d_idxg : nullptr, out->vcap, out->icap,
-                 batch_keys(b) ? b->d_vkey : nullptr, b->d_vedge};
+                 batch_keys(b) ? b->d_vkey : nullptr, b->d_vadj};
 }
 
 // Enqueues the sweeps of one update; returns the kernels launched.
@@ -1294,7 +1290,7 @@ struct bmf_fit {
   ProcessScratch ps{};
   uint32_t *d_idxg = nullptr, *d_vkey = nullptr;
   uint8_t *d_valence = nullptr, *d_boundary = nullptr;
-  uint16_t* d_vedge = nullptr;
+  uint32_t* d_vadj = nullptr;
   float* d_g = nullptr;           // position-gradient work buffer
   SweepLists sweep;               // the chunk-by-chunk sweeps' work lists, and the adjoint's queue over them
   int* d_pqueue = nullptr;
@@ -1314,10 +1310,10 @@ extern "C" {
 
 bmf_status bmf_fit_destroy(bmf_fit* f) {
   if (!f) return BMF_ERR_INVALID_ARGUMENT;
-  void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.icnt,
-                  f->ws.gpl, f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
+  void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.rec,
+                  f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
                   f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
-                  f->d_pqueue, f->d_vedge, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team};
+                  f->d_pqueue, f->d_vadj, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (f->h_pinned) cudaFreeHost(f->h_pinned);
@@ -1372,8 +1368,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMemset(f->d_ticket, 0, sizeof(int)) == cudaSuccess &&
             cudaMalloc(&f->ws.pb, sizeof(uint2) * n_chunks * dim) == cudaSuccess &&
             cudaMalloc(&f->ws.vcnt, sizeof(uint32_t) * words) == cudaSuccess &&
-            cudaMalloc(&f->ws.icnt, sizeof(uint32_t) * words) == cudaSuccess &&
-            cudaMalloc(&f->ws.gpl, sizeof(uint32_t) * 3 * words) == cudaSuccess &&
+            cudaMalloc(&f->ws.rec, sizeof(uint4) * words) == cudaSuccess &&
             cudaMalloc(&f->ps.off, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->ps.adj, sizeof(uint32_t) * (np * 4 + 1)) == cudaSuccess &&
             cudaMalloc(&f->ps.dual_p, sizeof(float) * (4 * np + 4)) == cudaSuccess &&
@@ -1381,7 +1376,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_idxg, sizeof(uint32_t) * (icap + 1)) == cudaSuccess &&
             cudaMalloc(&f->d_vkey, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->d_valence, vcap + 1) == cudaSuccess && cudaMalloc(&f->d_boundary, vcap + 1) == cudaSuccess &&
-            cudaMalloc(&f->d_vedge, sizeof(uint16_t) * (vcap + 1)) == cudaSuccess &&
+            cudaMalloc(&f->d_vadj, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->ws.quads, sizeof(uint4) * words) == cudaSuccess &&
             cudaMalloc(&f->d_g, sizeof(float) * 3 * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->d_qlist, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
@@ -1423,7 +1418,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   launch_count(BMF_MODE_Q, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words, f->d_flags, f->ws, st);
   launch_chunk_scan(f->d_chunks, f->n, f->ws, f->d_tot, f->d_flags, f->vcap, f->icap, d_chunk_info, f->d_totals,
                     f->h_pinned, f->d_ticket, st, &f->sweep);
-  MeshOut mo{d_pos, nullptr, f->d_boundary, f->d_valence, d_idx, f->d_idxg, f->vcap, f->icap, f->d_vkey, f->d_vedge};
+  MeshOut mo{d_pos, nullptr, f->d_boundary, f->d_valence, d_idx, f->d_idxg, f->vcap, f->icap, f->d_vkey, f->d_vadj};
   if (f->d_qflag && f->placement == BMF_PLACE_QEF) {  // the wide adjoint reads the forward's QEF branches
     mo.qflag = f->d_qflag;
     mo.qlist = f->d_qlist;
@@ -1433,7 +1428,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   int k = 3 + launch_emit(BMF_MODE_Q, f->placement, f->d_chunks, f->n, f->d_units, f->n * f->dim, f->d_words,
                           d_density, f->d_flags, f->ws, mo, f->d_totals, st);
   if (f->iters > 0) {
-    StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->d_words, f->ws, f->d_vkey, f->d_vedge};
+    StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->ws, f->d_vkey, f->d_vadj};
     if (f->form == kSweepChunks) {
       sa.tot = f->d_tot;
       sa.lists = f->sweep;
@@ -1498,7 +1493,7 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
   if (ng > 0)
     BMF_CUDA(ctx, cudaMemcpyAsync(f->d_g, d_grad_pos, sizeof(float) * 3 * ng, cudaMemcpyDeviceToDevice, st));
   // with enough chunks to fill the GPU the adjoint sweeps run chunk by chunk
-  StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->d_words, f->ws, f->d_vkey, f->d_vedge};
+  StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->ws, f->d_vkey, f->d_vadj};
   if (f->n >= kChunkSweepBwdMinChunks) {
     sa.tot = f->d_tot;
     sa.lists = f->sweep;
@@ -1518,10 +1513,10 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
   if (!b) return BMF_ERR_INVALID_ARGUMENT;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   void* ptrs[] = {b->d_chunks, b->d_units, b->d_flags, b->d_tot, b->d_totals, b->d_dens, b->d_words,
-                  b->ws.vcnt, b->ws.icnt, b->ws.gpl, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
+                  b->ws.vcnt, b->ws.rec, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
                   b->d_fill_items, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
-                  b->d_cols, b->d_ticket, b->ws.pb, b->team, b->ws.quads, b->d_vedge, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
+                  b->d_cols, b->d_ticket, b->ws.pb, b->team, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);

@@ -300,10 +300,7 @@ __global__ void __launch_bounds__(THREADS) k_count(const ChunkDev* __restrict__ 
       if (act) {
         const int64_t o = ch.words + (int64_t)x * nw + wi;
         ws.vcnt[o] = bv + iv - vc;
-        ws.icnt[o] = bi + ii - ic;
-        ws.gpl[3 * o] = p0;
-        ws.gpl[3 * o + 1] = p1;
-        ws.gpl[3 * o + 2] = p2;
+        ws.rec[o] = make_uint4(p0, p1, p2, bi + ii - ic);
       }
     }
     if (MODE == 0 && ws.exact && __any_sync(kFull, (f00 | f10 | f01 | fnx) != 0u)) {
@@ -544,12 +541,12 @@ __device__ __forceinline__ uint32_t nb_vertex_id(const NbCache& c, int dim, int 
 }
 
 // Mode Q vertex base of cell (x, y, z).
-__device__ __forceinline__ uint32_t q_vertex_base(const uint32_t* vbase, const uint32_t* gpl, const uint2* pb, int dim,
+__device__ __forceinline__ uint32_t q_vertex_base(const uint32_t* vbase, const uint4* rec, const uint2* pb, int dim,
                                                   int zc, int x, int y, int z) {
   const int64_t wi = ((int64_t)x * dim + y) * zc + (z >> 5);
   const uint32_t lt = lane_lt(z & 31);
-  return __ldg(&pb[x].x) + __ldg(vbase + wi) + __popc(__ldg(gpl + 3 * wi) & lt) +
-         2 * __popc(__ldg(gpl + 3 * wi + 1) & lt) + 4 * __popc(__ldg(gpl + 3 * wi + 2) & lt);
+  const uint4 r = __ldg(rec + wi);
+  return __ldg(&pb[x].x) + __ldg(vbase + wi) + __popc(r.x & lt) + 2 * __popc(r.y & lt) + 4 * __popc(r.z & lt);
 }
 
 template <int MODE, int PLACE>
@@ -566,7 +563,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint32_t* W = words + ch.words;
   const uint32_t* vbase = ws.vcnt + ch.words;
-  const uint32_t* ibase = ws.icnt + ch.words;
+  const uint4* rec = ws.rec + ch.words;
   const uint2* pb = ws.pb + ch.unit0;
   const uint2 pbx = pb[x];
   const float* D = dens + ch.dens;
@@ -649,7 +646,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const int t3 = 3 * (int)(tw >> 60);
       if (__ballot_sync(kFull, t3 != 0) == 0u) continue;
       const int incl = warp_incl_scan(t3);
-      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(ibase + wo)) + (incl - t3);
+      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(&rec[wo].w)) + (incl - t3);
       for (int i = 0; i < t3; ++i, ++gi) {
         const int e = tri_edge(tw, i);
         const uint32_t vid = nb_vertex_id(nb, dim, x, y, zb, c_edge_owner[e][0], c_edge_owner[e][1],
@@ -664,10 +661,9 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const bool interior = x <= dim - 2 && y <= dim - 2 && z <= dim - 2;
       const int mask = interior ? lw.mask(lane) : 0;
       const int ng = group_count(mask);
-      const int64_t gpo = 3 * (ch.words + wo);
       if (ng) {
-        uint32_t vid = pbx.x + __ldg(vbase + wo) + __popc(__ldg(ws.gpl + gpo) & lt) +
-                       2 * __popc(__ldg(ws.gpl + gpo + 1) & lt) + 4 * __popc(__ldg(ws.gpl + gpo + 2) & lt);
+        const uint4 r = __ldg(rec + wo);
+        uint32_t vid = pbx.x + __ldg(vbase + wo) + __popc(r.x & lt) + 2 * __popc(r.y & lt) + 4 * __popc(r.z & lt);
         const int nc = dim - 1;
         const uint8_t bnd = (x == 0 || y == 0 || z == 0 || x == nc - 1 || y == nc - 1 || z == nc - 1);
         for (int g = 0; g < ng; ++g, ++vid) {
@@ -704,7 +700,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
       const int nq = __popc(own);
       if (__ballot_sync(kFull, nq != 0) == 0u) continue;
       const int incl = warp_incl_scan(4 * nq);
-      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(ibase + wo)) + (incl - 4 * nq);
+      int64_t gi = ch.iout + (int64_t)(pbx.y + __ldg(&rec[wo].w)) + (incl - 4 * nq);
       const bool in0 = ((lw.w00 >> lane) & 1u) != 0u;
       for (int a = 0; a < 3; ++a) {
         if (!((own >> a) & 1)) continue;
@@ -721,7 +717,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
           lo[cax] = -oc;
           const int e = a == 0 ? 2 * lo[1] + lo[2] : (a == 1 ? 4 + 2 * lo[0] + lo[2] : 8 + 2 * lo[0] + lo[1]);
           const int cm = cell_mask_at(W, dim, zc, cc[0], cc[1], cc[2]);
-          q[k] = q_vertex_base(vbase, ws.gpl + 3 * ch.words, pb, dim, zc, cc[0], cc[1], cc[2]) +
+          q[k] = q_vertex_base(vbase, rec, pb, dim, zc, cc[0], cc[1], cc[2]) +
                  (uint32_t)group_of(cm, e);
         }
         if (!in0) {
@@ -775,130 +771,80 @@ int launch_place_bwd(int placement, int wide, const ChunkDev* d_chunks, int n_ch
 // sort, deterministic.
 // ---------------------------------------------------------------------------
 
-// Three consecutive inside bits z0..z0+2 of line (x, y) (zero outside the
-// chunk); W is the chunk's words, 32-bit offsets.
-__device__ __forceinline__ uint32_t line_bits3(const uint32_t* __restrict__ W, int dim, int zc, int x, int y, int z0) {
-  if (x < 0 || y < 0 || x >= dim || y >= dim) return 0u;
-  const int b0 = z0 >> 5, s = z0 & 31;  // arithmetic shift: block -1 for z0 = -1
-  const uint32_t* L = W + (x * dim + y) * zc;
-  uint32_t bits = (b0 >= 0 && b0 < zc) ? __ldg(L + b0) >> s : 0u;
-  if (s > 29 && b0 + 1 < zc) bits |= __ldg(L + b0 + 1) << (32 - s);  // the three bits cross into the next word
-  return bits & 7u;
-}
-
-// Mode R's adjacency table in shared memory: per case and edge e, bits
-// [5 e, 5 e + 5) mark the triangles that use e.
-struct SmemTabs {
-  uint64_t etris[256];
-};
-template <int MODE>
-__device__ __forceinline__ void load_tabs(SmemTabs& t) {
-  if (MODE != 0) return;
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) t.etris[i] = g_edge_tris.w[i];
-  __syncthreads();
-}
-
-// The adjacency list of one vertex (key: its packed grid position; edges: Mode Q,
-// its edges with a quad) of chunk ch, at most room entries, into out.
+// The adjacency list of one vertex (key: its packed grid position; bits: its
+// MeshOut::vadj) of chunk ch, at most room entries, into out.  An entry is its
+// word's first primitive plus its rank in the word: one 16-byte record of the emit
+// per cell (Mode R) or quad (Mode Q).
 // OUT = uint16_t with rel = the chunk's first primitive: the list holds
 // chunk-relative ids (the chunk-by-chunk sweeps, for chunks of at most 65535
 // primitives: half the bytes in the gathers' working set).
+// Rebuilding the crossings around the vertex from the occupancy words instead was
+// 80% of the instructions of a Mode Q mesh's sweeps, at 18 lanes each: k_sweep_chunks
+// on 512 x 65^3, eight sweeps, 1090 us against 689, a 512-chunk QEF update, four, 750
+// against 402; in Mode R (23 words against 4 records) a 4096-chunk update, four sweeps,
+// 4250 against 4090.
 template <int MODE, typename OUT = uint32_t>
-__device__ __forceinline__ void adj_vertex(const SmemTabs& T, const ChunkDev& ch, const uint32_t* __restrict__ words,
-                                           const WordScratch& ws, uint32_t key, uint32_t edges,
+__device__ __forceinline__ void adj_vertex(const ChunkDev& ch, const WordScratch& ws, uint32_t key, uint32_t bits,
                                            OUT* __restrict__ out, int room, int64_t rel = 0) {
   const int dim = ch.dim, zc = ch.zc;
-  const int64_t iout = ch.iout;
-  const uint32_t* W = words + ch.words;
-  const uint32_t* ibase = ws.icnt + ch.words;
-  const uint32_t* pl = ws.gpl + 3 * ch.words;  // (Mode R: ibase holds primitive bases by now)
   int x, y, z, k;
   vertex_key_decode(key, x, y, z, k);
+  // (a vertex past the work list's capacity has no key: stay inside the chunk)
+  if (max(x, max(y, z)) > dim - (MODE == 0 ? 1 : 2)) return;
   // the chunk's first primitive (its index offset and word bases are
   // multiples of the primitive size)
-  const int64_t pbase = iout / (MODE == 0 ? 3 : 4);
+  const int64_t pbase = ch.iout / (MODE == 0 ? 3 : 4) - rel;
   int n = 0;
   if (MODE == 0) {
-    const int a = k;
-    // inside bits of lines (x-1+i, y-1+j), samples z-1..z+1, packed 3 bits per
-    // line at bit 3 (3i + j): every corner of the four cells around the edge
-    uint32_t nbits = 0u;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j)
-        if (a == 0 ? i >= 1 : (a == 1 ? j >= 1 : true))
-          nbits |= line_bits3(W, dim, zc, x - 1 + i, y - 1 + j, z - 1) << (3 * (3 * i + j));
+    const uint4* P = ws.rec + ch.words;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {  // cells around the edge, ascending linear order
+      uint32_t tm = (bits >> (5 * q)) & 31u;  // the cell's triangles that use the edge, ascending
       const int d1 = (q >> 1) ^ 1, d2 = (q & 1) ^ 1;
-      int ox = 0, oy = 0, oz = 0;
-      if (a == 0) { oy = -d1; oz = -d2; }
-      else if (a == 1) { ox = -d1; oz = -d2; }
-      else { ox = -d1; oy = -d2; }
-      const int e = 4 * a + 2 * d1 + d2;
-      const int cx = x + ox, cy = y + oy, cz = z + oz;
-      if (cx < 0 || cy < 0 || cz < 0 || cx > dim - 2 || cy > dim - 2 || cz > dim - 2) continue;
-      // corner (dx, dy, dz): line (1 + ox + dx, 1 + oy + dy), bit 1 + oz + dz
-      const uint32_t base = nbits >> (3 * (3 * (1 + ox) + (1 + oy)) + 1 + oz);
-      const int m = (int)((base & 3u) | (((base >> 3) & 3u) << 2) | (((base >> 9) & 3u) << 4) |
-                          (((base >> 12) & 3u) << 6));
-      // the cell's triangles that use edge e, ascending (polygonize_cell order)
-      uint32_t tm = (uint32_t)(T.etris[m] >> (5 * e)) & 31u;
-      if (!tm) continue;
-      const int wi = (cx * dim + cy) * zc + (cz >> 5);
+      const int cx = x - (k == 0 ? 0 : d1), cy = y - (k == 0 ? d1 : (k == 1 ? 0 : d2)), cz = z - (k == 2 ? 0 : d2);
+      if (tm == 0u || (cx | cy | cz) < 0) continue;
+      const uint4 r = __ldg(P + ((cx * dim + cy) * zc + (cz >> 5)));
       const uint32_t lt = lane_lt(cz & 31);
-      const uint32_t pre = __popc(__ldg(pl + 3 * wi) & lt) + 2 * __popc(__ldg(pl + 3 * wi + 1) & lt) +
-                           4 * __popc(__ldg(pl + 3 * wi + 2) & lt);
-      const int64_t first = pbase + __ldg(ibase + wi) + pre;
-      for (; tm && n < room; tm &= tm - 1u) out[n++] = (OUT)(first + __ffs(tm) - 1 - rel);
+      const int64_t first = pbase + r.w + __popc(r.x & lt) + 2 * __popc(r.y & lt) + 4 * __popc(r.z & lt);
+      for (; tm && n < room; tm &= tm - 1u) out[n++] = (OUT)(first + __ffs(tm) - 1);
     }
   } else {
-    // The vertex's edges with a quad, ascending by the quad's id; a quad's id is its
-    // rank in the owner sample's word, one 16-byte record of the emit.  (Rebuilding
-    // the crossings of the owner's word for each of the 12 edges in turn cost 80% of
-    // the sweeps' instructions at 18 lanes each: k_sweep_chunks on 512 x 65^3, eight
-    // sweeps, 1090 us against 789; a 512-chunk QEF update, four, 750 against 501.)
-    if (x > dim - 2 || y > dim - 2 || z > dim - 2) return;  // a vertex past the work list's capacity has no key
     constexpr uint64_t kCorner = 0x654432211000ull;  // owner sample 4 dx + 2 dy + dz per edge in quad order
     constexpr uint32_t kAxis = 0x992124u;            // and axis
     const uint4* Q = ws.quads + ch.words;
 #pragma unroll 1
-    for (uint32_t set = edges; set; set &= set - 1u) {
+    for (uint32_t set = bits & 0xFFFu; set; set &= set - 1u) {
       const int i = __ffs(set) - 1, c0 = (int)(kCorner >> (4 * i)) & 7, a = (int)(kAxis >> (2 * i)) & 3;
       const int sz = z + (c0 & 1);
-      const uint4 q = __ldcg(Q + (((x + (c0 >> 2)) * dim + (y + ((c0 >> 1) & 1))) * zc + (sz >> 5)));
+      const uint4 q = __ldg(Q + (((x + (c0 >> 2)) * dim + (y + ((c0 >> 1) & 1))) * zc + (sz >> 5)));
       const int l = sz & 31;
       const uint32_t bit = 1u << l, lt = bit - 1u, lx = a >= 1 ? lt | bit : lt, ly = a >= 2 ? lt | bit : lt;
       const uint32_t pre = __popc(q.x & lx) + __popc(q.y & ly) + __popc(q.z & lt);
-      if (n < room) out[n++] = (OUT)(pbase + q.w + pre - rel);
+      if (n < room) out[n++] = (OUT)(pbase + q.w + pre);
     }
   }
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256) k_adj_build(const ChunkDev* __restrict__ chunks, int n_chunks,
-                                                   const uint32_t* __restrict__ words, WordScratch ws,
+__global__ void __launch_bounds__(256) k_adj_build(const ChunkDev* __restrict__ chunks, int n_chunks, WordScratch ws,
                                                    const uint32_t* __restrict__ vkey,
-                                                   const uint16_t* __restrict__ vedge, const uint32_t* __restrict__ off,
+                                                   const uint32_t* __restrict__ vadj, const uint32_t* __restrict__ off,
                                                    const int64_t* __restrict__ d_counts, int64_t vcap,
                                                    uint32_t* __restrict__ adj) {
-  __shared__ SmemTabs T;
-  load_tabs<MODE>(T);
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= (d_counts ? min(vcap, d_counts[0]) : vcap)) return;
   const int c = find_chunk_by_vertex(chunks, n_chunks, v);
   // the vertex's CSR range (the exclusive scan of init_valence): never write past it
-  adj_vertex<MODE>(T, chunks[c], words, ws, vkey[v], MODE ? vedge[v] : 0u, adj + off[v], (int)(off[v + 1] - off[v]));
+  adj_vertex<MODE>(chunks[c], ws, vkey[v], vadj[v], adj + off[v], (int)(off[v + 1] - off[v]));
 }
 
-void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, WordScratch ws,
-                      const uint32_t* vkey, const uint16_t* vedge, const uint32_t* off, const int64_t* d_counts,
+void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, WordScratch ws, const uint32_t* vkey,
+                      const uint32_t* vadj, const uint32_t* off, const int64_t* d_counts,
                       int64_t vcap, uint32_t* adj, cudaStream_t st) {
   const int blocks = (int)((vcap + 255) / 256);
   if (blocks == 0) return;
-  if (mode == 0) k_adj_build<0><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, vedge, off, d_counts, vcap, adj);
-  else k_adj_build<1><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, words, ws, vkey, vedge, off, d_counts, vcap, adj);
+  if (mode == 0) k_adj_build<0><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, ws, vkey, vadj, off, d_counts, vcap, adj);
+  else k_adj_build<1><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, ws, vkey, vadj, off, d_counts, vcap, adj);
 }
 
 // ---------------------------------------------------------------------------
@@ -921,10 +867,9 @@ struct SweepArgs {
   const ChunkDev* __restrict__ chunks;
   const uint32_t* __restrict__ tot;
   SweepLists lists;
-  const uint32_t* __restrict__ words;
   WordScratch ws;
   const uint32_t* __restrict__ vkey;
-  const uint16_t* __restrict__ vedge;
+  const uint32_t* __restrict__ vadj;
   int64_t nv, n_prims, adj_cap;
   const int64_t* __restrict__ d_counts;
   uint32_t* __restrict__ off;
@@ -1013,20 +958,17 @@ __device__ __forceinline__ void sweep_older(const SweepArgs& A, ChunkPart c, int
 template <int MODE, int N>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
     const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, SweepLists lists,
-    const uint32_t* __restrict__ words, WordScratch ws, const uint32_t* __restrict__ vkey,
-    const uint16_t* __restrict__ vedge, int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
+    WordScratch ws, const uint32_t* __restrict__ vkey, const uint32_t* __restrict__ vadj, int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
     const uint8_t* __restrict__ valence, uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary,
     const uint32_t* __restrict__ idx, SweepBufs b_, float* __restrict__ dual_p, float* __restrict__ dual_n, int iters,
     int process_boundary, int sn, int wide_adj) {
-  const SweepArgs A{chunks, tot, lists, words, ws, vkey, vedge, nv, n_prims, adj_cap, d_counts, off, valence, adj, boundary,
+  const SweepArgs A{chunks, tot, lists, ws, vkey, vadj, nv, n_prims, adj_cap, d_counts, off, valence, adj, boundary,
                     idx, b_, dual_p, dual_n, iters, process_boundary, sn, wide_adj};
   constexpr int kThreads = kSweepThreads, kWarps = kThreads / 32;
-  __shared__ SmemTabs T;
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_total;
   __shared__ uint32_t s_item;
   __shared__ uint32_t s_seg[8];  // valence sum of each CTA's vertices
-  load_tabs<MODE>(T);
   cluster_barrier();  // every CTA of the cluster has started before its shared memory is written
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_big = A.lists.head[0], n_list = A.lists.head[1];
@@ -1127,10 +1069,10 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
       const uint32_t o = A.off[v];
       const int room = (int)max((int64_t)0, min((int64_t)__ldg(A.valence + v), A.adj_cap - (int64_t)o));
       if (compact)
-        adj_vertex<MODE, uint16_t>(T, ch, A.words, A.ws, __ldg(A.vkey + v), MODE ? __ldg(A.vedge + v) : 0u,
+        adj_vertex<MODE, uint16_t>(ch, A.ws, __ldg(A.vkey + v), __ldg(A.vadj + v),
                                    const_cast<uint16_t*>(sweep_list<uint16_t>(A, c, o)), room, (int64_t)c.p0);
       else
-        adj_vertex<MODE>(T, ch, A.words, A.ws, __ldg(A.vkey + v), MODE ? __ldg(A.vedge + v) : 0u, A.adj + o, room);
+        adj_vertex<MODE>(ch, A.ws, __ldg(A.vkey + v), __ldg(A.vadj + v), A.adj + o, room);
     }
     for (int m = 0; m < A.iters; ++m) {
       const SweepStep st = sweep_step(m, A.iters, A.sn, A.b.keep(), A.b);
@@ -1169,10 +1111,9 @@ constexpr int kTeamRegs = 6;     // list entries gathered at once (and kept for 
 struct TeamArgs {
   const ChunkDev* chunks;
   int n_chunks;
-  const uint32_t* words;
   WordScratch ws;
   const uint32_t* vkey;
-  const uint16_t* vedge;
+  const uint32_t* vadj;
   int64_t nv, n_prims;
   const int64_t* d_counts;
   uint32_t* off;
@@ -1220,7 +1161,6 @@ __device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed,
 template <int MODE, int N>
 __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_constant__ TeamArgs A) {
   constexpr int kWarps = kTeamThreads / 32;
-  __shared__ SmemTabs T;
   __shared__ uint32_t s_warp[kWarps], s_total;
   const uint32_t nv = (uint32_t)(A.d_counts ? min(A.nv, A.d_counts[0]) : A.nv);
   const uint32_t np = (uint32_t)(A.d_counts ? min(A.n_prims, A.d_counts[1] / N) : A.n_prims);
@@ -1231,7 +1171,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
     if (threadIdx.x == 0) *(volatile unsigned*)A.host_failed = 1u;
     return;
   }
-  load_tabs<MODE>(T);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
   const int iters = A.iters;
   unsigned target = 0;
@@ -1274,8 +1213,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
       const uint32_t o = carry + s_warp[warp] + incl - x;
       A.off[v] = o;
       const int room = o < cap ? (int)min(x, cap - o) : 0;
-      adj_vertex<MODE>(T, A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.words, A.ws, __ldg(A.vkey + v),
-                       MODE ? __ldg(A.vedge + v) : 0u, A.adj + o, room);
+      adj_vertex<MODE>(A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.ws, __ldg(A.vkey + v),
+                       __ldg(A.vadj + v), A.adj + o, room);
     }
     carry += s_total;
     __syncthreads();
@@ -1366,7 +1305,7 @@ void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_pri
                        float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
                        int iters, int process_boundary, int smooth_normals, const ProcessScratch& s,
                        cudaStream_t st) {
-  TeamArgs A{sa.chunks, sa.n_chunks, sa.words, sa.ws, sa.vkey, sa.vedge, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
+  TeamArgs A{sa.chunks, sa.n_chunks, sa.ws, sa.vkey, sa.vadj, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
              idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
              smooth_normals, sa.team, sa.team_failed};
   cudaLaunchConfig_t cfg{};
@@ -1410,7 +1349,7 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st) {
-  SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.words, sa.ws, sa.vkey, sa.vedge, nv, n_prims, n_prims * N, d_counts, s.off,
+  SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.ws, sa.vkey, sa.vadj, nv, n_prims, n_prims * N, d_counts, s.off,
               valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters,
               process_boundary, smooth_normals, sa.wide_adj ? 1 : 0};
   cudaLaunchConfig_t cfg{};
@@ -1424,7 +1363,7 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   const auto go = [&](auto kernel) {
-    cudaLaunchKernelEx(&cfg, kernel, A.chunks, A.tot, A.lists, A.words, A.ws, A.vkey, A.vedge, A.nv, A.n_prims,
+    cudaLaunchKernelEx(&cfg, kernel, A.chunks, A.tot, A.lists, A.ws, A.vkey, A.vadj, A.nv, A.n_prims,
                        A.adj_cap,
                        A.d_counts, A.off, A.valence, A.adj, A.boundary, A.idx, A.b, A.dual_p, A.dual_n, A.iters,
                        A.process_boundary, A.sn, A.wide_adj);
@@ -1556,6 +1495,14 @@ __device__ __forceinline__ void stage_async(uint32_t* dst, const uint32_t* src) 
   *dst = __ldg(src);
 #endif
 }
+__device__ __forceinline__ void stage_async(uint4* dst, const uint4* src) {
+#if BMF_EMIT_ASYNC
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(src) : "memory");
+#else
+  *dst = __ldg(src);
+#endif
+}
 __device__ __forceinline__ void stage_wait() {
 #if BMF_EMIT_ASYNC
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -1563,8 +1510,8 @@ __device__ __forceinline__ void stage_wait() {
 }
 
 struct RTile {
+  uint4 rec[kTileWords];  // the words' records, the last with the plane's base added
   NbCache nb[kTileWords];
-  uint32_t ib[kTileWords], p0[kTileWords], p1[kTileWords], p2[kTileWords];
   uint32_t X[kTileWords], Y[kTileWords], Z[kTileWords];
   int x[kTileWords], y[kTileWords], zb[kTileWords], dim[kTileWords], zc[kTileWords];
   int64_t cw[kTileWords], dens[kTileWords], vout[kTileWords], iout[kTileWords];
@@ -1616,7 +1563,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
                                                                  const uint32_t* __restrict__ words,
                                                                  const float* __restrict__ dens, WordScratch ws,
                                                                  MeshOut out) {
-  __shared__ uint64_t s_tri[256], s_uses[256];
+  __shared__ uint64_t s_tri[256], s_etris[256];
   __shared__ RTile s_tiles[kEmitWarps];
   const int64_t n = min((int64_t)*ws.ccount, ws.clist_cap);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1631,7 +1578,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
   if ((spread ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kEmitWarps) * tw >= n) return;  // no warp has a tile
   for (int i = threadIdx.x; i < 256; i += blockDim.x) {
     s_tri[i] = __ldg(g_tri_cases + i);
-    s_uses[i] = __ldg(g_edge_uses + i);
+    s_etris[i] = g_edge_tris.w[i];
   }
   __syncthreads();
   for (int64_t t0 = w0 * tw; t0 < n; t0 += nwarps * tw) {
@@ -1696,10 +1643,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
     }
     if (lane < nt) {
       const int64_t wi = R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane];
-      stage_async(&R.ib[lane], ws.icnt + wi);
-      stage_async(&R.p0[lane], ws.gpl + 3 * wi);
-      stage_async(&R.p1[lane], ws.gpl + 3 * wi + 1);
-      stage_async(&R.p2[lane], ws.gpl + 3 * wi + 2);
+      stage_async(&R.rec[lane], ws.rec + wi);
     }
     stage_wait();
     __syncwarp();
@@ -1710,15 +1654,15 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
       if (lane < nt) {
         NbCache& nb = R.nb[lane];
         // word bases: within the plane + the plane's
-        const uint32_t ib = R.ib[lane] + pb0.y;
+        const uint32_t ib = R.rec[lane].w + pb0.y;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           nb.vb[k] += pb0.x;
           nb.vb[4 + k] += pv1;
         }
-        R.ib[lane] = ib;
+        R.rec[lane].w = ib;
         if (out.vkey)  // the adjacency build reads the word's primitive base
-          ws.icnt[R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane]] = ib / 3u;
+          ws.rec[R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane]].w = ib / 3u;
         const int dim = R.dim[lane], x = R.x[lane], y = R.y[lane], zb = R.zb[lane];
         const uint32_t wc = nb.w[(1 * 4 + 1) * 3 + 1];
         const uint32_t X = (x + 1 < dim) ? wc ^ nb.w[(2 * 4 + 1) * 3 + 1] : 0u;
@@ -1745,7 +1689,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
           R.oz_[lane][q] = Zq;
         }
         const uint32_t nv = __popc(X) + __popc(Y) + __popc(Z);
-        const uint32_t ntri = __popc(R.p0[lane]) + 2u * __popc(R.p1[lane]) + 4u * __popc(R.p2[lane]);
+        const uint32_t ntri = __popc(R.rec[lane].x) + 2u * __popc(R.rec[lane].y) + 4u * __popc(R.rec[lane].z);
         packed = nv | (ntri << 16);  // at most 96 and 160 per word
       }
       uint32_t incl = packed;
@@ -1816,9 +1760,9 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
             const uint64_t q = ((uint64_t)w[b + 1] << 32) | w[b];
             nbits |= ((uint32_t)(q >> (zr0 & 31)) & 7u) << (3 * (3 * i + jj));
           }
-        // init_valence: uses of this edge by the (up to) four interior cells
-        // around it (polygonize skips far-face cells, DMCChunk.cpp:528)
-        int val = 0;
+        // init_valence: the triangles that use this edge in the (up to) four interior
+        // cells around it (polygonize skips far-face cells, DMCChunk.cpp:528)
+        uint32_t bits = 0u;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const int d1 = c >> 1, d2 = c & 1;
@@ -1826,9 +1770,10 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
           const int e = 4 * a + 2 * d1 + d2;
           const int cx = x + ox, cy = y + oy, cz = z + oz;
           if (cx < 0 || cy < 0 || cz < 0 || cx > dim - 2 || cy > dim - 2 || cz > dim - 2) continue;
-          val += (int)((s_uses[packed_mask(nbits, ox, oy, oz)] >> (4 * e)) & 0xF);
+          bits |= ((uint32_t)(s_etris[packed_mask(nbits, ox, oy, oz)] >> (5 * e)) & 31u) << (5 * (3 - c));
         }
-        out.valence[gv] = (uint8_t)val;
+        out.valence[gv] = (uint8_t)__popc(bits);
+        if (out.vadj) out.vadj[gv] = bits;
       }
     }
     // 5. one lane per triangle: the k-th triangle of word t is in the cell l
@@ -1837,7 +1782,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
     for (int j = lane; j < ntt; j += 32) {
       const int t = tile_word(R.toff, nt, j);
       const int k = j - R.toff[t];
-      const uint32_t c0 = R.p0[t], c1 = R.p1[t], c2 = R.p2[t];
+      const uint32_t c0 = R.rec[t].x, c1 = R.rec[t].y, c2 = R.rec[t].z;
       int l = 0;
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1) {
@@ -1858,7 +1803,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
       const uint64_t tw = s_tri[mask];
       if (3 * r + 3 > 3 * (int)(tw >> 60)) continue;  // the planes and the case table agree
       const int z = 32 * R.zb[t] + l;
-      const int64_t gi = R.iout[t] + (int64_t)R.ib[t] + 3 * (int64_t)k;
+      const int64_t gi = R.iout[t] + (int64_t)R.rec[t].w + 3 * (int64_t)k;
       const int64_t vout = R.vout[t];
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
@@ -1888,8 +1833,9 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
 // thread-per-cell form it replaces read each quad's four cells from global
 // memory behind bounds checks (512 x 65^3 fitting grids: 607 us).
 struct QTile {
+  uint4 rec[kTileWords][8];        // [2i+j][b]: record of cell line (x-1+i, y-1+j), block zb-1+b
   uint32_t w[kTileWords][27];      // [i][j][b]: line (x-1+i, y-1+j), block zb-1+b
-  uint32_t cv[kTileWords][8][4];   // [2i+j][b]: cell line (x-1+i, y-1+j), block zb-1+b: vertex base, planes
+  uint32_t vb[kTileWords][8];      // and its vertex base
   uint32_t ib[kTileWords], X[kTileWords], Y[kTileWords], Z[kTileWords];
   int x[kTileWords], y[kTileWords], zb[kTileWords], dim[kTileWords], zc[kTileWords];
   int64_t cw[kTileWords], dens[kTileWords], vout[kTileWords], iout[kTileWords];
@@ -1972,15 +1918,8 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
       const int xx = R.x[t] - 1 + (l >> 2), yy = R.y[t] - 1 + ((l >> 1) & 1);
       if (xx < 0 || yy < 0 || zb < 0) continue;  // no cell there: never read
       const int64_t wi = R.cw[t] + (xx * dim + yy) * zc + zb;
-      uint32_t* dst = R.cv[t][l];
-      stage_async(dst, ws.vcnt + wi);
-      stage_async(dst + 1, ws.gpl + 3 * wi);
-      stage_async(dst + 2, ws.gpl + 3 * wi + 1);
-      stage_async(dst + 3, ws.gpl + 3 * wi + 2);
-    }
-    if (lane < nt) {
-      const int64_t wi = R.cw[lane] + (R.x[lane] * R.dim[lane] + R.y[lane]) * R.zc[lane] + R.zb[lane];
-      stage_async(&R.ib[lane], ws.icnt + wi);
+      stage_async(&R.vb[t][l], ws.vcnt + wi);
+      stage_async(&R.rec[t][l], ws.rec + wi);
     }
     stage_wait();
     __syncwarp();
@@ -2002,13 +1941,13 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
         R.Z[lane] = Z;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-          R.cv[lane][b][0] += pv0;
-          R.cv[lane][4 + b][0] += pb1.x;
+          R.vb[lane][b] += pv0;
+          R.vb[lane][4 + b] += pb1.x;
         }
-        R.ib[lane] += pb1.y;
+        const uint4 own = R.rec[lane][7];
+        R.ib[lane] = own.w + pb1.y;
         if (ws.quads) ws.quads[R.cw[lane] + (x * dim + R.y[lane]) * R.zc[lane] + zb] = make_uint4(X, Y, Z, R.ib[lane] / 4u);
-        const uint32_t* own = R.cv[lane][7];
-        const uint32_t nv = __popc(own[1]) + 2u * __popc(own[2]) + 4u * __popc(own[3]);
+        const uint32_t nv = __popc(own.x) + 2u * __popc(own.y) + 4u * __popc(own.z);
         packed = nv | ((__popc(X) + __popc(Y) + __popc(Z)) << 16);  // at most 128 and 96 per word
       }
       uint32_t incl = packed;
@@ -2032,8 +1971,8 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
       bool in = j < nvt;
       const int t = tile_word(R.voff, nt, in ? j : 0);
       const int k = in ? j - R.voff[t] : 0;
-      const uint32_t* own = R.cv[t][7];
-      const uint32_t c0 = own[1], c1 = own[2], c2 = own[3];
+      const uint4 own = R.rec[t][7];
+      const uint32_t c0 = own.x, c1 = own.y, c2 = own.z;
       int l = 0;
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1) {
@@ -2042,7 +1981,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
       }
       const uint32_t lt = lane_lt(l);
       const int g = k - (int)(__popc(c0 & lt) + 2 * __popc(c1 & lt) + 4 * __popc(c2 & lt));
-      const int64_t gv = R.vout[t] + (int64_t)own[0] + k;
+      const int64_t gv = R.vout[t] + (int64_t)R.vb[t][7] + k;
       in = in && gv < out.vcap;
       const int dim = R.dim[t], x = R.x[t], y = R.y[t], z = 32 * R.zb[t] + l;
       const int mask = qtile_mask(R.w[t], 1, 1, 32 + l);
@@ -2073,7 +2012,7 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
           cut(z > 0, kQuadDz0);
           cut(z + 1 <= dim - 2, kQuadDz1);
           out.valence[gv] = (uint8_t)__popc(set);
-          if (out.vedge) out.vedge[gv] = (uint16_t)set;
+          if (out.vadj) out.vadj[gv] = set;
         }
       }
       __syncwarp();
@@ -2107,9 +2046,10 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
         const int e = a == 0 ? 2 * dy + dz : (a == 1 ? 4 + 2 * dx + dz : 8 + 2 * dx + dy);
         const int i = 1 - dx, jj = 1 - dy, zr = 32 + l - dz;
         const int m = qtile_mask(w, i, jj, zr);
-        const uint32_t* cv = R.cv[t][(i * 2 + jj) * 2 + (zr >> 5)];
+        const int at = (i * 2 + jj) * 2 + (zr >> 5);
+        const uint4 cv = R.rec[t][at];
         const uint32_t ct = lane_lt(zr & 31);
-        q[c] = cv[0] + __popc(cv[1] & ct) + 2 * __popc(cv[2] & ct) + 4 * __popc(cv[3] & ct) +
+        q[c] = R.vb[t][at] + __popc(cv.x & ct) + 2 * __popc(cv.y & ct) + 4 * __popc(cv.z & ct) +
                (uint32_t)((s_grp[m] >> (4 * e)) & 0xF);
       }
       if (!((w[13] >> l) & 1u)) {  // lower sample outside: reversed

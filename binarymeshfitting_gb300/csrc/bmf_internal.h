@@ -41,9 +41,11 @@ struct MeshOut {
   // k = crossing axis (Mode R) or vertex group (Mode Q); the key the analytic
   // adjacency build starts from.
   uint32_t* vkey = nullptr;
-  // optional (Mode Q): per vertex the edges of its group that have a quad, as a
-  // 12-bit set in quad order (valence is its size); the adjacency reads it
-  uint16_t* vedge = nullptr;
+  // optional: per vertex what the adjacency starts from (valence is its number of
+  // bits).  Mode R: the triangles that use it in each of the four cells around its
+  // edge, 5 bits per cell, ascending; Mode Q: the edges of its group that have a
+  // quad, 12 bits in quad order.
+  uint32_t* vadj = nullptr;
   // optional (QEF placement with keys): the record the QEF adjoint reads --
   // per vertex whether it took the QEF branch, the list of those vertices
   // (count in *qcount) and their FP32 eigenvectors (9 floats per entry)
@@ -56,12 +58,13 @@ struct MeshOut {
 // Per-word scratch of the extraction kernels, indexed like the occupancy
 // words (chunk.words + (x*dim + y)*zc + zb).
 struct WordScratch {
-  // The count kernel writes these three for busy words only (words that own a
+  // The count kernel writes these two for busy words only (words that own a
   // vertex or emit a primitive); nothing reads them for any other word.
-  uint32_t* vcnt;   // vertices of the x-plane's words before this one (a word's base is pb[plane].x + vcnt)
-  uint32_t* icnt;   // indices of the x-plane's words before this one; Mode R's emit replaces it by the word's
-                    // chunk-local primitive base, which the adjacency reads
-  uint32_t* gpl;    // 3 bit-planes of the per-cell triangle (Mode R) / vertex-group (Mode Q) count
+  uint32_t* vcnt;  // vertices of the x-plane's words before this one (a word's base is pb[plane].x + vcnt)
+  // {3 bit-planes of the per-cell triangle (Mode R) / vertex-group (Mode Q) count,
+  // indices of the x-plane's words before this one}; Mode R's emit replaces the
+  // last by the word's first primitive (of the chunk), for the adjacency
+  uint4* rec;
   // Work list (nullable) of the busy words (those that own a vertex or emit a
   // primitive) as {chunk, word index in the chunk}, in no particular order;
   // *ccount (zeroed before the count kernel) entries, at most clist_cap kept:
@@ -272,10 +275,9 @@ struct StructuredAdj {
   int mode;                  // BMF_MODE_R / BMF_MODE_Q
   const ChunkDev* chunks;    // with vout / iout set
   int n_chunks;
-  const uint32_t* words;
-  WordScratch ws;            // scanned counts + per-word bit-planes
+  WordScratch ws;            // scanned counts + per-word records
   const uint32_t* vkey;      // per-vertex keys written by the emit kernel
-  const uint16_t* vedge;     // Mode Q: MeshOut::vedge (and ws.quads)
+  const uint32_t* vadj;      // MeshOut::vadj
   // optional (tot and lists.order, or neither): the sweeps run chunk by chunk
   const uint32_t* tot = nullptr;  // per chunk {vertices, indices}
   SweepLists lists;               // filled by launch_chunk_scan
@@ -287,8 +289,8 @@ struct StructuredAdj {
   // adjacency (the fit's adjoint sweeps want 32-bit mesh-wide ids)
   bool wide_adj = false;
 };
-void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, WordScratch ws,
-                      const uint32_t* vkey, const uint16_t* vedge, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
+void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, WordScratch ws, const uint32_t* vkey,
+                      const uint32_t* vadj, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
                       uint32_t* adj, cudaStream_t st);
 // The chunk-by-chunk form of launch_process for StructuredAdj with tot and
 // lists set: CSR offsets, adjacency and all sweeps in one launch.

@@ -41,10 +41,10 @@ namespace {
 constexpr int kNoAllocMaxDim = BMF_NOALLOC_MAX_DIM;
 constexpr int64_t kMaxWords = (int64_t)kNoAllocMaxDim * kNoAllocMaxDim * ((kNoAllocMaxDim + 31) / 32);
 // Layout (u32 units): [0, 64) chunk record + unit range + flags + chunk totals
-// + device totals; then the plane bases (2 per x-plane), vcnt, icnt and the 3
-// bit-planes, one entry per word.
+// + device totals; then the plane bases (2 per x-plane), the word records (4 per
+// word) and vcnt, one entry per word.
 constexpr int64_t kHeader = 64;
-constexpr int64_t kPlanes = kHeader + 2 * kNoAllocMaxDim;
+constexpr int64_t kPlanes = (kHeader + 2 * kNoAllocMaxDim + 3) / 4 * 4;
 constexpr int64_t kScratchWords = kPlanes + 5 * kMaxWords;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kScratchWords];
@@ -91,7 +91,8 @@ extern "C" bmf_status bmf_polygonize_noalloc(int32_t dim, const float* d_density
   int64_t* d_totals = (int64_t*)(base + 40);            // [40, 46), 8-byte aligned
   const int zc = (dim + 31) / 32;
   const int64_t nw = (int64_t)dim * dim * zc;
-  WordScratch ws{base + kPlanes, base + kPlanes + nw, base + kPlanes + 2 * nw};
+  static_assert(kPlanes % 4 == 0, "word records are 16-byte aligned");
+  WordScratch ws{base + kPlanes + 4 * nw, (uint4*)(base + kPlanes)};
   ws.pb = (uint2*)(base + kHeader);
 
   ChunkDev c{};
