@@ -1292,6 +1292,7 @@ struct bmf_fit {
   uint8_t *d_valence = nullptr, *d_boundary = nullptr;
   uint32_t* d_vadj = nullptr;
   float* d_g = nullptr;           // position-gradient work buffer
+  float* d_h = nullptr;           // and its scaled form between the adjoint's sweeps (4 per vertex)
   SweepLists sweep;               // the chunk-by-chunk sweeps' work lists, and the adjoint's queue over them
   int* d_pqueue = nullptr;
   SweepForm form = kSweepLaunches;  // the forward's sweeps
@@ -1312,7 +1313,7 @@ bmf_status bmf_fit_destroy(bmf_fit* f) {
   if (!f) return BMF_ERR_INVALID_ARGUMENT;
   void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.rec,
                   f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
-                  f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
+                  f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_h, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
                   f->d_pqueue, f->d_vadj, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1379,6 +1380,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_vadj, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->ws.quads, sizeof(uint4) * words) == cudaSuccess &&
             cudaMalloc(&f->d_g, sizeof(float) * 3 * (vcap + 1)) == cudaSuccess &&
+            cudaMalloc(&f->d_h, sizeof(float) * 4 * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->d_qlist, sizeof(uint32_t) * (vcap + 1)) == cudaSuccess &&
             cudaMalloc(&f->sweep.order, sizeof(int) * (n_chunks + kSweepHead)) == cudaSuccess &&
             cudaMalloc(&f->d_pqueue, sizeof(int)) == cudaSuccess &&
@@ -1489,18 +1491,25 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_fit_backward: null buffer or no forward yet");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t ng = n_grad_verts < f->vcap ? n_grad_verts : f->vcap;
-  BMF_CUDA(ctx, cudaMemsetAsync(f->d_g, 0, sizeof(float) * 3 * f->vcap, st));
-  if (ng > 0)
-    BMF_CUDA(ctx, cudaMemcpyAsync(f->d_g, d_grad_pos, sizeof(float) * 3 * ng, cudaMemcpyDeviceToDevice, st));
   // with enough chunks to fill the GPU the adjoint sweeps run chunk by chunk
   StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->ws, f->d_vkey, f->d_vadj};
   if (f->n >= kChunkSweepBwdMinChunks) {
     sa.tot = f->d_tot;
     sa.lists = f->sweep;
     sa.bwd_queue = f->d_pqueue;
+  } else if (f->form == kSweepTeam) {
+    sa.team = f->team;
+    sa.team_failed = ctx->team_failed();
   }
-  int k = launch_process_bwd(4, f->vcap, f->icap / 4, f->d_totals, f->d_boundary, f->d_valence, f->d_idxg, f->iters,
-                             0, f->ps, f->d_g, &sa, st);
+  int k = 0;
+  if (f->iters > 0 && f->icap >= 4) {
+    k = launch_process_bwd(f->vcap, f->icap / 4, f->d_totals, f->d_boundary, f->d_valence, f->d_idxg, f->iters, 0,
+                           f->ps, d_grad_pos, ng, f->d_g, f->d_h, &sa, st);
+  } else {
+    BMF_CUDA(ctx, cudaMemsetAsync(f->d_g, 0, sizeof(float) * 3 * f->vcap, st));
+    if (ng > 0)
+      BMF_CUDA(ctx, cudaMemcpyAsync(f->d_g, d_grad_pos, sizeof(float) * 3 * ng, cudaMemcpyDeviceToDevice, st));
+  }
   BMF_CUDA(ctx, cudaMemsetAsync(d_grad_density, 0, sizeof(float) * (size_t)f->n * f->dim * f->dim * f->dim, st));
   const int wide = (f->flags & BMF_FIT_ADJOINT_F64) ? 1 : ((f->flags & BMF_FIT_ADJOINT_DF) ? 2 : 0);
   k += launch_place_bwd(f->placement, wide, f->d_chunks, f->n, f->d_words, f->last_density, f->d_vkey, f->d_totals,

@@ -1104,10 +1104,6 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
 // wrote), the sums in list order, and the barrier.  Values and order of the
 // sums are those of k_adj_build, k_dual and k_primal.
 // ---------------------------------------------------------------------------
-constexpr int kTeamThreads = 512;
-constexpr int kTeamVerts = 256;  // vertices per CTA that make the team one CTA larger
-constexpr int kTeamRegs = 6;     // list entries gathered at once (and kept for a thread's first vertex)
-
 struct TeamArgs {
   const ChunkDev* chunks;
   int n_chunks;
@@ -1127,36 +1123,6 @@ struct TeamArgs {
   TeamSync* sync;
   unsigned* host_failed;  // pinned host memory
 };
-
-// Barrier over the team's CTAs (all resident: a cooperative launch).  The wait
-// is bounded: after kTeamSpins polls (a second or so) or once another CTA has
-// given up, the CTA marks the team failed and no longer waits anywhere; the
-// host finds the mark after its synchronisation.  Thread 0 releases the CTA's
-// stores with its arrival and acquires the others' with its polls, and the block
-// barriers carry both to the other threads; sequentially consistent fences around
-// a relaxed arrival cost 0.3 us more a meeting (129^3 chunk: 117.8 against 113.8 us).
-constexpr unsigned kTeamSpins = 1u << 22;
-__device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed, unsigned& target, unsigned team,
-                                             bool& dead) {
-  __syncthreads();
-  target += team;
-  if (threadIdx.x == 0 && team > 1 && !dead) {
-    // release: the CTA's stores (ordered before by the block barrier) come before the arrival
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&y->arrived) : "memory");
-    unsigned v = 0;
-    for (unsigned spins = 0;; ++spins) {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&y->arrived) : "memory");
-      if (v >= target) break;
-      if (spins >= kTeamSpins || ((spins & 1023u) == 1023u && *(volatile unsigned*)&y->failed)) {
-        *(volatile unsigned*)&y->failed = 1u;
-        *(volatile unsigned*)host_failed = 1u;
-        dead = true;  // this CTA waits nowhere any more
-        break;
-      }
-    }
-  }
-  __syncthreads();
-}
 
 template <int MODE, int N>
 __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_constant__ TeamArgs A) {

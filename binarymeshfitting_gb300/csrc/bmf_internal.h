@@ -318,12 +318,14 @@ int lod_generate(const bmf_lod_params& p, bmf_chunk_desc* d_descs, int cap, int3
 int launch_format(const ChunkDev* d_chunks, int n_chunks, int64_t nv, int64_t ni, const int64_t* d_counts,
                   const float* pos, const float* nrm, const uint32_t* idx, int unwind, int smooth, float* p, float* n,
                   float* c, int64_t cap, cudaStream_t st);
-// Adjoint of the position sweeps of launch_process (needs its CSR in s.off /
-// s.adj; uses s.dual_p as scratch).  g holds dL/d(final positions) on entry and
-// dL/d(initial positions) on return.  Returns the number of kernels launched.
-int launch_process_bwd(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,
+// Adjoint of a Mode Q mesh's position sweeps (needs launch_process's CSR in s.off /
+// s.adj; uses s.dual_p and h, 4 * nv floats, as scratch): dL/d(initial positions)
+// into g from dL/d(final positions) of the first n_grad vertices (0 for the
+// others); n_prims > 0, iters > 0.  Returns the number of kernels launched.
+int launch_process_bwd(int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,
                        const uint8_t* valence, const uint32_t* idx, int iters, int process_boundary,
-                       const ProcessScratch& s, float* g, const StructuredAdj* sa, cudaStream_t st);
+                       const ProcessScratch& s, const float* grad, int64_t n_grad, float* g, float* h,
+                       const StructuredAdj* sa, cudaStream_t st);
 // Adjoint of Mode Q placement (placement 1 mass point, 2 QEF); accumulates into
 // grad_dens (the caller clears it).  wide (QEF): 0 FP32 adjoint, 1 the QEF
 // derivative from an FP64 re-solve, 2 from a double-float re-solve; these read

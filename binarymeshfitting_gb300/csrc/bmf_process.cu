@@ -298,77 +298,154 @@ int launch_format(const ChunkDev* d_chunks, int n_chunks, int64_t nv, int64_t ni
 // transposes, last sweep first.  Both transposes are gathers (per primitive /
 // per vertex through the CSR), so they need no atomics.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ bool primal_updates(const uint8_t* valence, const uint8_t* boundary, int64_t v,
-                                               int process_boundary) {
-  return valence[v] != 0 && (process_boundary || !boundary[v]);
-}
+//
+// What the gathers read is stored ready for them, as float4: h[v] = g[v] / count(v)
+// (0 for a vertex that is not updated) and g_dual[t] / N.  A primitive then
+// sums four 16-byte gathers and a vertex its list's, instead of three 4-byte
+// gathers, a valence, a boundary flag and a division per corner; the products
+// and the order of the sums are the same.  Quads only (Mode Q).  Eight sweeps of
+// 512 x 65^3: 780 -> 650 us chunk by chunk, bound by the L1's wavefronts; of one 65^3
+// grid: sixteen launches of 4 us and the gaps between them -> 27 us as a team.
+struct BwdArgs {
+  int64_t nv, n_prims;
+  const int64_t* __restrict__ d_counts;
+  const uint32_t* __restrict__ off;
+  const uint8_t *__restrict__ valence, *__restrict__ boundary;
+  const uint32_t* __restrict__ adj;
+  const uint32_t* __restrict__ idx;  // mesh-wide
+  const float* __restrict__ grad;    // dL/d(final positions) of the first n_grad vertices (0 for the others)
+  int64_t n_grad;
+  float* g;       // dL/d(initial positions), and between the steps g of the vertices that are not updated
+  float4* h;      // g / count of the updated ones
+  float4* gd;     // g_dual / N
+  int iters, process_boundary;
+};
 
-// g_dual[t] = sum over the primitive's slots of g[v] / count(v), updated v only.
-template <int N>
-__global__ void k_primal_bwd(int64_t n_prims, int64_t nv, const int64_t* __restrict__ d_counts,
-                             const uint32_t* __restrict__ idx, const uint8_t* __restrict__ valence,
-                             const uint8_t* __restrict__ boundary, int process_boundary, const float* __restrict__ g,
-                             float* __restrict__ g_dual) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (d_counts ? min(n_prims, d_counts[1] / N) : n_prims)) return;
-  const int64_t nvb = d_counts ? min(nv, d_counts[0]) : nv;
+// Vertex v's list: its length on return; updated: whether the primal step moves it.
+__device__ __forceinline__ uint32_t bwd_list(const BwdArgs& A, uint32_t v, uint32_t cap, uint32_t& o, uint32_t& val,
+                                             bool& updated) {
+  o = __ldg(A.off + v);
+  val = __ldg(A.valence + v);
+  updated = val != 0u && (A.process_boundary || !__ldg(A.boundary + v));
+  return o < cap ? min(val, cap - o) : 0u;
+}
+__device__ __forceinline__ void bwd_put(const BwdArgs& A, uint32_t v, const float s[3], uint32_t val, bool updated,
+                                        bool last) {
+  if (updated && !last) {
+    const float inv = 1.0f / (float)val;
+    A.h[v] = make_float4(s[0] * inv, s[1] * inv, s[2] * inv, 0.0f);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) A.g[3 * (size_t)v + c] = s[c];
+  }
+}
+// Before the first step.
+__device__ __forceinline__ void bwd_begin(const BwdArgs& A, uint32_t v) {
+  float s[3] = {0.0f, 0.0f, 0.0f};
+  if ((int64_t)v < A.n_grad) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] = __ldg(A.grad + 3 * (size_t)v + c);
+  }
+  const uint32_t val = __ldg(A.valence + v);
+  const bool updated = val != 0u && (A.process_boundary || !__ldg(A.boundary + v));
+  if (!updated) A.h[v] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  bwd_put(A, v, s, val, updated, false);
+}
+// g_dual[t] / N from the sum over its corners.
+__device__ __forceinline__ void bwd_prim(const BwdArgs& A, uint32_t t, const uint4 v, uint32_t nv) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  float4 q[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) q[k] = w[k] < nv ? __ldca(A.h + w[k]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float s[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const uint32_t v = __ldg(idx + N * t + k);
-    if ((int64_t)v >= nvb || !primal_updates(valence, boundary, v, process_boundary)) continue;
-    const float inv = 1.0f / (float)valence[v];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) s[c] += __ldg(g + 3 * v + c) * inv;
+  for (int k = 0; k < 4; ++k) {
+    s[0] += q[k].x;
+    s[1] += q[k].y;
+    s[2] += q[k].z;
   }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) g_dual[3 * t + c] = s[c];
+  A.gd[t] = make_float4(s[0] * 0.25f, s[1] * 0.25f, s[2] * 0.25f, 0.0f);
 }
-
-// g[v] <- (updated(v) ? 0 : g[v]) + sum over t in adj(v) of g_dual[t] / N (in place).
-__global__ void k_dual_bwd(int N, int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts,
-                           const uint32_t* __restrict__ off, const uint8_t* __restrict__ valence,
-                           const uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary, int process_boundary,
-                           const float* __restrict__ g_dual, float* __restrict__ g) {
-  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= (d_counts ? min(nv, d_counts[0]) : nv)) return;
-  const int64_t room = adj_cap - (int64_t)off[v];
-  const uint32_t n = (uint32_t)max((int64_t)0, min((int64_t)valence[v], room));
+// s += the list's g_dual / N, kBwdGather at once, in list order; all lanes of the warp call it.
+constexpr int kBwdGather = 4;
+template <int G>
+__device__ __forceinline__ void bwd_sums(const BwdArgs& A, uint32_t o, uint32_t n, uint32_t np, float s[3],
+                                         const uint32_t* first = nullptr) {
+#pragma unroll 1
+  for (uint32_t k0 = 0; k0 < n; k0 += G) {
+    uint32_t t[G];
+    float4 q[G];
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+      t[k] = first && k0 == 0 ? first[k] : (k0 + k < n ? __ldg(A.adj + o + k0 + k) : 0xffffffffu);
+#pragma unroll
+    for (int k = 0; k < G; ++k) q[k] = t[k] < np ? __ldca(A.gd + t[k]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+      if (t[k] < np) {
+        s[0] += q[k].x;
+        s[1] += q[k].y;
+        s[2] += q[k].z;
+      }
+  }
+  __syncwarp();
+}
+// A backward primal step's vertex (whole warps; in: v is one).
+__device__ __forceinline__ void bwd_vert(const BwdArgs& A, uint32_t v, bool in, uint32_t cap, uint32_t np, bool last) {
+  uint32_t o = 0u, n = 0u, val = 0u;
+  bool updated = true;
   float s[3] = {0.0f, 0.0f, 0.0f};
-  if (!primal_updates(valence, boundary, v, process_boundary)) {
+  if (in) {
+    n = bwd_list(A, v, cap, o, val, updated);
+    if (!updated) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) s[c] = g[3 * v + c];
+      for (int c = 0; c < 3; ++c) s[c] = A.g[3 * (size_t)v + c];
+    }
   }
-  const float invN = 1.0f / (float)N;
-  for (uint32_t k = 0; k < n; ++k) {
-    const uint32_t t = __ldg(adj + off[v] + k);
-    if ((int64_t)t >= n_prims) continue;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) s[c] += __ldg(g_dual + 3 * t + c) * invN;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) g[3 * v + c] = s[c];
+  bwd_sums<kBwdGather>(A, o, n, np, s);
+  if (in) bwd_put(A, v, s, val, updated, last);
 }
 
-// Both transposes chunk by chunk: one CTA per chunk (from the queue) runs
-// every backward step of its chunk with block barriers in between -- a
-// chunk's primitives only read its own vertices and the reverse.  Per item the
-// operations are those of k_primal_bwd / k_dual_bwd, so the results are the
-// same; g and g_dual, which the kernel itself writes, are read with coherent
-// L1 loads.
+__device__ __forceinline__ void bwd_extent(const BwdArgs& A, uint32_t& nv, uint32_t& np) {
+  nv = (uint32_t)(A.d_counts ? min(A.nv, A.d_counts[0]) : A.nv);
+  np = (uint32_t)(A.d_counts ? min(A.n_prims, A.d_counts[1] / 4) : A.n_prims);
+}
+
+// The steps one launch each.
+__global__ void k_bwd_begin(BwdArgs A) {
+  uint32_t nv, np;
+  bwd_extent(A, nv, np);
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < nv) bwd_begin(A, v);
+}
+__global__ void k_primal_bwd(BwdArgs A) {
+  uint32_t nv, np;
+  bwd_extent(A, nv, np);
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < np) bwd_prim(A, t, __ldg(reinterpret_cast<const uint4*>(A.idx) + t), nv);
+}
+__global__ void k_dual_bwd(BwdArgs A, bool last) {
+  uint32_t nv, np;
+  bwd_extent(A, nv, np);
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  bwd_vert(A, v, v < nv, (uint32_t)min(4 * A.n_prims, (int64_t)UINT32_MAX), np, last);
+}
+
+// Chunk by chunk: one CTA per chunk (from the queue) runs every backward step
+// of its chunk with block barriers in between -- a chunk's primitives only
+// read its own vertices and the reverse.
 constexpr int kBwdChunkThreads = 512;
 
-template <int N>
-__global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(
-    const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, const int* __restrict__ order,
-    const int* __restrict__ head, int* __restrict__ queue, int64_t nv, int64_t n_prims, int64_t adj_cap,
-    const int64_t* __restrict__ d_counts, const uint32_t* __restrict__ off, const uint8_t* __restrict__ valence,
-    const uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary, int process_boundary,
-    const uint32_t* __restrict__ idx, float* __restrict__ g, float* __restrict__ g_dual, int iters) {
+__global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(const ChunkDev* __restrict__ chunks,
+                                                                         const uint32_t* __restrict__ tot,
+                                                                         const int* __restrict__ order,
+                                                                         const int* __restrict__ head,
+                                                                         int* __restrict__ queue,
+                                                                         const __grid_constant__ BwdArgs A) {
   __shared__ int s_item;
-  const int64_t nvb = d_counts ? min(nv, d_counts[0]) : nv;
-  const int64_t npb = d_counts ? min(n_prims, d_counts[1] / N) : n_prims;
-  const float invN = 1.0f / (float)N;
+  uint32_t nv, np;
+  bwd_extent(A, nv, np);
+  const uint32_t cap = (uint32_t)min(4 * A.n_prims, (int64_t)UINT32_MAX);
   const int n_list = head[1];
   for (;;) {
     if (threadIdx.x == 0) s_item = atomicAdd(queue, 1);
@@ -377,82 +454,122 @@ __global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(
     __syncthreads();  // everyone has read s_item before thread 0 takes the next
     if (it >= n_list) break;
     const int c = order[it];
-    const int64_t v0 = chunks[c].vout, v1 = min(v0 + (int64_t)tot[2 * c], nvb);
-    const int64_t p0 = chunks[c].iout / N, p1 = min((chunks[c].iout + (int64_t)tot[2 * c + 1]) / N, npb);
-    for (int m = iters - 1; m >= 0; --m) {
-      for (int64_t t = p0 + threadIdx.x; t < p1; t += kBwdChunkThreads) {
-        float sd[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          const uint32_t v = __ldg(idx + N * t + k);
-          if ((int64_t)v >= nvb || !primal_updates(valence, boundary, v, process_boundary)) continue;
-          const float inv = 1.0f / (float)valence[v];
-#pragma unroll
-          for (int cc = 0; cc < 3; ++cc) sd[cc] += __ldca(g + 3 * v + cc) * inv;
-        }
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc) g_dual[3 * t + cc] = sd[cc];
-      }
+    const int64_t vo = chunks[c].vout, po = chunks[c].iout / 4;
+    const uint32_t v0 = (uint32_t)vo, v1 = (uint32_t)min(vo + (int64_t)tot[2 * c], (int64_t)nv);
+    const uint32_t p0 = (uint32_t)po, p1 = (uint32_t)min(po + (int64_t)(tot[2 * c + 1] / 4), (int64_t)np);
+    for (uint32_t v = v0 + threadIdx.x; v < v1; v += kBwdChunkThreads) bwd_begin(A, v);
+    __syncthreads();
+    for (int m = A.iters - 1; m >= 0; --m) {
+      for (uint32_t t = p0 + threadIdx.x; t < p1; t += kBwdChunkThreads)
+        bwd_prim(A, t, __ldg(reinterpret_cast<const uint4*>(A.idx) + t), nv);
       __syncthreads();
-      for (int64_t v = v0 + threadIdx.x; v < v1; v += kBwdChunkThreads) {
-        const int64_t room = adj_cap - (int64_t)off[v];
-        const uint32_t n = (uint32_t)max((int64_t)0, min((int64_t)valence[v], room));
-        float sv[3] = {0.0f, 0.0f, 0.0f};
-        if (!primal_updates(valence, boundary, v, process_boundary)) {
-#pragma unroll
-          for (int cc = 0; cc < 3; ++cc) sv[cc] = g[3 * v + cc];
-        }
-        for (uint32_t k = 0; k < n; ++k) {
-          const uint32_t t = __ldg(adj + off[v] + k);
-          if ((int64_t)t >= n_prims) continue;
-#pragma unroll
-          for (int cc = 0; cc < 3; ++cc) sv[cc] += __ldca(g_dual + 3 * t + cc) * invN;
-        }
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc) g[3 * v + cc] = sv[cc];
-      }
+      for (uint32_t v = v0 + threadIdx.x; v - (threadIdx.x & 31u) < v1; v += kBwdChunkThreads)
+        bwd_vert(A, v, v < v1, cap, np, m == 0);
       __syncthreads();
     }
   }
 }
 
-int launch_process_bwd(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,
+// The whole mesh in one cooperative launch (as the forward's team, which also
+// says when): the team's CTAs keep their vertices and primitives, a thread its
+// first vertex's list and its first primitive's corners.
+__global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_bwd_team(const __grid_constant__ BwdArgs A, TeamSync* sync,
+                                                                   unsigned* host_failed) {
+  uint32_t nv, np;
+  bwd_extent(A, nv, np);
+  const uint32_t cap = (uint32_t)min(4 * A.n_prims, (int64_t)UINT32_MAX);
+  const unsigned team = min(gridDim.x, max(1u, (nv + kTeamVerts - 1u) / kTeamVerts)), rank = blockIdx.x;
+  if (rank >= team || nv == 0u) return;
+  if (*(volatile unsigned*)&sync->failed) {  // a launch before gave up and the host has not seen it yet
+    if (threadIdx.x == 0) *(volatile unsigned*)host_failed = 1u;
+    return;
+  }
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
+  unsigned target = 0;
+  bool dead = false;
+  const uint32_t vs = (nv + team - 1u) / team, ps = (np + team - 1u) / team;
+  const uint32_t va = min(rank * vs, nv), ve = min(va + vs, nv), pa = min(rank * ps, np), pe = min(pa + ps, np);
+  for (uint32_t v = va + tid; v < ve; v += kTeamThreads) bwd_begin(A, v);
+  const uint4* quads = reinterpret_cast<const uint4*>(A.idx);
+  const uint32_t v_own = va + tid, p_own = pa + tid;
+  const uint4 c_own = p_own < pe ? __ldg(quads + p_own) : make_uint4(0u, 0u, 0u, 0u);
+  uint32_t o_own = 0u, n_own = 0u, val_own = 0u, ids[kTeamRegs] = {};
+  bool upd_own = true;
+  if (v_own < ve) {
+    n_own = bwd_list(A, v_own, cap, o_own, val_own, upd_own);
+#pragma unroll
+    for (int k = 0; k < kTeamRegs; ++k) ids[k] = k < (int)n_own ? __ldg(A.adj + o_own + k) : 0xffffffffu;
+  }
+  team_barrier(sync, host_failed, target, team, dead);
+  for (int m = A.iters - 1; m >= 0; --m) {
+    for (uint32_t t = p_own; t < pe; t += kTeamThreads) bwd_prim(A, t, t == p_own ? c_own : __ldg(quads + t), nv);
+    team_barrier(sync, host_failed, target, team, dead);
+    float s[3] = {0.0f, 0.0f, 0.0f};
+    if (v_own < ve && !upd_own) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) s[c] = A.g[3 * (size_t)v_own + c];
+    }
+    bwd_sums<kTeamRegs>(A, o_own, n_own, np, s, ids);
+    if (v_own < ve) bwd_put(A, v_own, s, val_own, upd_own, m == 0);
+    for (uint32_t v = v_own + kTeamThreads; v - lane < ve; v += kTeamThreads) bwd_vert(A, v, v < ve, cap, np, m == 0);
+    if (m > 0) team_barrier(sync, host_failed, target, team, dead);
+  }
+  // the last CTA leaves the barrier ready for the next launch
+  __syncthreads();
+  if (tid == 0 && atomicAdd(&sync->left, 1u) == team - 1u) {
+    sync->arrived = 0u;
+    sync->left = 0u;
+  }
+}
+
+int launch_process_bwd(int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,
                        const uint8_t* valence, const uint32_t* idx, int iters, int process_boundary,
-                       const ProcessScratch& s, float* g, const StructuredAdj* sa, cudaStream_t st) {
-  if (nv == 0 || n_prims == 0 || iters <= 0) return 0;
-  if (sa && sa->tot && sa->lists.order && sa->bwd_queue) {
-    // one slot array per primitive size: the two kernels' occupancies may differ
-    static std::atomic<int> grid3[64] = {}, grid4[64] = {};
-    const int grid = per_device_once(N == 3 ? grid3 : grid4, [N](int dev) {
+                       const ProcessScratch& s, const float* grad, int64_t n_grad, float* g, float* h,
+                       const StructuredAdj* sa, cudaStream_t st) {
+  BwdArgs A{nv,  n_prims, d_counts, s.off, valence, boundary, s.adj, idx, grad, n_grad, g, reinterpret_cast<float4*>(h),
+            reinterpret_cast<float4*>(s.dual_p), iters, process_boundary};
+  if (sa->tot && sa->bwd_queue) {
+    static std::atomic<int> slots[64] = {};
+    const int grid = per_device_once(slots, [](int dev) {
       int sms = 0, per_sm = 0;
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      if (N == 3)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_bwd_chunks<3>, kBwdChunkThreads, 0);
-      else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_bwd_chunks<4>, kBwdChunkThreads, 0);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_bwd_chunks, kBwdChunkThreads, 0);
       return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
     });
     cudaMemsetAsync(sa->bwd_queue, 0, sizeof(int), st);
-    if (N == 3)
-      k_sweep_bwd_chunks<3><<<grid, kBwdChunkThreads, 0, st>>>(
-          sa->chunks, sa->tot, sa->lists.order, sa->lists.head, sa->bwd_queue, nv, n_prims, n_prims * N, d_counts, s.off,
-          valence, s.adj, boundary, process_boundary, idx, g, s.dual_p, iters);
-    else
-      k_sweep_bwd_chunks<4><<<grid, kBwdChunkThreads, 0, st>>>(
-          sa->chunks, sa->tot, sa->lists.order, sa->lists.head, sa->bwd_queue, nv, n_prims, n_prims * N, d_counts, s.off,
-          valence, s.adj, boundary, process_boundary, idx, g, s.dual_p, iters);
+    k_sweep_bwd_chunks<<<grid, kBwdChunkThreads, 0, st>>>(sa->chunks, sa->tot, sa->lists.order, sa->lists.head,
+                                                         sa->bwd_queue, A);
     return 1;
   }
-  const int vb = (int)((nv + 255) / 256), pb = (int)((n_prims + 255) / 256);
-  for (int m = iters - 1; m >= 0; --m) {
-    if (N == 3)
-      k_primal_bwd<3><<<pb, 256, 0, st>>>(n_prims, nv, d_counts, idx, valence, boundary, process_boundary, g, s.dual_p);
-    else
-      k_primal_bwd<4><<<pb, 256, 0, st>>>(n_prims, nv, d_counts, idx, valence, boundary, process_boundary, g, s.dual_p);
-    k_dual_bwd<<<vb, 256, 0, st>>>(N, nv, n_prims, n_prims * N, d_counts, s.off, valence, s.adj, boundary,
-                                   process_boundary, s.dual_p, g);
+  if (sa->team) {
+    static std::atomic<int> slots[64] = {};
+    const int grid = per_device_once(slots, [](int dev) {
+      int sms = 0, per_sm = 0;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sweep_bwd_team, kTeamThreads, 0);
+      return per_sm > 0 ? min(sms, kTeamMax) : -1;
+    });
+    if (grid > 0) {
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeCooperative;
+      at.val.cooperative = 1;
+      cfg.gridDim = dim3(grid);
+      cfg.blockDim = dim3(kTeamThreads);
+      cfg.stream = st;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, k_sweep_bwd_team, A, sa->team, sa->team_failed);
+      return 1;
+    }
   }
-  return 2 * iters;
+  const int vb = (int)((nv + 255) / 256), pb = (int)((n_prims + 255) / 256);
+  k_bwd_begin<<<vb, 256, 0, st>>>(A);
+  for (int m = iters - 1; m >= 0; --m) {
+    k_primal_bwd<<<pb, 256, 0, st>>>(A);
+    k_dual_bwd<<<vb, 256, 0, st>>>(A, m == 0);
+  }
+  return 2 * iters + 1;
 }
 
 int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, float* pos, float* nrm,
