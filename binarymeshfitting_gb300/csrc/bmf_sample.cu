@@ -856,15 +856,24 @@ int columns2d_item() { return kColumnItem; }
 // The 2D heightmap's occupancy words from its column heights, no densities
 // (the column fill).  One warp per x-plane at a time (persistent; a warp's
 // planes ascend, so it finds each plane's chunk by searching forward from
-// the previous one, 32 candidates a step).  Per block zb a lane holds the
-// height of column z = 32 zb + lane; per line y every lane evaluates its
-// sample's density sign with the full fill's operations and a ballot forms
-// the word, which lane y % 32 keeps, so each lane stores one word per 32 lines.
-__global__ void __launch_bounds__(256) k_words2d(const ChunkDev* __restrict__ chunks, int n_chunks,
-                                                 const int* __restrict__ unit_start, int n_units, FieldDev field,
-                                                 const float* __restrict__ cols, uint32_t* __restrict__ words,
-                                                 uint32_t* __restrict__ flags) {
-  const int lane = threadIdx.x & 31;
+// the previous one, 32 candidates a step).  With positive scales a column's density
+// falls with y -- also as rounded: a product with a positive factor, a sum and a
+// difference keep the order -- so it is inside from some line on, which a binary
+// search finds with the full fill's operations.  A block of 32 columns then has
+// empty words below its lowest such line, full ones from its highest on, and a
+// ballot per line in between.  The words of 32 lines are staged in shared memory
+// and leave in order.  1024 chunks: 313 -> 120 us (every sample's sign by itself: a
+// dozen instructions and a ballot per line).
+constexpr int kWords2dWarps = 8;
+
+__global__ void __launch_bounds__(32 * kWords2dWarps) k_words2d(const ChunkDev* __restrict__ chunks, int n_chunks,
+                                                              const int* __restrict__ unit_start, int n_units,
+                                                              FieldDev field, const float* __restrict__ cols,
+                                                              uint32_t* __restrict__ words,
+                                                              uint32_t* __restrict__ flags) {
+  __shared__ uint16_t s_first[kWords2dWarps][512];      // per column its first inside line (dim: none)
+  __shared__ uint32_t s_words[kWords2dWarps][32 * 16];  // the words of 32 lines, in order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   int c = 0;
   for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n_units; u += nwarps) {
@@ -879,30 +888,52 @@ __global__ void __launch_bounds__(256) k_words2d(const ChunkDev* __restrict__ ch
     const float oy = ch.oy, scale = ch.scale;
     const float* colx = cols + ch.words + (int64_t)x * dim;
     uint32_t* wx = words + ch.words + (int64_t)x * dim * zc;
+    const auto inside = [&](int y, float n) { return terrain2d_density(field, oy + (float)y * scale, n) < 0.0f; };
+    const bool mono = scale > 0.0f && field.p[0] > 0.0f;
+    if (mono) {
+      for (int z = lane; z < dim; z += 32) {
+        const float n = __ldg(colx + z);
+        int lo = 0, hi = dim;
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (inside(mid, n)) hi = mid; else lo = mid + 1;
+        }
+        s_first[warp][z] = (uint16_t)lo;
+      }
+      __syncwarp();
+    }
     uint32_t f = 0u;
-    for (int zb = 0; zb < zc; ++zb) {
-      const int z = 32 * zb + lane;
-      const bool zin = z < dim;
-      const float n = zin ? __ldg(colx + z) : 0.0f;
-      for (int yb = 0; yb < dim; yb += 32) {
+    for (int yb = 0; yb < dim; yb += 32) {
+      const int ny = min(32, dim - yb);
+      for (int zb = 0; zb < zc; ++zb) {
+        const int z = 32 * zb + lane;
+        const bool zin = z < dim;
         uint32_t mine = 0u;
-        const int ny = min(32, dim - yb);
-        for (int j = 0; j < ny; ++j) {
-          const float py = oy + (float)(yb + j) * scale;
-          const uint32_t w = __ballot_sync(kFull, zin && terrain2d_density(field, py, n) < 0.0f);
-          if (lane == j) mine = w;
+        if (mono) {
+          const int first = zin ? s_first[warp][z] : INT_MAX;
+          const int lowest = __reduce_min_sync(kFull, first), highest = __reduce_max_sync(kFull, zin ? first : 0);
+          if (yb + lane >= highest) mine = zbits_upto(dim - 1, zb);
+          for (int y = max(yb, lowest), e = min(yb + ny, highest); y < e; ++y) {
+            const uint32_t w = __ballot_sync(kFull, first <= y);
+            if (yb + lane == y) mine = w;
+          }
+        } else {
+          const float n = zin ? __ldg(colx + z) : 0.0f;
+          for (int j = 0; j < ny; ++j) {
+            const uint32_t w = __ballot_sync(kFull, zin && inside(yb + j, n));
+            if (lane == j) mine = w;
+          }
         }
         if (lane < ny) {
-          wx[(int64_t)(yb + lane) * zc + zb] = mine;
-          f |= (mine != 0u && mine != kFull) ? 1u : (mine == kFull ? 2u : 4u);
+          s_words[warp][lane * zc + zb] = mine;
+          f |= word_class(mine);
         }
       }
+      __syncwarp();
+      for (int i = lane; i < ny * zc; i += 32) wx[yb * zc + i] = s_words[warp][i];
+      __syncwarp();
     }
-    f |= __shfl_xor_sync(kFull, f, 16);
-    f |= __shfl_xor_sync(kFull, f, 8);
-    f |= __shfl_xor_sync(kFull, f, 4);
-    f |= __shfl_xor_sync(kFull, f, 2);
-    f |= __shfl_xor_sync(kFull, f, 1);
+    f = __reduce_or_sync(kFull, f);
     if (lane == 0 && f) atomicOr(flags + c, f);
   }
 }
@@ -913,12 +944,13 @@ void launch_words2d(const ChunkDev* d_chunks, int n_chunks, const int* d_unit_st
   const int g = per_device_once(grid, [](int dev) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_words2d, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_words2d, 32 * kWords2dWarps, 0);
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   });
-  const int need = (n_units + 7) / 8;  // eight warps per CTA, one plane each at a time
-  if (need > 0) k_words2d<<<min(g, need), 256, 0, st>>>(d_chunks, n_chunks, d_unit_start, n_units, field, cols, words,
-                                                       flags);
+  const int need = (n_units + kWords2dWarps - 1) / kWords2dWarps;
+  if (need > 0)
+    k_words2d<<<min(g, need), 32 * kWords2dWarps, 0, st>>>(d_chunks, n_chunks, d_unit_start, n_units, field, cols, words,
+                                                         flags);
 }
 
 // The fill of one terrain chunk (k_fill_block): a thread takes one run of a
