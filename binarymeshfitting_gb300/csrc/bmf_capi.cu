@@ -368,6 +368,12 @@ bmf_status process_mesh(bmf_ctx* ctx, bmf_mesh* mesh, int iters, int pb, int sn,
   // MeshProcessor::init returns early without work on an empty mesh (MeshProcessor.cpp:28-29)
   // (kept positions have to reach the output even then)
   if (iters <= 0 || nv == 0 || (mesh->n_idx < N && !x)) return BMF_OK;
+  StructuredAdj any{2};
+  if (!sa && sweep_team_mesh(N, nv, n_prims)) {
+    any.team = ctx->team;
+    any.team_failed = ctx->team_failed();
+    sa = &any;
+  }
   return process_scratch(ctx, N, nv, n_prims, x, [&](const ProcessScratch& ps) {
     return launch_process(N, nv, n_prims, nullptr, mesh->d_pos, mesh->d_nrm, mesh->d_boundary, mesh->d_valence,
                           mesh->d_idx, iters, pb, sn, ps, sa, st);

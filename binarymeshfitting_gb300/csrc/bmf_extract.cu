@@ -1223,6 +1223,7 @@ struct TeamArgs {
   int64_t nv, n_prims;
   const int64_t* d_counts;
   uint32_t* off;
+  uint32_t* cursor;  // MODE 2: entries of each vertex's list so far
   const uint8_t* valence;
   uint32_t* adj;
   const uint8_t* boundary;
@@ -1234,6 +1235,36 @@ struct TeamArgs {
   unsigned* host_failed;  // pinned host memory
 };
 
+// Ascending order of a list of n entries: by rank in registers, or (long
+// lists) by insertion in place.
+__device__ __forceinline__ void sort_list(uint32_t* a, uint32_t n) {
+  constexpr int kRegs = 10;
+  if (n <= kRegs) {
+    uint32_t e[kRegs];
+#pragma unroll
+    for (int k = 0; k < kRegs; ++k) e[k] = k < (int)n ? a[k] : 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < kRegs; ++k) {
+      int rank = 0;
+#pragma unroll
+      for (int j = 0; j < kRegs; ++j) rank += j < k ? e[j] <= e[k] : (j > k ? e[j] < e[k] : 0);
+      if (k < (int)n) a[rank] = e[k];
+    }
+    return;
+  }
+  for (uint32_t i = 1; i < n; ++i) {
+    const uint32_t key = a[i];
+    int j = (int)i - 1;
+    while (j >= 0 && a[j] > key) {
+      a[j + 1] = a[j];
+      --j;
+    }
+    a[j + 1] = key;
+  }
+}
+
+// MODE 2: any mesh, its lists filled from the indices through cursors and put in
+// ascending order (set_adj, MeshRecursion.hpp:173-190).
 template <int MODE, int N>
 __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_constant__ TeamArgs A) {
   constexpr int kWarps = kTeamThreads / 32;
@@ -1256,7 +1287,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
   const uint32_t cap = np * N;  // slots of adj
   // CSR offsets (MeshProcessor.cpp:32-40): the CTAs' valence sums, then a scan of the own range
   uint32_t sum = 0u;
-  for (uint32_t v = va + tid; v < ve; v += kTeamThreads) sum += __ldg(A.valence + v);
+  for (uint32_t v = va + tid; v < ve; v += kTeamThreads) {
+    sum += __ldg(A.valence + v);
+    if (MODE == 2) A.cursor[v] = 0u;
+  }
   sum = __reduce_add_sync(kFull, sum);
   if (lane == 0) s_warp[warp] = sum;
   __syncthreads();
@@ -1288,17 +1322,34 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
     if (v < ve) {
       const uint32_t o = carry + s_warp[warp] + incl - x;
       A.off[v] = o;
-      const int room = o < cap ? (int)min(x, cap - o) : 0;
-      adj_vertex<MODE>(A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.ws, __ldg(A.vkey + v),
-                       __ldg(A.vadj + v), A.adj + o, room);
+      if (MODE != 2) {
+        const int room = o < cap ? (int)min(x, cap - o) : 0;
+        adj_vertex<MODE>(A.chunks[find_chunk_by_vertex(A.chunks, A.n_chunks, v)], A.ws, __ldg(A.vkey + v),
+                         __ldg(A.vadj + v), A.adj + o, room);
+      }
     }
     carry += s_total;
     __syncthreads();
+  }
+  if (MODE == 2) {
+    team_barrier(A.sync, A.host_failed, target, team, dead);  // every offset and cursor
+    for (uint32_t j = pa * N + tid; j < pe * N; j += kTeamThreads) {
+      const uint32_t v = __ldg(A.idx + j);
+      if (v >= nv) continue;  // an index outside the mesh is ignored
+      const uint32_t k = atomicAdd(A.cursor + v, 1u), o = A.off[v] + k;
+      if (k < __ldg(A.valence + v) && o < cap) A.adj[o] = j / N;  // a caller's valences may not add up
+    }
+    team_barrier(A.sync, A.host_failed, target, team, dead);
+    for (uint32_t v = va + tid; v < ve; v += kTeamThreads) {
+      const uint32_t o = A.off[v];
+      if (o < cap) sort_list(A.adj + o, min(min(A.cursor[v], (uint32_t)__ldg(A.valence + v)), cap - o));
+    }
   }
   // what a thread keeps over all steps: its first vertex's list and its first two primitives' corners
   const auto list_of = [&](uint32_t v, uint32_t& n, uint32_t& o) {
     o = A.off[v];
     n = o < cap ? min((uint32_t)__ldg(A.valence + v), cap - o) : 0u;
+    if (MODE == 2) n = min(n, A.cursor[v]);
     if (!A.process_boundary && __ldg(A.boundary + v)) n = 0u;
   };
   const auto load_ids = [&](uint32_t o, uint32_t n, uint32_t ids[kTeamRegs]) {
@@ -1377,24 +1428,41 @@ static int team_grid() {
   });
 }
 
+static int sweep_team_grid(int mode, int N) {
+  if (mode == 0) return team_grid<0, 3>();
+  if (mode == 1) return team_grid<1, 4>();
+  return N == 3 ? team_grid<2, 3>() : team_grid<2, 4>();
+}
+
+// Any mesh (the lists filled from its indices): one launch instead of 7 + 2 iters
+// small ones, up to kTeamMeshVerts vertices.  Polygonize + smoothing + layout, us,
+// launches / team: 33^3 121 / 91, 100^3 137 / 104, 160^3 178 / 136, 256^3 (~195 k
+// vertices) 221 / 186; Mode Q, 65^3 188 / 136, 320^3 270 / 239.
+constexpr int64_t kTeamMeshVerts = 200000;
+bool sweep_team_mesh(int N, int64_t nv, int64_t n_prims) {
+  return nv <= kTeamMeshVerts && n_prims <= 3 * kTeamMeshVerts && sweep_team_grid(2, N) > 0;
+}
+
 void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,
                        float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
                        int iters, int process_boundary, int smooth_normals, const ProcessScratch& s,
                        cudaStream_t st) {
-  TeamArgs A{sa.chunks, sa.n_chunks, sa.ws, sa.vkey, sa.vadj, nv, n_prims, d_counts, s.off, valence, s.adj, boundary,
+  TeamArgs A{sa.chunks, sa.n_chunks, sa.ws, sa.vkey, sa.vadj, nv, n_prims, d_counts, s.off, s.cursor, valence, s.adj, boundary,
              idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
              smooth_normals, sa.team, sa.team_failed};
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
-  cfg.gridDim = dim3(sa.mode == 0 ? team_grid<0, 3>() : team_grid<1, 4>());
+  cfg.gridDim = dim3(sweep_team_grid(sa.mode, N));
   cfg.blockDim = dim3(kTeamThreads);
   cfg.stream = st;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   if (sa.mode == 0) cudaLaunchKernelEx(&cfg, k_sweep_team<0, 3>, A);
-  else cudaLaunchKernelEx(&cfg, k_sweep_team<1, 4>, A);
+  else if (sa.mode == 1) cudaLaunchKernelEx(&cfg, k_sweep_team<1, 4>, A);
+  else if (N == 3) cudaLaunchKernelEx(&cfg, k_sweep_team<2, 3>, A);
+  else cudaLaunchKernelEx(&cfg, k_sweep_team<2, 4>, A);
 }
 
 // Clusters of `size` (1, 2, 4 or 8) CTAs that can be resident at once (negative: none).
@@ -1469,7 +1537,7 @@ constexpr int64_t kTeamColumns = 140000;
 constexpr int kChunkSweepMin = 320, kChunkSweepPairs = 1024;
 
 SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s) {
-  if (columns <= kTeamColumns && (mode == 0 ? team_grid<0, 3>() : team_grid<1, 4>()) > 0) return kSweepTeam;
+  if (columns <= kTeamColumns && sweep_team_grid(mode, mode == 0 ? 3 : 4) > 0) return kSweepTeam;
   if (n_chunks >= kChunkSweepMin) {
     for (int size = n_chunks >= kChunkSweepPairs ? 2 : 4; size >= 1; size >>= 1) {
       const int clusters = mode == 0 ? sweep_max_clusters<0, 3>(size) : sweep_max_clusters<1, 4>(size);

@@ -272,7 +272,7 @@ struct ProcessScratch {
 // (grid structure known: built analytically per vertex) or any mesh (atomic
 // scatter + per-vertex sort).
 struct StructuredAdj {
-  int mode;                  // BMF_MODE_R / BMF_MODE_Q
+  int mode;                  // BMF_MODE_R / BMF_MODE_Q; 2: any mesh, as one team (team set, the rest unused)
   const ChunkDev* chunks;    // with vout / iout set
   int n_chunks;
   WordScratch ws;            // scanned counts + per-word records
@@ -298,6 +298,8 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st);
+// Whether any mesh of this size takes the whole-mesh form (StructuredAdj mode 2).
+bool sweep_team_mesh(int N, int64_t nv, int64_t n_prims);
 // The whole-mesh form of launch_process in one cooperative launch (sa.team set).
 void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,
                        float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence, const uint32_t* idx,
