@@ -494,7 +494,26 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
   __shared__ int s_bin[64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int mine = blockIdx.x * kScanWarps + warp;
-  if (mine < n) {
+  if (n == 1) {
+    // one chunk: a thread per plane (at most 512), all of them loaded at once
+    // (129 planes by one warp: 5.2 against 3.8 us)
+    const int dim = chunks[0].dim, at = threadIdx.x;
+    uint2* p = pb + chunks[0].unit0;
+    const uint2 t = at < dim ? p[at] : make_uint2(0u, 0u);
+    const uint32_t iv = warp_incl_sum(t.x, lane), ii = warp_incl_sum(t.y, lane);
+    if (lane == 31) {
+      s_v[warp] = iv;
+      s_i[warp] = ii;
+    }
+    __syncthreads();
+    const uint32_t bv = __reduce_add_sync(kFull, lane < warp ? (uint32_t)s_v[lane] : 0u);
+    const uint32_t bi = __reduce_add_sync(kFull, lane < warp ? (uint32_t)s_i[lane] : 0u);
+    if (at < dim) p[at] = make_uint2(bv + iv - t.x, bi + ii - t.y);
+    if (at == kScanThreads - 1) {
+      tot[0] = bv + iv;
+      tot[1] = bi + ii;
+    }
+  } else if (mine < n) {
     const int dim = chunks[mine].dim;
     uint2* p = pb + chunks[mine].unit0;
     uint32_t cv = 0u, ci = 0u;
@@ -511,12 +530,12 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
       tot[2 * mine + 1] = ci;
     }
   }
-  __threadfence();  // this CTA's totals before its ticket
+  if (gridDim.x > 1) __threadfence();  // this CTA's totals before its ticket
   __syncthreads();
   if (threadIdx.x == 0) s_last = gridDim.x == 1 || atomicAdd(ticket, 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!s_last) return;
-  __threadfence();  // the other CTAs' totals after their tickets
+  if (gridDim.x > 1) __threadfence();  // the other CTAs' totals after their tickets
   int64_t carry_v = 0, carry_i = 0;
   for (int base = 0; base < n; base += kScanThreads) {
     const int c = base + threadIdx.x;
