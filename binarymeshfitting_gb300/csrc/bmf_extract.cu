@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
   const int mine = blockIdx.x * kScanWarps + warp;
   if (n == 1) {
     // one chunk: a thread per plane (at most 512), all of them loaded at once
-    // (129 planes by one warp: 5.2 against 3.8 us)
+    // (129 planes: 4.0 us; by one warp's steps, and with the fences, 5.2)
     const int dim = chunks[0].dim, at = threadIdx.x;
     uint2* p = pb + chunks[0].unit0;
     const uint2 t = at < dim ? p[at] : make_uint2(0u, 0u);
