@@ -437,7 +437,7 @@ def run_fit(ctx, args, stream):
                            "per step",
            "peak_mem_bytes": int(peak), "loss_first": loss_first, "loss_last": loss_last,
            "loss_last_lr_0.1": loss_last_lr01,
-           "note": "fwd = bmf_fit_forward (label, count, scan, offsets, emit with QEF, 8 sweeps); bwd = "
+           "note": "fwd = bmf_fit_forward (label, count, chunk scan, emit with QEF, 8 sweeps); bwd = "
                    "bmf_fit_backward (sweep adjoint + QEF/hermite adjoint); step_ms = CUDA-event time of a "
                    "replayed step, step_ms_host = host clock over the same replays; loss_last_lr_0.1 = the same "
                    "200 steps at lr 0.1"}
@@ -525,16 +525,18 @@ def run_gb300(args):
     fill_ops = fill_fp32_ops(rows, workloads.TERRAIN_PARAMS) if args.field == "fbm" else 0
     s_scale, i_scale = samples / DRAM_UPDATE_SAMPLES, ni / DRAM_UPDATE_INDICES
     dram = {k: v * (s_scale if k in ("fill", "count") else i_scale) for k, v in DRAM_BYTES.items()}
-    # algorithmic HBM bytes of the extraction kernels (count + scan + offsets + emit)
-    per_vertex = 12 + 1 + 1 + 8 + (12 if normals else 0)
-    ext_bytes = words * (4 + 8 + 8 + 4) + nv * per_vertex + ni * 4
+    # algorithmic HBM bytes of the extraction kernels (count + chunk scan + emit): every word read
+    # once, per vertex its end densities, position, flags, key and adjacency bits (the sweeps set
+    # the normals), the indices
+    per_vertex = 12 + 1 + 1 + 8 + (8 if args.iters else 0)
+    ext_bytes = words * 4 + nv * per_vertex + ni * 4
     ext_ms = st_ms[1] + st_ms[2] + st_ms[3] + st_ms[4]
     ext_gbs = ext_bytes / (ext_ms / 1000.0) / 1e9
     ext_dram = dram["count"] + dram["scan"] + dram["emit"]
     # logical bytes of the mesh processing (CSR scan + adjacency + iters x (dual, primal)),
-    # each array counted once per pass: dual reads indices + positions (+ normals) and writes
-    # dual points + normals; primal reads offsets, adjacency, dual points + normals, flags and
-    # writes positions + normals
+    # each array counted once per pass: dual reads indices + positions and writes dual points;
+    # primal reads offsets, adjacency, dual points, flags and writes positions.  Normals go with
+    # all passes but the face sweeps left out before the last (at most two)
     n_per = 3 if args.mode == "R" else 4
     n_prims = ni // n_per
     nb = 12 if normals else 0
@@ -542,12 +544,15 @@ def run_gb300(args):
     # defines them; the chunk-by-chunk sweeps store 16-bit lists for chunks of
     # at most 65535 primitives, so the bytes that kernel's own layout touches
     # (own_bytes) are fewer
-    chunk_path = args.chunks >= (512 if args.mode == "R" else 2048)
+    chunk_path = args.chunks >= 320 and float((rows[:, 4] ** 2).sum()) > 140000
     ic = bufs["info"][:, 3].cpu().numpy()
     adj16_entries = int(ic[ic // n_per <= 65535].sum()) if chunk_path else 0
-    dual_b = 4 * ni + 12 * nv + nb * nv + (12 + nb) * n_prims
-    primal_b = 4 * nv + 4 * ni + (12 + nb) * n_prims + 2 * nv + (12 + nb) * nv
-    proc_bytes = args.iters * (dual_b + primal_b) + (1 + 4) * nv + (4 + 4) * nv + 4 * ni
+    face = min(max(3, min(args.iters // 2 - 3, 10)), args.iters)
+    left_out = face - 1 if 1 <= face <= 3 else 0
+    dual_b = 4 * ni + 12 * nv + 12 * n_prims
+    primal_b = 4 * nv + 4 * ni + 12 * n_prims + 2 * nv + 12 * nv
+    normal_b = nb * (2 * n_prims + nv) * (args.iters - left_out) + nb * nv * max(0, args.iters - face)
+    proc_bytes = args.iters * (dual_b + primal_b) + normal_b + (1 + 4) * nv + (4 + 4 + 4) * nv + 4 * ni
     own_bytes = proc_bytes - (args.iters + 1) * 2 * adj16_entries
     proc_gbs = proc_bytes / (st_ms[5] / 1000.0) / 1e9 if st_ms[5] > 0 else 0.0
     sweep_name = ("k_sweep_chunks (CSR scan, adjacency, %d x (dual, primal), chunk by chunk)" if chunk_path
@@ -565,14 +570,15 @@ def run_gb300(args):
                 "dram_achieved": dram["sweeps"] / (st_ms[5] / 1000.0) / 1e9,
                 "dram_frac": dram["sweeps"] / (st_ms[5] / 1000.0) / 1e9 / hbm_peak,
                 "ms_per_launch": st_ms[5],
-                "fill": {"kernels": ("k_columns2d (one thread per (x, z) column height) + k_sample_label "
-                                     "(occupancy words from the heights) + k_fill_fixup (densities at the ends of "
-                                     "crossings only)" if args.field == "2d" and args.mode == "R" else
-                                     "k_sample_label (x-plane CTAs; one height evaluation per (x, z) column)"
+                "fill": {"kernels": ("k_columns2d (one thread per (x, z) column height) + k_words2d "
+                                     "(occupancy words from the heights; the emit computes the densities at the ends "
+                                     "of crossings)" if args.field == "2d" and args.mode == "R" else
+                                     "k_columns2d + k_sample_plane (every density, from the column heights)"
                                      if args.field == "2d" else
                                      "k_fill_terrain<16, band> + k_fill_fixup (terrain FBM, occupancy words, exact "
                                      "densities at the ends of crossings)" if args.mode == "R" else
-                                     "k_fill_terrain<16> (every density exact)"),
+                                     "k_fill_terrain<16, band> + k_fill_need (terrain FBM, occupancy words, exact "
+                                     "densities where the placement reads)"),
                          "ms": st_ms[0], "samples_per_s": samples / (st_ms[0] / 1000.0),
                          "dram_bytes": dram["fill"] if (args.mode == "R" and args.field == "fbm") else None,
                          "density_write_gbs": (4 * samples + 4 * words) / (st_ms[0] / 1000.0) / 1e9
@@ -586,7 +592,7 @@ def run_gb300(args):
                          "note": "the band fill stops a run's octaves once their bound fixes every sign, so its "
                                  "own FP32 work is data-dependent; full_fill_* is the work of evaluating every "
                                  "octave of every sample, divided by the band fill's time"},
-                "extraction_hbm": {"kernels": "count+scan+offsets+emit", "achieved": ext_gbs, "peak": hbm_peak,
+                "extraction_hbm": {"kernels": "count+chunk scan+emit", "achieved": ext_gbs, "peak": hbm_peak,
                                    "unit": "GB/s", "frac": ext_gbs / hbm_peak, "bytes": ext_bytes,
                                    "dram_bytes": ext_dram, "dram_frac": ext_dram / (ext_ms / 1000.0) / 1e9 / hbm_peak,
                                    "ms": ext_ms, "peak_kind": peak_kind,

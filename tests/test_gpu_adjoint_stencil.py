@@ -1,9 +1,8 @@
-"""The wide QEF adjoint's stencil (32 samples around a cell, met in shared
-memory) where it is clamped: surfaces cut by the chunk's faces, chunks of a few
-samples, lists of any length.  Its gradient against the FP32 adjoint, a separate
-code path without the stencil, within that path's own bar (1e-2 relative L2:
-1/s^2 times the ~1e-6 FP32 error of small kept eigenvalues); double-float
-against FP64 within 2e-5."""
+"""The wide QEF adjoint where its stencil (the 32 samples around a cell) is clamped:
+surfaces cut by the chunk's faces, chunks of a few samples, lists of any length.
+Its gradient against the FP32 adjoint, a separate code path, within that path's
+own bar (1e-2 relative L2: 1/s^2 times the ~1e-6 FP32 error of small kept
+eigenvalues); double-float against FP64 within 2e-5."""
 import numpy as np
 import pytest
 import torch
