@@ -44,9 +44,9 @@ OPS_PER_LAYER = 20          # 4 corners (mul + fma), alpha and beta (3 lerps of 
 # count by samples, the emit, scan and sweeps by output indices.
 DRAM_UPDATE_SAMPLES = 1_785_478_272
 DRAM_UPDATE_INDICES = 167_847_141
-DRAM_BYTES = {"fill": 390.0e6 + 1311.7e6 + 19.9e6 + 10.4e6,   # k_fill_terrain<16, band> + k_fill_fixup
-              "count": 331.0e6 + 1462.8e6, "scan": 590.5e6 + 530.9e6, "emit": 1865.2e6 + 2281.4e6,
-              "sweeps": 11777.4e6 + 8051.2e6}
+DRAM_BYTES = {"fill": 397.2e6 + 1331.3e6 + 20.2e6 + 10.6e6,   # k_fill_terrain<16, band> + k_fill_fixup
+              "count": 475.6e6 + 212.6e6, "scan": 2.2e6, "emit": 1541.1e6 + 1476.6e6,
+              "sweeps": 11426.8e6 + 6894.6e6}
 
 
 def fill_fp32_ops(rows, params):
@@ -257,7 +257,7 @@ def config(args):
             "mode Q (DMC quads, placement %d)" % args.placement,
             "smoothing_iters": args.iters, "smoothed_normals": not args.no_normals,
             "l2": "working set larger than L2: a step moves about %.0f GB through DRAM (ncu on the 4096-chunk "
-                  "update: 29 GB, scaled by chunks), no flush between steps" % (29.0 * args.chunks / 4096),
+                  "update: 24 GB, scaled by chunks), no flush between steps" % (24.0 * args.chunks / 4096),
             "parallelism": "replicas" if
             args.gpus == 1 else "weak: one independent update per GPU"}
 

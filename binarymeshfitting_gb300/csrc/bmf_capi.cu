@@ -311,7 +311,7 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk
   if (sa) {
     if (mode == BMF_MODE_Q && (s = scratch(ctx, S_QUADS, (size_t)words_total, &ws.quads)) != BMF_OK) return s;
     *sa = StructuredAdj{mode, d_chunks, n_chunks, ws, mo.vkey, mo.vadj};
-    if (sweep_form(mode, 1, (int64_t)n_units * n_units, &sa->lists) == kSweepTeam) {
+    if (sweep_form(mode, 1, (int64_t)n_units * n_units, false, &sa->lists) == kSweepTeam) {
       sa->team = ctx->team;
       sa->team_failed = ctx->team_failed();
     }
@@ -733,7 +733,7 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if (opts->iters > 0) {
     int64_t columns = 0;
     for (const ChunkDev& c : b->h_chunks) columns += (int64_t)c.dim * c.dim;
-    b->form = sweep_form(opts->mode, n_chunks, columns, &b->sweep);
+    b->form = sweep_form(opts->mode, n_chunks, columns, false, &b->sweep);
     if (b->form == kSweepChunks) {
       if ((s = bail(cudaMalloc(&b->sweep.order, sizeof(int) * (n_chunks + kSweepHead)), "sweep lists")) != BMF_OK)
         return s;
@@ -1399,7 +1399,8 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMemcpy(f->d_chunks, hc.data(), sizeof(ChunkDev) * n_chunks, cudaMemcpyHostToDevice) == cudaSuccess &&
             cudaMemcpy(f->d_units, units.data(), sizeof(int) * (n_chunks + 1), cudaMemcpyHostToDevice) == cudaSuccess;
   f->sweep.head = f->sweep.order + n_chunks;
-  f->form = iters > 0 ? sweep_form(BMF_MODE_Q, n_chunks, (int64_t)n_chunks * dim * dim, &f->sweep) : kSweepLaunches;
+  f->form = iters > 0 ? sweep_form(BMF_MODE_Q, n_chunks, (int64_t)n_chunks * dim * dim, true, &f->sweep)
+                      : kSweepLaunches;
   if (!ok) {
     bmf_fit_destroy(f);
     return fail(ctx, BMF_ERR_OUT_OF_MEMORY, "bmf_fit_create: device allocation failed");

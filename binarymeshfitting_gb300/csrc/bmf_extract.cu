@@ -1537,27 +1537,31 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
 
 // Where the lines lie (whole passes, us; launches / team / chunks with the
 // cluster size chosen here):
-//   one 33^3 chunk, Mode R            152 /  121 /    -
-//   one 257^3 chunk, Mode R           267 /  244 /    -       (66 k columns)
-//   fit, 8 x 65^3 (adjoint in all)    370 /  332 /  375
-//   fit, 32 x 65^3                    608 /  590 /  567       (135 k columns)
-//   mixed update, 48 chunks           299 /  328 /  460       (214 k columns)
-//   128 chunks Mode R / Q       522 / 771   631 / 833   688 / 1034
-//   256                       1019 / 1551  1389 / 1813 1004 / 1663
-//   384                       1414 / 2248  1967 / 2658 1333 / 2247
-//   512                       1779 / 2938  2465 / 3441 1643 / 2879
-//   1024                      3423 / 5629  4819 / 6657 2954 / 5459
+//   one 33^3 chunk, Mode R            110 /   74 /    -
+//   one 257^3 chunk, Mode R           244 /  213 /    -       (66 k columns)
+//   fit, 8 x 65^3 (adjoint in all)    290 /  214 /  279
+//   fit, 32 x 65^3                    526 /  473 /  476       (135 k columns)
+//   fit, 64 x 65^3                    771 /  721 /  701
+//   mixed update, 48 chunks           272 /  296 /  426       (214 k columns)
+//   128 chunks Mode R / Q        464 / 541   552 / 588   618 / 632
+//   256                         918 / 1082 1223 / 1298  898 / 1068
+//   384                        1275 / 1546 1728 / 1877 1209 / 1475
+//   512                        1604 / 1954 2181 / 2368 1518 / 1837
+//   1024                       3086 / 3819 4256 / 4635 2630 / 3465
+//   300, 2D heightmap, two sweeps     710 /    - /  739
+//   fit, 64 x 97^3, 128 x 65^3 (four sweeps), 200 x 33^3  923, 1044, 866 / - / 815, 1009, 860
 // A team pays off while a step is shorter than a launch; its 16 warps per SM
 // carry fewer gathers than full occupancy once steps are long.  A chunk per CTA
-// or cluster needs several chunks per resident CTA to balance.  Clusters of 4
-// against 2 and 1: 512 chunks 1643 / 1802 / 2434 us, 1024 chunks 2996 / 2954 /
+// or cluster needs several chunks per resident CTA to balance, or equal ones (a
+// fit plan's) that fill the GPU as clusters.  Clusters of 4 against 2 and 1 (taken with the adjacency built from
+// the occupancy words): 512 chunks 1643 / 1802 / 2434 us, 1024 chunks 2996 / 2954 /
 // 3456, 2048 chunks 5805 / 5764 / 5781.
 constexpr int64_t kTeamColumns = 140000;
-constexpr int kChunkSweepMin = 320, kChunkSweepPairs = 1024;
+constexpr int kChunkSweepMin = 320, kChunkSweepEqual = 64, kChunkSweepPairs = 1024;
 
-SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s) {
+SweepForm sweep_form(int mode, int n_chunks, int64_t columns, bool equal, SweepLists* s) {
   if (columns <= kTeamColumns && sweep_team_grid(mode, mode == 0 ? 3 : 4) > 0) return kSweepTeam;
-  if (n_chunks >= kChunkSweepMin) {
+  if (n_chunks >= (equal ? kChunkSweepEqual : kChunkSweepMin)) {
     for (int size = n_chunks >= kChunkSweepPairs ? 2 : 4; size >= 1; size >>= 1) {
       const int clusters = mode == 0 ? sweep_max_clusters<0, 3>(size) : sweep_max_clusters<1, 4>(size);
       if (clusters <= 0) continue;

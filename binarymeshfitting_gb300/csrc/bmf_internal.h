@@ -196,9 +196,10 @@ void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_
                        cudaStream_t st, const SweepLists* sweep = nullptr);
 // How the sweeps of n_chunks chunks with `columns` (sum of dim^2) columns in all
 // run: one launch per step, one cooperative launch over the whole mesh, or
-// chunk by chunk (then cluster and ctas of *s are filled).
+// chunk by chunk (then cluster and ctas of *s are filled).  equal: all chunks have
+// the same dim and about as large meshes.
 enum SweepForm { kSweepLaunches, kSweepTeam, kSweepChunks };
-SweepForm sweep_form(int mode, int n_chunks, int64_t columns, SweepLists* s);
+SweepForm sweep_form(int mode, int n_chunks, int64_t columns, bool equal, SweepLists* s);
 // Returns the kernels launched: Mode Q QEF placement with vertex keys and
 // d_counts (total vertices on the device) adds the per-vertex k_place_qef.
 int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start,

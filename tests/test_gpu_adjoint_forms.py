@@ -1,8 +1,9 @@
 """The adjoint sweeps' three forms (whole mesh in one launch, step by step, chunk by
-chunk) against a plan of the one chunk, whose gradient the oracle tests pin.
-The sweeps' values are the same in every form; the placement adjoint adds a
-sample's at most 64 contributions by atomics in any order, 64 * 2^-24 = 4e-6
-of their magnitudes, so a chunk's gradient agrees within 2e-5 (relative L2)."""
+chunk), after each of the forward's, against a plan of the one chunk, whose
+gradient the oracle tests pin.  The sweeps' values are the same in every form;
+the placement adjoint adds a sample's at most 64 contributions by atomics in
+any order, 64 * 2^-24 = 4e-6 of their magnitudes, so a chunk's gradient agrees
+within 2e-5 (relative L2)."""
 import numpy as np
 import pytest
 import torch
@@ -24,7 +25,7 @@ def _grids(n, dim, seed):
     return torch.cat(out)
 
 
-@pytest.mark.parametrize("n,dim", [(3, 33), (150, 17), (36, 65), (256, 9), (300, 12)])
+@pytest.mark.parametrize("n,dim", [(3, 33), (150, 17), (36, 65), (70, 49), (260, 25), (256, 9), (300, 12)])
 @pytest.mark.parametrize("iters", [1, 4])
 def test_forms_match_single_chunk(ctx, n, dim, iters):
     dens = _grids(n, dim, 7 * n + dim)
