@@ -17,7 +17,7 @@
 // the three rotations of a sweep share one copy of the code (the axes change
 // places), and 128 registers keep the matrices out of local memory.  512 x 65^3
 // (3.9 M vertices): 2.40 -> 1.35 ms against one free-running thread per vertex at
-// 8 x 128 threads; one 65^3 grid 85 -> 48 us.
+// 8 x 128 threads; one 65^3 grid 85 -> 44 us.
 //
 // The wide operations and their order are what they were there: with the largest
 // gradients 1000 times the rms, a last bit of dL/dA is 1e-3 of the rms after the
@@ -63,16 +63,14 @@ __device__ __forceinline__ void swap_axes(W B[3][3], W V[3][3], int i, int j) {
   }
 }
 
-constexpr int kQefBwdThreads = 256;
-
-template <typename W>
-__global__ void __launch_bounds__(kQefBwdThreads, 2) k_qef_bwd(
+template <typename W, int THREADS>
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_qef_bwd(
     const ChunkDev* __restrict__ chunks, int n_chunks, const uint32_t* __restrict__ words,
     const float* __restrict__ dens, const uint32_t* __restrict__ vkey, const float* __restrict__ grad_pos,
     float* __restrict__ grad_dens, const uint32_t* __restrict__ qlist, const uint32_t* __restrict__ qcount,
     const float* __restrict__ qseed) {
   const int64_t n = *qcount;
-  for (int64_t s0 = (int64_t)blockIdx.x * kQefBwdThreads; s0 < n; s0 += (int64_t)gridDim.x * kQefBwdThreads) {
+  for (int64_t s0 = (int64_t)blockIdx.x * THREADS; s0 < n; s0 += (int64_t)gridDim.x * THREADS) {
     const int64_t slot = s0 + threadIdx.x;
     const bool in = slot < n;
     const uint32_t v = in ? qlist[slot] : 0u;
@@ -314,29 +312,42 @@ __global__ void __launch_bounds__(kQefBwdThreads, 2) k_qef_bwd(
   }
 }
 
-template <typename W>
+// The resident CTAs, and the launch.
+template <typename W, int THREADS>
 int qef_bwd_grid() {
   static std::atomic<int> grid[64] = {};
   return per_device_once(grid, [](int dev) {
     int sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qef_bwd<W>, kQefBwdThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qef_bwd<W, THREADS>, THREADS, 0);
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   });
+}
+template <typename W, int THREADS, typename... A>
+void qef_bwd_run(int64_t vcap, cudaStream_t st, A... args) {
+  const int64_t need = (vcap + THREADS - 1) / THREADS, grid = qef_bwd_grid<W, THREADS>();
+  if (need > 0) k_qef_bwd<W, THREADS><<<(int)(need < grid ? need : grid), THREADS, 0, st>>>(args...);
 }
 
 }  // namespace
 
+// Double-float: lists that one or two waves of 128-thread CTAs take (the capacity is
+// about twice the list) go out in those, spread over more SMs with half the warps per
+// barrier (fit steps, us, 128 / 256 threads: 1 x 65^3 173 / 181, 4 x 192 / 201, 16 x
+// 284 / 291); longer ones in 256-thread CTAs, whose warps share more of the code's
+// fetches (512 x 4310 / 4020).
 void launch_qef_bwd(int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, const float* dens,
                     const uint32_t* vkey, int64_t vcap, const float* grad_pos, float* grad_dens, const uint32_t* qlist,
                     const uint32_t* qcount, const float* qseed, cudaStream_t st) {
-  const int64_t need = (vcap + kQefBwdThreads - 1) / kQefBwdThreads;
-  if (need == 0) return;
-#define BMF_QEF_BWD(W)                                                                                              \
-  k_qef_bwd<W><<<(int)(need < qef_bwd_grid<W>() ? need : qef_bwd_grid<W>()), kQefBwdThreads, 0, st>>>(              \
-      d_chunks, n_chunks, words, dens, vkey, grad_pos, grad_dens, qlist, qcount, qseed)
-  if (wide == 2) BMF_QEF_BWD(DF); else BMF_QEF_BWD(double);
-#undef BMF_QEF_BWD
+  const auto run = [&](auto go) {
+    go(vcap, st, d_chunks, n_chunks, words, dens, vkey, grad_pos, grad_dens, qlist, qcount, qseed);
+  };
+  if (wide != 2)
+    run([](auto... a) { qef_bwd_run<double, 256>(a...); });
+  else if (vcap <= 4ll * 128 * qef_bwd_grid<DF, 128>())
+    run([](auto... a) { qef_bwd_run<DF, 128>(a...); });
+  else
+    run([](auto... a) { qef_bwd_run<DF, 256>(a...); });
 }
 
 }  // namespace bmf

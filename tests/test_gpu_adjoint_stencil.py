@@ -26,7 +26,7 @@ def _grids(n, dim, seed):
     return np.concatenate([d.reshape(-1) for d in out]).astype(np.float32)
 
 
-@pytest.mark.parametrize("n,dim", [(64, 3), (40, 5), (7, 9), (3, 17), (2, 33)])
+@pytest.mark.parametrize("n,dim", [(64, 3), (40, 5), (7, 9), (3, 17), (2, 33), (12, 33)])
 def test_stencil_at_chunk_faces(ctx, n, dim):
     dens = torch.from_numpy(_grids(n, dim, 100 + dim)).cuda()
     grads, gp = {}, None
