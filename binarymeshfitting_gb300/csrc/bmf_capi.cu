@@ -26,7 +26,7 @@ enum Slot {
 constexpr int kMaxDim = 512;
 constexpr int kCounters = 3;  // list counters behind a plan's chunk flags
 // fit plans: the adjoint sweeps run chunk by chunk from this many chunks (one
-// 512-thread CTA per chunk, four per SM)
+// 1024-thread CTA per chunk, two per SM)
 constexpr int kChunkSweepBwdMinChunks = 256;
 
 struct DevBuf {

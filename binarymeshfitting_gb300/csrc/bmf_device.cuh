@@ -27,7 +27,6 @@ static __constant__ uint64_t c_edge_uses[256] = BMF_EDGE_USES_INIT;
 // (thread-indexed constant loads would serialise).
 static __device__ uint64_t g_tri_cases[256] = BMF_TRI_CASES_INIT;
 static __device__ uint64_t g_group_cases[256] = BMF_GROUP_CASES_INIT;
-static __device__ uint64_t g_edge_uses[256] = BMF_EDGE_USES_INIT;
 
 __device__ __forceinline__ int tri_edge(uint64_t w, int i) { return (int)((w >> (4 * i)) & 0xF); }
 __device__ __forceinline__ int group_count(int mask) { return (int)((c_group_cases[mask] >> 48) & 0xF); }

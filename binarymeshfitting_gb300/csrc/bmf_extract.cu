@@ -1607,20 +1607,6 @@ void launch_chunk_scan(ChunkDev* d_chunks, int n_chunks, WordScratch ws, uint32_
       sweep ? *sweep : SweepLists{});
 }
 
-// k-th set bit (from 0) of m; m must have more than k set bits.
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int k) {
-  int pos = 0, c = __popc(m & 0xFFFFu);
-  if (k >= c) { k -= c; m >>= 16; pos += 16; }
-  c = __popc(m & 0xFFu);
-  if (k >= c) { k -= c; m >>= 8; pos += 8; }
-  c = __popc(m & 0xFu);
-  if (k >= c) { k -= c; m >>= 4; pos += 4; }
-  c = __popc(m & 0x3u);
-  if (k >= c) { k -= c; m >>= 2; pos += 2; }
-  if (k >= (int)(m & 1u)) pos += 1;
-  return pos;
-}
-
 // Corner mask of the cell at offset (ox, oy, oz) in {-1, 0} from sample
 // (x, y, z), from the inside bits of lines (x-1+i, y-1+j) at samples z-1..z+1
 // packed 3 bits per line at bit 3 (3i + j): corner (dx, dy, dz) is bit

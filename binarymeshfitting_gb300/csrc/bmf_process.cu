@@ -304,7 +304,7 @@ int launch_format(const ChunkDev* d_chunks, int n_chunks, int64_t nv, int64_t ni
 // sums four 16-byte gathers and a vertex its list's, instead of three 4-byte
 // gathers, a valence, a boundary flag and a division per corner; the products
 // and the order of the sums are the same.  Quads only (Mode Q).  Eight sweeps of
-// 512 x 65^3: 780 -> 650 us chunk by chunk, bound by the L1's wavefronts; of one 65^3
+// 512 x 65^3: 780 -> 613 us chunk by chunk, bound by the L1's wavefronts; of one 65^3
 // grid: sixteen launches of 4 us and the gaps between them -> 27 us as a team.
 struct BwdArgs {
   int64_t nv, n_prims;
@@ -433,10 +433,12 @@ __global__ void k_dual_bwd(BwdArgs A, bool last) {
 
 // Chunk by chunk: one CTA per chunk (from the queue) runs every backward step
 // of its chunk with block barriers in between -- a chunk's primitives only
-// read its own vertices and the reverse.
-constexpr int kBwdChunkThreads = 512;
+// read its own vertices and the reverse.  1024 threads, two CTAs per SM (fit steps, us,
+// against 512 threads, four: 256 x 33^3 934 / 1004, 300 x 65^3 2497 / 2680, 512 x 65^3
+// 3978 / 4016): fewer chunks at a time, and the last ones end sooner.
+constexpr int kBwdChunkThreads = 1024;
 
-__global__ void __launch_bounds__(kBwdChunkThreads, 4) k_sweep_bwd_chunks(const ChunkDev* __restrict__ chunks,
+__global__ void __launch_bounds__(kBwdChunkThreads, 2) k_sweep_bwd_chunks(const ChunkDev* __restrict__ chunks,
                                                                          const uint32_t* __restrict__ tot,
                                                                          const int* __restrict__ order,
                                                                          const int* __restrict__ head,
