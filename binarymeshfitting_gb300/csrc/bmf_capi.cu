@@ -26,8 +26,10 @@ enum Slot {
 constexpr int kMaxDim = 512;
 constexpr int kCounters = 3;  // list counters behind a plan's chunk flags
 // fit plans: the adjoint sweeps run chunk by chunk from this many chunks (one
-// 1024-thread CTA per chunk, two per SM)
-constexpr int kChunkSweepBwdMinChunks = 256;
+// 1024-thread CTA per chunk, two per SM): fewer leave SMs idle (fit steps, us, step
+// by step / chunk by chunk: 100 x 65^3 988 / 1049, 152 x 1449 / 1448, 200 x 1807 /
+// 1716, 250 x 2213 / 2043; 200 x 33^3 865 / 826, 152 x 97^3 1717 / 1606)
+constexpr int kChunkSweepBwdMinChunks = 160;
 
 struct DevBuf {
   void* p = nullptr;

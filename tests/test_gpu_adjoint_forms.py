@@ -25,7 +25,7 @@ def _grids(n, dim, seed):
     return torch.cat(out)
 
 
-@pytest.mark.parametrize("n,dim", [(3, 33), (150, 17), (36, 65), (70, 49), (260, 25), (256, 9), (300, 12)])
+@pytest.mark.parametrize("n,dim", [(3, 33), (150, 17), (36, 65), (70, 49), (260, 25), (256, 9), (300, 12), (165, 30)])
 @pytest.mark.parametrize("iters", [1, 4])
 def test_forms_match_single_chunk(ctx, n, dim, iters):
     dens = _grids(n, dim, 7 * n + dim)
