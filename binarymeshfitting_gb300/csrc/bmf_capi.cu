@@ -881,8 +881,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   if (const int skip = field_skipped(b->field.kind, b->opts.iters, b->opts.smooth_normals))
     for (int k = 0; k <= skip; ++k) BMF_CUDA(ctx, cudaMalloc(&b->ps.x[k], sizeof(float) * 3 * (vcap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->ps.tmp, sizeof(uint32_t) * (vcap / 4096 + 2)));
-  if (b->opts.iters > 0 && b->form != kSweepChunks)
-    BMF_CUDA(ctx, cudaMalloc(&b->d_idxg, sizeof(uint32_t) * (icap + 1)));
+  if (b->opts.iters > 0) BMF_CUDA(ctx, cudaMalloc(&b->d_idxg, sizeof(uint32_t) * (icap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->d_valence, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_boundary, vcap + 1));
   BMF_CUDA(ctx, cudaMalloc(&b->d_vkey, sizeof(uint32_t) * (vcap + 1)));
@@ -920,10 +919,11 @@ MeshOut batch_mesh_out(const bmf_batch* b, const bmf_batch_out* out) {
   const bool proc = b->opts.iters > 0;
   const ProcessScratch ps = batch_sweep_scratch(b, out);
   const bool keep = proc && ps.x[0];
-  // the chunk-by-chunk sweeps read the chunk-local indices
+  // the sweeps read the plan's own mesh-wide indices: the caller's are final after
+  // the extraction and may be rewritten while the sweeps run
   return MeshOut{keep ? ps.x[0] : out->d_pos, keep ? nullptr : out->d_nrm,
                  proc && !out->d_boundary ? b->d_boundary : out->d_boundary, proc ? b->d_valence : nullptr, out->d_idx,
-                 proc && b->form != kSweepChunks ? b->d_idxg : nullptr, out->vcap, out->icap,
+                 proc ? b->d_idxg : nullptr, out->vcap, out->icap,
                  batch_keys(b) ? b->d_vkey : nullptr, b->d_vadj};
 }
 
@@ -932,9 +932,8 @@ int batch_sweeps(bmf_batch* b, const bmf_batch_out* out, cudaStream_t st) {
   const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
   const StructuredAdj sa = batch_adj(b);
   return launch_process(N, out->vcap, out->icap / N, b->d_totals, out->d_pos, out->d_nrm,
-                        out->d_boundary ? out->d_boundary : b->d_boundary, b->d_valence,
-                        b->form == kSweepChunks ? out->d_idx : b->d_idxg, b->opts.iters, b->opts.process_boundary,
-                        b->opts.smooth_normals, batch_sweep_scratch(b, out), &sa, st);
+                        out->d_boundary ? out->d_boundary : b->d_boundary, b->d_valence, b->d_idxg, b->opts.iters,
+                        b->opts.process_boundary, b->opts.smooth_normals, batch_sweep_scratch(b, out), &sa, st);
 }
 
 // Enqueues one whole update on st (captured into the graph, or run directly).
@@ -1448,8 +1447,8 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
       sa.team = f->team;
       sa.team_failed = ctx->team_failed();
     }
-    k += launch_process(4, f->vcap, f->icap / 4, f->d_totals, d_pos, nullptr, f->d_boundary, f->d_valence,
-                        f->form == kSweepChunks ? d_idx : f->d_idxg, f->iters, 0, 0, f->ps, &sa, st);
+    k += launch_process(4, f->vcap, f->icap / 4, f->d_totals, d_pos, nullptr, f->d_boundary, f->d_valence, f->d_idxg,
+                        f->iters, 0, 0, f->ps, &sa, st);
   }
   BMF_LAUNCHED(ctx, k);
   f->last_density = d_density;

@@ -1005,7 +1005,7 @@ struct SweepArgs {
   const uint8_t* __restrict__ valence;
   uint32_t* __restrict__ adj;
   const uint8_t* __restrict__ boundary;
-  const uint32_t* __restrict__ idx;  // chunk-local
+  const uint32_t* __restrict__ idx;  // mesh-wide
   SweepBufs b;
   float *__restrict__ dual_p, *__restrict__ dual_n;
   int iters, process_boundary, sn, wide_adj;
@@ -1016,7 +1016,8 @@ struct SweepArgs {
 // few registers (the kernel has 32).
 struct ChunkPart {
   uint32_t v0, p0, io;  // the chunk's first vertex, primitive and index
-  uint32_t nv, np;      // its vertices and primitives
+  uint32_t nv, np;      // its vertices and primitives, of those the arena holds
+  uint32_t nvb;         // the mesh's vertices, of those the arena holds
   uint32_t va, ve, pa, pe;  // this CTA's (from v0 / p0)
 };
 
@@ -1041,9 +1042,7 @@ __device__ __forceinline__ void sweep_dual(const SweepArgs& A, const ChunkPart& 
                                            int normals) {
   for (uint32_t t = c.pa + threadIdx.x; t < c.pe; t += kSweepThreads) {
     uint32_t v[N];
-    prim_corners<N, uint32_t>(c.p0 + t, c.nv, A.idx, v);
-#pragma unroll
-    for (int k = 0; k < N; ++k) v[k] += c.v0;
+    prim_corners<N, uint32_t>(c.p0 + t, c.nvb, A.idx, v);
     dual_corners<N, true, uint32_t>(c.p0 + t, v, src, A.b.nrm, A.dual_p, A.dual_n, normals);
   }
 }
@@ -1079,7 +1078,7 @@ __device__ __forceinline__ void sweep_older(const SweepArgs& A, ChunkPart c, int
     const uint32_t o = A.off[v], n = sweep_list_len(A, v, o);
     const float* q = A.b.nrm + 3 * (int64_t)v;
     if (n == 0 || q[0] != 0.0f || q[1] != 0.0f || q[2] != 0.0f) continue;
-    primal_older_normal<N, true>(v, sweep_list<AT>(A, c, o), n, lim, rel, A.idx, c.v0, c.nv, skipped, A.b.x[0],
+    primal_older_normal<N, true>(v, sweep_list<AT>(A, c, o), n, lim, rel, A.idx, c.nvb, skipped, A.b.x[0],
                                  A.b.x[1], A.iters, A.b.nrm);
   }
 }
@@ -1132,6 +1131,7 @@ __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
       const int64_t nvb = A.d_counts ? min(A.nv, A.d_counts[0]) : A.nv;
       const int64_t npb = A.d_counts ? min(A.n_prims, A.d_counts[1] / N) : A.n_prims;
       const int64_t v0 = ch.vout, p0 = ch.iout / N;
+      c.nvb = (uint32_t)nvb;
       c.v0 = (uint32_t)v0;
       c.p0 = (uint32_t)p0;
       c.io = (uint32_t)ch.iout;
@@ -1422,7 +1422,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
         list_of(v, n, o);
         const float* nv3 = A.b.nrm + 3 * (int64_t)v;
         if (n == 0u || nv3[0] != 0.0f || nv3[1] != 0.0f || nv3[2] != 0.0f) continue;
-        primal_older_normal<N, true>(v, A.adj + o, n, np, 0u, A.idx, 0u, nv, st.skipped, A.b.x[0], A.b.x[1], iters, A.b.nrm);
+        primal_older_normal<N, true>(v, A.adj + o, n, np, 0u, A.idx, nv, st.skipped, A.b.x[0], A.b.x[1], iters, A.b.nrm);
       }
     }
     if (m + 1 < iters) team_barrier(A.sync, A.host_failed, target, team, dead);

@@ -173,7 +173,7 @@ __global__ void k_primal(int64_t nv, int64_t n_prims, int64_t adj_cap, const int
   } else if (st.normals == 0) {
     primal_store<false>((uint32_t)v, n, p, nn, st.dst, b.nrm, st.set_colors, 0);
   } else if (primal_store<true>((uint32_t)v, n, p, nn, st.dst, b.nrm, st.set_colors, st.skipped)) {
-    primal_older_normal<N, false>(v, adj + o, n, np_lim, 0u, idx, 0u, (uint32_t)min(nvb, (int64_t)UINT32_MAX),
+    primal_older_normal<N, false>(v, adj + o, n, np_lim, 0u, idx, (uint32_t)min(nvb, (int64_t)UINT32_MAX),
                                   st.skipped, b.x[0], b.x[1], iters, b.nrm);
   }
 }

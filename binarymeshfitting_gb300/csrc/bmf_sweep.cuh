@@ -216,14 +216,13 @@ __device__ __forceinline__ void primal_frozen(uint32_t v, const SweepStep& s, fl
 // The normal of vertex v whose n.y was 0 in the last face sweep: that of the
 // last left-out face sweep whose n.y is not 0, from the positions before it
 // (the sums in list order, as that sweep would have made them); it stays 0
-// when none has.  Rare (walls exactly along y).  rel, v0: the primitive and
-// vertex that the list's ids and the corners count from.
+// when none has.  Rare (walls exactly along y).  rel: the primitive that the
+// list's ids count from.
 template <int N, bool COH, typename AT>
 __device__ __noinline__ void primal_older_normal(int64_t v, const AT* __restrict__ list, uint32_t n, uint32_t np_lim,
-                                                 uint32_t rel, const uint32_t* __restrict__ idx, uint32_t v0,
-                                                 uint32_t nvb, int skipped,
-                                                 const float* __restrict__ x0, const float* __restrict__ x1, int iters,
-                                                 float* __restrict__ nrm) {
+                                                 uint32_t rel, const uint32_t* __restrict__ idx, uint32_t nvb,
+                                                 int skipped, const float* __restrict__ x0,
+                                                 const float* __restrict__ x1, int iters, float* __restrict__ nrm) {
 #pragma unroll 1
   for (int j = skipped - 1; j >= 0; --j) {
     const float* x = j == 1 ? x1 : x0;
@@ -236,7 +235,7 @@ __device__ __noinline__ void primal_older_normal(int64_t v, const AT* __restrict
       float P[N][3], o[3];
       prim_corners<N, uint32_t>(rel + t, nvb, idx, w);
       for (int q = 0; q < N; ++q)
-        for (int c = 0; c < 3; ++c) P[q][c] = sweep_ld<COH>(x + 3 * ((int64_t)v0 + w[q]) + c);
+        for (int c = 0; c < 3; ++c) P[q][c] = sweep_ld<COH>(x + 3 * (int64_t)w[q] + c);
       face_normal<N>(w, P, o);
       for (int c = 0; c < 3; ++c) nn[c] = nn[c] + o[c];
     }
