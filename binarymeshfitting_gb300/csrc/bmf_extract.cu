@@ -959,21 +959,23 @@ __global__ void __launch_bounds__(256) k_adj_build(const ChunkDev* __restrict__ 
                                                    const uint32_t* __restrict__ vkey,
                                                    const uint32_t* __restrict__ vadj, const uint32_t* __restrict__ off,
                                                    const int64_t* __restrict__ d_counts, int64_t vcap,
-                                                   uint32_t* __restrict__ adj) {
+                                                   int64_t adj_cap, uint32_t* __restrict__ adj) {
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= (d_counts ? min(vcap, d_counts[0]) : vcap)) return;
   const int c = find_chunk_by_vertex(chunks, n_chunks, v);
-  // the vertex's CSR range (the exclusive scan of init_valence): never write past it
-  adj_vertex<MODE>(chunks[c], ws, vkey[v], vadj[v], adj + off[v], (int)(off[v + 1] - off[v]));
+  // the vertex's CSR range (the exclusive scan of init_valence), and of that what
+  // the slots hold (an index arena that is too small has fewer): never write past it
+  const int64_t o = off[v], room = min((int64_t)off[v + 1], adj_cap) - o;
+  if (room > 0) adj_vertex<MODE>(chunks[c], ws, vkey[v], vadj[v], adj + o, (int)room);
 }
 
 void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, WordScratch ws, const uint32_t* vkey,
                       const uint32_t* vadj, const uint32_t* off, const int64_t* d_counts,
-                      int64_t vcap, uint32_t* adj, cudaStream_t st) {
+                      int64_t vcap, int64_t adj_cap, uint32_t* adj, cudaStream_t st) {
   const int blocks = (int)((vcap + 255) / 256);
   if (blocks == 0) return;
-  if (mode == 0) k_adj_build<0><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, ws, vkey, vadj, off, d_counts, vcap, adj);
-  else k_adj_build<1><<<blocks, 256, 0, st>>>(d_chunks, n_chunks, ws, vkey, vadj, off, d_counts, vcap, adj);
+  const auto kernel = mode == 0 ? k_adj_build<0> : k_adj_build<1>;
+  kernel<<<blocks, 256, 0, st>>>(d_chunks, n_chunks, ws, vkey, vadj, off, d_counts, vcap, adj_cap, adj);
 }
 
 // ---------------------------------------------------------------------------

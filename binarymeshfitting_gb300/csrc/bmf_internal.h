@@ -292,7 +292,7 @@ struct StructuredAdj {
 };
 void launch_adj_build(int mode, const ChunkDev* d_chunks, int n_chunks, WordScratch ws, const uint32_t* vkey,
                       const uint32_t* vadj, const uint32_t* off, const int64_t* d_counts, int64_t vcap,
-                      uint32_t* adj, cudaStream_t st);
+                      int64_t adj_cap, uint32_t* adj, cudaStream_t st);
 // The chunk-by-chunk form of launch_process for StructuredAdj with tot and
 // lists set: CSR offsets, adjacency and all sweeps in one launch.
 void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_prims, const int64_t* d_counts,

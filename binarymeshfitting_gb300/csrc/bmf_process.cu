@@ -599,7 +599,8 @@ int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, 
   const int vbt = (int)((nv + tb - 1) / tb), pbt = (int)((n_prims + tb - 1) / tb);
   const uint32_t* cursor = nullptr;
   if (sa) {
-    launch_adj_build(sa->mode, sa->chunks, sa->n_chunks, sa->ws, sa->vkey, sa->vadj, s.off, d_counts, nv, s.adj, st);
+    launch_adj_build(sa->mode, sa->chunks, sa->n_chunks, sa->ws, sa->vkey, sa->vadj, s.off, d_counts, nv, n_slots, s.adj,
+                     st);
     launched += 1;
   } else {
     cudaMemsetAsync(s.cursor, 0, (size_t)nv * sizeof(uint32_t), st);

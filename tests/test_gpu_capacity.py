@@ -67,12 +67,11 @@ def whole(ctx):
     return get
 
 
-@pytest.mark.parametrize("mode", [L.MODE_R, L.MODE_Q])
-@pytest.mark.parametrize("share", [0.0, 0.4, 0.999])
-def test_chunk_sweeps_with_too_few_vertices(ctx, whole, mode, share):
-    (nv, ni), want, _ = whole("chunks", mode)
-    b = _plan(ctx, "chunks", mode)
-    intact = _arena(b, max(1, int(share * nv)), 6 * nv)
+def _short(ctx, form, mode, vcap, icap, totals, want):
+    """A plan whose arena is too small at first."""
+    nv, ni = totals
+    b = _plan(ctx, form, mode)
+    intact = _arena(b, vcap, icap)
     for graph in (False, True):
         with pytest.raises(L.BmfError) as e:
             b.run(use_graph=graph)
@@ -81,6 +80,22 @@ def test_chunk_sweeps_with_too_few_vertices(ctx, whole, mode, share):
     b.allocate(nv, ni, normals=True)
     assert b.run() == (nv, ni) and _equal(_mesh(b, nv, ni), want)
     b.close()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("mode", [L.MODE_R, L.MODE_Q])
+@pytest.mark.parametrize("share", [0.0, 0.4, 0.999])
+def test_too_few_vertices(ctx, whole, form, mode, share):
+    totals, want, _ = whole(form, mode)
+    _short(ctx, form, mode, max(1, int(share * totals[0])), 6 * totals[0], totals, want)
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("mode", [L.MODE_R, L.MODE_Q])
+@pytest.mark.parametrize("share", [0.0, 0.4, 0.999])
+def test_too_few_indices(ctx, whole, form, mode, share):
+    totals, want, _ = whole(form, mode)
+    _short(ctx, form, mode, totals[0], max(1, int(share * totals[1])), totals, want)
 
 
 def test_fit_chunk_sweeps_with_too_few_vertices(ctx):
