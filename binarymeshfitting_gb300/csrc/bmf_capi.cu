@@ -108,9 +108,7 @@ struct bmf_batch {
   float* d_cols = nullptr;
   uint2* d_fix = nullptr;  // samples to make exact (+ counter), sized 2 vcap + 1
   int64_t fix_cap = 0;
-  // Mode R work list, sized by the output capacity (vcap + icap / 3 + 1)
-  uint2* d_clist = nullptr;
-  int64_t clist_cap = 0;
+  uint2* d_clist = nullptr;  // work list of the busy words, with room for every word
 };
 
 namespace {
@@ -305,8 +303,7 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk
   if ((s = scratch(ctx, S_PB, (size_t)n_units, &ws.pb)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_TOT, (size_t)n_chunks * 2, &tot)) != BMF_OK) return s;
   {
-    // work list of active cells: each one owns a vertex or emits a primitive
-    ws.clist_cap = mo.vcap + mo.icap / (mode == BMF_MODE_R ? 3 : 4) + 1;
+    ws.clist_cap = words_total;
     if ((s = scratch(ctx, S_CLIST, (size_t)ws.clist_cap, &ws.clist)) != BMF_OK) return s;
     ws.ccount = c.ccount;
   }
@@ -722,6 +719,10 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if ((s = bail(cudaMalloc(&b->d_words, sizeof(uint32_t) * words), "words")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->ws.vcnt, sizeof(uint32_t) * words), "vcnt")) != BMF_OK) return s;
   if ((s = bail(cudaMalloc(&b->ws.rec, sizeof(uint4) * words), "word records")) != BMF_OK) return s;
+  if ((s = bail(cudaMalloc(&b->d_clist, sizeof(uint2) * words), "work list")) != BMF_OK) return s;
+  b->ws.clist = b->d_clist;
+  b->ws.ccount = b->d_flags + n_chunks;
+  b->ws.clist_cap = words;
   if (opts->mode == BMF_MODE_Q && opts->iters > 0 &&
       (s = bail(cudaMalloc(&b->ws.quads, sizeof(uint4) * words), "quads per word")) != BMF_OK)
     return s;
@@ -797,19 +798,9 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
 
 namespace {
 
-// The work list of active cells for an output arena of (vcap, icap) (+ its counter).
-bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
-  const int64_t cap = vcap + icap / (b->opts.mode == BMF_MODE_R ? 3 : 4) + 1;
-  if (cap > b->clist_cap) {
-    if (b->d_clist) cudaFree(b->d_clist);
-    b->d_clist = nullptr;
-    b->clist_cap = 0;
-    BMF_CUDA(b->ctx, cudaMalloc(&b->d_clist, sizeof(uint2) * cap));
-    b->clist_cap = cap;
-  }
-  b->ws.clist = b->d_clist;
-  b->ws.ccount = b->d_flags + b->n;
-  b->ws.clist_cap = b->clist_cap;
+// The fix-up list for an output arena of vcap vertices, and the scratch's optional parts
+// as the tuning asks for them.
+bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap) {
   if (b->d_exact && b->opts.mode == BMF_MODE_R) {
     // band fill: every crossing (one vertex each in Mode R) lists at most its two ends
     const int64_t fcap = 2 * vcap + 1;
@@ -983,7 +974,7 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
   cudaStream_t st = (cudaStream_t)stream;
   bmf_status s;
   if (batch_keys(b) && (s = batch_proc_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
-  if ((s = batch_list_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
+  if ((s = batch_list_scratch(b, out->vcap)) != BMF_OK) return s;
   if (use_graph) {
     if (!b->exec || !same_out(b->graph_out, *out)) {
       if (b->exec) {
@@ -1101,7 +1092,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   bmf_status s;
   const bool proc = b->opts.iters > 0;
   if (batch_keys(b) && (s = batch_proc_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
-  if ((s = batch_list_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
+  if ((s = batch_list_scratch(b, out->vcap)) != BMF_OK) return s;
   cudaEvent_t ev[8];
   for (auto& e : ev) BMF_CUDA(ctx, cudaEventCreate(&e));
   BMF_CUDA(ctx, cudaEventRecord(ev[0], st));
@@ -1307,7 +1298,7 @@ struct bmf_fit {
   uint32_t* d_qlist = nullptr;    // QEF-placed vertices of the forward, for the wide backward (+ counter at [vcap])
   float* d_qseed = nullptr;       // their FP32 eigenvectors (9 per entry), recorded by the forward
   uint8_t* d_qflag = nullptr;     // per vertex: took the QEF branch in the forward
-  uint2* d_clist = nullptr;       // work list of active cells (+ counter after it)
+  uint2* d_clist = nullptr;       // work list of the busy words, with room for every word
   const float* last_density = nullptr;
   int64_t* h_pinned = nullptr;
   float* d_lpart = nullptr;       // per-block partial sums of bmf_fit_loss_spheres
@@ -1394,7 +1385,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             (!(flags & (BMF_FIT_ADJOINT_F64 | BMF_FIT_ADJOINT_DF)) ||
              (cudaMalloc(&f->d_qseed, sizeof(float) * 9 * (vcap + 1)) == cudaSuccess &&
               cudaMalloc(&f->d_qflag, vcap + 1) == cudaSuccess)) &&
-            cudaMalloc(&f->d_clist, sizeof(uint2) * (vcap + icap / 4 + 2)) == cudaSuccess &&
+            cudaMalloc(&f->d_clist, sizeof(uint2) * words) == cudaSuccess &&
             cudaMalloc(&f->d_lpart, sizeof(float) * kFitLossPartials) == cudaSuccess &&
             cudaMallocHost(&f->h_pinned, sizeof(int64_t) * 4) == cudaSuccess &&
             cudaMemcpy(f->d_chunks, hc.data(), sizeof(ChunkDev) * n_chunks, cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -1407,7 +1398,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
     return fail(ctx, BMF_ERR_OUT_OF_MEMORY, "bmf_fit_create: device allocation failed");
   }
   f->ws.clist = f->d_clist;
-  f->ws.clist_cap = vcap + icap / 4 + 1;
+  f->ws.clist_cap = words;
   f->ws.ccount = f->d_flags + n_chunks;
   *out = f;
   return BMF_OK;

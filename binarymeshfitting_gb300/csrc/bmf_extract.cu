@@ -918,8 +918,6 @@ __device__ __forceinline__ void adj_vertex(const ChunkDev& ch, const WordScratch
   const int dim = ch.dim, zc = ch.zc;
   int x, y, z, k;
   vertex_key_decode(key, x, y, z, k);
-  // (a vertex past the work list's capacity has no key: stay inside the chunk)
-  if (max(x, max(y, z)) > dim - (MODE == 0 ? 1 : 2)) return;
   // the chunk's first primitive (its index offset and word bases are
   // multiples of the primitive size)
   const int64_t pbase = ch.iout / (MODE == 0 ? 3 : 4) - rel;

@@ -67,8 +67,10 @@ struct WordScratch {
   uint4* rec;
   // Work list (nullable) of the busy words (those that own a vertex or emit a
   // primitive) as {chunk, word index in the chunk}, in no particular order;
-  // *ccount (zeroed before the count kernel) entries, at most clist_cap kept:
-  // vcap + icap / prim_size + 1 suffice.
+  // *ccount (zeroed before the count kernel) entries, at most clist_cap kept.
+  // With room for every word no arena is too small for it: each vertex that the
+  // arena holds then gets its key, which the QEF placement, the adjacency and
+  // the adjoint take for a cell inside the chunk.
   uint2* clist;
   uint32_t* ccount;
   int64_t clist_cap;

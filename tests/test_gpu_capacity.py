@@ -13,8 +13,8 @@ from binarymeshfitting_gb300.fitting import FitPlan
 pytestmark = pytest.mark.gpu
 
 GUARD = 4096
-# (chunks, dim): one launch per step, and chunk by chunk
-FORMS = {"launches": (100, 41), "chunks": (330, 24)}
+# (chunks, dim): one cooperative launch, one launch per step, and chunk by chunk
+FORMS = {"team": (40, 33), "launches": (100, 41), "chunks": (330, 24)}
 
 
 def _plan(ctx, form, mode, place=L.PLACE_MASSPOINT, iters=4):
@@ -134,3 +134,44 @@ def test_indices_may_be_rewritten_behind_the_extraction(ctx, whole, mode):
         torch.cuda.synchronize()
         assert torch.equal(got, want[3]) and _equal(_mesh(b, nv, ni)[:3], want[:3])
     b.close()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("mode,place", [(L.MODE_Q, L.PLACE_QEF), (L.MODE_Q, L.PLACE_MASSPOINT)])
+@pytest.mark.parametrize("share", [0.05, 0.15])
+def test_chunks_that_fit_are_whole(ctx, whole, form, mode, place, share):
+    """Far too small an arena (fewer entries than busy words): the chunks whose status
+    is 0 are complete, and every vertex of the arena has a cell to be placed in."""
+    (nv, ni), want, wtab = whole(form, mode, place)
+    b = _plan(ctx, form, mode, place)
+    intact = _arena(b, int(share * nv), int(share * ni))
+    for graph in (False, True):
+        with pytest.raises(L.BmfError) as e:
+            b.run(use_graph=graph)
+        torch.cuda.synchronize()
+        assert e.value.status == L.ERR_CAPACITY and (b.out.n_verts, b.out.n_idx) == (nv, ni) and intact()
+        tab = b.bufs["info"].cpu().numpy()
+        fit = np.flatnonzero((tab[:, 5] == 0) & (tab[:, 1] > 0))
+        assert len(fit) > 0 and np.array_equal(tab[:, :5], wtab[:, :5])
+        for i in fit:
+            vo, vc, io, ic = tab[i, :4]
+            got = [b.bufs[k][vo:vo + vc] for k in ("pos", "nrm", "boundary")] + [b.bufs["idx"][io:io + ic]]
+            assert _equal(got, [t[vo:vo + vc] for t in want[:3]] + [want[3][io:io + ic]]), i
+    b.close()
+
+
+@pytest.mark.parametrize("n,dim", [(1, 33), (200, 33)])
+@pytest.mark.parametrize("adjoint", ["f32", "df"])
+def test_fit_step_in_a_small_arena_stays_inside(ctx, n, dim, adjoint):
+    """A whole fitting step without a host sync, on vertices that partly have no room."""
+    dens, sph = workloads.fit_batch(n, dim=dim, seed=9, device=ctx.device)
+    plan = FitPlan(ctx, n, dim, iters=2, adjoint=adjoint, vcap=40 * n, icap=40 * n)
+    loss, grad_pos = torch.zeros(1, device=ctx.device), torch.zeros((plan.vcap, 3), device=ctx.device)
+    grad = torch.full((dens.numel() + 2 * GUARD,), -7.0, device=ctx.device)
+    plan.step_grad(dens, sph, loss, grad_pos, grad[GUARD:-GUARD])
+    torch.cuda.synchronize()
+    assert (grad[:GUARD] == -7.0).all() and (grad[-GUARD:] == -7.0).all()
+    with pytest.raises(L.BmfError) as e:
+        plan.forward(dens)
+    assert e.value.status == L.ERR_CAPACITY
+    plan.close()
