@@ -137,7 +137,8 @@ def test_indices_may_be_rewritten_behind_the_extraction(ctx, whole, mode):
 
 
 @pytest.mark.parametrize("form", list(FORMS))
-@pytest.mark.parametrize("mode,place", [(L.MODE_Q, L.PLACE_QEF), (L.MODE_Q, L.PLACE_MASSPOINT)])
+@pytest.mark.parametrize("mode,place", [(L.MODE_R, L.PLACE_MASSPOINT), (L.MODE_Q, L.PLACE_QEF),
+                                        (L.MODE_Q, L.PLACE_MASSPOINT)])
 @pytest.mark.parametrize("share", [0.05, 0.15])
 def test_chunks_that_fit_are_whole(ctx, whole, form, mode, place, share):
     """Far too small an arena (fewer entries than busy words): the chunks whose status
