@@ -798,6 +798,12 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
 
 namespace {
 
+// A captured graph holds the scratch's addresses: dropped before any of it is freed.
+void batch_drop_graph(bmf_batch* b) {
+  if (b->exec) cudaGraphExecDestroy(b->exec);
+  b->exec = nullptr;
+}
+
 // The fix-up list for an output arena of vcap vertices, and the scratch's optional parts
 // as the tuning asks for them.
 bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap) {
@@ -805,6 +811,7 @@ bmf_status batch_list_scratch(bmf_batch* b, int64_t vcap) {
     // band fill: every crossing (one vertex each in Mode R) lists at most its two ends
     const int64_t fcap = 2 * vcap + 1;
     if (fcap > b->fix_cap) {
+      batch_drop_graph(b);
       if (b->d_fix) cudaFree(b->d_fix);
       b->d_fix = nullptr;
       b->fix_cap = 0;
@@ -853,6 +860,7 @@ void batch_fill(bmf_batch* b, cudaStream_t st) {
 
 bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   if (vcap <= b->proc_vcap && icap <= b->proc_icap) return BMF_OK;
+  batch_drop_graph(b);
   bmf_ctx* ctx = b->ctx;
   const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
   const int64_t np = icap / N;
@@ -977,10 +985,7 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
   if ((s = batch_list_scratch(b, out->vcap)) != BMF_OK) return s;
   if (use_graph) {
     if (!b->exec || !same_out(b->graph_out, *out)) {
-      if (b->exec) {
-        cudaGraphExecDestroy(b->exec);
-        b->exec = nullptr;
-      }
+      batch_drop_graph(b);
       cudaStream_t cap;
       BMF_CUDA(ctx, cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
       cudaGraph_t g;
@@ -1172,10 +1177,7 @@ bmf_status bmf_batch_set_tuning(bmf_batch* b, const bmf_batch_tuning* t) {
   b->fill_band = t->fill_band;
   if (terrain) b->fill_grid = fill_terrain_resident_ctas(b->fill_run, (int)b->field.p[5], batch_band(b));
   b->ps.block = t->sweep_block;
-  if (b->exec) {
-    cudaGraphExecDestroy(b->exec);
-    b->exec = nullptr;
-  }
+  batch_drop_graph(b);
   return BMF_OK;
 }
 

@@ -176,3 +176,24 @@ def test_fit_step_in_a_small_arena_stays_inside(ctx, n, dim, adjoint):
         plan.forward(dens)
     assert e.value.status == L.ERR_CAPACITY
     plan.close()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("mode", [L.MODE_R, L.MODE_Q])
+@pytest.mark.parametrize("between", ["run", "profile"])
+def test_a_graph_does_not_outlive_its_scratch(ctx, whole, form, mode, between):
+    """A graph captured for one arena, replayed after a direct run on a larger one."""
+    (nv, ni), want, _ = whole(form, mode)
+    b = _plan(ctx, form, mode)
+    b.allocate(nv, ni, normals=True)
+    small = b.out, b.bufs
+    assert b.run() == (nv, ni)
+    b.allocate(2 * nv, 2 * ni, normals=True)
+    if between == "run":
+        assert b.run(use_graph=False) == (nv, ni) and _equal(_mesh(b, nv, ni), want)
+    else:
+        b.profile()
+    b.out, b.bufs = small
+    b.bufs["pos"].zero_()
+    assert b.run() == (nv, ni) and _equal(_mesh(b, nv, ni), want)
+    b.close()
