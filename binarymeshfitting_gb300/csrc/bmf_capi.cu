@@ -146,6 +146,7 @@ bmf_status fail(bmf_ctx* ctx, bmf_status s, const std::string& msg) {
 
 bmf_status cuda_check(bmf_ctx* ctx, cudaError_t e, const char* what) {
   if (e == cudaSuccess) return BMF_OK;
+  cudaGetLastError();  // reported here: the next call's launch check starts clean (an allocation that failed)
   return fail(ctx, e == cudaErrorMemoryAllocation ? BMF_ERR_OUT_OF_MEMORY : BMF_ERR_CUDA,
               std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -1396,6 +1397,7 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
   f->form = iters > 0 ? sweep_form(BMF_MODE_Q, n_chunks, (int64_t)n_chunks * dim * dim, true, &f->sweep)
                       : kSweepLaunches;
   if (!ok) {
+    cudaGetLastError();  // (as cuda_check)
     bmf_fit_destroy(f);
     return fail(ctx, BMF_ERR_OUT_OF_MEMORY, "bmf_fit_create: device allocation failed");
   }

@@ -136,3 +136,32 @@ def test_bounded_wait_times_out_then_completes(ctx):
         idle.wait(0)  # never ran
     assert e.value.status == L.ERR_INVALID_ARGUMENT
     idle.close()
+
+
+def test_calls_work_after_an_allocation_that_failed(ctx):
+    """A request for more memory than any GPU has: BMF_ERR_OUT_OF_MEMORY from the call
+    that asked, and only from it."""
+    huge = 1 << 40  # vertices
+    desc, field = L.ChunkDesc.make((0.0, 48.0, 0.0), 1.0, 33), workloads.terrain_field()
+    want = ctx.extract_chunk(desc, field, iters=2, smooth_normals=True)
+    b = Batch(ctx, [desc], field, mode=L.MODE_R, iters=2, smooth_normals=True)
+    b.allocate(1 << 16, 1 << 18, normals=True)
+    totals = b.run(use_graph=True)
+    room = b.out
+    b.out = L.BatchOut(room.d_pos, room.d_nrm, room.d_boundary, room.d_idx, huge, 6 * huge, room.d_chunk_info, 0, 0)
+    fit = ctypes.c_void_p()
+
+    def asks():
+        yield lambda: b.run(use_graph=True)
+        yield lambda: L.check(ctx.lib.bmf_fit_create(ctx.h, 1, 33, L.PLACE_QEF, 2, huge, 4 * huge, 0, ctypes.byref(fit)),
+                              ctx.h, ctx.lib)
+    for ask in asks():
+        with pytest.raises(L.BmfError) as e:
+            ask()
+        assert e.value.status == L.ERR_OUT_OF_MEMORY
+        got = ctx.extract_chunk(desc, field, iters=2, smooth_normals=True)
+        assert torch.equal(got.pos, want.pos) and torch.equal(got.idx, want.idx)
+    b.out = room
+    assert b.run(use_graph=True) == totals == (want.n_verts, want.n_idx)
+    assert torch.equal(b.bufs["pos"][:totals[0]], want.pos)
+    b.close()
