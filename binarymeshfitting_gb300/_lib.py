@@ -134,6 +134,7 @@ SIGNATURES = {
     "bmf_fit_adam": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_float, c_float,
                                c_float, c_float, c_void_p]),
     "bmf_fit_destroy": (c_int32, [c_void_p]),
+    "bmf_debug_sweep_timeout": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p]),
 }
 
 _lib = None

@@ -38,7 +38,16 @@ struct DevBuf {
 
 }  // namespace
 
-constexpr int kPinned = 64, kPinnedFailed = 32;  // h_pinned: entries, and the one that holds the sweeps' failure mark
+constexpr int kPinned = 64;      // entries of a context's h_pinned
+constexpr int kPlanPinned = 64;  // and of a plan's: the totals, and on a line of its own the mark
+constexpr int kPinnedMark = 32;  // the entry that holds the sweeps' mark
+
+// The barrier of the one-launch sweeps of a context or a plan, and its mark in pinned
+// memory, which the kernel sets when a wait runs out.
+struct Team {
+  TeamSync* sync = nullptr;
+  unsigned* mark = nullptr;
+};
 
 struct bmf_ctx {
   int device = 0;
@@ -46,8 +55,7 @@ struct bmf_ctx {
   int64_t launches = 0;
   DevBuf bufs[S_NUM];
   int64_t* h_pinned = nullptr;  // readback staging
-  TeamSync* team = nullptr;     // barrier of the whole-mesh sweep kernel
-  unsigned* team_failed() const { return (unsigned*)(h_pinned + kPinnedFailed); }
+  Team team;                    // of bmf_process and bmf_extract_chunk
 };
 
 struct bmf_batch {
@@ -91,7 +99,7 @@ struct bmf_batch {
   int* d_queue = nullptr;
   SweepForm form = kSweepLaunches;
   SweepLists sweep;  // the chunk-by-chunk sweeps' work lists
-  TeamSync* team = nullptr;  // barrier of the whole-mesh sweep kernel
+  Team team;
   int fill_grid = 0;
   int fill_mode = 0;
   int fill_run = 16;  // the tile height the autotuner picks on the mixed-LOD update
@@ -164,13 +172,23 @@ bmf_status cuda_check(bmf_ctx* ctx, cudaError_t e, const char* what) {
     if (_s != BMF_OK) return _s;                                               \
   } while (0)
 
-// After a synchronisation: did a wait of the whole-mesh sweep kernel run out?
-// (Only when its CTAs could not all make progress; the barrier is set anew.)
-bmf_status team_check(bmf_ctx* ctx, TeamSync* team) {
-  if (!team || !*(volatile unsigned*)ctx->team_failed()) return BMF_OK;
-  *ctx->team_failed() = 0;
-  cudaMemset(team, 0, sizeof(TeamSync));
-  return fail(ctx, BMF_ERR_CUDA, "a wait of the smoothing sweeps ran out: the mesh is not smoothed");
+// Did a wait of this object's one-launch sweeps run out (only when their CTAs could
+// not all make progress)?  Asked after a synchronisation, and, for the calls that did
+// not synchronise, before the object's next sweeps; reported once.
+bmf_status team_check(bmf_ctx* ctx, const Team& t) {
+  if (!*(volatile unsigned*)t.mark) return BMF_OK;
+  *t.mark = 0;
+  return fail(ctx, BMF_ERR_CUDA,
+              "a wait of the smoothing sweeps ran out, in this call or in an earlier one on the same object that did "
+              "not synchronise: that mesh (or gradient) is not valid");
+}
+
+// The barrier, zeroed, and its mark (in pinned memory of at least kPinnedMark + 1 entries).
+cudaError_t team_create(Team* t, int64_t* pinned) {
+  t->mark = (unsigned*)(pinned + kPinnedMark);
+  *t->mark = 0;
+  const cudaError_t e = cudaMalloc(&t->sync, sizeof(TeamSync));
+  return e == cudaSuccess ? cudaMemset(t->sync, 0, sizeof(TeamSync)) : e;
 }
 
 template <class T>
@@ -312,8 +330,8 @@ bmf_status extract_core(bmf_ctx* ctx, int mode, int placement, const SingleChunk
     if (mode == BMF_MODE_Q && (s = scratch(ctx, S_QUADS, (size_t)words_total, &ws.quads)) != BMF_OK) return s;
     *sa = StructuredAdj{mode, d_chunks, n_chunks, ws, mo.vkey, mo.vadj};
     if (sweep_form(mode, 1, (int64_t)n_units * n_units, false, &sa->lists) == kSweepTeam) {
-      sa->team = ctx->team;
-      sa->team_failed = ctx->team_failed();
+      sa->team = ctx->team.sync;
+      sa->team_failed = ctx->team.mark;
     }
   }
   launch_count(mode, d_chunks, n_chunks, d_units, n_units, d_words, flags_ready ? d_flags : nullptr, ws, st,
@@ -370,8 +388,8 @@ bmf_status process_mesh(bmf_ctx* ctx, bmf_mesh* mesh, int iters, int pb, int sn,
   if (iters <= 0 || nv == 0 || (mesh->n_idx < N && !x)) return BMF_OK;
   StructuredAdj any{2};
   if (!sa && sweep_team_mesh(N, nv, n_prims)) {
-    any.team = ctx->team;
-    any.team_failed = ctx->team_failed();
+    any.team = ctx->team.sync;
+    any.team_failed = ctx->team.mark;
     sa = &any;
   }
   return process_scratch(ctx, N, nv, n_prims, x, [&](const ProcessScratch& ps) {
@@ -412,9 +430,7 @@ bmf_status bmf_create(const bmf_config* cfg, bmf_ctx** out) {
     delete ctx;
     return BMF_ERR_OUT_OF_MEMORY;
   }
-  std::memset(ctx->h_pinned, 0, kPinned * sizeof(int64_t));
-  if (cudaMalloc(&ctx->team, sizeof(TeamSync)) != cudaSuccess ||
-      cudaMemset(ctx->team, 0, sizeof(TeamSync)) != cudaSuccess) {
+  if (team_create(&ctx->team, ctx->h_pinned) != cudaSuccess) {
     bmf_destroy(ctx);
     return BMF_ERR_OUT_OF_MEMORY;
   }
@@ -428,7 +444,7 @@ bmf_status bmf_destroy(bmf_ctx* ctx) {
   for (auto& b : ctx->bufs)
     if (b.p) cudaFree(b.p);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
-  if (ctx->team) cudaFree(ctx->team);
+  if (ctx->team.sync) cudaFree(ctx->team.sync);
   delete ctx;
   return BMF_OK;
 }
@@ -458,6 +474,7 @@ bmf_status bmf_sample_label(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf_
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
     const uint32_t f = *(const uint32_t*)ctx->h_pinned;
     *h_contains_mesh = ((f & 1u) || ((f & 6u) == 6u)) ? 1 : 0;
+    return team_check(ctx, ctx->team);  // (a bmf_process before)
   }
   return BMF_OK;
 }
@@ -529,7 +546,7 @@ bmf_status bmf_polygonize(bmf_ctx* ctx, int32_t dim, const float* d_density, con
   out->prim_size = mode == BMF_MODE_R ? 3 : 4;
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_polygonize: output capacity exceeded (needed counts reported)");
-  return BMF_OK;
+  return team_check(ctx, ctx->team);  // (a bmf_process before)
 }
 
 bmf_status bmf_process(bmf_ctx* ctx, bmf_mesh* mesh, int32_t iters, int32_t process_boundary,
@@ -540,6 +557,7 @@ bmf_status bmf_process(bmf_ctx* ctx, bmf_mesh* mesh, int32_t iters, int32_t proc
   if ((s = mesh_valid(ctx, mesh)) != BMF_OK) return s;
   if (mesh->n_verts > mesh->vcap || mesh->n_idx > mesh->icap || iters < 0)
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_process: counts exceed capacities or negative iters");
+  if ((s = team_check(ctx, ctx->team)) != BMF_OK) return s;
   return process_mesh(ctx, mesh, iters, process_boundary, smooth_normals, (cudaStream_t)stream);
 }
 
@@ -579,6 +597,7 @@ bmf_status bmf_format(bmf_ctx* ctx, const bmf_mesh* mesh, int32_t unwind, int32_
   if (h_count) {
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
     *h_count = count;
+    return team_check(ctx, ctx->team);  // (a bmf_process before)
   }
   return BMF_OK;
 }
@@ -648,15 +667,15 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   out->prim_size = N;
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_extract_chunk: output capacity exceeded (needed counts reported)");
-  if (one_sync) return team_check(ctx, sa.team);
+  if (one_sync) return team_check(ctx, ctx->team);
   // ChunkGenerator.cpp:112: processing only when the chunk has a mesh
   if (opts->iters > 0 && out->contains_mesh && out->n_verts && (out->n_idx || skip)) {
     if ((s = process_mesh(ctx, out, opts->iters, opts->process_boundary, opts->smooth_normals, st, &sa,
                           skip ? x : nullptr)) != BMF_OK)
       return s;
     BMF_CUDA(ctx, cudaStreamSynchronize(st));
-    return team_check(ctx, sa.team);
   }
+  return team_check(ctx, ctx->team);
   return BMF_OK;
 }
 
@@ -727,7 +746,8 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
   if (opts->mode == BMF_MODE_Q && opts->iters > 0 &&
       (s = bail(cudaMalloc(&b->ws.quads, sizeof(uint4) * words), "quads per word")) != BMF_OK)
     return s;
-  if ((s = bail(cudaMallocHost(&b->h_pinned, sizeof(int64_t) * 4), "pinned")) != BMF_OK) return s;
+  if ((s = bail(cudaMallocHost(&b->h_pinned, sizeof(int64_t) * kPlanPinned), "pinned")) != BMF_OK) return s;
+  if ((s = bail(team_create(&b->team, b->h_pinned), "sweep barrier")) != BMF_OK) return s;
   if ((s = bail(cudaMemcpy(b->d_chunks, b->h_chunks.data(), sizeof(ChunkDev) * n_chunks, cudaMemcpyHostToDevice),
                 "upload chunks")) != BMF_OK)
     return s;
@@ -744,8 +764,6 @@ bmf_status bmf_batch_create(bmf_ctx* ctx, const bmf_chunk_desc* h_descs, int32_t
       b->sweep.head = b->sweep.order + n_chunks;
     }
   }
-  if ((s = bail(cudaMalloc(&b->team, sizeof(TeamSync)), "sweep barrier")) != BMF_OK) return s;
-  if ((s = bail(cudaMemset(b->team, 0, sizeof(TeamSync)), "sweep barrier")) != BMF_OK) return s;
   // chunks by size, largest first (longest-processing-time order for the
   // work queue of the fill)
   std::vector<int> order(n_chunks);
@@ -898,8 +916,8 @@ StructuredAdj batch_adj(const bmf_batch* b) {
     sa.tot = b->d_tot;
     sa.lists = b->sweep;
   } else if (b->form == kSweepTeam) {
-    sa.team = b->team;
-    sa.team_failed = b->ctx->team_failed();
+    sa.team = b->team.sync;
+    sa.team_failed = b->team.mark;
   }
   return sa;
 }
@@ -982,6 +1000,7 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_batch_run: output arena needs d_pos and d_idx");
   cudaStream_t st = (cudaStream_t)stream;
   bmf_status s;
+  if ((s = team_check(ctx, b->team)) != BMF_OK) return s;
   if (batch_keys(b) && (s = batch_proc_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
   if ((s = batch_list_scratch(b, out->vcap)) != BMF_OK) return s;
   if (use_graph) {
@@ -1019,7 +1038,7 @@ bmf_status bmf_batch_run(bmf_batch* b, bmf_batch_out* out, int32_t use_graph, in
     out->n_idx = b->h_pinned[1];
     if (out->n_verts > out->vcap || out->n_idx > out->icap)
       return fail(ctx, BMF_ERR_CAPACITY, "bmf_batch_run: output capacity exceeded (needed totals reported)");
-    if (b->form == kSweepTeam) return team_check(ctx, b->team);
+    return team_check(ctx, b->team);
   }
   return BMF_OK;
 }
@@ -1045,7 +1064,7 @@ bmf_status bmf_batch_wait(bmf_batch* b, bmf_batch_out* out, int32_t timeout_ms) 
   out->n_idx = b->h_pinned[1];
   if (out->n_verts > out->vcap || out->n_idx > out->icap)
     return fail(ctx, BMF_ERR_CAPACITY, "bmf_batch_wait: output capacity exceeded (needed totals reported)");
-  return b->form == kSweepTeam ? team_check(ctx, b->team) : BMF_OK;
+  return team_check(ctx, b->team);
 }
 
 bmf_status bmf_batch_wait_extraction(bmf_batch* b, void* stream) {
@@ -1132,7 +1151,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   for (int k = 3; k < 6; ++k) BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[k], ev[k], ev[k + 1]));
   for (auto& e : ev) cudaEventDestroy(e);
   ctx->launches += 3 + fixups + (b->d_cols ? 1 : 0) + ek + pk;
-  return BMF_OK;
+  return team_check(ctx, b->team);
 }
 
 bmf_status bmf_batch_format(bmf_batch* b, const bmf_batch_out* out, int32_t unwind, int32_t smooth_normals,
@@ -1297,7 +1316,7 @@ struct bmf_fit {
   SweepLists sweep;               // the chunk-by-chunk sweeps' work lists, and the adjoint's queue over them
   int* d_pqueue = nullptr;
   SweepForm form = kSweepLaunches;  // the forward's sweeps
-  TeamSync* team = nullptr;       // barrier of the whole-mesh sweep kernel
+  Team team;
   uint32_t* d_qlist = nullptr;    // QEF-placed vertices of the forward, for the wide backward (+ counter at [vcap])
   float* d_qseed = nullptr;       // their FP32 eigenvectors (9 per entry), recorded by the forward
   uint8_t* d_qflag = nullptr;     // per vertex: took the QEF branch in the forward
@@ -1315,7 +1334,7 @@ bmf_status bmf_fit_destroy(bmf_fit* f) {
   void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.rec,
                   f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
                   f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_h, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
-                  f->d_pqueue, f->d_vadj, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team};
+                  f->d_pqueue, f->d_vadj, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team.sync};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (f->h_pinned) cudaFreeHost(f->h_pinned);
@@ -1365,8 +1384,6 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
             cudaMalloc(&f->d_words, sizeof(uint32_t) * words) == cudaSuccess &&
             cudaMalloc(&f->d_totals, sizeof(int64_t) * kTotals) == cudaSuccess &&
             cudaMalloc(&f->d_ticket, sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&f->team, sizeof(TeamSync)) == cudaSuccess &&
-            cudaMemset(f->team, 0, sizeof(TeamSync)) == cudaSuccess &&
             cudaMemset(f->d_ticket, 0, sizeof(int)) == cudaSuccess &&
             cudaMalloc(&f->ws.pb, sizeof(uint2) * n_chunks * dim) == cudaSuccess &&
             cudaMalloc(&f->ws.vcnt, sizeof(uint32_t) * words) == cudaSuccess &&
@@ -1390,7 +1407,8 @@ bmf_status bmf_fit_create(bmf_ctx* ctx, int32_t n_chunks, int32_t dim, int32_t p
               cudaMalloc(&f->d_qflag, vcap + 1) == cudaSuccess)) &&
             cudaMalloc(&f->d_clist, sizeof(uint2) * words) == cudaSuccess &&
             cudaMalloc(&f->d_lpart, sizeof(float) * kFitLossPartials) == cudaSuccess &&
-            cudaMallocHost(&f->h_pinned, sizeof(int64_t) * 4) == cudaSuccess &&
+            cudaMallocHost(&f->h_pinned, sizeof(int64_t) * kPlanPinned) == cudaSuccess &&
+            team_create(&f->team, f->h_pinned) == cudaSuccess &&
             cudaMemcpy(f->d_chunks, hc.data(), sizeof(ChunkDev) * n_chunks, cudaMemcpyHostToDevice) == cudaSuccess &&
             cudaMemcpy(f->d_units, units.data(), sizeof(int) * (n_chunks + 1), cudaMemcpyHostToDevice) == cudaSuccess;
   f->sweep.head = f->sweep.order + n_chunks;
@@ -1415,6 +1433,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
   bmf_ctx* ctx = f->ctx;
   if (!d_density || !d_pos || !d_idx) return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_fit_forward: null buffer");
   cudaStream_t st = (cudaStream_t)stream;
+  if (const bmf_status s = team_check(ctx, f->team); s != BMF_OK) return s;
   FieldDev fd{};
   fd.kind = BMF_FIELD_GRID;
   BMF_CUDA(ctx, cudaMemsetAsync(f->d_flags, 0, sizeof(uint32_t) * (f->n + kCounters), st));
@@ -1439,8 +1458,8 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
       sa.lists = f->sweep;
       sa.wide_adj = true;  // bmf_fit_backward's adjoint sweeps read it
     } else if (f->form == kSweepTeam) {
-      sa.team = f->team;
-      sa.team_failed = ctx->team_failed();
+      sa.team = f->team.sync;
+      sa.team_failed = f->team.mark;
     }
     k += launch_process(4, f->vcap, f->icap / 4, f->d_totals, d_pos, nullptr, f->d_boundary, f->d_valence, f->d_idxg,
                         f->iters, 0, 0, f->ps, &sa, st);
@@ -1453,7 +1472,7 @@ bmf_status bmf_fit_forward(bmf_fit* f, const float* d_density, float* d_pos, uin
     h_counts[1] = f->h_pinned[1];
     if (h_counts[0] > f->vcap || h_counts[1] > f->icap)
       return fail(ctx, BMF_ERR_CAPACITY, "bmf_fit_forward: output capacity exceeded (needed totals reported)");
-    if (f->form == kSweepTeam) return team_check(ctx, f->team);
+    return team_check(ctx, f->team);
   }
   return BMF_OK;
 }
@@ -1493,6 +1512,7 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
   if (!d_grad_pos || !d_grad_density || !f->last_density || n_grad_verts < 0)
     return fail(ctx, BMF_ERR_INVALID_ARGUMENT, "bmf_fit_backward: null buffer or no forward yet");
   cudaStream_t st = (cudaStream_t)stream;
+  if (const bmf_status s = team_check(ctx, f->team); s != BMF_OK) return s;
   const int64_t ng = n_grad_verts < f->vcap ? n_grad_verts : f->vcap;
   // with enough chunks to fill the GPU the adjoint sweeps run chunk by chunk
   StructuredAdj sa{BMF_MODE_Q, f->d_chunks, f->n, f->ws, f->d_vkey, f->d_vadj};
@@ -1501,8 +1521,8 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
     sa.lists = f->sweep;
     sa.bwd_queue = f->d_pqueue;
   } else if (f->form == kSweepTeam) {
-    sa.team = f->team;
-    sa.team_failed = ctx->team_failed();
+    sa.team = f->team.sync;
+    sa.team_failed = f->team.mark;
   }
   int k = 0;
   if (f->iters > 0 && f->icap >= 4) {
@@ -1521,6 +1541,15 @@ bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_
   return BMF_OK;
 }
 
+bmf_status bmf_debug_sweep_timeout(bmf_ctx* ctx, bmf_batch* b, bmf_fit* f, void* stream) {
+  BMF_TRACE("bmf_debug_sweep_timeout");
+  if (!ctx) return BMF_ERR_INVALID_ARGUMENT;
+  const Team& t = b ? b->team : (f ? f->team : ctx->team);
+  launch_team_timeout(t.sync, t.mark, (cudaStream_t)stream);
+  BMF_LAUNCHED(ctx, 1);
+  return BMF_OK;
+}
+
 bmf_status bmf_batch_destroy(bmf_batch* b) {
   if (!b) return BMF_ERR_INVALID_ARGUMENT;
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -1528,7 +1557,7 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
                   b->ws.vcnt, b->ws.rec, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
                   b->d_fill_items, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
-                  b->d_cols, b->d_ticket, b->ws.pb, b->team, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
+                  b->d_cols, b->d_ticket, b->ws.pb, b->team.sync, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);

@@ -1293,10 +1293,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
   const unsigned team = min(gridDim.x, max(1u, (nv + kTeamVerts - 1u) / kTeamVerts));
   const unsigned rank = blockIdx.x;
   if (rank >= team || nv == 0) return;
-  if (*(volatile unsigned*)&A.sync->failed) {  // a launch before gave up and the host has not seen it yet
-    if (threadIdx.x == 0) *(volatile unsigned*)A.host_failed = 1u;
-    return;
-  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
   const int iters = A.iters;
   unsigned target = 0;
@@ -1427,12 +1423,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_team(const __grid_con
     }
     if (m + 1 < iters) team_barrier(A.sync, A.host_failed, target, team, dead);
   }
-  // the last CTA leaves the barrier ready for the next launch
-  __syncthreads();
-  if (tid == 0 && atomicAdd(&A.sync->left, 1u) == team - 1u) {
-    A.sync->arrived = 0u;
-    A.sync->left = 0u;
-  }
+  team_leave(A.sync, team);
 }
 
 template <int MODE, int N>

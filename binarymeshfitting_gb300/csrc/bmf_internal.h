@@ -185,7 +185,7 @@ struct SweepLists {
 };
 constexpr int kSweepHead = 4;
 // The barrier of the whole-mesh sweep kernel's team of CTAs (zeroed once; each
-// launch leaves arrived and left zero) and the CTAs' valence sums.
+// launch leaves its counters zero) and the CTAs' valence sums.
 constexpr int kTeamMax = 256;
 struct TeamSync {
   unsigned arrived, left, failed, pad;
@@ -301,6 +301,9 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          float* pos, float* nrm, const uint8_t* boundary, const uint8_t* valence,
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st);
+// Makes the wait of a team's barrier run out, in one CTA that returns after about
+// a millisecond: what a failed launch leaves behind.
+void launch_team_timeout(TeamSync* sync, unsigned* host_failed, cudaStream_t st);
 // Whether any mesh of this size takes the whole-mesh form (StructuredAdj mode 2).
 bool sweep_team_mesh(int N, int64_t nv, int64_t n_prims);
 // The whole-mesh form of launch_process in one cooperative launch (sa.team set).

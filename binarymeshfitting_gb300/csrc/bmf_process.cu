@@ -482,10 +482,6 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_bwd_team(const __grid
   const uint32_t cap = (uint32_t)min(4 * A.n_prims, (int64_t)UINT32_MAX);
   const unsigned team = min(gridDim.x, max(1u, (nv + kTeamVerts - 1u) / kTeamVerts)), rank = blockIdx.x;
   if (rank >= team || nv == 0u) return;
-  if (*(volatile unsigned*)&sync->failed) {  // a launch before gave up and the host has not seen it yet
-    if (threadIdx.x == 0) *(volatile unsigned*)host_failed = 1u;
-    return;
-  }
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   unsigned target = 0;
   bool dead = false;
@@ -516,12 +512,18 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_sweep_bwd_team(const __grid
     for (uint32_t v = v_own + kTeamThreads; v - lane < ve; v += kTeamThreads) bwd_vert(A, v, v < ve, cap, np, m == 0);
     if (m > 0) team_barrier(sync, host_failed, target, team, dead);
   }
-  // the last CTA leaves the barrier ready for the next launch
-  __syncthreads();
-  if (tid == 0 && atomicAdd(&sync->left, 1u) == team - 1u) {
-    sync->arrived = 0u;
-    sync->left = 0u;
-  }
+  team_leave(sync, team);
+}
+
+// One CTA of a team of two: its wait runs out after `limit` polls, and it leaves.
+__global__ void __launch_bounds__(32) k_team_timeout(TeamSync* sync, unsigned* host_failed, unsigned limit) {
+  unsigned target = 0;
+  bool dead = false;
+  team_barrier(sync, host_failed, target, 2u, dead, limit);
+  team_leave(sync, 1u);
+}
+void launch_team_timeout(TeamSync* sync, unsigned* host_failed, cudaStream_t st) {
+  k_team_timeout<<<1, 32, 0, st>>>(sync, host_failed, 1024u);
 }
 
 int launch_process_bwd(int64_t nv, int64_t n_prims, const int64_t* d_counts, const uint8_t* boundary,

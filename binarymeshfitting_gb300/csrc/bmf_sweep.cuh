@@ -47,15 +47,15 @@ constexpr int kTeamVerts = 256;  // vertices per CTA that make the team one CTA 
 constexpr int kTeamRegs = 6;     // list entries gathered at once (and kept for a thread's first vertex)
 
 // Barrier over the team's CTAs (all resident: a cooperative launch).  The wait
-// is bounded: after kTeamSpins polls (a second or so) or once another CTA has
-// given up, the CTA marks the team failed and no longer waits anywhere; the
-// host finds the mark after its synchronisation.  Thread 0 releases the CTA's
+// is bounded: after `limit` polls (a second or so) or once another CTA has
+// given up, the CTA marks the team failed and no longer waits anywhere, so that
+// every CTA comes to team_leave; the host finds the object's mark.  Thread 0 releases the CTA's
 // stores with its arrival and acquires the others' with its polls, and the block
 // barriers carry both to the other threads; sequentially consistent fences around
 // a relaxed arrival cost 0.3 us more a meeting (129^3 chunk: 117.8 against 113.8 us).
 constexpr unsigned kTeamSpins = 1u << 22;
 __device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed, unsigned& target, unsigned team,
-                                             bool& dead) {
+                                             bool& dead, unsigned limit = kTeamSpins) {
   __syncthreads();
   target += team;
   if (threadIdx.x == 0 && team > 1 && !dead) {
@@ -65,15 +65,25 @@ __device__ __forceinline__ void team_barrier(TeamSync* y, unsigned* host_failed,
     for (unsigned spins = 0;; ++spins) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&y->arrived) : "memory");
       if (v >= target) break;
-      if (spins >= kTeamSpins || ((spins & 1023u) == 1023u && *(volatile unsigned*)&y->failed)) {
+      if (spins >= limit || ((spins & 1023u) == 1023u && *(volatile unsigned*)&y->failed)) {
         *(volatile unsigned*)&y->failed = 1u;
         *(volatile unsigned*)host_failed = 1u;
+        __threadfence();  // before this CTA leaves
         dead = true;  // this CTA waits nowhere any more
         break;
       }
     }
   }
   __syncthreads();
+}
+// The team's last CTA leaves the barrier as the first launch found it, also after a
+// wait that ran out: nothing of a failed launch is left for the next one.
+__device__ __forceinline__ void team_leave(TeamSync* y, unsigned team) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(&y->left, 1u) == team - 1u) {
+    __threadfence();  // behind the others' last words
+    y->arrived = y->left = y->failed = 0u;
+  }
 }
 
 // COH selects the load for data that the same kernel also writes (positions,

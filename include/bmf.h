@@ -172,7 +172,7 @@ BMF_API bmf_status bmf_polygonize_noalloc(int32_t dim, const float* d_density, c
 /* MeshProcessor<N>::init/optimize_dual_grid/optimize_primal_grid/flush
  * (MeshProcessor.cpp:26-306) in the order ChunkGenerator::extract_chunk uses
  * (ChunkGenerator.cpp:112-124).  Updates d_pos (and d_nrm when non-NULL) in
- * place; N = mesh->prim_size. */
+ * place; N = mesh->prim_size.  Asynchronous (see "bounded waits" below). */
 BMF_API bmf_status bmf_process(bmf_ctx* ctx, bmf_mesh* mesh, int32_t iters, int32_t process_boundary,
                        int32_t smooth_normals, void* stream);
 
@@ -358,6 +358,21 @@ BMF_API bmf_status bmf_fit_adam(bmf_fit* f, float* d_param, const float* d_grad,
 BMF_API bmf_status bmf_fit_backward(bmf_fit* f, const float* d_grad_pos, int64_t n_grad_verts, float* d_grad_density,
                                     void* stream);
 BMF_API bmf_status bmf_fit_destroy(bmf_fit* f);
+
+/* ---- bounded waits ----
+ * The smoothing sweeps of small meshes (bmf_process, bmf_extract_chunk, plans of
+ * few chunks, forward and adjoint) run as one kernel whose blocks wait for one
+ * another.  Each wait gives up after a second or so -- which takes blocks that
+ * make no progress for that long -- and the kernel then ends without its result.
+ * The call that synchronises on it returns BMF_ERR_CUDA; where the call did not
+ * synchronise (bmf_process, bmf_batch_run with sync == 0, bmf_fit_forward without
+ * h_counts, bmf_fit_backward, a replayed graph), the next call on the same object
+ * that synchronises, or that is about to run the sweeps again (it then does
+ * nothing else), returns it.  Reported once, and only by the object -- context,
+ * batch or fit plan -- whose sweeps they were; all of them stay usable.
+ * For tests: makes such a wait run out, after about a millisecond, in a kernel of
+ * one block that then returns, for plan b, else plan f, else the context. */
+BMF_API bmf_status bmf_debug_sweep_timeout(bmf_ctx* ctx, bmf_batch* b, bmf_fit* f, void* stream);
 
 #ifdef __cplusplus
 }

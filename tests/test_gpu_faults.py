@@ -14,6 +14,7 @@ import torch
 from binarymeshfitting_gb300 import _lib as L
 from binarymeshfitting_gb300 import workloads
 from binarymeshfitting_gb300.engine import Batch
+from binarymeshfitting_gb300.fitting import FitPlan
 
 pytestmark = pytest.mark.gpu
 
@@ -165,3 +166,83 @@ def test_calls_work_after_an_allocation_that_failed(ctx):
     assert b.run(use_graph=True) == totals == (want.n_verts, want.n_idx)
     assert torch.equal(b.bufs["pos"][:totals[0]], want.pos)
     b.close()
+
+
+def test_a_sweep_wait_that_runs_out_is_reported_by_its_owner(ctx):
+    """The bounded waits of the one-launch sweeps, made to run out in a one-block kernel
+    that returns: only the object whose wait it was reports it, once, and its next
+    call is right again -- also where no call synchronised."""
+    field = workloads.terrain_field()
+    desc = L.ChunkDesc.make((0.0, 48.0, 0.0), 1.0, 33)
+    descs = [L.ChunkDesc.make((40.0 * i, 48.0, 0.0), 1.0, 33) for i in range(4)]
+    plans = [Batch(ctx, descs, field, mode=L.MODE_R, iters=4, smooth_normals=True) for _ in range(2)]
+    dens, sph = workloads.fit_batch(1, dim=33, seed=2, device=ctx.device)
+    fits = [FitPlan(ctx, 1, 33, iters=2) for _ in range(2)]
+    loss, grad = torch.zeros(1, device=ctx.device), torch.zeros_like(dens)
+    grad_pos = torch.zeros((fits[0].vcap, 3), device=ctx.device)
+    for b in plans:
+        b.allocate(1 << 16, 1 << 18, normals=True)
+
+    def chunk():
+        m = ctx.extract_chunk(desc, field, iters=4, smooth_normals=True)
+        return m.pos.clone(), m.nrm.clone()
+
+    def smoothed():
+        m = ctx.extract_chunk(desc, field)
+        m.nrm = torch.zeros_like(m.pos)
+        ctx.process(m, 4, False, True)
+        return m.pos.clone(), m.nrm.clone()
+
+    def update(b):
+        nv, _ = b.run()
+        return b.bufs["pos"][:nv].clone(), b.bufs["nrm"][:nv].clone()
+
+    def later(b):
+        b.run(sync=False)
+        nv, _ = b.wait(10_000)
+        return b.bufs["pos"][:nv].clone(), b.bufs["nrm"][:nv].clone()
+
+    def step(f):
+        f.step_grad(dens, sph, loss, grad_pos, grad)
+        return (f.pos[:int(f.info[:, 1].sum())].clone(),)
+
+    def counted(f):
+        return (f.forward(dens)[0].clone(),)
+
+    def adjoint(f):
+        assert f.backward(torch.ones_like(grad_pos)).abs().sum() > 0
+        return ()
+
+    calls = [(None, None, chunk), (None, None, smoothed), (plans[0], None, lambda: update(plans[0])),
+             (plans[0], None, lambda: later(plans[0])), (plans[1], None, lambda: update(plans[1])),
+             (None, fits[0], lambda: step(fits[0])), (None, fits[0], lambda: counted(fits[0])),
+             (None, fits[0], lambda: adjoint(fits[0])), (None, fits[1], lambda: counted(fits[1]))]
+    want = [c[2]() for c in calls]
+    handle = lambda o: o.h if o is not None else None
+    owners = {(id(b), id(f)): (b, f) for b, f, _ in calls}
+    for b, f in owners.values():
+        for k, (ob, of, call) in enumerate(calls):
+            L.check(ctx.lib.bmf_debug_sweep_timeout(ctx.h, handle(b), handle(f), None), ctx.h, ctx.lib)
+            torch.cuda.synchronize()
+            if (ob, of) == (b, f):
+                with pytest.raises(L.BmfError) as e:
+                    call()
+                assert e.value.status == L.ERR_CUDA and "ran out" in str(e.value)
+            assert all(torch.equal(x, y) for x, y in zip(call(), want[k])), k
+            # (take the mark of an owner that was not called)
+            for ob, of, call in calls:
+                if (ob, of) == (b, f):
+                    try:
+                        call()
+                    except L.BmfError:
+                        pass
+                    break
+    # a call that does not run the sweeps reports it as well, behind its own result
+    m = ctx.extract_chunk(desc, field)
+    L.check(ctx.lib.bmf_debug_sweep_timeout(ctx.h, None, None, None), ctx.h, ctx.lib)
+    with pytest.raises(L.BmfError) as e:
+        ctx.format(m)
+    assert e.value.status == L.ERR_CUDA
+    assert len(ctx.format(m)[0]) == m.n_verts
+    for o in plans + fits:
+        o.close()
