@@ -189,8 +189,9 @@ class WorldOctreeNode:
 class ChunkGenerator:
     """ChunkGenerator::process_queue (ChunkGenerator.cpp:27-147): the whole
     queue goes through one batched, graph-captured update.  The plan and its
-    output arena are kept while queues keep their shape (same chunk count and
-    resolution): the next queue's descriptors are swapped in with
+    output arena are kept while queues keep their shape and what the plan was made
+    from (chunk count, resolution, mode, placement, the properties that it bakes in
+    and the field): the next queue's descriptors are swapped in with
     bmf_batch_set_descs and the captured graph replays."""
 
     def __init__(self, properties: WorldProperties, sampler: Sampler, dim=RESOLUTION, mode=L.MODE_R,
@@ -201,6 +202,7 @@ class ChunkGenerator:
         self.mode = mode
         self.placement = placement
         self._plan: Optional[Batch] = None
+        self._plan_key = None
         self.plans_reused = 0
 
     def overlap_for(self, node: WorldOctreeNode):
@@ -225,14 +227,16 @@ class ChunkGenerator:
         descs = self._descs(batch)
         ctx = context()
         b = self._plan
-        if b is not None and b.n == len(batch):
+        key = (len(batch), self.dim, self.mode, self.placement, p.process_iters, bool(p.boundary_processing),
+               bool(p.smooth_normals), bytes(self.sampler.field))
+        if b is not None and key == self._plan_key:
             b.set_descs(descs)
             self.plans_reused += 1
         else:
             self.close()
             b = Batch(ctx, descs, self.sampler.field, mode=self.mode, placement=self.placement,
                       iters=p.process_iters, process_boundary=p.boundary_processing, smooth_normals=p.smooth_normals)
-            self._plan = b
+            self._plan, self._plan_key = b, key
             vcap, icap = max(4096, len(batch) * self.dim ** 2 * 4), max(16384, len(batch) * self.dim ** 2 * 24)
             b.allocate(vcap, icap, normals=p.smooth_normals)
         nv = ni = 0
@@ -252,4 +256,4 @@ class ChunkGenerator:
     def close(self):
         if self._plan is not None:
             self._plan.close()
-            self._plan = None
+            self._plan = self._plan_key = None

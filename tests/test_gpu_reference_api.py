@@ -91,3 +91,47 @@ def test_process_queue_reuses_its_plan(ctx):
         checked += 1
     assert checked >= 2
     gen.close()
+
+
+def _other_field(gen):  # another seed of the terrain
+    params = list(workloads.TERRAIN_PARAMS)
+    params[6] += 1
+    gen.sampler = R.Sampler(L.Field.make(L.FIELD_TERRAIN_FBM, params))
+
+
+def _moved_field(gen):  # the same Field object, changed in place
+    gen.sampler.field.params[0] += 3.0
+
+
+CHANGES = {"iters": lambda g: setattr(g.properties, "process_iters", 3),
+           "boundary": lambda g: setattr(g.properties, "boundary_processing", True),
+           "normals": lambda g: setattr(g.properties, "smooth_normals", False),
+           "dim": lambda g: setattr(g, "dim", 40), "mode": lambda g: setattr(g, "mode", L.MODE_Q),
+           "placement": lambda g: setattr(g, "placement", L.PLACE_QEF), "sampler": _other_field, "field": _moved_field}
+
+
+@pytest.mark.parametrize("change", list(CHANGES))
+def test_process_queue_follows_a_change_between_equal_queues(ctx, change):
+    """The kept plan serves queues of its own making only: what a changed generator
+    gives is what a new one gives."""
+    def nodes():
+        return [R.WorldOctreeNode(pos=(1000.0 + 64 * i, 16.0 - 24 * i, 2000.0), size=64.0, level=2) for i in range(4)]
+
+    def generator(mode):
+        props = R.WorldProperties(max_level=3, process_iters=2, boundary_processing=False, smooth_normals=True)
+        return R.ChunkGenerator(props, R.Sampler(workloads.terrain_field()), dim=33, mode=mode)
+
+    mode = L.MODE_Q if change == "placement" else L.MODE_R
+    gen, fresh = generator(mode), generator(mode)
+    gen.process_queue(nodes())
+    for g in (gen, fresh):
+        CHANGES[change](g)
+    got, want = gen.process_queue(nodes()), fresh.process_queue(nodes())
+    assert sum(len(n.vi["pos"]) for n in want) > 0
+    for a, b in zip(got, want):
+        for k in ("pos", "nrm", "boundary", "idx"):
+            assert (a.vi[k] is None) == (b.vi[k] is None)
+            assert a.vi[k] is None or a.vi[k].equal(b.vi[k]), k
+    assert gen.plans_reused == 0
+    gen.close()
+    fresh.close()
