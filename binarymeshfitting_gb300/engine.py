@@ -340,15 +340,22 @@ class Batch:
                     idx=b["idx"][io:io + ic], contains_mesh=bool(info[4]), status=int(info[5]))
 
     def chunk_meshes(self, n_verts, n_idx):
-        """chunk_mesh of every chunk of the last run, over one copy of its n_verts
-        vertices and n_idx indices (the arena may be overwritten): one read of
-        the chunk table and one copy per attribute, whatever the chunk count."""
+        """chunk_mesh of every chunk of the last run (n_verts vertices, n_idx indices) as
+        copies (the arena may be overwritten), each a tensor of its own, so that a kept
+        mesh keeps no other alive: one read of the chunk table and one grouped
+        copy per attribute.  Of 64 chunks 0.8 ms, most of it the 256 tensors; a clone
+        each takes 2.1 ms, views into one copy of the arena 0.3 ms."""
         info = self.bufs["info"].cpu().tolist()
         vc, ic = [r[1] for r in info], [r[3] for r in info]
         b = self.bufs
 
         def parts(t, n, sizes):
-            return t[:n].clone().split(sizes) if t is not None else [None] * len(sizes)
+            if t is None:
+                return [None] * len(sizes)
+            views = t[:n].split(sizes)
+            own = [torch.empty_like(v) for v in views]
+            torch._foreach_copy_(own, views)
+            return own
 
         return [dict(pos=p, nrm=q, boundary=f, idx=i, contains_mesh=bool(r[4]), status=int(r[5]))
                 for r, p, q, f, i in zip(info, parts(b["pos"], n_verts, vc), parts(b["nrm"], n_verts, vc),

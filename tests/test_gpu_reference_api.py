@@ -135,3 +135,24 @@ def test_process_queue_follows_a_change_between_equal_queues(ctx, change):
     assert gen.plans_reused == 0
     gen.close()
     fresh.close()
+
+
+@pytest.mark.parametrize("normals", [False, True])
+def test_a_queue_mesh_owns_its_memory(ctx, normals):
+    """A node's arrays hold its own mesh and nothing of the rest of the queue."""
+    props = R.WorldProperties(max_level=3, process_iters=2, smooth_normals=normals)
+    gen = R.ChunkGenerator(props, R.Sampler(workloads.terrain_field()), dim=33)
+    nodes = [R.WorldOctreeNode(pos=(1000.0 + 64 * i, 16.0 + 200.0 * (i % 2), 2000.0), size=64.0, level=2) for i in range(6)]
+    gen.process_queue(nodes)
+    sizes = [len(n.vi["pos"]) for n in nodes]
+    assert sum(s > 0 for s in sizes) >= 3 and 0 in sizes  # chunks with a surface, and without
+    for i, n in enumerate(nodes):
+        view = gen._plan.chunk_mesh(i)
+        for k in ("pos", "nrm", "boundary", "idx"):
+            t = n.vi[k]
+            assert (t is None) == (k == "nrm" and not normals)
+            if t is None:
+                continue
+            assert t.equal(view[k]) and t.untyped_storage().nbytes() == t.numel() * t.element_size()
+            assert t.numel() == 0 or t.data_ptr() != view[k].data_ptr()
+    gen.close()
