@@ -1274,7 +1274,7 @@ bmf_status bmf_batch_autotune(bmf_batch* b, bmf_batch_out* out, int32_t reps, vo
       s = time_it([&] { batch_sweeps(b, out, st); }, &ms);
       if (s != BMF_OK) return s;
       report.push_back(ms);
-      if (ms < best_ms) {
+      if (b->form == kSweepLaunches && ms < best_ms) {  // (the other forms have their own block size)
         best_ms = ms;
         best.sweep_block = bs;
       }

@@ -597,7 +597,6 @@ __global__ void __launch_bounds__(kScanThreads) k_chunk_scan(ChunkDev* __restric
     if (lane == 31) {
       sweep.head[0] = big;
       sweep.head[1] = incl;
-      sweep.head[2] = sweep.head[3] = 0;
     }
   }
   __syncthreads();
@@ -1506,6 +1505,7 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
   SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.ws, sa.vkey, sa.vadj, nv, n_prims, n_prims * N, d_counts, s.off,
               valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters,
               process_boundary, smooth_normals, sa.wide_adj ? 1 : 0};
+  cudaMemsetAsync(sa.lists.head + 2, 0, 2 * sizeof(int), st);  // the queues: each launch takes the whole lists
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;

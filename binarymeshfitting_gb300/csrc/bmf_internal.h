@@ -179,7 +179,7 @@ constexpr int kTotals = 3;
 // clusters, the others by single CTAs.
 struct SweepLists {
   int* order = nullptr;  // [n_chunks]
-  int* head = nullptr;   // {n_big, listed chunks, cluster queue, CTA queue}; the queues are zeroed with the lists
+  int* head = nullptr;   // {n_big, listed chunks, cluster queue, CTA queue}; launch_sweep_chunks zeroes the queues
   int cluster = 1;       // CTAs per cluster and CTAs in all of the launch that will take the lists
   int ctas = 1;
 };

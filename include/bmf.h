@@ -285,7 +285,8 @@ typedef struct {
   int32_t fill_mode;   /* terrain fill: 0 x-plane kernel, 1 one CTA per line item, 2 persistent CTAs taking
                           line items (largest chunks first) from a device work queue */
   int32_t fill_run;    /* line kernel tile height: z-samples per thread step, 4, 8 or 16 */
-  int32_t sweep_block; /* threads per CTA of the dual / primal sweeps: 128, 256 or 512 */
+  int32_t sweep_block; /* threads per CTA of the dual / primal sweeps: 128, 256 or 512 (plans that run them as
+                          one launch per step; the others have a size of their own) */
   int32_t fill_band;   /* 1: band fill (Mode R terrain plans, fill_mode 1 or 2): a run stops evaluating octaves
                           once the bound on the remaining octaves fixes every sample's sign, and only the ends of
                           sign-changing edges get exact densities (the mesh reads no others); for Mode R plans of
@@ -303,7 +304,8 @@ BMF_API bmf_status bmf_batch_set_tuning(bmf_batch* b, const bmf_batch_tuning* t)
 /* Autotuner: times every fill candidate (terrain fields) and every sweep block
  * size (iters > 0) on this plan and output arena, `reps` runs each (median of
  * CUDA-event times on `stream`), keeps the fastest of each stage and returns
- * the choice in *chosen (nullable).  h_ms (nullable) receives the median
+ * the choice in *chosen (nullable; sweep_block unchanged where it reaches
+ * nothing).  h_ms (nullable) receives the median
  * times in candidate order (fill candidates, then sweep candidates), at most
  * max_report of them; *n_report (nullable) their count.  Synchronises; on
  * return `out` holds a correct update made with the chosen tuning. */
