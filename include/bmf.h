@@ -306,7 +306,8 @@ BMF_API bmf_status bmf_batch_set_tuning(bmf_batch* b, const bmf_batch_tuning* t)
  * CUDA-event times on `stream`), keeps the fastest of each stage and returns
  * the choice in *chosen (nullable; sweep_block unchanged where it reaches
  * nothing).  h_ms (nullable) receives the median
- * times in candidate order (fill candidates, then sweep candidates), at most
+ * times in candidate order (fill candidates, a band fill with the pass that
+ * makes exact what the mesh reads; then sweep candidates), at most
  * max_report of them; *n_report (nullable) their count.  Synchronises; on
  * return `out` holds a correct update made with the chosen tuning. */
 BMF_API bmf_status bmf_batch_autotune(bmf_batch* b, bmf_batch_out* out, int32_t reps, void* stream,

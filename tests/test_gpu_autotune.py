@@ -35,3 +35,20 @@ def test_sweep_candidates_are_timed(ctx, n, mode):
     assert chosen["sweep_block"] == block or n == 200  # only one launch per step has a choice
     assert b.run() == want and torch.equal(b.bufs["pos"][:want[0]], mesh)
     b.close()
+
+
+@pytest.mark.parametrize("mode,place", [(L.MODE_R, L.PLACE_CENTER), (L.MODE_Q, L.PLACE_QEF),
+                                        (L.MODE_Q, L.PLACE_MASSPOINT), (L.MODE_Q, L.PLACE_CENTER)])
+def test_fill_candidates_are_timed_whole(ctx, mode, place):
+    """A band fill with what it leaves to the pass behind the count (Mode Q's QEF
+    placement: about half as much again), a full fill by itself."""
+    b = _plan(ctx, 400, mode, place)
+    want = b.run()
+    mesh = b.bufs["pos"][:want[0]].clone()
+    _, ms = b.autotune(reps=5)
+    for (fm, fr), t in zip([(0, 8), (1, 4), (1, 8), (1, 16), (2, 4), (2, 8), (2, 16)], ms):
+        b.set_tuning(fill_mode=fm, fill_run=fr)
+        fill = _stage(b, 0)
+        assert 0.85 * fill < t < 1.5 * fill, (fm, fr, t, fill)
+    assert b.run() == want and torch.equal(b.bufs["pos"][:want[0]], mesh)
+    b.close()
