@@ -20,7 +20,7 @@ namespace {
 
 enum Slot {
   S_CHUNKS, S_TOT, S_TOTALS, S_WORDS, S_DENS, S_VCNT, S_REC,
-  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_X2, S_COLS, S_VADJ, S_QUADS, S_NUM
+  S_OFF, S_CURSOR, S_ADJ, S_DUALP, S_DUALN, S_SCANTMP, S_VKEY, S_CLIST, S_LOD, S_PB, S_X0, S_X1, S_COLS, S_VADJ, S_QUADS, S_NUM
 };
 
 constexpr int kMaxDim = 512;
@@ -369,7 +369,7 @@ bmf_status process_scratch(bmf_ctx* ctx, int N, int64_t nv, int64_t n_prims, flo
   if ((s = scratch(ctx, S_ADJ, (size_t)n_prims * N, &ps.adj)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_DUALP, (size_t)n_prims * 4, &ps.dual_p)) != BMF_OK) return s;
   if ((s = scratch(ctx, S_DUALN, (size_t)n_prims * 2, &ps.dual_n)) != BMF_OK) return s;
-  for (int k = 0; x && k < 3; ++k) ps.x[k] = x[k];
+  for (int k = 0; x && k < 2; ++k) ps.x[k] = x[k];
   if ((s = scratch(ctx, S_SCANTMP, (size_t)(nv / 4096 + 2), &ps.tmp)) != BMF_OK) return s;
   BMF_LAUNCHED(ctx, launch(ps));
   return BMF_OK;
@@ -641,9 +641,9 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   const int64_t ib = std::min(out->icap, chunk_max_idx(dim, opts->mode));
   const bool bounded = 40 * vb + 4 * ib + 24 * (ib / N) <= kOneSyncBytes;
   // sweeps that leave steps out read the mesh from x[0] and write out->d_pos
-  float* x[3] = {};
+  float* x[2] = {};
   const int skip = bounded ? field_skipped(field->kind, opts->iters, opts->smooth_normals && out->d_nrm) : 0;
-  for (int k = 0; skip && k <= skip; ++k)
+  for (int k = 0; k < skip; ++k)
     if ((s = scratch(ctx, (Slot)(S_X0 + k), (size_t)vb * 3, &x[k])) != BMF_OK) return s;
   if (skip) {
     mo.pos = x[0];
@@ -884,7 +884,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   const int N = b->opts.mode == BMF_MODE_R ? 3 : 4;
   const int64_t np = icap / N;
   void** ptrs[] = {(void**)&b->ps.off, (void**)&b->ps.adj, (void**)&b->ps.dual_p, (void**)&b->ps.dual_n,
-                   (void**)&b->ps.tmp, (void**)&b->ps.x[0], (void**)&b->ps.x[1], (void**)&b->ps.x[2],
+                   (void**)&b->ps.tmp, (void**)&b->ps.x[0], (void**)&b->ps.x[1],
                    (void**)&b->d_idxg, (void**)&b->d_valence, (void**)&b->d_boundary, (void**)&b->d_vkey,
                    (void**)&b->d_vadj};
   for (void** p : ptrs) {
@@ -897,7 +897,7 @@ bmf_status batch_proc_scratch(bmf_batch* b, int64_t vcap, int64_t icap) {
   BMF_CUDA(ctx, cudaMalloc(&b->ps.dual_p, sizeof(float) * (4 * np + 4)));
   if (b->opts.smooth_normals) BMF_CUDA(ctx, cudaMalloc(&b->ps.dual_n, sizeof(float) * (2 * np + 2)));
   if (const int skip = field_skipped(b->field.kind, b->opts.iters, b->opts.smooth_normals))
-    for (int k = 0; k <= skip; ++k) BMF_CUDA(ctx, cudaMalloc(&b->ps.x[k], sizeof(float) * 3 * (vcap + 1)));
+    for (int k = 0; k < skip; ++k) BMF_CUDA(ctx, cudaMalloc(&b->ps.x[k], sizeof(float) * 3 * (vcap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->ps.tmp, sizeof(uint32_t) * (vcap / 4096 + 2)));
   if (b->opts.iters > 0) BMF_CUDA(ctx, cudaMalloc(&b->d_idxg, sizeof(uint32_t) * (icap + 1)));
   BMF_CUDA(ctx, cudaMalloc(&b->d_valence, vcap + 1));
@@ -1564,7 +1564,7 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
                   b->ws.vcnt, b->ws.rec, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
                   b->d_fill_items, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
-                  b->d_cols, b->d_ticket, b->ws.pb, b->team.sync, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1], b->ps.x[2]};
+                  b->d_cols, b->d_ticket, b->ws.pb, b->team.sync, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1]};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);

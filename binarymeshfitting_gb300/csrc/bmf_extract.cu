@@ -1457,7 +1457,7 @@ void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_pri
                        int iters, int process_boundary, int smooth_normals, const ProcessScratch& s,
                        cudaStream_t st) {
   TeamArgs A{sa.chunks, sa.n_chunks, sa.ws, sa.vkey, sa.vadj, nv, n_prims, d_counts, s.off, s.cursor, valence, s.adj, boundary,
-             idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
+             idx, SweepBufs{{s.x[0], s.x[1]}, pos, nrm}, s.dual_p, s.dual_n, iters, process_boundary,
              smooth_normals, sa.team, sa.team_failed};
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at{};
@@ -1503,7 +1503,7 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
                          const uint32_t* idx, int iters, int process_boundary, int smooth_normals,
                          const ProcessScratch& s, cudaStream_t st) {
   SweepArgs A{sa.chunks, sa.tot, sa.lists, sa.ws, sa.vkey, sa.vadj, nv, n_prims, n_prims * N, d_counts, s.off,
-              valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1], s.x[2]}, pos, nrm}, s.dual_p, s.dual_n, iters,
+              valence, s.adj, boundary, idx, SweepBufs{{s.x[0], s.x[1]}, pos, nrm}, s.dual_p, s.dual_n, iters,
               process_boundary, smooth_normals, sa.wide_adj ? 1 : 0};
   cudaMemsetAsync(sa.lists.head + 2, 0, 2 * sizeof(int), st);  // the queues: each launch takes the whole lists
   cudaLaunchConfig_t cfg{};

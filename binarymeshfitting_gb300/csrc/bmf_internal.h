@@ -214,11 +214,10 @@ int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks,
 // anew, so with at most three face sweeps they are computed in the last of
 // them alone.  A vertex keeps its older normal when its new one has n.y == 0
 // (MeshProcessor.cpp:287): the positions before the left-out sweeps are kept,
-// x[0] before the first, x[1] before the second, x[2] (src) before the last,
-// and primal_older_normal takes the normal of such a vertex from them.  Left out: the square roots and divisions of two of three
+// x[0] before the first, x[1] before the second, and primal_older_normal takes the normal of such a vertex from them.  Left out: the square roots and divisions of two of three
 // sweeps, a float2 gather per list entry and a normal written per vertex.
 struct SweepBufs {
-  float* x[3] = {nullptr, nullptr, nullptr};  // positions before the left-out sweeps and the last face sweep (null: none left out, in place)
+  float* x[2] = {nullptr, nullptr};  // positions before the left-out sweeps (null: none left out)
   float* pos = nullptr;                       // positions out
   float* nrm = nullptr;                       // normals out (null: none)
   __host__ __device__ bool keep() const { return x[0] != nullptr; }
@@ -247,8 +246,8 @@ __host__ __device__ inline SweepStep sweep_step(int m, int iters, int sn, bool k
   SweepStep s;
   s.normals = !sn ? 0 : (m > last ? 2 : (m < k ? 0 : 1));
   s.set_colors = m < k ? 0 : sweep_colors(m, iters);
-  s.src = k == 0 || m > k ? b.pos : (m == 0 ? b.x[0] : (m == 1 ? b.x[1] : b.x[2]));
-  s.dst = k == 0 || m >= k ? b.pos : (m == 0 ? b.x[1] : b.x[2]);
+  s.src = m >= k ? b.pos : (m == 0 ? b.x[0] : b.x[1]);
+  s.dst = m + 1 < k ? b.x[1] : b.pos;
   s.skipped = m == k ? k : 0;
   return s;
 }
@@ -262,7 +261,7 @@ struct ProcessScratch {
   float* dual_n;      // 2 * n_prims: normal y, z (unused without normals)
   // positions before the left-out face sweeps (3 * nv each; null: none are left
   // out): x[0] is where the emit put the mesh
-  float* x[3] = {nullptr, nullptr, nullptr};
+  float* x[2] = {nullptr, nullptr};
   uint32_t* tmp;      // scan scratch (block totals)
   int block;          // threads per CTA of the dual / primal sweeps (0 = 256)
 };

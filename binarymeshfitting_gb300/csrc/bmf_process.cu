@@ -612,7 +612,7 @@ int launch_process(int N, int64_t nv, int64_t n_prims, const int64_t* d_counts, 
     cursor = s.cursor;
     launched += 2;
   }
-  const SweepBufs b{{s.x[0], s.x[1], s.x[2]}, pos, nrm};
+  const SweepBufs b{{s.x[0], s.x[1]}, pos, nrm};
   for (int m = 0; m < iters; ++m) {
     const SweepStep step = sweep_step(m, iters, sn ? 1 : 0, b.keep(), b);
     if (pbt == 0) {
