@@ -331,11 +331,12 @@ void qef_bwd_run(int64_t vcap, cudaStream_t st, A... args) {
 
 }  // namespace
 
-// Double-float: lists that one or two waves of 128-thread CTAs take (the capacity is
-// about twice the list) go out in those, spread over more SMs with half the warps per
+// Double-float: lists that one or two waves of 128-thread CTAs take go out in those, spread over more SMs with half the warps per
 // barrier (fit steps, us, 128 / 256 threads: 1 x 65^3 173 / 181, 4 x 192 / 201, 16 x
 // 284 / 291); longer ones in 256-thread CTAs, whose warps share more of the code's
-// fetches (512 x 4310 / 4020).
+// fetches (512 x 4310 / 4020).  The host knows the arena's capacity, not the list (which is
+// about half of it in the usual arena): a small list in a far larger arena takes the
+// longer lists' form, and its 8 us.
 void launch_qef_bwd(int wide, const ChunkDev* d_chunks, int n_chunks, const uint32_t* words, const float* dens,
                     const uint32_t* vkey, int64_t vcap, const float* grad_pos, float* grad_dens, const uint32_t* qlist,
                     const uint32_t* qcount, const float* qseed, cudaStream_t st) {

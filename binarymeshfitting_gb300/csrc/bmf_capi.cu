@@ -635,7 +635,9 @@ bmf_status bmf_extract_chunk(bmf_ctx* ctx, const bmf_chunk_desc* desc, const bmf
   // What the capacities, bounded by the chunk's size, ask of the sweeps'
   // scratch: within kOneSyncBytes the sweeps are enqueued behind the emit with
   // the counts on the device, and positions are kept for left-out face
-  // sweeps; beyond (large chunks) they wait for the counts and are sized by them.
+  // sweeps; beyond (capacities far above a chunk's needs, large chunks) they wait for
+  // the counts and are sized by them.  The second wait costs 8 us at 33^3 and 129^3
+  // (74 / 83, 107 / 116), 11 at 257^3 (212 / 222): the bound is there for the memory.
   constexpr int64_t kOneSyncBytes = 256ll << 20;
   const int64_t vb = std::min(out->vcap, chunk_max_verts(dim, opts->mode));
   const int64_t ib = std::min(out->icap, chunk_max_idx(dim, opts->mode));
@@ -1118,7 +1120,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   const bool proc = b->opts.iters > 0;
   if (batch_keys(b) && (s = batch_proc_scratch(b, out->vcap, out->icap)) != BMF_OK) return s;
   if ((s = batch_list_scratch(b, out->vcap)) != BMF_OK) return s;
-  cudaEvent_t ev[8];
+  cudaEvent_t ev[7];
   for (auto& e : ev) BMF_CUDA(ctx, cudaEventCreate(&e));
   BMF_CUDA(ctx, cudaEventRecord(ev[0], st));
   BMF_CUDA(ctx, cudaMemsetAsync(b->d_flags, 0, sizeof(uint32_t) * (b->n + kCounters), st));
@@ -1128,8 +1130,7 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaEventRecord(ev[2], st));
   // the band fill's exact-density fix-up belongs to the fill stage
   const int fixups = batch_fixup(b, st);
-  BMF_CUDA(ctx, cudaEventRecord(ev[7], st));
-  BMF_CUDA(ctx, cudaEventRecord(ev[3], st));  // the word scan is part of the count
+  BMF_CUDA(ctx, cudaEventRecord(ev[3], st));
   launch_chunk_scan(b->d_chunks, b->n, b->ws, b->d_tot, b->d_flags, out->vcap, out->icap, out->d_chunk_info,
                     b->d_totals, b->h_pinned, b->d_ticket, st, &b->sweep);
   BMF_CUDA(ctx, cudaEventRecord(ev[4], st));
@@ -1144,10 +1145,10 @@ bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms
   BMF_CUDA(ctx, cudaPeekAtLastError());
   float fix = 0.0f;
   BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[0], ev[0], ev[1]));
-  BMF_CUDA(ctx, cudaEventElapsedTime(&fix, ev[2], ev[7]));
+  BMF_CUDA(ctx, cudaEventElapsedTime(&fix, ev[2], ev[3]));
   h_stage_ms[0] += fix;
   BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[1], ev[1], ev[2]));
-  BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[2], ev[7], ev[3]));
+  h_stage_ms[2] = 0.0f;  // (the word scan is part of the count)
   for (int k = 3; k < 6; ++k) BMF_CUDA(ctx, cudaEventElapsedTime(&h_stage_ms[k], ev[k], ev[k + 1]));
   for (auto& e : ev) cudaEventDestroy(e);
   ctx->launches += 3 + fixups + (b->d_cols ? 1 : 0) + ek + pk;
@@ -1339,7 +1340,7 @@ extern "C" {
 bmf_status bmf_fit_destroy(bmf_fit* f) {
   if (!f) return BMF_ERR_INVALID_ARGUMENT;
   void* ptrs[] = {f->d_chunks, f->d_units, f->d_flags, f->d_tot, f->d_words, f->d_totals, f->ws.vcnt, f->ws.rec,
-                  f->ps.off, f->ps.cursor, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
+                  f->ps.off, f->ps.adj, f->ps.dual_p, f->ps.dual_n, f->ps.tmp, f->d_idxg,
                   f->d_vkey, f->d_valence, f->d_boundary, f->d_g, f->d_h, f->d_qlist, f->d_qseed, f->d_clist, f->sweep.order,
                   f->d_pqueue, f->d_vadj, f->ws.quads, f->d_qflag, f->d_lpart, f->d_ticket, f->ws.pb, f->team.sync};
   for (void* p : ptrs)
@@ -1561,7 +1562,7 @@ bmf_status bmf_batch_destroy(bmf_batch* b) {
   if (!b) return BMF_ERR_INVALID_ARGUMENT;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   void* ptrs[] = {b->d_chunks, b->d_units, b->d_flags, b->d_tot, b->d_totals, b->d_dens, b->d_words,
-                  b->ws.vcnt, b->ws.rec, b->ps.off, b->ps.cursor, b->ps.adj, b->ps.dual_p,
+                  b->ws.vcnt, b->ws.rec, b->ps.off, b->ps.adj, b->ps.dual_p,
                   b->ps.dual_n, b->ps.tmp, b->d_idxg, b->d_valence, b->d_boundary, b->d_vkey,
                   b->d_fill_items, b->sweep.order, b->d_clist, b->d_exact, b->d_fix,
                   b->d_cols, b->d_ticket, b->ws.pb, b->team.sync, b->ws.quads, b->d_vadj, b->ps.x[0], b->ps.x[1]};

@@ -179,7 +179,9 @@ static __device__ const EdgeTris g_edge_tris = make_edge_tris();
 
 // With few planes (a chunk or a small batch) a CTA of 256 threads per plane shortens
 // the walk over its words (129^3: 645 words); a whole update's planes fill the GPU
-// with a warp each, which leaves out the block's barriers and the quiet words.
+// with a warp each, which leaves out the block's barriers and the quiet words.  Mixed
+// updates without sweeps, us, a warp / a CTA per plane: 20 chunks (1.3 k planes) 183 /
+// 175, 32 (2.0 k) 192 / 189, 48 (2.9 k) 174 / 177, 96 243 / 259, 400 625 / 714.
 constexpr int kCountThreads = 256;
 constexpr int kCountFewUnits = 2048;
 
@@ -677,6 +679,8 @@ __device__ __forceinline__ uint32_t q_vertex_base(const uint32_t* vbase, const u
   return __ldg(&pb[x].x) + __ldg(vbase + wi) + __popc(r.x & lt) + 2 * __popc(r.y & lt) + 4 * __popc(r.z & lt);
 }
 
+// Without a work list (the allocation-free call, which keeps no vertex keys either): a
+// CTA per x-plane, a warp per busy word.
 template <int MODE, int PLACE>
 __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunks, int n_chunks,
                                               const int* __restrict__ unit_start, const uint32_t* __restrict__ words,
@@ -748,7 +752,6 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
             out.boundary[gv] = (x == 0 || y == 0 || z == 0 || x == dim - 1 || y == dim - 1 || z == dim - 1 ||
                                 x1 == dim - 1 || y1 == dim - 1 || z1 == dim - 1);
           if (out.nrm) { out.nrm[3 * gv] = 0.0f; out.nrm[3 * gv + 1] = 0.0f; out.nrm[3 * gv + 2] = 0.0f; }
-          if (out.vkey) out.vkey[gv] = vertex_key(x, y, z, a);
           if (out.valence) {
             // init_valence: uses of this edge by the (up to) four interior
             // cells around it (polygonize skips far-face cells, DMCChunk.cpp:528).
@@ -779,10 +782,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
         const int e = tri_edge(tw, i);
         const uint32_t vid = nb_vertex_id(nb, dim, x, y, zb, c_edge_owner[e][0], c_edge_owner[e][1],
                                           z + c_edge_owner[e][2], c_edge_owner[e][3]);
-        if (gi < out.icap) {
-          out.idx[gi] = vid;
-          if (out.idx_global) out.idx_global[gi] = (uint32_t)(ch.vout + vid);
-        }
+        if (gi < out.icap) out.idx[gi] = vid;
       }
     } else {
       // ---- Mode Q vertices: one per vertex group of each interior surface cell ----
@@ -797,19 +797,13 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
         for (int g = 0; g < ng; ++g, ++vid) {
           const int64_t gv = ch.vout + vid;
           if (gv >= out.vcap) continue;
-          // QEF positions come from k_place_qef (thread per vertex) when the
-          // vertex keys are kept; only here on the few lanes of surface cells
-          // otherwise
-          if (PLACE != 2 || !out.vkey) {
-            float P[3];
-            q_place<PLACE, false>(D, dim, x, y, z, group_edges(mask, g), P);
-            out.pos[3 * gv] = P[0];
-            out.pos[3 * gv + 1] = P[1];
-            out.pos[3 * gv + 2] = P[2];
-          }
+          float P[3];
+          q_place<PLACE, false>(D, dim, x, y, z, group_edges(mask, g), P);
+          out.pos[3 * gv] = P[0];
+          out.pos[3 * gv + 1] = P[1];
+          out.pos[3 * gv + 2] = P[2];
           if (out.nrm) { out.nrm[3 * gv] = 0.0f; out.nrm[3 * gv + 1] = 0.0f; out.nrm[3 * gv + 2] = 0.0f; }
           if (out.boundary) out.boundary[gv] = bnd;
-          if (out.vkey) out.vkey[gv] = vertex_key(x, y, z, g);
           if (out.valence) {
             int val = 0;
             for (int e = 0; e < 12; ++e) {
@@ -855,10 +849,7 @@ __global__ void __launch_bounds__(256) k_emit(const ChunkDev* __restrict__ chunk
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k, ++gi)
-          if (gi < out.icap) {
-            out.idx[gi] = q[k];
-            if (out.idx_global) out.idx_global[gi] = (uint32_t)(ch.vout + q[k]);
-          }
+          if (gi < out.icap) out.idx[gi] = q[k];
       }
     }
     }
@@ -1085,7 +1076,8 @@ __device__ __forceinline__ void sweep_older(const SweepArgs& A, ChunkPart c, int
 template <int MODE, int N>
 __global__ void __launch_bounds__(kSweepThreads, kSweepCtas) k_sweep_chunks(
     const ChunkDev* __restrict__ chunks, const uint32_t* __restrict__ tot, SweepLists lists,
-    WordScratch ws, const uint32_t* __restrict__ vkey, const uint32_t* __restrict__ vadj, int64_t nv, int64_t n_prims, int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
+    WordScratch ws, const uint32_t* __restrict__ vkey, const uint32_t* __restrict__ vadj, int64_t nv, int64_t n_prims,
+    int64_t adj_cap, const int64_t* __restrict__ d_counts, uint32_t* __restrict__ off,
     const uint8_t* __restrict__ valence, uint32_t* __restrict__ adj, const uint8_t* __restrict__ boundary,
     const uint32_t* __restrict__ idx, SweepBufs b_, float* __restrict__ dual_p, float* __restrict__ dual_n, int iters,
     int process_boundary, int sn, int wide_adj) {
@@ -1474,10 +1466,10 @@ void launch_sweep_team(const StructuredAdj& sa, int N, int64_t nv, int64_t n_pri
   else cudaLaunchKernelEx(&cfg, k_sweep_team<2, 4>, A);
 }
 
-// Clusters of `size` (1, 2, 4 or 8) CTAs that can be resident at once (negative: none).
+// Clusters of `size` (1, 2 or 4) CTAs that can be resident at once (negative: none).
 template <int MODE, int N>
 static int sweep_max_clusters(int size) {
-  static std::atomic<int> slots[4][64] = {};
+  static std::atomic<int> slots[3][64] = {};
   int lg = 0;
   while ((1 << lg) < size) ++lg;
   return per_device_once(slots[lg], [size](int dev) {
@@ -1544,7 +1536,9 @@ void launch_sweep_chunks(const StructuredAdj& sa, int N, int64_t nv, int64_t n_p
 // A team pays off while a step is shorter than a launch; its 16 warps per SM
 // carry fewer gathers than full occupancy once steps are long.  A chunk per CTA
 // or cluster needs several chunks per resident CTA to balance, or equal ones (a
-// fit plan's) that fill the GPU as clusters.  Clusters of 4 against 2 and 1 (taken with the adjacency built from
+// fit plan's) that fill the GPU as clusters.  Between 256 and 384 mixed chunks the two
+// forms are within 5 % of each other, and which is ahead depends on the field and
+// the number of sweeps as well: 320 is the middle.  Clusters of 4 against 2 and 1 (taken with the adjacency built from
 // the occupancy words): 512 chunks 1643 / 1802 / 2434 us, 1024 chunks 2996 / 2954 /
 // 3456, 2048 chunks 5805 / 5764 / 5781.
 constexpr int64_t kTeamColumns = 140000;
@@ -1715,7 +1709,10 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
   const int64_t nwarps = (int64_t)gridDim.x * kEmitWarps;
   // A short list (a chunk) is spread over the whole grid, few words per warp:
   // a tile's time is the chain of its phases and rounds, whatever its size
-  // (33^3 chunk, ~300 busy words: 16 us as 16-word tiles on 19 warps).
+  // (33^3 chunk, ~300 busy words: 16 us as 16-word tiles on 19 warps).  Whole calls
+  // without sweeps, us, spread / not: 33^3 48 / 58, 65^3 50 / 62, 129^3 75 / 85, 257^3
+  // 158 / 164, Mode Q 129^3 73 / 77; longer lists fill the tiles (32 chunks 188 / 189),
+  // and a line at whole instead of half tiles changes nothing (within 0.5 us).
   const bool spread = n <= nwarps * (kTileWords / 2);
   const int64_t tw = spread ? (n + nwarps - 1) / nwarps : kTileWords;
   const int64_t w0 = spread ? (int64_t)warp * gridDim.x + blockIdx.x : (int64_t)blockIdx.x * kEmitWarps + warp;
@@ -2129,10 +2126,9 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_q(const Chunk
       in = in && gv < out.vcap;
       const int dim = R.dim[t], x = R.x[t], y = R.y[t], z = 32 * R.zb[t] + l;
       const int mask = qtile_mask(R.w[t], 1, 1, 32 + l);
-      const uint32_t edges = in && (PLACE != 2 || !out.vkey) ? group_edges(mask, g & 3) : 0u;
-      if (PLACE != 2 || !out.vkey) {
+      if (PLACE != 2) {  // (QEF positions come from k_place_qef)
         float P[3];
-        q_place<PLACE, true>(dens + R.dens[t], dim, x, y, z, edges, P);
+        q_place<PLACE, true>(dens + R.dens[t], dim, x, y, z, in ? group_edges(mask, g & 3) : 0u, P);
         if (in) {
           out.pos[3 * gv] = P[0];
           out.pos[3 * gv + 1] = P[1];
@@ -2318,11 +2314,10 @@ int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks,
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_emit_words_q<1>, 32 * kEmitWarps, 0);
       return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
     });
-    if (placement == 2 && (!out.vkey || !d_counts)) out.vkey = nullptr;
     if (placement == 0) k_emit_words_q<0><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
     else if (placement == 1) k_emit_words_q<1><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
     else k_emit_words_q<2><<<g, 32 * kEmitWarps, 0, st>>>(d_chunks, words, dens, ws, out);
-    if (placement == 2 && out.vkey && out.vcap > 0) {
+    if (placement == 2 && out.vcap > 0) {
       launch_place_qef(d_chunks, n_chunks, words, dens, out, d_counts, st);
       return 2;
     }
@@ -2331,12 +2326,7 @@ int launch_emit(int mode, int placement, const ChunkDev* d_chunks, int n_chunks,
   } else if (placement == 1) {
     k_emit<1, 1><<<n_units, 256, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, dens, flags, ws, out);
   } else {
-    if (!out.vkey || !d_counts) out.vkey = nullptr;  // no keys: the emit places in place
     k_emit<1, 2><<<n_units, 256, 0, st>>>(d_chunks, n_chunks, d_unit_start, words, dens, flags, ws, out);
-    if (out.vkey && out.vcap > 0) {
-      launch_place_qef(d_chunks, n_chunks, words, dens, out, d_counts, st);
-      return 2;
-    }
   }
   return 1;
 }

@@ -43,7 +43,10 @@ __device__ __forceinline__ void cluster_store(uint32_t* p, uint32_t rank, uint32
 }
 
 constexpr int kTeamThreads = 512;
-constexpr int kTeamVerts = 256;  // vertices per CTA that make the team one CTA larger
+// Vertices per CTA that make the team one CTA larger.  Whole calls, us, at 128 / 256 / 512 /
+// 1024: 33^3 75 / 75 / 79 / 91, 65^3 76 / 77 / 81 / 98, 129^3 110 / 110 / 112 / 128, Mode Q
+// 65^3 with eight sweeps 92 / 94 / 97 / 116, fit step 65^3 167 / 165 / 171 / 202.
+constexpr int kTeamVerts = 256;
 constexpr int kTeamRegs = 6;     // list entries gathered at once (and kept for a thread's first vertex)
 
 // Barrier over the team's CTAs (all resident: a cooperative launch).  The wait

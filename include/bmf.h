@@ -230,8 +230,8 @@ BMF_API bmf_status bmf_batch_wait_extraction(bmf_batch* b, void* stream);
 BMF_API bmf_status bmf_batch_set_descs(bmf_batch* b, const bmf_chunk_desc* h_descs, int32_t n_chunks, void* stream);
 /* Runs one update stage by stage (no graph) with CUDA events between the
  * stages on `stream` and returns the stage times in ms:
- * h_stage_ms[0] fill+label, [1] count (with the word scan), [2] nothing any
- * more (a separate word scan once), [3] chunk scan and offsets, [4] emit,
+ * h_stage_ms[0] fill+label, [1] count (with the word scan), [2] 0 (a separate
+ * word scan once), [3] chunk scan and offsets, [4] emit,
  * [5] mesh processing. */
 BMF_API bmf_status bmf_batch_profile(bmf_batch* b, bmf_batch_out* out, float* h_stage_ms, void* stream);
 
