@@ -10,7 +10,9 @@
 //          polygonize and MeshProcessor<3>::init / optimize_dual_grid /
 //          optimize_primal_grid / flush, which must give the same bytes;
 //       3. ChunkGenerator::process_queue on two queues of the same shape (the
-//          second reuses the plan: new descriptors, graph replay).
+//          second reuses the plan: new descriptors, graph replay), and the
+//          last one again after each change of the properties, which must give
+//          what a new generator gives.
 //       Prints one JSON object with the counts and chunk frames, so a test can
 //       check them against the oracle.
 //
@@ -165,6 +167,20 @@ int check() {
                   (long long)nodes[i].vertex_count, (long long)nodes[i].index_count);
     }
     std::printf("]}");
+  }
+  std::printf("], \"after_changes\": [");
+  for (int k = 0; k < 3; ++k) {
+    if (k == 0) gen.props.process_iters = 4;
+    if (k == 1) gen.props.boundary_processing = true;
+    if (k == 2) gen.props.smooth_normals = false;
+    gen.process_queue(queue);
+    std::vector<float> got = gen.pos.to_host((size_t)gen.n_verts * 3, ctx.stream());
+    bmf::ChunkGenerator fresh(ctx, gen.props, {terrain(), 4096.0f}, 33);
+    fresh.process_queue(queue);
+    std::vector<float> want = fresh.pos.to_host((size_t)fresh.n_verts * 3, ctx.stream());
+    std::printf("%s{\"plans_reused\": %d, \"n_verts\": %lld, \"match_fresh\": %d}", k ? ", " : "", gen.plans_reused,
+                (long long)gen.n_verts,
+                (int)(got.size() == want.size() && std::memcmp(got.data(), want.data(), want.size() * 4) == 0));
   }
   std::printf("]}\n");
   return classes_match ? 0 : 1;

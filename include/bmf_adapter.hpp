@@ -308,8 +308,9 @@ struct WorldOctreeNode {
 
 /* ChunkGenerator::process_queue (ChunkGenerator.hpp:23) as one batched,
  * graph-replayed update.  The plan is kept while the queue keeps its shape
- * (same chunk count and resolution): the next queue's descriptors are swapped
- * in with bmf_batch_set_descs and the captured graph replays. */
+ * (same chunk count) and props keep what the plan was made from (the sweeps, the
+ * boundary, the normals): the next queue's descriptors are swapped in with
+ * bmf_batch_set_descs and the captured graph replays. */
 class ChunkGenerator {
  public:
   ChunkGenerator(Context& ctx, const WorldProperties& props, const Sampler& sampler, int dim = 33,
@@ -338,7 +339,10 @@ class ChunkGenerator {
       descs[i] = {{op.x, op.y, op.z}, delta, dim_, batch[i]->level};
     }
     bool fresh = false;
-    if (plan_ && plan_chunks_ == n) {
+    const bool same = props.process_iters == planned_.process_iters &&
+                      props.boundary_processing == planned_.boundary_processing &&
+                      props.smooth_normals == planned_.smooth_normals;
+    if (plan_ && plan_chunks_ == n && same) {
       check(bmf_batch_set_descs(plan_, descs.data(), n, ctx_->stream()), ctx_->get());
       ++plans_reused;
     } else {
@@ -348,6 +352,7 @@ class ChunkGenerator {
                             props.smooth_normals ? 1 : 0, 0};
       check(bmf_batch_create(ctx_->get(), descs.data(), n, &sampler_.field, &o, &plan_), ctx_->get());
       plan_chunks_ = n;
+      planned_ = props;
       info.reserve((size_t)n * 6);
       fresh = true;
     }
@@ -400,6 +405,7 @@ class ChunkGenerator {
   int dim_, mode_, placement_;
   bmf_batch* plan_ = nullptr;
   int plan_chunks_ = 0;
+  WorldProperties planned_;  // what plan_ was made from
   int64_t vcap_ = 0, icap_ = 0;
 };
 

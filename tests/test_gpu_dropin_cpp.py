@@ -62,6 +62,14 @@ def test_process_queue_reuses_its_plan_and_matches_oracle(report):
     assert checked >= 4
 
 
+def test_process_queue_follows_changed_properties(report):
+    """After a change of the sweeps, the boundary or the normals between two equal
+    queues: the meshes of a generator made with the new properties."""
+    assert len(report["after_changes"]) == 3
+    for c in report["after_changes"]:
+        assert c["match_fresh"] == 1 and c["n_verts"] > 0 and c["plans_reused"] == 1
+
+
 def test_time_loop_runs(tmp_path):
     """The per-chunk timing mode (used by bench.py) on a few chunks."""
     build.build()
