@@ -37,16 +37,15 @@ OPS_PER_SAMPLE = 1          # fma(-a, sum, py - h)
 OPS_PER_LINE_OCTAVE = 20    # xs, ys, 2 floor, xf, yf, 2 fade (5 each), x1, y1, fr, amp
 OPS_PER_LINE = 1            # py - h
 OPS_PER_LAYER = 20          # 4 corners (mul + fma), alpha and beta (3 lerps of 2 each)
-# DRAM bytes (read + write) of one launch of each kernel on the 4096-chunk update
-# (seed 2024, Mode R, 4 sweeps + normals), from one ncu capture of
-# dram__bytes_read.sum + dram__bytes_write.sum (one pass; profiles/
-# dram_bytes_lod_update_4096.txt).  Other workloads scale them: the fill and
+# DRAM bytes (read + write) of one launch of each kernel on a 1024-chunk update of the
+# same layout (Mode R, 4 sweeps + normals), one kernel per ncu capture (profiles/
+# dram_bytes_lod_update_1024.txt).  A workload scales them: the fill and
 # count by samples, the emit, scan and sweeps by output indices.
-DRAM_UPDATE_SAMPLES = 1_785_478_272
-DRAM_UPDATE_INDICES = 167_847_141
-DRAM_BYTES = {"fill": 397.2e6 + 1331.3e6 + 20.2e6 + 10.6e6,   # k_fill_terrain<16, band> + k_fill_fixup
-              "count": 475.6e6 + 212.6e6, "scan": 2.2e6, "emit": 1541.1e6 + 1476.6e6,
-              "sweeps": 11426.8e6 + 6894.6e6}
+DRAM_UPDATE_SAMPLES = 447_305_600
+DRAM_UPDATE_INDICES = 42_336_141
+DRAM_BYTES = {"fill": 93.6e6 + 292.5e6 + 3.3e6 + 0.7e6,   # k_fill_terrain<16, band> + k_fill_fixup
+              "count": 109.7e6 + 37.2e6, "scan": 0.6e6, "emit": 323.5e6 + 491.8e6,
+              "sweeps": 2801.0e6 + 1672.7e6}
 
 
 def fill_fp32_ops(rows, params):
@@ -256,8 +255,8 @@ def config(args):
             "topology": "mode R (reference Marching-Cubes triangles)" if args.mode == "R" else
             "mode Q (DMC quads, placement %d)" % args.placement,
             "smoothing_iters": args.iters, "smoothed_normals": not args.no_normals,
-            "l2": "working set larger than L2: a step moves about %.0f GB through DRAM (ncu on the 4096-chunk "
-                  "update: 24 GB, scaled by chunks), no flush between steps" % (24.0 * args.chunks / 4096),
+            "l2": "working set larger than L2: a step moves about %.0f GB through DRAM (scaled from ncu captures of "
+                  "each kernel on 1024 chunks), no flush between steps" % (23.0 * args.chunks / 4096),
             "parallelism": "replicas" if
             args.gpus == 1 else "weak: one independent update per GPU"}
 
@@ -566,7 +565,8 @@ def run_gb300(args):
                 if st_ms[5] > 0 else 0.0,
                 "own_bytes_note": "the logical bytes with the kernel's 16-bit adjacency lists (%d entries) "
                                   "counted at 2 B" % adj16_entries,
-                "traffic": dram["sweeps"], "traffic_unit": "DRAM bytes per launch (ncu, scaled to this update)",
+                "traffic": dram["sweeps"],
+                "traffic_unit": "DRAM bytes per launch (ncu capture of 1024 chunks, scaled to this update by indices)",
                 "dram_achieved": dram["sweeps"] / (st_ms[5] / 1000.0) / 1e9,
                 "dram_frac": dram["sweeps"] / (st_ms[5] / 1000.0) / 1e9 / hbm_peak,
                 "ms_per_launch": st_ms[5],

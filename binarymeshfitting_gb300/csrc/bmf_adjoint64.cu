@@ -10,14 +10,15 @@
 // pseudo-inverse are wide.  What remains, the chain rule into the density, is
 // a product of well-conditioned factors in FP32 on the forward's own hermite data.
 //
-// Bound by issue and by instruction fetch: the double-float code is larger than
-// the instruction caches, and warps at different places of it stall on fetches (8
-// of 12.6 cycles per issue with free-running warps).  So a CTA's warps go through
+// Bound by what 16 warps per SM leave uncovered of the latencies (0.59 of the issue
+// slots, the FMA pipe half busy).  The double-float code is larger than the
+// instruction caches, and free-running warps, at different places of it, stall on
+// fetches instead (8 of 12.6 cycles per issue; now 0.9).  So a CTA's warps go through
 // the parts together, with a block barrier between them and between the sweeps,
 // the three rotations of a sweep share one copy of the code (the axes change
 // places), and 128 registers keep the matrices out of local memory.  512 x 65^3
 // (3.9 M vertices): 2.40 -> 1.35 ms against one free-running thread per vertex at
-// 8 x 128 threads; one 65^3 grid 85 -> 44 us.
+// 8 x 128 threads; one 65^3 grid 85 -> 76 us.
 //
 // The wide operations and their order are what they were there: with the largest
 // gradients 1000 times the rms, a last bit of dL/dA is 1e-3 of the rms after the

@@ -1969,10 +1969,11 @@ __global__ void __launch_bounds__(32 * kEmitWarps, 4) k_emit_words_r(const Chunk
 // planes of the cell lines (x-1..x, y-1..y) in blocks zb-1, zb), then writes one
 // lane per vertex (the k-th vertex group of a word, from its group-count
 // planes) and one lane per quad (the k-th interior crossing edge; its four
-// cells' masks, groups and vertex ids from the staged lines).  Issue-bound: 512 x
-// 65^3 fitting grids (3.9 M vertices) 352 us, 512 mixed terrain chunks 180 us; the
-// thread-per-cell form it replaces read each quad's four cells from global
-// memory behind bounds checks (512 x 65^3 fitting grids: 607 us).
+// cells' masks, groups and vertex ids from the staged lines).  Bound by
+// shared-memory wavefronts (0.73 of peak) and issue (0.67): 512 x 65^3 fitting grids
+// (3.9 M vertices) 231 us, 512 mixed terrain chunks 132 us; the thread-per-cell form it
+// replaces read each quad's four cells from global memory behind bounds checks (512 x
+// 65^3 fitting grids: 607 us).
 struct QTile {
   uint4 rec[kTileWords][8];        // [2i+j][b]: record of cell line (x-1+i, y-1+j), block zb-1+b
   uint32_t w[kTileWords][27];      // [i][j][b]: line (x-1+i, y-1+j), block zb-1+b

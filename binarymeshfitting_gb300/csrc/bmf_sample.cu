@@ -36,9 +36,10 @@ __device__ __forceinline__ uint32_t word_class(uint32_t w) { return (w != 0u && 
 // and stores are whole 128-byte rows whatever the dim; a ballot gives 32
 // consecutive inside bits, the CTA's bit stream stays in shared memory, and each
 // occupancy word is cut out of it with a funnel shift (a line of 65 samples
-// is three words, the last of one bit).  Bound by HBM: 4 bytes per sample.
-// Runs of four samples per thread with a shared atomicOr each reached 1.5 TB/s
-// on a grid (512 x 65^3: 380 us).
+// is three words, the last of one bit).  4 bytes per sample of HBM traffic, bound by
+// the latency of the loads in flight (200 x 65^3: DRAM at 0.38 of its peak).  512 x
+// 65^3: 180 to 204 us; runs of four samples per thread with a shared atomicOr each took
+// 380.
 constexpr int kPlaneThreads = 256;
 constexpr int kPlaneUnroll = 8;  // rows in flight per warp
 
