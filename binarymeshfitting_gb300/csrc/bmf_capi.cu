@@ -134,7 +134,7 @@ bool batch_band(const bmf_batch* b) {
 int batch_fixup(bmf_batch* b, cudaStream_t st) {
   if (!batch_band(b) || b->field.kind != BMF_FIELD_TERRAIN_FBM) return 0;  // the 2D column fill needs none
   if (b->opts.mode == BMF_MODE_R)
-    launch_fill_fixup(b->d_chunks, b->ws, b->field, b->d_dens, st);
+    launch_fill_fixup(b->d_chunks, b->d_words, b->ws, b->field, b->d_dens, st);
   else if (b->opts.placement == BMF_PLACE_CENTER)
     return 0;  // reads no density
   else

@@ -144,8 +144,8 @@ int launch_adam(float* p, const float* g, float* m, float* v, int64_t n, int* st
                 float eps, cudaStream_t st);
 // exact densities for the samples the count kernel listed in ws.fix (the
 // inexact ends of crossings; after launch_count, before launch_emit)
-void launch_fill_fixup(const ChunkDev* d_chunks, const WordScratch& ws, const FieldDev& field, float* dens,
-                       cudaStream_t st);
+void launch_fill_fixup(const ChunkDev* d_chunks, const uint32_t* words, const WordScratch& ws, const FieldDev& field,
+                       float* dens, cudaStream_t st);
 // the same for a Mode Q mesh: the ends of all crossings, with grad also their
 // neighbours along the axes (what the QEF's central differences read)
 void launch_fill_need(bool grad, const ChunkDev* d_chunks, int n_chunks, const int* d_unit_start, int n_units,

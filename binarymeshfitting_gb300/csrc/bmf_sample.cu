@@ -664,8 +664,11 @@ __device__ float terrain_exact(const FieldDev& f, const int* __restrict__ perm2,
   return __fmaf_rn(-ampl, sum, py - h0);
 }
 
-__global__ void __launch_bounds__(256) k_fill_fixup(const ChunkDev* __restrict__ chunks, const uint2* __restrict__ list,
-                                                    const uint32_t* __restrict__ count, int64_t cap, FieldDev field,
+// One thread per listed sample.  An output arena that is too small for the mesh can
+// leave the list too short: the ends are then formed anew from the busy words (some of
+// them several times), so that the chunks that do fit are exact.
+__global__ void __launch_bounds__(256) k_fill_fixup(const ChunkDev* __restrict__ chunks,
+                                                    const uint32_t* __restrict__ words, WordScratch ws, FieldDev field,
                                                     float* __restrict__ dens) {
   __shared__ int perm2[512];
   __shared__ float4 gtab[512];
@@ -674,9 +677,33 @@ __global__ void __launch_bounds__(256) k_fill_fixup(const ChunkDev* __restrict__
     gtab[i] = grad_coeffs(field.perm[i & 255]);
   }
   __syncthreads();
-  const int64_t n = min((int64_t)*count, cap);
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    const uint2 ent = list[e];
+  const int64_t e0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  const int64_t n = *ws.fcount;
+  if (n > ws.fix_cap) {
+    const int64_t nb = min((int64_t)*ws.ccount, ws.clist_cap);
+    for (int64_t e = e0; e < nb; e += step) {
+      const uint2 ent = ws.clist[e];
+      const ChunkDev ch = chunks[ent.x];
+      const int dim = ch.dim, zc = ch.zc, xy = (int)ent.y / zc, zb = (int)ent.y - xy * zc, x = xy / dim, y = xy - x * dim;
+      const uint32_t* W = words + ch.words;
+      const auto fix = [&](uint32_t m, int xx, int yy, int zz) {  // the samples m of word (xx, yy, zz)
+        if (m) m &= ~__ldg(ws.exact + ch.words + ((int64_t)xx * dim + yy) * zc + zz);
+        for (; m; m &= m - 1u) {
+          const int z = 32 * zz + __ffs(m) - 1;
+          dens[ch.dens + ((int64_t)xx * dim + yy) * dim + z] = terrain_exact(field, perm2, gtab, ch, xx, yy, z);
+        }
+      };
+      const uint32_t X = xcross_word(W, dim, zc, x, y, zb), Y = ycross_word(W, dim, zc, x, y, zb);
+      const uint32_t Z = zcross_word(W, dim, zc, x, y, zb);
+      fix(X | Y | Z | (Z << 1), x, y, zb);
+      fix(X, x + 1, y, zb);
+      fix(Y, x, y + 1, zb);
+      fix(Z >> 31, x, y, zb + 1);
+    }
+    return;
+  }
+  for (int64_t e = e0; e < n; e += step) {
+    const uint2 ent = ws.fix[e];
     const ChunkDev ch = chunks[ent.x];
     const uint32_t dim = (uint32_t)ch.dim, line = ent.y / dim;
     const int z = (int)(ent.y - line * dim), x = (int)(line / dim), y = (int)(line - (uint32_t)x * dim);
@@ -684,8 +711,8 @@ __global__ void __launch_bounds__(256) k_fill_fixup(const ChunkDev* __restrict__
   }
 }
 
-void launch_fill_fixup(const ChunkDev* d_chunks, const WordScratch& ws, const FieldDev& field, float* dens,
-                       cudaStream_t st) {
+void launch_fill_fixup(const ChunkDev* d_chunks, const uint32_t* words, const WordScratch& ws, const FieldDev& field,
+                       float* dens, cudaStream_t st) {
   static std::atomic<int> grid[64] = {};
   const int g = per_device_once(grid, [](int dev) {
     int sms = 0, per_sm = 0;
@@ -693,7 +720,7 @@ void launch_fill_fixup(const ChunkDev* d_chunks, const WordScratch& ws, const Fi
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fill_fixup, 256, 0);
     return (sms > 0 ? sms : 1) * (per_sm > 0 ? per_sm : 1);
   });
-  k_fill_fixup<<<g, 256, 0, st>>>(d_chunks, ws.fix, ws.fcount, ws.fix_cap, field, dens);
+  k_fill_fixup<<<g, 256, 0, st>>>(d_chunks, words, ws, field, dens);
 }
 
 // ---------------------------------------------------------------------------

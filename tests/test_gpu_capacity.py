@@ -197,3 +197,22 @@ def test_a_graph_does_not_outlive_its_scratch(ctx, whole, form, mode, between):
     b.bufs["pos"].zero_()
     assert b.run() == (nv, ni) and _equal(_mesh(b, nv, ni), want)
     b.close()
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+def test_first_chunks_are_exact_when_the_fixup_list_overflows(ctx, whole, form):
+    """Room for the first chunks' vertices only: far fewer entries than the band fill
+    leaves ends to make exact."""
+    _, want, wtab = whole(form, L.MODE_R)
+    k = int(np.flatnonzero(wtab[:, 1] > 0)[1])  # the second chunk with a mesh is the last that fits
+    vcap, icap = int(wtab[k, 0] + wtab[k, 1]), int(wtab[k, 2] + wtab[k, 3])
+    b = _plan(ctx, form, L.MODE_R)
+    assert b.tuning()["fill_band"] == 1
+    intact = _arena(b, vcap, icap)
+    with pytest.raises(L.BmfError) as e:
+        b.run()
+    torch.cuda.synchronize()
+    assert e.value.status == L.ERR_CAPACITY and intact() and (b.bufs["info"][:k + 1, 5] == 0).all()
+    got = [b.bufs["pos"][:vcap], b.bufs["nrm"][:vcap], b.bufs["boundary"][:vcap], b.bufs["idx"][:icap]]
+    assert _equal(got, [want[0][:vcap], want[1][:vcap], want[2][:vcap], want[3][:icap]])
+    b.close()
